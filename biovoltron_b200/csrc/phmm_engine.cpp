@@ -47,6 +47,9 @@ void DevBuf::release() {
 namespace {
 constexpr int kMaxRowsPerLane = 8;
 constexpr int kMaxVariants = 32;
+// Launches in flight beside each other.  Two, four and eight lanes took 1.77, 1.74 and 1.72 ms for the
+// call on 48 uneven regions; every lane is a stream that a new context has to make (0.3 ms for four).
+constexpr int kMaxLanes = 4;
 constexpr int kRescaleTarget = 1000;  // FP64 boundary rows are scaled to ~2^1000
 
 int64_t round_up(int64_t x, int64_t m) { return (x + m - 1) / m * m; }
@@ -79,6 +82,9 @@ Engine::~Engine() {
       if (e) cudaEventDestroy(e);
     for (auto& e : tune_ev_)
       if (e) cudaEventDestroy(e);
+    for (auto& e : side_done_) cudaEventDestroy(e);
+    if (fork_ev_) cudaEventDestroy(fork_ev_);
+    for (auto& s : side_) cudaStreamDestroy(s);
     cudaStreamDestroy(stream_);
   }
 }
@@ -161,6 +167,36 @@ bv_status Engine::init() {
   return BV_OK;
 }
 
+bv_status Engine::reserve_lanes(int n) {
+  if (n > 1 && !fork_ev_) BV_CUDA(cudaEventCreateWithFlags(&fork_ev_, cudaEventDisableTiming), "event");
+  while ((int)side_.size() < n - 1) {
+    cudaStream_t s;
+    BV_CUDA(cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking), "stream");
+    side_.push_back(s);
+  }
+  while (side_done_.size() < side_.size()) {
+    cudaEvent_t e;
+    BV_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming), "event");
+    side_done_.push_back(e);
+  }
+  return BV_OK;
+}
+
+bv_status Engine::fork(int n) {
+  if (n < 2) return BV_OK;
+  BV_CUDA(cudaEventRecord(fork_ev_, stream_), "event");
+  for (int i = 1; i < n; ++i) BV_CUDA(cudaStreamWaitEvent(lane(i), fork_ev_, 0), "fork");
+  return BV_OK;
+}
+
+bv_status Engine::join(int n) {
+  for (int i = 1; i < n; ++i) {
+    BV_CUDA(cudaEventRecord(side_done_[i - 1], lane(i)), "event");
+    BV_CUDA(cudaStreamWaitEvent(stream_, side_done_[i - 1], 0), "join");
+  }
+  return BV_OK;
+}
+
 bv_status Engine::reserve_chunk_offsets(int64_t n) {
   if (n <= chunk_off_cap_) return BV_OK;
   if (h_chunk_off_) {
@@ -234,7 +270,7 @@ bv_status Engine::plan(const bv_region_batch& b) {
   n_results_ = 0;
   n_cells_ = 0;
   max_hap_ = 0;
-  const int per_unit = std::max(1, opt_.haps_per_unit > 0 ? opt_.haps_per_unit : 8);
+  const int max_unit = std::max(1, opt_.haps_per_unit > 0 ? opt_.haps_per_unit : 8);
   const bool all_f64 = opt_.precision == BV_PRECISION_F64;
   const int v_multi = variant_index(false, 8, true);
   std::vector<int64_t> count(kMaxVariants, 0);
@@ -248,6 +284,25 @@ bv_status Engine::plan(const bv_region_batch& b) {
     region_max_hap[g] = mh;
     max_hap_ = std::max(max_hap_, mh);
   }
+  // Haplotypes per unit: as many as the options allow when the batch still
+  // gives every resident warp (about 16 an SM) eight units, so that the last
+  // units of a launch do not leave the chip idle; fewer for smaller batches
+  // (the row set-up a unit shares is ~1 % of one haplotype's sweep).  An even
+  // count of at least two, for the paired kernels; one, with one haplotype per
+  // warp, when the pairs do not even fill half the resident warps: a warp then
+  // runs alone on its scheduler and only the length of its dependent chain
+  // counts.  (FP32 kernels' time, ms, with 8 / 2 / 1 haplotypes a unit, the bins
+  // one after the other: 64 reads x 8 haplotypes 0.108 / 0.035 / 0.027; 46 k
+  // uneven pairs 2.07 / 1.26 / 1.28; 349 k 7.6 / 6.75 / 7.7, and with the bins
+  // side by side 6.59 / 6.50 / 7.56.)
+  int64_t n_pairs = 0;
+  for (int64_t g = 0; g < b.num_regions; ++g)
+    n_pairs += (b.region_reads[g + 1] - b.region_reads[g]) * (b.region_haps[g + 1] - b.region_haps[g]);
+  const int64_t warps = (int64_t)sms_ * 16;
+  const bool few = n_pairs * 2 <= warps && opt_.haps_per_warp != 2 && !band_enabled() && !tuning_;
+  const int per_unit = band_enabled() ? max_unit
+                       : few          ? 1
+                                      : (int)std::min<int64_t>(max_unit, std::max<int64_t>(2, n_pairs / (warps * 8) / 2 * 2));
   // two haplotypes per warp (paired variants) unless the options or the bin's tuning ask for one
   auto pair_rows = [&](int64_t rt) {
     if (opt_.haps_per_warp == 1 || per_unit < 2 || rt < 1 || rt > kTuneBins) return false;
@@ -324,6 +379,7 @@ bv_status Engine::plan(const bv_region_batch& b) {
       int rt = 0;
       for (int t = 1; t <= kTuneBins; ++t)
         if (v == variant_index(false, t, false, false) || v == variant_index(false, t, false, true)) rt = t;
+      lp.rows = rt;
       lp.warps_per_block = rt ? tune_[rt].warps_per_block : kThreadsPerBlock / kWarp;
     }
     const int smem_block = lp.warp_smem * lp.warps_per_block;
@@ -336,6 +392,12 @@ bv_status Engine::plan(const bv_region_batch& b) {
     lp.bnd_cols = lp.multi ? bnd_cols_for(var_max_hap[v]) : 0;
     plans_.push_back(lp);
   }
+  // The launches run beside each other (enqueue_kernels), the ones with the
+  // longest units first: the shorter ones then fill their last waves.
+  std::stable_sort(plans_.begin(), plans_.end(), [&](const LaunchPlan& x, const LaunchPlan& y) {
+    return x.multi != y.multi ? x.multi : x.rows > y.rows;
+  });
+  if (bv_status ls = reserve_lanes(std::min((int)plans_.size(), kMaxLanes)); ls != BV_OK) return ls;
   // FP64 launch: persistent over the whole device, whatever the FP32 passes flag
   LaunchPlan rp;
   rp.variant = variant_index(true, 4, true);
@@ -524,10 +586,16 @@ bv_status Engine::enqueue_kernels(bool capturing) {
       tune_ev_.push_back(e);
     }
   }
+  // The bins side by side on the lanes' streams (one after the other while the
+  // tuner times them): 48 uneven regions' eight bins, 46 k pairs, take 0.96
+  // instead of 1.26 ms, since no bin waits for the last warps of another.
+  const bool timed = tune_timing_ && !capturing;
+  const int lanes = band_enabled() || timed ? 1 : std::min((int)plans_.size(), kMaxLanes);
+  if (bv_status fs = fork(lanes); fs != BV_OK) return fs;
+  cudaError_t le = cudaSuccess;  // a failed launch still joins the lanes that started
   for (size_t pi = 0; pi < plans_.size(); ++pi) {
     const LaunchPlan& lp = plans_[pi];
     if (band_enabled()) break;
-    const bool timed = tune_timing_ && !capturing;
     if (timed) BV_CUDA(cudaEventRecord(tune_ev_[2 * pi], stream_), "event");
     p.unit_base = lp.unit_base;
     p.n_units = lp.n_units;
@@ -541,9 +609,12 @@ bv_status Engine::enqueue_kernels(bool capturing) {
     p.bnd_cols = lp.bnd_cols;
     p.rescale = 0;
     p.rescale_target = 0;
-    BV_CUDA(launch_forward(lp.variant, p, lp.grid, stream_), "FP32 forward launch");
+    le = launch_forward(lp.variant, p, lp.grid, lane((int)pi % lanes));
+    if (le != cudaSuccess) break;
     if (timed) BV_CUDA(cudaEventRecord(tune_ev_[2 * pi + 1], stream_), "event");
   }
+  if (bv_status js = join(lanes); js != BV_OK) return js;
+  BV_CUDA(le, "FP32 forward launch");
   BV_CUDA(rec(ev_[3]), "event");
   {
     const LaunchPlan& lp = rescue_plan_;

@@ -43,6 +43,7 @@ constexpr int kTuneBins = 8;  // rows per lane 1..8
 
 struct LaunchPlan {
   int variant = -1;
+  int rows = 0;  // rows per lane of a single-strip variant (0: multi-strip)
   int slot = 0;
   long long unit_base = 0;
   long long n_units = 0;
@@ -208,11 +209,22 @@ class Engine {
   bv_status enqueue_band(bool capturing, KernelParams& p);
   bv_status band_stats(bv_phmm_stats* stats);
   void destroy_graph();
+  // Side streams: independent launches (the bins of a full-DP pass) run beside
+  // each other.  reserve_lanes() makes streams for n launches in flight (before
+  // any capture); fork() lets lanes 1 .. n-1 start behind the work queued on
+  // the context's stream (lane 0), join() makes that stream wait for them.
+  bv_status reserve_lanes(int n);
+  bv_status fork(int n);
+  bv_status join(int n);
+  cudaStream_t lane(int i) const { return i == 0 ? stream_ : side_[i - 1]; }
 
   bv_phmm_options opt_;
   int sms_ = 0;
   cudaStream_t stream_ = nullptr;
   cudaEvent_t ev_[8] = {};
+  std::vector<cudaStream_t> side_;
+  std::vector<cudaEvent_t> side_done_;
+  cudaEvent_t fork_ev_ = nullptr;
   std::string err_;
 
   std::unique_ptr<Tables> h_tables_;  // host copy of d_tables_
@@ -270,6 +282,7 @@ class Engine {
   // per-bin launch parameters; per-launch timing while tuning
   BinTune tune_[kTuneBins + 1];
   bool tune_timing_ = false;
+  bool tuning_ = false;  // autotune is staging trial shapes: plan() takes them as they are
   std::vector<cudaEvent_t> tune_ev_;
 
   cudaGraph_t graph_ = nullptr;

@@ -56,6 +56,7 @@ bv_status Engine::autotune(const bv_region_batch& sample, int repeats, bv_phmm_t
   if (opt_.precision == BV_PRECISION_F64) return fail(BV_ERR_INVALID_ARG, "autotune needs FP32 precision");
   const int saved_hpw = opt_.haps_per_warp;
   opt_.haps_per_warp = 0;  // the per-bin table decides
+  tuning_ = true;
   BinTune saved[kTuneBins + 1];
   std::copy(tune_, tune_ + kTuneBins + 1, saved);
   struct Cand {
@@ -123,6 +124,7 @@ bv_status Engine::autotune(const bv_region_batch& sample, int repeats, bv_phmm_t
       }
     }
   }
+  tuning_ = false;
   opt_.haps_per_warp = saved_hpw;
   std::copy(saved, saved + kTuneBins + 1, tune_);
   staged_ = false;  // the sample was staged with trial shapes

@@ -67,9 +67,10 @@ typedef struct bv_phmm_options {
   int32_t precision;        /* bv_phmm_precision */
   int32_t mode;             /* bv_phmm_mode */
   double rescue_threshold;  /* FP32 value (scaled by 2^120) below which FP64 runs; default 1e-28 */
-  int32_t haps_per_unit;    /* haplotypes one warp scores against a read before taking new work; default 8 */
+  int32_t haps_per_unit;    /* most haplotypes one warp scores against a read before taking new work; default 8
+                               (batches too small to fill the device use fewer) */
   int32_t haps_per_warp;    /* 2: a warp scores two haplotypes of a read at once (packed FP32x2), 1: one;
-                               0 (default): 2 */
+                               0 (default): 2, or 1 when the pairs do not fill the device */
   int32_t pipeline_chunks;  /* bv_phmm_compute_regions on a batch of at least pipeline_min_pairs pairs:
                                region chunks scored by two alternating contexts on the device, one
                                chunk's copies and planning overlapping the previous chunk's kernels;

@@ -1,0 +1,44 @@
+"""The full-DP launch rules on either side of their edges, against the FP64
+oracle and against forced unit sizes (bit for bit)."""
+import numpy as np
+import pytest
+
+from biovoltron_b200 import workloads as W
+from oracle.oracle import TestcaseArray
+
+pytestmark = pytest.mark.gpu
+
+TOL_FP32 = 1e-4  # FP32 rounding against 64 bits, as the parity tests allow
+
+
+def _region(rng, n_reads, n_haps, read_lens, hap_len):
+    base = W._random_seq(rng, hap_len)
+    haps = [W._apply_indels(rng, W._substitute(rng, base, 0.01), k % 3, 1, 8) for k in range(n_haps)]
+    reads = []
+    for k in range(n_reads):
+        src = haps[k % n_haps]
+        n = min(int(read_lens[k % len(read_lens)]), len(src))
+        at = int(rng.integers(0, len(src) - n + 1))
+        r = W._substitute(rng, src[at:at + n], 0.01)
+        reads.append((r, *W._quals(rng, n, 10, 40)))
+    return reads, haps
+
+
+# pairs on either side of half the resident warps (148 SMs x 16 / 2 = 1184: one haplotype a unit or two),
+# a single pair, an odd haplotype count, and reads of every bin and of two strips in one batch
+@pytest.mark.parametrize("n_reads,n_haps,lens", [(1, 1, [1]), (37, 32, [90, 150]), (79, 15, [29, 30, 61, 62, 150]),
+                                                 (60, 33, [29, 30, 61, 93, 125, 157, 189, 221, 253, 254, 300])])
+def test_unit_sizes_and_lanes(engine, oracle, n_reads, n_haps, lens):
+    from biovoltron_b200.pairhmm import PairHMMEngine
+    rng = np.random.default_rng(n_reads * 100 + n_haps)
+    b = W._build([_region(rng, n_reads, n_haps, lens, 380)], "dispatch")
+    got = engine.compute_regions(b)
+    truth = oracle.log10_rescaled(TestcaseArray.for_batch(b))
+    assert np.max(np.abs(got - truth)) <= TOL_FP32
+    for unit, warp in ((32, 2), (1, 1)):
+        with PairHMMEngine(haps_per_unit=unit, haps_per_warp=warp) as e:
+            assert np.array_equal(e.compute_regions(b), got)
+            n = e.stage(b)
+            for _ in range(3):  # direct launches, then the captured graph with its parallel branches
+                e.run()
+                assert np.array_equal(e.fetch(n), got)
