@@ -850,14 +850,7 @@ __device__ __forceinline__ void band_outcome(const BandParams& p, int cls, const
       atomicOr(&p.ctr->status, 4ull);
     }
   } else if (rescue) {
-    const unsigned long long slot = atomicAdd(&p.ctr->rescue_count, 1ull);
-    if (slot < (unsigned long long)p.rescue_cap) {
-      p.rescue[slot].read = it.read;
-      p.rescue[slot].hap = it.hap;
-      p.rescue[slot].out = it.out;
-    } else {
-      atomicOr(&p.ctr->status, 1ull);
-    }
+    push_rescue(p.ctr, p.rescue, p.rescue_cap, p.long_rows, R, it.read, it.hap, it.out);
     p.out[it.out] = __longlong_as_double(0x7ff8000000000000ll);
   } else {
     p.out[it.out] = (double)(log10f(tot) - p.tables->log10_init_f);

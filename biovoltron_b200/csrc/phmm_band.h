@@ -128,6 +128,7 @@ struct BandParams {
   double* audit_out;          // full-DP log10 of the audit pairs
   PairRef* rescue;
   long long rescue_cap;
+  int long_rows;              // > 0: rescues of reads this long or longer go to the FP64 list's long part
 };
 
 // Words of the per-haplotype 11-mer hash tables of a batch.

@@ -653,18 +653,8 @@ __device__ __forceinline__ void write_result(const KernelParams& p, int read, in
     if (!p.rescue && (!(res >= (T)kMinAccepted) || isinf((double)res))) {
       p.out[o] = __longlong_as_double(0x7ff8000000000000ll);
     } else if (!(res >= (T)kMinAccepted) || isinf((double)res)) {
-      // reads of at least long_rows bases go to the long list, filled from the
-      // list's far end for the several-warps-per-pair FP64 kernel
-      const bool lng = p.long_rows > 0 && p.batch.read_off[read + 1] - p.batch.read_off[read] >= p.long_rows;
-      const unsigned long long slot = atomicAdd(lng ? &p.ctr->rescue_long_count : &p.ctr->rescue_count, 1ull);
-      if (slot < (unsigned long long)p.rescue_cap) {
-        const long long at = lng ? p.rescue_cap - 1 - (long long)slot : (long long)slot;
-        p.rescue[at].read = read;
-        p.rescue[at].hap = hap;
-        p.rescue[at].out = o;
-      } else {
-        atomicOr(&p.ctr->status, 1ull);
-      }
+      push_rescue(p.ctr, p.rescue, p.rescue_cap, p.long_rows, (int)(p.batch.read_off[read + 1] - p.batch.read_off[read]),
+                  read, hap, o);
       p.out[o] = __longlong_as_double(0x7ff8000000000000ll);
     } else {
       p.out[o] = (double)(log10_((float)res) - p.tables->log10_init_f);

@@ -46,7 +46,11 @@ void DevBuf::release() {
 
 namespace {
 constexpr int kMaxRowsPerLane = 8;
-constexpr int kMaxVariants = 32;
+// Launch bins: the FP32 variants (variant_index), then FP64 mode's bins of 1 .. 8 rows a lane; reads of
+// several strips go to the FP64 list.
+constexpr int kF64Bin0 = 19;
+constexpr int kF64List = 28;
+constexpr int kMaxVariants = 28;
 // Launches in flight beside each other.  Two, four and eight lanes took 1.77, 1.74 and 1.72 ms for the
 // call on 48 uneven regions; every lane is a stream that a new context has to make (0.3 ms for four).
 constexpr int kMaxLanes = 4;
@@ -275,6 +279,7 @@ bv_status Engine::plan(const bv_region_batch& b) {
   const int v_multi = variant_index(false, 8, true);
   std::vector<int64_t> count(kMaxVariants, 0);
   std::vector<int> var_max_hap(kMaxVariants, 0);
+  int64_t n_long = 0, long_rows_sum = 0;  // pairs the long-read kernel may get, and their reads' bases
   // pass 1: count units per variant
   std::vector<int> region_max_hap(std::max<int64_t>(b.num_regions, 1), 0);
   for (int64_t g = 0; g < b.num_regions; ++g) {
@@ -299,8 +304,11 @@ bv_status Engine::plan(const bv_region_batch& b) {
   for (int64_t g = 0; g < b.num_regions; ++g)
     n_pairs += (b.region_reads[g + 1] - b.region_reads[g]) * (b.region_haps[g + 1] - b.region_haps[g]);
   const int64_t warps = (int64_t)sms_ * 16;
+  // FP64 mode: reads that fit a strip run in units too, one haplotype at a time
+  const bool f64_units = all_f64 && !band_enabled();
   const bool few = n_pairs * 2 <= warps && opt_.haps_per_warp != 2 && !band_enabled() && !tuning_;
   const int per_unit = band_enabled() ? max_unit
+                       : f64_units    ? (int)std::min<int64_t>(max_unit, std::max<int64_t>(1, n_pairs / (warps * 8)))
                        : few          ? 1
                                       : (int)std::min<int64_t>(max_unit, std::max<int64_t>(2, n_pairs / (warps * 8) / 2 * 2));
   // two haplotypes per warp (paired variants) unless the options or the bin's tuning ask for one
@@ -309,6 +317,7 @@ bv_status Engine::plan(const bv_region_batch& b) {
     return opt_.haps_per_warp == 2 || tune_[rt].haps_per_warp == 2;
   };
   auto variant_of = [&](int64_t rlen) {
+    if (f64_units) return rlen <= kF64ShortMax ? kF64Bin0 + (int)((rlen + 3 + kWarp - 1) / kWarp) : kF64List;
     // rows of the single-strip FP32 kernel: row 0, the read, the summing row
     // and one padding row on top (phmm_device.cuh, rows_needed)
     const int64_t rows = rows_needed((int)std::min<int64_t>(rlen, 1 << 24), true, true);
@@ -321,14 +330,20 @@ bv_status Engine::plan(const bv_region_batch& b) {
     if (nh == 0 || nr == 0) continue;
     const int64_t chunks = (nh + per_unit - 1) / per_unit;
     for (int64_t r = b.region_reads[g]; r < b.region_reads[g + 1]; ++r) {
-      const int v = variant_of(b.read_offsets[r + 1] - b.read_offsets[r]);
+      const int64_t rl = b.read_offsets[r + 1] - b.read_offsets[r];
+      if (rl >= long_rows()) {
+        n_long += nh;
+        long_rows_sum += nh * rl;
+      }
+      const int v = variant_of(rl);
+      if (v == kF64List) continue;
       count[v] += chunks;
       var_max_hap[v] = std::max(var_max_hap[v], region_max_hap[g]);
     }
   }
   std::vector<int64_t> start(kMaxVariants + 1, 0);
   for (int v = 0; v < kMaxVariants; ++v) start[v + 1] = start[v] + count[v];
-  if (!all_f64) units_.resize(start[kMaxVariants]);
+  if (!all_f64 || f64_units) units_.resize(start[kMaxVariants]);
   std::vector<int64_t> fill(start.begin(), start.end() - 1);
   // pass 2: fill units (or FP64 items) in result order within each bucket
   int64_t res = 0;
@@ -340,13 +355,13 @@ bv_status Engine::plan(const bv_region_batch& b) {
       const int64_t rl = b.read_offsets[r + 1] - b.read_offsets[r];
       n_cells_ += rl * hap_bases;
       max_read = std::max(max_read, rl);
-      if (all_f64) {
+      const int v = variant_of(rl);
+      if (all_f64 && (!f64_units || v == kF64List)) {
         auto& list = rl >= long_rows() ? f64_long_items_ : f64_items_;
         for (int64_t k = 0; k < nh; ++k)
           list.push_back(PairRef{(int32_t)r, (int32_t)(h0 + k), res + (r - r0) * nh + k});
         continue;
       }
-      const int v = variant_of(rl);
       for (int64_t k = 0; k < nh; k += per_unit) {
         Unit u{};
         u.read = (int32_t)r;
@@ -361,7 +376,7 @@ bv_status Engine::plan(const bv_region_batch& b) {
   n_results_ = res;
   // launch plans
   int slot = 0;
-  for (int v = 0; v < kMaxVariants && !all_f64; ++v) {
+  for (int v = 0; v < kMaxVariants && (!all_f64 || f64_units); ++v) {
     if (count[v] == 0) continue;
     LaunchPlan lp;
     lp.variant = v;
@@ -369,7 +384,18 @@ bv_status Engine::plan(const bv_region_batch& b) {
     lp.unit_base = start[v];
     lp.n_units = count[v];
     lp.multi = (v == v_multi);
-    lp.f64 = false;
+    lp.f64 = v > kF64Bin0;
+    if (lp.f64) {
+      lp.rows = v - kF64Bin0;
+      lp.hap_bytes = hap_bytes_for(var_max_hap[v], 8);
+      lp.warp_smem = f64_warp_smem(lp.rows, lp.hap_bytes);
+      const int smem = lp.warp_smem * lp.warps_per_block;
+      if (smem > 227 * 1024) return fail(BV_ERR_INVALID_ARG, "haplotype too long for shared-memory staging");
+      const int64_t need = (count[v] + lp.warps_per_block - 1) / lp.warps_per_block;
+      lp.grid = (int)std::min<int64_t>(need, (int64_t)sms_ * std::max(1, f64_blocks_per_sm(lp.rows, smem)));
+      plans_.push_back(lp);
+      continue;
+    }
     lp.code_row_bytes = hap_bytes_for(var_max_hap[v], lp.multi ? 32 : 8);
     // a paired variant stages one 32-bit entry (both haplotypes' table offsets) per column
     lp.hap_bytes = variant_paired(v) ? 4 * lp.code_row_bytes : lp.code_row_bytes;
@@ -398,36 +424,43 @@ bv_status Engine::plan(const bv_region_batch& b) {
     return x.multi != y.multi ? x.multi : x.rows > y.rows;
   });
   if (bv_status ls = reserve_lanes(std::min((int)plans_.size(), kMaxLanes)); ls != BV_OK) return ls;
-  // FP64 launch: persistent over the whole device, whatever the FP32 passes flag
+  // FP64 list: persistent over the whole device, whatever the other passes send there
   LaunchPlan rp;
-  rp.variant = variant_index(true, 4, true);
-  rp.slot = 15;
   rp.multi = true;
   rp.f64 = true;
   rp.hap_bytes = hap_bytes_for(std::max(max_hap_, 1), 32);
-  rp.warp_smem = warp_smem_bytes(rp.variant, rp.hap_bytes);
+  rp.warp_smem = f64_warp_smem(0, rp.hap_bytes);
   const int smem_block = rp.warp_smem * (kThreadsPerBlock / kWarp);
   if (smem_block > 227 * 1024) return fail(BV_ERR_INVALID_ARG, "haplotype too long for shared-memory staging");
-  BV_CUDA(prepare_variant(rp.variant, smem_block), "kernel attribute");
-  const int bps = std::max(1, blocks_per_sm(rp.variant, smem_block));
-  rp.grid = sms_ * bps;
+  rp.grid = sms_ * std::max(1, f64_blocks_per_sm(0, smem_block));
   rp.bnd_cols = bnd_cols_for(std::max(max_hap_, 1));
   rescue_plan_ = rp;
   // FP64 long reads: one block per pair, longest pairs first (the long list is
-  // read from its far end, so the host list is in ascending order of cells)
+  // read from its far end, so the host list is in ascending order of cells).
+  // The block's warps, unless they are set: twice as many while the pairs then
+  // still fit the device's resident warps (16 an SM) at once and the longest
+  // read has strips for them -- a pair then ends sooner -- and while the
+  // average read gives every warp at least two strips.  FP64 pass, ms, with
+  // 4 / 8 / 16 warps: 40 reads of up to 10 kb 28 / 17 / 12, 2000 of them 86 / 79 /
+  // 77, 3000 of up to 1.5 kb 8.7 / 9.3 / 10.3, 400 of 400 bases 0.47 / 0.65 / 0.82.
   long_plan_ = LaunchPlan{};
-  if (max_read >= long_rows()) {
-    long_smem_ = long_smem_bytes(rp.hap_bytes, long_warps_);
+  if (max_read >= long_rows() && n_long > 0) {
+    const int64_t strips = (max_read + 1 + 127) / 128, strips_mean = long_rows_sum / n_long / 128 + 1;
+    long_block_ = long_set_ ? long_warps_ : 2;
+    while (!long_set_ && long_block_ < 16 &&
+           ((2 * long_block_ * n_long <= warps && long_block_ < strips) || 4 * long_block_ <= strips_mean))
+      long_block_ *= 2;
+    long_smem_ = long_smem_bytes(rp.hap_bytes, long_block_);
     if (long_smem_ <= 227 * 1024) {
-      BV_CUDA(prepare_long(long_smem_, long_warps_), "kernel attribute");
-      long_plan_.grid = sms_ * std::max(1, long_blocks_per_sm(long_smem_, long_warps_));
+      BV_CUDA(prepare_long(long_smem_, long_block_), "kernel attribute");
+      long_plan_.grid = (int)std::min<int64_t>(n_long, (int64_t)sms_ * std::max(1, long_blocks_per_sm(long_smem_, long_block_)));
       long_plan_.hap_bytes = rp.hap_bytes;
       long_plan_.bnd_cols = rp.bnd_cols;
       long_plan_.f64 = true;
       long_plan_.multi = true;
     }
   }
-  if (long_plan_.grid == 0) {  // no long kernel: the long reads stay on the one-warp FP64 kernel
+  if (long_plan_.grid == 0) {  // no long kernel: the long reads stay on k_f64_list
     f64_items_.insert(f64_items_.end(), f64_long_items_.begin(), f64_long_items_.end());
     f64_long_items_.clear();
   }
@@ -545,6 +578,48 @@ bv_status Engine::stage(const bv_region_batch& b, bool wait) {
   return BV_OK;
 }
 
+// The staged bins' launches (of FP32 units, or of FP64 mode's).
+bv_status Engine::enqueue_plans(bool capturing, bool f64, KernelParams& p) {
+  if (band_enabled() || plans_.empty() || plans_[0].f64 != f64) return BV_OK;
+  if (tune_timing_ && !capturing) {
+    while (tune_ev_.size() < 2 * plans_.size()) {
+      cudaEvent_t e;
+      BV_CUDA(cudaEventCreate(&e), "event");
+      tune_ev_.push_back(e);
+    }
+  }
+  // The bins side by side on the lanes' streams (one after the other while the
+  // tuner times them): 48 uneven regions' eight bins, 46 k pairs, take 0.96
+  // instead of 1.26 ms, since no bin waits for the last warps of another.
+  const bool timed = tune_timing_ && !capturing;
+  const int lanes = timed ? 1 : std::min((int)plans_.size(), kMaxLanes);
+  if (bv_status fs = fork(lanes); fs != BV_OK) return fs;
+  cudaError_t le = cudaSuccess;  // a failed launch still joins the lanes that started
+  for (size_t pi = 0; pi < plans_.size(); ++pi) {
+    const LaunchPlan& lp = plans_[pi];
+    if (lp.f64 != f64) continue;
+    if (timed) BV_CUDA(cudaEventRecord(tune_ev_[2 * pi], stream_), "event");
+    p.unit_base = lp.unit_base;
+    p.n_units = lp.n_units;
+    p.slot = lp.slot;
+    p.hap_bytes = lp.hap_bytes;
+    p.code_row_bytes = lp.code_row_bytes;
+    p.warps_per_block = lp.warps_per_block;
+    p.warp_smem_bytes = lp.warp_smem;
+    p.bnd = lp.multi ? d_bnd32_.get() : nullptr;
+    p.bnd_cols = lp.bnd_cols;
+    p.rescale = 0;
+    p.rescale_target = 0;
+    const cudaStream_t st = lane((int)pi % lanes);
+    le = f64 ? launch_f64(lp.rows, p, lp.grid, st) : launch_forward(lp.variant, p, lp.grid, st);
+    if (le != cudaSuccess) break;
+    if (timed) BV_CUDA(cudaEventRecord(tune_ev_[2 * pi + 1], stream_), "event");
+  }
+  if (bv_status js = join(lanes); js != BV_OK) return js;
+  BV_CUDA(le, "forward launch");
+  return BV_OK;
+}
+
 bv_status Engine::enqueue_kernels(bool capturing) {
   // Inside stream capture, timing events become event-record nodes of the
   // graph only when recorded as external events.
@@ -579,49 +654,13 @@ bv_status Engine::enqueue_kernels(bool capturing) {
     bv_status bs = enqueue_band(capturing, p);
     if (bs != BV_OK) return bs;
   }
-  if (tune_timing_ && !capturing) {
-    while (tune_ev_.size() < 2 * plans_.size()) {
-      cudaEvent_t e;
-      BV_CUDA(cudaEventCreate(&e), "event");
-      tune_ev_.push_back(e);
-    }
-  }
-  // The bins side by side on the lanes' streams (one after the other while the
-  // tuner times them): 48 uneven regions' eight bins, 46 k pairs, take 0.96
-  // instead of 1.26 ms, since no bin waits for the last warps of another.
-  const bool timed = tune_timing_ && !capturing;
-  const int lanes = band_enabled() || timed ? 1 : std::min((int)plans_.size(), kMaxLanes);
-  if (bv_status fs = fork(lanes); fs != BV_OK) return fs;
-  cudaError_t le = cudaSuccess;  // a failed launch still joins the lanes that started
-  for (size_t pi = 0; pi < plans_.size(); ++pi) {
-    const LaunchPlan& lp = plans_[pi];
-    if (band_enabled()) break;
-    if (timed) BV_CUDA(cudaEventRecord(tune_ev_[2 * pi], stream_), "event");
-    p.unit_base = lp.unit_base;
-    p.n_units = lp.n_units;
-    p.slot = lp.slot;
-    p.from_rescue = 0;
-    p.hap_bytes = lp.hap_bytes;
-    p.code_row_bytes = lp.code_row_bytes;
-    p.warps_per_block = lp.warps_per_block;
-    p.warp_smem_bytes = lp.warp_smem;
-    p.bnd = lp.multi ? d_bnd32_.get() : nullptr;
-    p.bnd_cols = lp.bnd_cols;
-    p.rescale = 0;
-    p.rescale_target = 0;
-    le = launch_forward(lp.variant, p, lp.grid, lane((int)pi % lanes));
-    if (le != cudaSuccess) break;
-    if (timed) BV_CUDA(cudaEventRecord(tune_ev_[2 * pi + 1], stream_), "event");
-  }
-  if (bv_status js = join(lanes); js != BV_OK) return js;
-  BV_CUDA(le, "FP32 forward launch");
+  if (bv_status ps = enqueue_plans(capturing, false, p); ps != BV_OK) return ps;
   BV_CUDA(rec(ev_[3]), "event");
+  if (bv_status ps = enqueue_plans(capturing, true, p); ps != BV_OK) return ps;
   {
     const LaunchPlan& lp = rescue_plan_;
     p.unit_base = 0;
     p.n_units = 0;
-    p.slot = lp.slot;
-    p.from_rescue = 1;
     p.hap_bytes = lp.hap_bytes;
     p.code_row_bytes = 0;
     p.warps_per_block = kThreadsPerBlock / kWarp;
@@ -635,9 +674,9 @@ bv_status Engine::enqueue_kernels(bool capturing) {
       KernelParams q = p;
       q.hap_bytes = long_plan_.hap_bytes;
       q.bnd_cols = long_plan_.bnd_cols;
-      BV_CUDA(launch_forward_long(q, long_plan_.grid, long_smem_, long_warps_, stream_), "FP64 long-read launch");
+      BV_CUDA(launch_forward_long(q, long_plan_.grid, long_smem_, long_block_, stream_), "FP64 long-read launch");
     }
-    BV_CUDA(launch_forward(lp.variant, p, lp.grid, stream_), "FP64 forward launch");
+    BV_CUDA(launch_f64(0, p, lp.grid, stream_), "FP64 forward launch");
     p.cells_ctr = nullptr;
   }
   BV_CUDA(rec(ev_[4]), "event");
@@ -716,6 +755,10 @@ bv_status Engine::finish(bv_phmm_stats* stats) {
     stats->cells = n_cells_;
     stats->rescued = (int64_t)(c.rescue_count + c.rescue_long_count);
     stats->rescued_cells = (int64_t)c.rescued_cells;
+    if (opt_.precision == BV_PRECISION_F64 && !band_enabled()) {  // every pair, on the list or in units
+      stats->rescued = n_results_;
+      stats->rescued_cells = n_cells_;
+    }
     stats->fp32_skipped_cells = (int64_t)c.fp32_skipped_cells;
     stats->underflow = (int64_t)c.underflow_count;
     // band mode: k-mer tables, nibble image, read k-mers, gap check, two featurisers, MLP, route,
@@ -724,7 +767,7 @@ bv_status Engine::finish(bv_phmm_stats* stats) {
     stats->kernel_launches = band_enabled()
                                  ? 9 + (band_opt_.use_mlp ? 1 : 0) + kBandWidths + 9 + (band_opt_.cap_margin > 0 ? 10 : 0) +
                                        (band_opt_.audit_period > 0 ? 11 : 0) + 1
-                                 : (int64_t)plans_.size() + 1;
+                                 : (int64_t)plans_.size() + 1 + (long_plan_.grid > 0);
     stats->ms_fp32 = ms32;
     stats->ms_fp64 = ms64;
     if (band_enabled()) {

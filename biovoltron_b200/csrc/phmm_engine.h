@@ -205,6 +205,7 @@ class Engine {
   bv_status upload_inputs(const bv_region_batch& b);
   bv_status upload_plan();
   bv_status enqueue_kernels(bool capturing);
+  bv_status enqueue_plans(bool capturing, bool f64, KernelParams& p);
   bv_status band_prepare();
   bv_status enqueue_band(bool capturing, KernelParams& p);
   bv_status band_stats(bv_phmm_stats* stats);
@@ -241,8 +242,12 @@ class Engine {
   std::vector<LaunchPlan> plans_;
   LaunchPlan rescue_plan_;
   LaunchPlan long_plan_;  // FP64 long reads, a block of long_warps_ warps per pair (grid 0: none)
-  int long_warps_ = kLongWarps;  // 2, 4 or 8; reads of at least long_rows() bases take the long kernel
-  int long_rows() const { return long_warps_ * 128; }
+  // Warps per pair of the long-read kernel as set or tuned (2, 4 or 8), and whether they were: until
+  // then plan() picks the block (long_block_) and every read longer than a strip takes the kernel.
+  int long_warps_ = kLongWarps;
+  bool long_set_ = false;
+  int long_block_ = kLongWarps;
+  int long_rows() const { return long_set_ ? long_warps_ * 128 : kF64ShortMax + 1; }
   int long_smem_ = 0;
   int64_t n_results_ = 0;
   int64_t n_cells_ = 0;

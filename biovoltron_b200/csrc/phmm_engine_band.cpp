@@ -78,6 +78,7 @@ BandParams Engine::band_params() const {
   p.audit_out = d_audit_out_.as<double>();
   p.rescue = d_rescue_.as<PairRef>();
   p.rescue_cap = std::max<int64_t>(n_results_, 1);
+  p.long_rows = long_plan_.grid > 0 ? long_rows() : 0;
   return p;
 }
 
@@ -162,7 +163,6 @@ bv_status Engine::enqueue_band(bool capturing, KernelParams& kp) {
     kp.n_units = 0;
     kp.n_units_dev = &d_bctr_.as<BandCounters>()->full_count[v];
     kp.slot = lp.slot;
-    kp.from_rescue = 0;
     kp.hap_bytes = lp.hap_bytes;
     kp.warp_smem_bytes = lp.warp_smem;
     kp.bnd = lp.multi ? d_bnd32_.get() : nullptr;
@@ -181,8 +181,7 @@ bv_status Engine::enqueue_band(bool capturing, KernelParams& kp) {
       kp.n_units = 0;
       kp.n_units_dev = &d_bctr_.as<BandCounters>()->cap_count[v];
       kp.slot = kCapSlot0 + v;
-      kp.from_rescue = 0;
-      kp.hap_bytes = lp.hap_bytes;
+        kp.hap_bytes = lp.hap_bytes;
       kp.warp_smem_bytes = lp.warp_smem;
       kp.bnd = lp.multi ? d_bnd32_.get() : nullptr;
       kp.bnd_cols = lp.bnd_cols;

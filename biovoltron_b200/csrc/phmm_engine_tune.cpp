@@ -148,9 +148,10 @@ bv_status Engine::autotune(const bv_region_batch& sample, int repeats, bv_phmm_t
 }
 
 bv_status Engine::set_long_warps(int warps) {
-  if (!long_warps_valid(warps)) return fail(BV_ERR_INVALID_ARG, "long-read warps per pair must be 2, 4 or 8");
-  if (warps != long_warps_) {
+  if (warps != 2 && warps != 4 && warps != 8) return fail(BV_ERR_INVALID_ARG, "long-read warps per pair must be 2, 4 or 8");
+  if (warps != long_warps_ || !long_set_) {
     long_warps_ = warps;
+    long_set_ = true;
     ++config_version_;
     staged_ = false;  // the FP64 lists and launch plan depend on it: stage again
     destroy_graph();
@@ -161,7 +162,7 @@ bv_status Engine::set_long_warps(int warps) {
 // The long-read kernel's shape: for each candidate warps per pair (and with
 // it the long-read edge, 128 x warps bases) the sample is staged in FP64 mode
 // -- every pair on the FP64 kernels, long reads on the long-read kernel, the
-// rest on the one-warp kernel -- and its FP64 pass timed (repeats runs after
+// rest on the short reads' kernels -- and its FP64 pass timed (repeats runs after
 // a warm-up, median); the fastest is installed.
 bv_status Engine::autotune_long(const bv_region_batch& sample, int repeats, int32_t* warps_out, double* ms_out) {
   if (!warps_out || !ms_out) return fail(BV_ERR_INVALID_ARG, "null output");
@@ -170,6 +171,8 @@ bv_status Engine::autotune_long(const bv_region_batch& sample, int repeats, int3
   const int cands[3] = {2, 4, 8};
   for (int c = 0; c < 3; ++c) ms_out[c] = 0.0;
   const int saved_warps = long_warps_;
+  const bool saved_set = long_set_;
+  long_set_ = true;
   const int32_t saved_precision = opt_.precision;
   opt_.precision = BV_PRECISION_F64;
   int best = saved_warps;
@@ -213,6 +216,7 @@ bv_status Engine::autotune_long(const bv_region_batch& sample, int repeats, int3
   }
   opt_.precision = saved_precision;
   long_warps_ = s == BV_OK ? best : saved_warps;
+  if (s != BV_OK) long_set_ = saved_set;
   staged_ = false;  // the sample was staged in FP64 mode
   destroy_graph();
   ++config_version_;

@@ -43,10 +43,9 @@
 //   Columns outside the haplotype have code 5 and e = 0, which makes the
 //   wavefront's ramp-up and ramp-down reproduce the DP boundary exactly.
 // * Pairs whose FP32 result is below MIN_ACCEPTED (1e-28, pairhmm_common.h:16)
-//   or not finite are appended to a list that the FP64 kernel recomputes, as
-//   AvxPairHMM::computeLikelihoodsNative does (pairhmm_avx.hpp:140-149).  The
-//   FP64 kernel renormalises the strip boundary row by an exact power of two
-//   so reads of many kilobases stay finite.
+//   or not finite are appended to a list that the FP64 kernels (phmm_f64.cu,
+//   phmm_long.cu) recompute, as AvxPairHMM::computeLikelihoodsNative does
+//   (pairhmm_avx.hpp:140-149).
 #include <cuda_runtime.h>
 
 #include <map>
@@ -89,43 +88,14 @@ __global__ void __launch_bounds__(kThreadsPerBlock) k_forward(KernelParams p) {
   const int warp_global = blockIdx.x * p.warps_per_block + wib;
   unsigned char* wsm = smem + (size_t)wib * p.warp_smem_bytes;
   T* bnd = MULTI ? reinterpret_cast<T*>(p.bnd) + (size_t)warp_global * p.bnd_cols * 4 : nullptr;
-  // only the FP64 variants drain the FP64 list
-  constexpr bool kList = sizeof(T) == 8;
-  const bool from_list = kList && p.from_rescue;
-  const unsigned long long n = from_list ? p.ctr->rescue_count
-                               : p.n_units_dev ? *p.n_units_dev : (unsigned long long)p.n_units;
-  const unsigned long long n_short = from_list && n > (unsigned long long)p.rescue_cap ? p.rescue_cap : n;
-  // FP64 pass: after the short list, the long list's entries the long-read
-  // kernel handed back (read index complemented)
-  const unsigned long long n_long =
-      from_list && p.long_rows > 0 ? min(p.ctr->rescue_long_count, (unsigned long long)p.rescue_cap) : 0ull;
-  const unsigned long long n_eff = n_short + n_long;
-  unsigned long long* next = from_list ? &p.ctr->rescue_next : &p.ctr->unit_next[p.slot];
+  const unsigned long long n = p.n_units_dev ? *p.n_units_dev : (unsigned long long)p.n_units;
   for (;;) {
     unsigned long long w = 0;
-    if (lane == 0) w = atomicAdd(next, 1ull);
+    if (lane == 0) w = atomicAdd(&p.ctr->unit_next[p.slot], 1ull);
     w = __shfl_sync(0xffffffffu, w, 0);
-    if (w >= n_eff) break;
-    Item it;
-    long long handed_back = -1;  // list slot of an entry the long-read kernel handed back
-    if (kList && from_list) {
-      PairRef pr;
-      if (w < n_short) {
-        pr = p.rescue[w];
-      } else {
-        handed_back = p.rescue_cap - 1 - (long long)(w - n_short);
-        pr = p.rescue[handed_back];
-        if (pr.read >= 0) continue;  // scored by the long-read kernel
-        pr.read = ~pr.read;
-      }
-      it.read = pr.read; it.hap0 = pr.hap; it.nh = 1; it.out0 = pr.out;
-    } else {
-      const Unit u = p.units[p.unit_base + w];
-      it.read = u.read; it.hap0 = u.hap0; it.nh = u.nh; it.out0 = u.out0;
-    }
-    process_item<T, RT, MULTI, PAIR>(p, it, wsm, lane, bnd);
-    // the mark is cleared: a replayed batch finds the list as it was staged
-    if (kList && handed_back >= 0 && lane == 0) p.rescue[handed_back].read = it.read;
+    if (w >= n) break;
+    const Unit u = p.units[p.unit_base + w];
+    process_item<T, RT, MULTI, PAIR>(p, Item{u.read, u.hap0, u.nh, u.out0}, wsm, lane, bnd);
   }
 }
 
@@ -182,11 +152,11 @@ static int occupancy_one(int smem_per_block, int threads) {
 
 // Variant order: indices 0..7 are FP32 single strip with 1..8 rows per lane
 // and 8 the FP32 multi-strip variant (the band path's fallback buckets use
-// these numbers); then the FP64 variants and the paired FP32 variants.
+// these numbers); then the paired FP32 variants.
 #define BV_VARIANTS(X)              \
   X(float, 1, false, false) X(float, 2, false, false) X(float, 3, false, false) X(float, 4, false, false) \
   X(float, 5, false, false) X(float, 6, false, false) X(float, 7, false, false) X(float, 8, false, false) \
-  X(float, 8, true, false) X(double, 4, true, false) X(double, 2, true, false)                           \
+  X(float, 8, true, false)                                                                              \
   X(float, 1, false, true) X(float, 2, false, true) X(float, 3, false, true) X(float, 4, false, true)     \
   X(float, 5, false, true) X(float, 6, false, true) X(float, 7, false, true) X(float, 8, false, true)
 

@@ -17,7 +17,6 @@ struct KernelParams {
   long long n_units;
   const unsigned long long* n_units_dev;  // if set, the unit count is read from device memory
   int slot;               // work-queue head used by this launch
-  int from_rescue;        // 1: items come from the FP64 list
   Counters* ctr;
   double* out;            // log10 likelihoods, one per result slot
   PairRef* rescue;        // null: pairs below the FP32 threshold get NaN (audit runs)
@@ -28,18 +27,26 @@ struct KernelParams {
   int warp_smem_bytes;    // per-warp dynamic shared memory
   void* bnd;              // per-warp strip-boundary buffers (multi-strip variants)
   long long bnd_cols;     // rows of 4 values per warp buffer
-  int rescale;            // renormalise between strips (FP64 variants)
+  int rescale;            // renormalise between strips (FP64, multi-strip)
   int rescale_target;     // binary exponent the boundary maximum is scaled to
   unsigned long long* cells_ctr;  // if set, FP64 launches add read x haplotype length per pair here
   int long_rows;          // > 0: FP32 results of reads this long or longer go to the FP64 list's long part
 };
 
-// Long reads in FP64: a block of `warps` warps per pair (phmm_long.cu; 2, 4
-// or 8, kLongWarps by default, chosen per context by the long-read tuner);
-// reads of at least warps x 128 bases (as many strips of 128 rows as the
-// block has warps) take it.
+// Reads of at most kF64ShortMax bases fit one strip of the FP64 wavefront
+// (eight rows a lane, phmm_f64.cu).  rt = 1 .. 8: the unit kernel of that many
+// rows a lane; rt = 0: the FP64 list.
+constexpr int kF64ShortMax = 8 * kWarp - 3;
+int f64_warp_smem(int rt, int hap_bytes);
+int f64_blocks_per_sm(int rt, int smem_per_block);
+cudaError_t launch_f64(int rt, const KernelParams& p, int grid, cudaStream_t st);
+
+// Long reads in FP64: a block of `warps` warps per pair (phmm_long.cu; 2, 4,
+// 8 or 16).  By default reads of more than kF64ShortMax bases take it, with as
+// many warps as Engine::plan finds for the batch; a context whose warps per
+// pair are set or tuned uses that many, for reads of at least 128 x warps
+// bases.
 constexpr int kLongWarps = 4;
-constexpr int kLongRows = kLongWarps * 128;
 bool long_warps_valid(int warps);
 int long_smem_bytes(int hap_bytes, int warps);
 cudaError_t prepare_long(int smem, int warps);
@@ -63,6 +70,25 @@ cudaError_t launch_pack_quals(const uint8_t* q, const uint8_t* i, const uint8_t*
 // The same with the insertion, deletion and continuation qualities constant.
 cudaError_t launch_pack_quals_uniform(const uint8_t* q, uint8_t gi, uint8_t gd, uint8_t gc, uchar4* out, long long n,
                                       int sms, cudaStream_t st);
+
+#if defined(__CUDACC__)
+// Appends a pair to the FP64 list: reads of at least long_rows bases to its
+// long part, filled from the list's far end for the several-warps-per-pair
+// kernel, the others to its front.
+__device__ __forceinline__ void push_rescue(Counters* c, PairRef* list, long long cap, int long_rows, int R, int read,
+                                            int hap, long long out) {
+  const bool lng = long_rows > 0 && R >= long_rows;
+  const unsigned long long slot = atomicAdd(lng ? &c->rescue_long_count : &c->rescue_count, 1ull);
+  if (slot < (unsigned long long)cap) {
+    PairRef& e = list[lng ? cap - 1 - (long long)slot : (long long)slot];
+    e.read = read;
+    e.hap = hap;
+    e.out = out;
+  } else {
+    atomicOr(&c->status, 1ull);
+  }
+}
+#endif
 
 // Writes one 64-bit value on the device (graph-capturable).
 cudaError_t launch_set_u64(unsigned long long* dst, unsigned long long v, cudaStream_t st);

@@ -4,285 +4,354 @@
 // every pair in FP64 mode) runs a long read strip after strip: strip s holds
 // read rows [128 s, 128 s + 128) (4 rows per lane).  With one warp per pair
 // the strips run one after the other and the longest pair sets the launch
-// time; here a block of kLongWarps warps takes one pair and warp w runs
-// strips w, w + K, w + 2K, ... as a pipelined wavefront: strip s + 1 starts a
-// 32-column chunk as soon as strip s has finished the next one.
+// time; here a block of K warps takes one pair and warp w runs strips w,
+// w + K, w + 2K, ... as a pipelined wavefront: strip s + 1 starts a 32-column
+// chunk as soon as strip s has finished the next one.  The cells are the
+// scaled, folded form of phmm_f64.cuh (five FP64 operations).
 //
-// Strip boundaries.  Inside a group of K consecutive strips (one per warp) a
-// strip's bottom row goes to the next warp through a shared-memory channel of
-// kLongSlots chunk slots; a slot's mbarriers say "full" (the producer's lane
-// 31 arrives after writing the chunk) and "empty" (the consumer's lane 0
-// arrives after reading it).  Between groups the bottom row goes through the
-// block's global boundary buffer, read back by the next group's first strip
-// with bulk (TMA) copies as in the one-warp kernel, and renormalised: the
-// row's maximum is scaled to 2^target by an exact power of two, the exponent
-// carried to the result.  So the values of a group share one scale and may
-// shrink over its 128 K rows before the next renormalisation (the one-warp
-// kernel renormalises every 128 rows).
+// Strip boundaries.  A strip hands the row below it, per column, the two sums
+// that row's first cell consumes (zx, zm; phmm_f64.cuh): 16 bytes.  Inside a
+// group of K consecutive strips (one per warp) they go to the next warp
+// through a shared-memory channel of kLongSlots chunk slots; a slot's mbarriers
+// say "full" (the producer's lane 31 arrives after writing the chunk) and
+// "empty" (the consumer's lane 0 arrives once its warp has copied it).  From
+// the group's last warp to the next group's first they go through the block's
+// global boundary buffer, read back one chunk ahead of their use; a counter in
+// shared memory says how many chunks are written, so the next group starts
+// while the last one is still running.
 //
-// A pair whose group-end row maximum falls below 2^kLongMinExp, or whose
-// result is not a positive finite number, is handed back to the one-warp FP64
-// kernel (its list entry marked), which runs after this one.
+// Scale.  Every strip keeps its own power of two E (true values are stored
+// values * 2^E) and a chunk carries the E it was written with.  Before a
+// chunk the warp looks at the largest exponent among its states and the
+// incoming sums and, when that has left [2^-100, 2^400], moves it to 2^200: all
+// states are multiplied by one exact power of two.  Inside a chunk (32
+// columns) a state grows by at most ~2^350 (a gap's continuation undone once a
+// column) and falls by at most 2^-500, so nothing that matters leaves the
+// range whatever the length of the read.
+//
+// A pair with a row that cannot be folded, or whose result is not a positive
+// finite number, is handed back to k_f64_list (its list entry marked), which
+// runs after this kernel.
+//
+// Bound by the issue slots of the FP64 instructions (two each): 40 reads of up to
+// 10 kb take 12.0 ms with 16 warps a pair (28 with 4), 2,000 of them 77 ms, where
+// the unscaled form with four warps, emissions in shared memory and one scale
+// a group of strips took 58 and 169.
 //
 // The haplotype codes are staged once per pair for all warps.  Every wait is
 // bounded (status bit 8 when one gives up); after the first wait of a block
 // that gives up the others are skipped, so a broken hand-over ends after one
-// time-out.  Single-GPU kernel: the bulk copies read this GPU's own memory,
-// without multicast.
+// time-out.
 #include <cuda_runtime.h>
 
 #include <algorithm>
 #include <cstdint>
 
-#include "phmm_device.cuh"
+#include "phmm_f64.cuh"
 #include "phmm_kernels.h"
 
 namespace bvphmm {
 namespace {
 
-constexpr int kLongRT = 4;     // rows per lane (FP64)
-// a group whose last row's maximum is below 2^kLongMinExp (relative to the
-// 2^1000 its first row started from, more than 1,600 binary orders) hands the
-// pair back: the one-warp kernel renormalises every 128 rows instead of 512
-constexpr int kLongMinExp = -600;
-constexpr int kLongSlots = 4;  // chunk slots per channel
-using LS = WarpSmem<double, kLongRT>;
-constexpr int kColB = LS::kColBytes;  // bytes per boundary column (M, X, Y, unused)
-constexpr int kChunkB = 32 * kColB;   // one 32-column chunk
+constexpr int kLongRT = 4;                // rows per lane
+constexpr int kStrip = kWarp * kLongRT;   // rows per strip
+constexpr int kLongSlots = 4;             // chunk slots per channel
+constexpr int kChunkB = 32 * 16;          // one 32-column chunk of (zx, zm)
+constexpr int kTop = 200;                 // exponent the largest state is moved to
+constexpr int kTopMax = 400, kTopMin = -100;
+constexpr int kNoExp = -(1 << 24);        // "no value": below every exponent
 
 // Dynamic shared memory of a block of K warps, after the staged haplotype
 // codes (hap_bytes, a multiple of 16):
-//   per warp: emission table, 32-column output staging (global output)
-//   warp 0:   64-column input ring (global input)
-//   channels 0 .. K-2: kLongSlots chunks each
-//   barriers: full / empty per channel slot, the group-done barrier, the two
-//   input-ring halves; then the shared scalars.
+//   per warp: the 32 (zx, zm) its lane 0 consumes in the current chunk;
+//   channels 0 .. K-2: kLongSlots chunks each, then their exponents;
+//   barriers: full / empty per channel slot; the shared scalars.
 template <int K>
 struct LongLayout {
-  static constexpr int kWarpBytes = LS::kEtabBytes + kChunkB;
-  static constexpr int kRingIn = K * kWarpBytes;
-  static constexpr int kChan = kRingIn + 2 * kChunkB;
-  static constexpr int kBars = kChan + (K - 1) * kLongSlots * kChunkB;
-  static constexpr int kNumBars = 2 * (K - 1) * kLongSlots + 3;
+  static constexpr int kChan = K * kChunkB;
+  static constexpr int kExp = kChan + (K - 1) * kLongSlots * kChunkB;
+  static constexpr int kBars = kExp + ((K - 1) * kLongSlots * 4 + 15) / 16 * 16;
+  static constexpr int kNumBars = 2 * (K - 1) * kLongSlots;
   static constexpr int kScalars = kBars + 8 * kNumBars;
   static constexpr int kBytes = kScalars + 64;
 };
 
 struct LongShared {  // at LongLayout::kScalars
-  double grp_max;    // the last group-end row's maximum (in its own scale)
-  long long kexp;    // current group's exponent: stored values are true values * 2^-kexp
   long long item;
+  int done;  // chunks the group-ending strips have written to the boundary buffer
   int fail;
-  int redo;          // the pair goes back to the one-warp FP64 kernel
+  int redo;  // the pair goes back to k_f64_list
 };
 
 struct LongIO {
-  int in_mode, out_mode;  // warp-uniform
-  const double* chin;
+  const double2* chin;  // input channel (warps 1 .. K-1)
+  const int* chin_e;
   uint64_t* in_full;
   uint64_t* in_empty;
-  double* chout;
+  double2* chout;       // output channel (warps 0 .. K-2)
+  int* chout_e;
   uint64_t* out_full;
   uint64_t* out_empty;
-  double* bnd;
-  double* ring_in;
-  uint64_t* ring_mb;
-  double* ring_out;
-  double in_scale, in_scale2;  // the group-start renormalisation, as two exact power-of-two factors
+  double2* bnd;         // the block's boundary buffer and its chunks' exponents
+  int* bnd_e;
+  double2* stage;       // the warp's staged chunk
 };
-constexpr int kInZero = 0, kInChan = 1, kInGlobal = 2;
-constexpr int kOutNone = 0, kOutChan = 1, kOutGlobal = 2;
+enum LongMode { kZero = 0, kChan = 1, kGlobal = 2 };  // where a strip's input comes from (kZero: none), its output goes
 
 __device__ __forceinline__ void mbar_arrive(uint64_t* mb) {
   asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_addr(mb)) : "memory");
 }
 // Waits for the barrier's phase of parity ((bits >> i) & 1) and flips that
 // bit.  Once any wait of the block has given up (*fail), waits are skipped.
-__device__ __forceinline__ bool wait_flip(uint64_t* mb, unsigned& bits, int i, volatile int* fail) {
-  bool ok = true;
-  if (!*fail) {
-    ok = mbar_wait(mb, (bits >> i) & 1u);
-    if (!ok) *fail = 1;
-  }
+__device__ __forceinline__ void wait_flip(uint64_t* mb, unsigned& bits, int i, volatile int* fail) {
+  if (!*fail && !mbar_wait(mb, (bits >> i) & 1u)) *fail = 1;
   bits ^= 1u << i;
-  return ok;
+}
+// Waits until the group-ending strips have written `need` chunks.
+__device__ __forceinline__ void wait_done(volatile int* done, int need, volatile int* fail) {
+  for (unsigned it = 0; it < kBulkWaitLimit && !*fail; ++it) {
+    if (*done >= need) {
+      __threadfence_block();
+      return;
+    }
+    __nanosleep(100);
+  }
+  *fail = 1;
 }
 
-// One FP64 strip of a long pair (the one-warp kernel's run_strip with the
-// boundary row taken from, and given to, the modes of `io`).  Column c of a
-// boundary row is row c + 31 of the boundary space: chunk j of a producer
-// (steps 32j .. 32j+31 of lane 31) holds rows 32j+1 .. 32j+32 (slot entry u:
-// step 32j+u); at step s lane 0 reads row s + 32, its diagonal starts at row
-// 31.  fph (lane 0) and eph (lane 31) are the parities of the channel
-// barriers' next phases; ok turns false when a wait gives up.
-template <int RT>
-__device__ __forceinline__ void run_strip_long(const Rows<double, RT>& rw, const ELane el,
-                                               const unsigned char* __restrict__ hc_lane, int nsteps, int lane,
-                                               const LongIO& io, unsigned& fph, unsigned& eph, double& sumM,
-                                               double& sumX, double& bmax, bool& ok, volatile int* fail) {
-  using T = double;
-  T M[RT], X[RT], Y[RT];
+// Exponent of a non-negative value (kNoExp for zero and below 2^-1022).
+__device__ __forceinline__ int exp_of(double v) {
+  const int e = (__double2hiint(v) >> 20) & 0x7ff;
+  return e == 0 ? kNoExp : e - 1023;
+}
+// 2^d, exact; zero below 2^-1000 (a value that far below the others does not count).
+__device__ __forceinline__ double pow2(int d) {
+  return d < -1000 ? 0.0 : __hiloint2double((min(d, 1000) + 1023) << 20, 0);
+}
+
+// The 32 steps of a chunk.  hc: the lane's first column code; stage: what lane
+// 0 consumes; o: where lane 31's last row goes (kChan: shared, kGlobal: global
+// memory).  RAMP: row 0 (lane l0, register j0) reaches column 0 at step l0 - 1.
+// LAST: the last row is summed over the columns up to H (lane 31 is at column
+// u + c31).  Specialised so that a step issues nothing but its cells, four
+// shuffles, one load and one store: with these choices made inside the loop a
+// step took 86 instructions, 23 of them FP64, instead of 60, and the 40 pairs
+// below 15.7 ms instead of 12.0.
+template <LongMode OUT, bool RAMP, bool LAST>
+__device__ __forceinline__ void run_chunk(const F64Rows<kLongRT>& w, F64State<kLongRT>& st, double2& z,
+                                          const unsigned char* __restrict__ hc, const double2* __restrict__ stage,
+                                          double2* __restrict__ o, int lane, int l0, int j0, double y0, int c31, int H,
+                                          double& sumM, double& sumX) {
+  const unsigned stage_at = smem_addr(stage);
+  const unsigned o_at = OUT == kChan ? smem_addr(o) : 0u;
+  const unsigned low = lane == 0, high = lane == kWarp - 1;
+#pragma unroll(RAMP ? 1 : 4)
+  for (int u = 0; u < 32; ++u) {
+    asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %2, 0;\n\t@p ld.shared.v2.f64 {%0, %1}, [%3];\n\t}"
+                 : "+d"(z.x), "+d"(z.y) : "r"(low), "r"(stage_at + 16 * u) : "memory");
+    st.zx = z.x;
+    st.zm = z.y;
+    double dm, dx, dy;
+    f64_cells(w, st, hc[u], dm, dx, dy);
+    if (RAMP && lane == l0 && u == l0 - 1) {
 #pragma unroll
-  for (int j = 0; j < RT; ++j) { M[j] = T(0); X[j] = T(0); Y[j] = rw.y0[j]; }
-  sumM = T(0); sumX = T(0); bmax = T(0);
-  T upM = __shfl_up_sync(0xffffffffu, M[RT - 1], 1);
-  T upX = __shfl_up_sync(0xffffffffu, X[RT - 1], 1);
-  T upY = __shfl_up_sync(0xffffffffu, Y[RT - 1], 1);
-  T dM = upM, dX = upX, dY = upY;
-  const int nch = nsteps / 32;
-  unsigned rphase = 0;  // lane 0, global input: parity bits of the two ring halves
-  if (lane == 0) {
-    if (io.in_mode == kInZero) {
-      dM = dX = dY = T(0);
-    } else if (io.in_mode == kInChan) {
-      ok &= wait_flip(io.in_full, fph, 0, fail);
-      if (nch > 1) ok &= wait_flip(io.in_full + 1, fph, 1, fail);
-      const T* r31 = io.chin + 30 * 4;  // row 31 = chunk 0, entry 30
-      dM = r31[0]; dX = r31[1]; dY = r31[2];
+      for (int j = 0; j < kLongRT; ++j)
+        if (j == j0) st.Y[j] = y0;
+    }
+    z = f64_sums(w, st, dm, dx, dy);
+    if (OUT == kChan)
+      asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %2, 0;\n\t@p st.shared.v2.f64 [%3], {%0, %1};\n\t}"
+                   ::"d"(z.x), "d"(z.y), "r"(high), "r"(o_at + 16 * u) : "memory");
+    if (OUT == kGlobal && high) o[u] = z;
+    if (LAST && u + c31 <= H) {
+      sumM += st.M[kLongRT - 1];
+      sumX += st.X[kLongRT - 1];
+    }
+    z = shfl_up_d2(z);
+  }
+}
+
+// One strip of a long pair.  Entry x of a boundary row is its column x - 30:
+// lane 31 is at that column at step x, and lane 0 consumes entry s + 31 at step
+// s; chunk k holds the entries 32 k .. 32 k + 31.  fph (lane 0) and eph (lane
+// 31) are the parities of the channel barriers' next phases.  Returns the
+// strip's exponent; sumM, sumX: lane 31's last row summed over the haplotype's
+// columns (last strip only).
+__device__ __forceinline__ int run_strip_long(const F64Rows<kLongRT>& w, const unsigned char* __restrict__ hc_lane, int H,
+                                              int nch, int lane, LongMode in, LongMode out, bool last, int in_done,
+                                              int out_done, int l0, int j0, double y0, int y0_exp, const LongIO& io,
+                                              LongShared& sh, unsigned& fph, unsigned& eph, double& sumM, double& sumX) {
+  volatile int* fail = &sh.fail;
+  F64State<kLongRT> st;
+  const bool first = in == kZero;
+#pragma unroll
+  for (int j = 0; j < kLongRT; ++j) {
+    st.M[j] = 0.0;
+    st.X[j] = 0.0;
+    st.Y[j] = (first && l0 == 0 && lane == 0 && j == j0) ? y0 : 0.0;
+  }
+  sumM = 0.0;
+  sumX = 0.0;
+  int E = y0_exp;
+  // carry: lane 31 keeps the last entry of the chunk before the one being staged
+  double2 carry = make_double2(0.0, 0.0);
+  int carry_e = E;
+  double2 ahead = make_double2(0.0, 0.0);  // global input: the chunk after the next, on its way
+  int ahead_e = 0;
+  if (in == kChan) {
+    if (lane == 0) wait_flip(io.in_full, fph, 0, fail);
+    __syncwarp();
+    carry = io.chin[lane];
+    carry_e = io.chin_e[0];
+    __syncwarp();
+    if (lane == 0) mbar_arrive(io.in_empty);
+  } else if (in == kGlobal) {
+    if (lane == 0) wait_done(&sh.done, in_done + min(2, nch), fail);
+    __syncwarp();
+    carry = __ldcg(io.bnd + lane);
+    carry_e = __ldcg(io.bnd_e);
+    if (nch > 1) {
+      ahead = __ldcg(io.bnd + 32 + lane);
+      ahead_e = __ldcg(io.bnd_e + 1);
     }
   }
-  if (io.in_mode == kInGlobal) {
-    fence_for_bulk();
-    __syncwarp();
-    if (lane == 0) {
-      mbar_init(io.ring_mb, 1);
-      mbar_init(io.ring_mb + 1, 1);
-      fence_for_bulk();
-      bulk_g2s(io.ring_in, io.bnd + (size_t)32 * 4, kChunkB, io.ring_mb);
-      dM = io.bnd[31 * 4 + 0] * io.in_scale * io.in_scale2;
-      dX = io.bnd[31 * 4 + 1] * io.in_scale * io.in_scale2;
-      dY = io.bnd[31 * 4 + 2] * io.in_scale * io.in_scale2;
-      if (!*fail && !mbar_wait(io.ring_mb, 0)) { ok = false; *fail = 1; }
-      rphase ^= 1u;
-    }
-    __syncwarp();
-  }
+  if (!first) E = carry_e;
+  else io.stage[lane] = make_double2(0.0, 0.0);
+  double2 z = make_double2(0.0, 0.0);  // nothing lies above column 0
   for (int k = 0; k < nch; ++k) {
-    const int s0 = 32 * k;
-    if (lane == 0) {
-      if (io.in_mode == kInChan && k >= 1 && k + 1 < nch)
-        ok &= wait_flip(io.in_full + (k + 1) % kLongSlots, fph, (k + 1) % kLongSlots, fail);
-      if (io.in_mode == kInGlobal)
-        bulk_g2s(io.ring_in + ((k + 1) & 1) * 32 * 4, io.bnd + (size_t)(32 * (k + 1) + 32) * 4, kChunkB,
-                 io.ring_mb + ((k + 1) & 1));
-    }
-    if (lane == kWarp - 1 && io.out_mode == kOutChan)
-      ok &= wait_flip(io.out_empty + k % kLongSlots, eph, k % kLongSlots, fail);
-    const T* cur = io.chin + (k % kLongSlots) * 32 * 4;
-    const T* nxt = io.chin + ((k + 1) % kLongSlots) * 32 * 4;
-    T* out_slot = io.chout + (k % kLongSlots) * 32 * 4;
-#pragma unroll 8  // a fully unrolled chunk (32 steps, five I/O modes) overflows the instruction cache
-    for (int u = 0; u < 32; ++u) {
-      if (lane == 0) {
-        if (io.in_mode == kInChan) {
-          if (u == 0) { upM = cur[31 * 4]; upX = cur[31 * 4 + 1]; upY = cur[31 * 4 + 2]; }
-          else if (k + 1 < nch) { upM = nxt[(u - 1) * 4]; upX = nxt[(u - 1) * 4 + 1]; upY = nxt[(u - 1) * 4 + 2]; }
-          else { upM = T(0); upX = T(0); upY = T(0); }
-        } else if (io.in_mode == kInGlobal) {
-          const T* rin = io.ring_in + ((k & 1) * 32 + u) * 4;
-          upM = rin[0] * io.in_scale * io.in_scale2;
-          upX = rin[1] * io.in_scale * io.in_scale2;
-          upY = rin[2] * io.in_scale * io.in_scale2;
-        } else {
-          upM = T(0); upX = T(0); upY = T(0);
-        }
+    // the next chunk's entries, one a lane
+    double2 nx = make_double2(0.0, 0.0);
+    int nx_e = carry_e;
+    if (in == kChan && k + 1 < nch) {
+      const int sl = (k + 1) % kLongSlots;
+      if (lane == 0) wait_flip(io.in_full + sl, fph, sl, fail);
+      __syncwarp();
+      nx = io.chin[sl * 32 + lane];
+      nx_e = io.chin_e[sl];
+      __syncwarp();
+      if (lane == 0) mbar_arrive(io.in_empty + sl);
+    } else if (in == kGlobal) {
+      if (k + 1 < nch) {
+        nx = ahead;
+        nx_e = ahead_e;
       }
-      T e[RT];
-      load_emissions<T, RT>(el, (unsigned)hc_lane[s0 + u] * LS::kCodeStride, e);
-      T um = upM, ux = upX;
-      T dm = dM, dx = dX, dy = dY;
+      if (k + 2 < nch) {
+        if (lane == 0) wait_done(&sh.done, in_done + k + 3, fail);
+        __syncwarp();
+        ahead = __ldcg(io.bnd + 32 * (k + 2) + lane);
+        ahead_e = __ldcg(io.bnd_e + k + 2);
+      }
+    }
+    {
+      // the scale of this chunk
+      int top = max(max(exp_of(z.x), exp_of(z.y)), max(exp_of(sumM), exp_of(sumX)));
 #pragma unroll
-      for (int j = 0; j < RT; ++j) {
-        const T mn = e[j] * fma_(rw.mm[j], dm, fma_(rw.cx[j], dx, rw.cy[j] * dy));
-        const T xn = fma_(rw.gx[j], ux, rw.kap[j] * um);
-        const T yn = fma_(rw.g[j], Y[j], rw.my[j] * M[j]);
-        dm = M[j]; dx = X[j]; dy = Y[j];
-        um = mn; ux = xn;
-        M[j] = mn; X[j] = xn; Y[j] = yn;
-      }
-      sumM += M[RT - 1];
-      sumX += X[RT - 1];
-      const T nM = __shfl_up_sync(0xffffffffu, M[RT - 1], 1);
-      const T nX = __shfl_up_sync(0xffffffffu, X[RT - 1], 1);
-      const T nY = __shfl_up_sync(0xffffffffu, Y[RT - 1], 1);
-      if (lane == kWarp - 1) {
-        if (io.out_mode == kOutChan) {
-          T* o = out_slot + u * 4;
-          o[0] = M[RT - 1]; o[1] = X[RT - 1]; o[2] = Y[RT - 1];
-        } else if (io.out_mode == kOutGlobal) {
-          T* o = io.ring_out + u * 4;
-          o[0] = M[RT - 1]; o[1] = X[RT - 1]; o[2] = Y[RT - 1];
-          bmax = fmax(bmax, fmax(M[RT - 1], fmax(X[RT - 1], Y[RT - 1])));
+      for (int j = 0; j < kLongRT; ++j) top = max(top, max(exp_of(st.M[j]), max(exp_of(st.X[j]), exp_of(st.Y[j]))));
+      top += E;
+      top = max(top, max(exp_of(nx.x), exp_of(nx.y)) + nx_e);
+      if (lane == kWarp - 1) top = max(top, max(exp_of(carry.x), exp_of(carry.y)) + carry_e);
+      top = __reduce_max_sync(0xffffffffu, top);
+      if (top > kNoExp / 2 && (top - E > kTopMax || top - E < kTopMin)) {
+        const int d = min(E - (top - kTop), 1000);  // stored values times 2^d
+        const double f = pow2(d);
+#pragma unroll
+        for (int j = 0; j < kLongRT; ++j) {
+          st.M[j] *= f;
+          st.X[j] *= f;
+          st.Y[j] *= f;
         }
+        z.x *= f;
+        z.y *= f;
+        sumM *= f;
+        sumX *= f;
+        y0 *= f;
+        E -= d;
       }
-      dM = upM; dX = upX; dY = upY;
-      upM = nM; upX = nX; upY = nY;
     }
-    // end of chunk k
-    if (lane == kWarp - 1 && io.out_mode == kOutChan) mbar_arrive(io.out_full + k % kLongSlots);
-    if (lane == 0 && io.in_mode == kInChan) mbar_arrive(io.in_empty + k % kLongSlots);
-    if (io.out_mode == kOutGlobal) {
-      __syncwarp();
-      T* dstb = io.bnd + (size_t)(s0 + 1 + lane) * 4;
-      const T* srco = io.ring_out + lane * 4;
-      reinterpret_cast<double2*>(dstb)[0] = reinterpret_cast<const double2*>(srco)[0];
-      reinterpret_cast<double2*>(dstb)[1] = reinterpret_cast<const double2*>(srco)[1];
-      __syncwarp();
-    }
-    if (io.in_mode == kInGlobal) {
-      if (lane == 0) {
-        const int h = (k + 1) & 1;
-        if (!*fail && !mbar_wait(io.ring_mb + h, (rphase >> h) & 1u)) { ok = false; *fail = 1; }
-        rphase ^= 1u << h;
+    if (!first) {
+      // lane 0's inputs of this chunk: the carried entry, then the next chunk's first 31
+      const double f = pow2(nx_e - E);
+      const double2 v = make_double2(nx.x * f, nx.y * f);
+      if (lane < kWarp - 1) {
+        io.stage[lane + 1] = v;
+      } else {
+        const double fc = pow2(carry_e - E);
+        io.stage[0] = make_double2(carry.x * fc, carry.y * fc);
       }
-      __syncwarp();
+      carry = nx;
+      carry_e = nx_e;
     }
+    const int slot = k % kLongSlots;
+    if (lane == kWarp - 1 && out == kChan) {
+      wait_flip(io.out_empty + slot, eph, slot, fail);
+      io.chout_e[slot] = E;
+    }
+    double2* o = out == kChan ? io.chout + slot * 32 : io.bnd + 32 * k;
+    __syncwarp();
+    const unsigned char* hc = hc_lane + 32 * k;
+    auto chunk = [&](auto mode, auto sum) {
+      if (first && k == 0)
+        run_chunk<decltype(mode)::value, true, decltype(sum)::value>(w, st, z, hc, io.stage, o, lane, l0, j0, y0,
+                                                                     32 * k - 30, H, sumM, sumX);
+      else
+        run_chunk<decltype(mode)::value, false, decltype(sum)::value>(w, st, z, hc, io.stage, o, lane, l0, j0, y0,
+                                                                      32 * k - 30, H, sumM, sumX);
+    };
+    using std::integral_constant;
+    if (last) chunk(integral_constant<LongMode, kZero>{}, std::true_type{});
+    else if (out == kChan) chunk(integral_constant<LongMode, kChan>{}, std::false_type{});
+    else chunk(integral_constant<LongMode, kGlobal>{}, std::false_type{});
+    if (lane == kWarp - 1) {
+      if (out == kChan) {
+        mbar_arrive(io.out_full + slot);
+      } else if (out == kGlobal) {
+        io.bnd_e[k] = E;
+        __threadfence_block();
+        *(volatile int*)&sh.done = out_done + k + 1;
+      }
+    }
+    __syncwarp();  // lane 0 has read the staged entries
   }
-  if (io.in_mode == kInGlobal && lane == 0 && ok) {
-    mbar_inval(io.ring_mb);
-    mbar_inval(io.ring_mb + 1);
-  }
-  __syncwarp();
+  return E;
 }
 
 // One block of K warps per long pair (the FP64 list's long part, read from
 // the list's far end).
 template <int K>
-__global__ void __launch_bounds__(K * kWarp) k_forward_long(KernelParams p) {
+__global__ void __launch_bounds__(K * kWarp, 16 / K) k_forward_long(KernelParams p) {
   using L = LongLayout<K>;
   extern __shared__ __align__(16) unsigned char smem[];
   const int lane = threadIdx.x & (kWarp - 1), w = threadIdx.x >> 5;
   unsigned char* hc = smem;
   unsigned char* base = smem + p.hap_bytes;
-  unsigned char* etab = base + w * L::kWarpBytes;
-  const ELane el = elane<double, kLongRT>(etab, lane);
   uint64_t* bars = reinterpret_cast<uint64_t*>(base + L::kBars);
-  uint64_t* full = bars;                                 // [(K-1) * slots]
-  uint64_t* empty = bars + (K - 1) * kLongSlots;         // [(K-1) * slots]
-  uint64_t* grp_done = bars + 2 * (K - 1) * kLongSlots;  // group-end row written
+  uint64_t* full = bars;                          // [(K-1) * slots]
+  uint64_t* empty = bars + (K - 1) * kLongSlots;  // [(K-1) * slots]
   LongShared& sh = *reinterpret_cast<LongShared*>(base + L::kScalars);
-  double* bnd = reinterpret_cast<double*>(p.bnd) + (size_t)blockIdx.x * p.bnd_cols * 4;
   if (threadIdx.x == 0) {
-    for (int i = 0; i < 2 * (K - 1) * kLongSlots + 1; ++i) mbar_init(bars + i, 1);
+    for (int i = 0; i < L::kNumBars; ++i) mbar_init(bars + i, 1);
     sh.fail = 0;
   }
-  fence_for_bulk();
   __syncthreads();
   LongIO io{};
-  io.chin = w >= 1 ? reinterpret_cast<const double*>(base + L::kChan + (w - 1) * kLongSlots * kChunkB) : nullptr;
-  io.in_full = w >= 1 ? full + (w - 1) * kLongSlots : nullptr;
-  io.in_empty = w >= 1 ? empty + (w - 1) * kLongSlots : nullptr;
-  io.chout = w + 1 < K ? reinterpret_cast<double*>(base + L::kChan + w * kLongSlots * kChunkB) : nullptr;
-  io.out_full = w + 1 < K ? full + w * kLongSlots : nullptr;
-  io.out_empty = w + 1 < K ? empty + w * kLongSlots : nullptr;
-  io.bnd = bnd;
-  io.ring_in = reinterpret_cast<double*>(base + L::kRingIn);
-  io.ring_mb = grp_done + 1;
-  io.ring_out = reinterpret_cast<double*>(etab + LS::kEtabBytes);
+  if (w >= 1) {
+    io.chin = reinterpret_cast<const double2*>(base + L::kChan) + (w - 1) * kLongSlots * 32;
+    io.chin_e = reinterpret_cast<const int*>(base + L::kExp) + (w - 1) * kLongSlots;
+    io.in_full = full + (w - 1) * kLongSlots;
+    io.in_empty = empty + (w - 1) * kLongSlots;
+  }
+  if (w + 1 < K) {
+    io.chout = reinterpret_cast<double2*>(base + L::kChan) + w * kLongSlots * 32;
+    io.chout_e = reinterpret_cast<int*>(base + L::kExp) + w * kLongSlots;
+    io.out_full = full + w * kLongSlots;
+    io.out_empty = empty + w * kLongSlots;
+  }
+  // bnd_cols rows of 32 bytes: 16 bytes an entry, the exponents behind them
+  io.bnd = reinterpret_cast<double2*>(p.bnd) + (size_t)blockIdx.x * p.bnd_cols * 2;
+  io.bnd_e = reinterpret_cast<int*>(io.bnd + p.bnd_cols);
+  io.stage = reinterpret_cast<double2*>(base) + w * 32;
   unsigned fph = 0;                        // lane 0: input channel slots' next full phases
   unsigned eph = (1u << kLongSlots) - 1u;  // lane 31: output slots; their first wait passes at once
-  unsigned gph = 0;                        // warp 0, lane 0: group-done barrier
-  bool ok = true;
   volatile int* fail = &sh.fail;
   const DeviceBatch& b = p.batch;
   const unsigned long long n_long = min(p.ctr->rescue_long_count, (unsigned long long)p.rescue_cap);
@@ -301,88 +370,47 @@ __global__ void __launch_bounds__(K * kWarp) k_forward_long(KernelParams p) {
       __syncthreads();
       continue;
     }
-    const double init_y = p.tables->init_d / (double)H;
-    const int nsteps = (H + kWarp - 1 + 31) / 32 * 32;
-    const int rows = R + 1;
-    const int nstrips = (rows + 32 * kLongRT - 1) / (32 * kLongRT);
-    const int pad = nstrips * 32 * kLongRT - rows;
-    stage_hap_block(b.hap_bases + ho, H, hc, nsteps + kHapLead);
-    // boundary rows past the last column, read as zeros by a group's first strip
-    for (int x = threadIdx.x; x < 96; x += blockDim.x) {
-      double* r = bnd + (size_t)(nsteps + 1 + x) * 4;
-      r[0] = 0.0; r[1] = 0.0; r[2] = 0.0;
-    }
-    fence_for_bulk();  // those rows are read by bulk copies
+    const int nch = (H + kWarp - 1 + 31) / 32;
+    const int nstrips = (R + 1 + kStrip - 1) / kStrip;
+    const int pad = nstrips * kStrip - (R + 1);  // padding rows on top of row 0
+    // initial row: init / H, stored with exponent y0_exp
+    const int y0_exp = kF64InitExp - kTop;
+    const double y0 = ldexp(p.tables->init_d, -y0_exp) / (double)H;
+    stage_hap_block(b.hap_bases + ho, H, hc, 32 * nch + kHapLead);
     if (threadIdx.x == 0) {
-      sh.kexp = 0;
+      sh.done = 0;
       sh.redo = 0;
     }
     __syncthreads();
     for (int s = w; s < nstrips; s += K) {
-      Rows<double, kLongRT> rw;
-      setup_rows<double, kLongRT>(p.tables, quals, bases, R, s * 32 * kLongRT + lane * kLongRT - pad, init_y, rw,
-                                  etab, lane);
-      __syncwarp();
-      io.in_mode = s == 0 ? kInZero : (s % K == 0 ? kInGlobal : kInChan);
-      io.out_mode = s == nstrips - 1 ? kOutNone : (s % K == K - 1 ? kOutGlobal : kOutChan);
-      io.in_scale = 1.0;
-      io.in_scale2 = 1.0;
-      if (io.in_mode == kInGlobal) {
-        // renormalise: the previous group's last row, maximum scaled to 2^target
-        // (a factor up to 2^2074 does not fit one double: two factors, each exact)
-        double m = 0.0;
-        if (lane == 0) {
-          ok &= wait_flip(grp_done, gph, 0, fail);
-          m = sh.grp_max;
-        }
-        m = __shfl_sync(0xffffffffu, m, 0);
-        if (m > 0.0) {
-          int e2;
-          frexp(m, &e2);
-          const int shift = e2 - p.rescale_target;
-          const int a = min(-shift, 1023), b2 = min(-shift - a, 1023);
-          io.in_scale = ldexp(1.0, a);
-          io.in_scale2 = ldexp(1.0, b2);
-          if (lane == 0) sh.kexp += shift;
-          // the group fell far below the one-warp kernel's per-strip range: that kernel redoes the pair
-          if (lane == 0 && e2 < kLongMinExp) sh.redo = 1;
-        } else if (lane == 0) {
+      F64Rows<kLongRT> rw;
+      const bool fold =
+          f64_setup<kLongRT, false>(p.tables, quals, bases, R, s * kStrip + lane * kLongRT - pad, rw);
+      if (!fold) sh.redo = 1;
+      const LongMode in = s == 0 ? kZero : (w == 0 ? kGlobal : kChan);
+      const bool last = s == nstrips - 1;
+      const LongMode out = last ? kZero : (w == K - 1 ? kGlobal : kChan);
+      double sumM, sumX;
+      const int E = run_strip_long(rw, hc + kHapLead - lane, H, nch, lane, in, out, last, (s / K - 1) * nch,
+                                   (s / K) * nch, pad / kLongRT, pad % kLongRT, y0, y0_exp, io, sh, fph, eph, sumM, sumX);
+      if (last && lane == kWarp - 1) {
+        const double pmx = p.tables->const_mode ? p.tables->cd[1] : p.tables->ph2pr_d[quals[R - 1].y & kQualMask];
+        const double res = sumM + pmx * sumX;
+        if (!(res > 0.0 && isfinite(res))) {
           sh.redo = 1;
-        }
-        __syncwarp();
-      }
-      double sumM, sumX, bmax;
-      run_strip_long<kLongRT>(rw, el, hc + kHapLead - lane, nsteps, lane, io, fph, eph, sumM, sumX, bmax, ok, fail);
-      if (io.out_mode == kOutGlobal) {
-        fence_for_bulk();  // the rows just written are read by bulk copies
-        __syncwarp();
-        if (lane == kWarp - 1) sh.grp_max = bmax;
-        __syncwarp();
-        if (lane == 0) mbar_arrive(grp_done);
-      }
-      if (s == nstrips - 1 && lane == kWarp - 1) {
-        const double res = sumM + sumX;
-        if (sh.redo || !(res > 0.0 && isfinite(res))) {
-          sh.redo = 1;
-        } else {
-          write_result<double>(p, pr.read, pr.hap, pr.out, res, sh.kexp);
+        } else if (!*(volatile int*)&sh.redo) {
+          write_result<double>(p, pr.read, pr.hap, pr.out, res, E);
           if (p.cells_ctr) atomicAdd(p.cells_ctr, (unsigned long long)R * (unsigned long long)H);
         }
       }
     }
     __syncthreads();
-    // handed back: the entry is marked (read index complemented) for the one-warp FP64 kernel
+    // handed back: the entry is marked (read index complemented) for k_f64_list
     if (threadIdx.x == 0 && sh.redo) p.rescue[p.rescue_cap - 1 - wi].read = ~pr.read;
   }
-  if (!ok) atomicOr(&p.ctr->status, 8ull);
+  if (threadIdx.x == 0 && *fail) atomicOr(&p.ctr->status, 8ull);
 }
 
-}  // namespace
-
-// The kernel for `warps` warps per pair (2, 4 or 8; long_warps_valid).
-namespace {
-template <int K>
-int smem_for(int hap_bytes) { return hap_bytes + LongLayout<K>::kBytes; }
 template <int K>
 int blocks_for(int smem) {
   int nb = 0;
@@ -392,27 +420,32 @@ int blocks_for(int smem) {
 }
 }  // namespace
 
-bool long_warps_valid(int warps) { return warps == 2 || warps == 4 || warps == 8; }
+bool long_warps_valid(int warps) { return warps == 2 || warps == 4 || warps == 8 || warps == 16; }
 
 int long_smem_bytes(int hap_bytes, int warps) {
-  return warps == 2 ? smem_for<2>(hap_bytes) : warps == 8 ? smem_for<8>(hap_bytes) : smem_for<4>(hap_bytes);
+  return hap_bytes + (warps == 2    ? LongLayout<2>::kBytes
+                      : warps == 4  ? LongLayout<4>::kBytes
+                      : warps == 8  ? LongLayout<8>::kBytes
+                                    : LongLayout<16>::kBytes);
 }
 
 cudaError_t prepare_long(int smem, int warps) {
   const void* f = warps == 2   ? reinterpret_cast<const void*>(&k_forward_long<2>)
+                  : warps == 4 ? reinterpret_cast<const void*>(&k_forward_long<4>)
                   : warps == 8 ? reinterpret_cast<const void*>(&k_forward_long<8>)
-                               : reinterpret_cast<const void*>(&k_forward_long<4>);
+                               : reinterpret_cast<const void*>(&k_forward_long<16>);
   return raise_dynamic_smem(f, smem);
 }
 
 int long_blocks_per_sm(int smem, int warps) {
-  return warps == 2 ? blocks_for<2>(smem) : warps == 8 ? blocks_for<8>(smem) : blocks_for<4>(smem);
+  return warps == 2 ? blocks_for<2>(smem) : warps == 4 ? blocks_for<4>(smem) : warps == 8 ? blocks_for<8>(smem) : blocks_for<16>(smem);
 }
 
 cudaError_t launch_forward_long(const KernelParams& p, int grid, int smem, int warps, cudaStream_t st) {
   if (warps == 2) k_forward_long<2><<<grid, 2 * kWarp, smem, st>>>(p);
+  else if (warps == 4) k_forward_long<4><<<grid, 4 * kWarp, smem, st>>>(p);
   else if (warps == 8) k_forward_long<8><<<grid, 8 * kWarp, smem, st>>>(p);
-  else k_forward_long<4><<<grid, 4 * kWarp, smem, st>>>(p);
+  else k_forward_long<16><<<grid, 16 * kWarp, smem, st>>>(p);
   return cudaGetLastError();
 }
 

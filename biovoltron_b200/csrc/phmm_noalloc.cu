@@ -10,7 +10,7 @@
 // into that memory without the library reserving anything.
 //
 // How.  bv_phmm_forward_f64_noalloc runs a variant of the FP64 multi-strip
-// forward kernel (k_forward<double, 4, multi-strip>, phmm_forward.cu): the
+// forward pass (process_item<double, 4, multi-strip>, phmm_device.cuh): the
 // scratch that kernel normally takes from context-owned allocations -- the
 // work-queue counters, the probability tables and one strip-boundary buffer
 // per resident warp -- lives here in one file-scope __device__ array of fixed
@@ -196,7 +196,6 @@ extern "C" bv_status bv_phmm_forward_f64_noalloc(int device, const bv_phmm_devic
     p.out = out_log10;
     p.rescue = const_cast<PairRef*>(static_cast<const PairRef*>(in->pairs));
     p.rescue_cap = in->num_pairs;
-    p.from_rescue = 1;
     p.hap_bytes = kHapBytes;
     p.warp_smem_bytes = kHapBytes + WarpSmem<double, kRT>::kEtabBytes + WarpSmem<double, kRT>::kRingBytes;
     p.bnd = scratch + kCountersBytes + kTablesBytes;

@@ -437,9 +437,11 @@ bv_status bv_phmm_autotune(bv_phmm_ctx* ctx, const bv_region_batch* sample, int3
  * not listed keep their values (defaults: two haplotypes per warp, 4 warps). */
 bv_status bv_phmm_set_tuning(bv_phmm_ctx* ctx, const bv_phmm_tune_entry* entries, int32_t num);
 bv_status bv_phmm_get_tuning(bv_phmm_ctx* ctx, bv_phmm_tune_entry* out, int32_t* num_out);
-/* The FP64 long-read kernel: a block of `warps` warps per pair (2, 4 or 8;
- * default 4) runs reads of at least 128 x warps bases, strip w of every
- * group of `warps` strips on warp w.  bv_phmm_autotune_long stages `sample`
+/* The FP64 long-read kernel: a block of `warps` warps per pair (2, 4 or 8)
+ * runs reads of at least 128 x warps bases, strip w of every group of `warps`
+ * strips on warp w.  Until it is set or tuned (get then says 4) every read of
+ * more than 253 bases takes the kernel, with 2 to 16 warps chosen from the
+ * batch.  bv_phmm_autotune_long stages `sample`
  * in FP64 mode for each choice (the long-read edge moves with it), times the
  * FP64 pass (`repeats` runs, median), installs the fastest and writes it to
  * *warps_out and the times to ms_out[0..2] (2, 4, 8 warps; 0 where the

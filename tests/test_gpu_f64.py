@@ -1,0 +1,123 @@
+"""FP64 kernels in the scaled, folded form (single strips, long reads) at the
+edges of their range, against the rescaled FP64 oracle: |d log10| <= 1e-9, the
+bound the unscaled FP64 kernels are held to."""
+import numpy as np
+import pytest
+
+from biovoltron_b200 import workloads as W
+from oracle.oracle import TestcaseArray
+
+pytestmark = pytest.mark.gpu
+
+TOL = 1e-9
+
+
+def _check(b, got, oracle):
+    truth = oracle.log10_rescaled(TestcaseArray.for_batch(b))
+    fin = np.isfinite(truth)
+    assert np.array_equal(np.isfinite(got), fin)
+    assert np.max(np.abs(got[fin] - truth[fin]), initial=0) <= TOL
+
+
+def _pair(rng, n, hap_len, related=True, gaps=(45, 45, 10), qlo=10, qhi=40):
+    hap = W._random_seq(rng, hap_len)
+    at = int(rng.integers(0, max(1, hap_len - n + 1)))
+    read = W._mutate_read(rng, hap, at, n, 0.02, 0.01, 1, 3) if related and hap_len >= n else W._random_seq(rng, n)
+    q, i, d, c = W._quals(rng, len(read), qlo, qhi, *gaps)
+    return [(read, q, i, d, c)], [hap]
+
+
+# every rows-per-lane bin's edges, the longest single strip (253) and the first two-strip reads, haplotypes
+# shorter and longer than the read, unrelated pairs (results far below the kept range: handed to the
+# unscaled kernel), rows that cannot fold (indel qualities of 0-3), varying gap qualities
+def _short_cases(rng):
+    regions = []
+    for n in (1, 2, 28, 29, 30, 61, 62, 93, 94, 125, 126, 157, 158, 189, 190, 221, 222, 252, 253, 254, 255, 300):
+        regions.append(_pair(rng, n, n + int(rng.integers(0, 200))))
+        regions.append(_pair(rng, n, 3 + n // 2, related=False))
+    for n in (150, 253):
+        regions.append(_pair(rng, n, 400, related=False, qlo=39, qhi=40))
+        regions.append(_pair(rng, n, 400, gaps=(2, 2, 10)))
+        regions.append(_pair(rng, n, 400, gaps=(0, 3, 0)))
+    reads, haps = _pair(rng, 200, 500)
+    r, q, i, d, c = reads[0]
+    i, d, c = (rng.integers(0, 128, len(r)).astype(np.uint8) for _ in range(3))
+    regions.append(([(r, q, i, d, c), (r, q, i | 16, d | 16, c)], haps * 3))
+    return W._build(regions, "short reads in FP64")
+
+
+def test_single_strip_edges(oracle):
+    from biovoltron_b200.pairhmm import PairHMMEngine
+    b = _short_cases(np.random.default_rng(3))
+    with PairHMMEngine(precision="f64") as e:
+        got, st = e.compute_regions(b, with_stats=True)
+        _check(b, got, oracle)
+        assert st["rescued"] == b.n_pairs and st["rescued_cells"] == b.n_cells()
+        n = e.stage(b)
+        for _ in range(3):  # the handed-back pairs are scored again by every replay
+            e.run()
+            assert np.array_equal(e.fetch(n), got)
+    with PairHMMEngine() as e:  # the rescue of the pairs FP32 cannot hold takes the same kernels
+        auto, st = e.compute_regions(b, with_stats=True)
+        assert 0 < st["rescued"] < b.n_pairs
+        fin = np.isfinite(got)
+        assert np.all(np.abs(auto[fin] - got[fin]) <= 1e-4)
+
+
+def test_units_of_several_haplotypes(oracle):
+    from biovoltron_b200.pairhmm import PairHMMEngine
+    rng = np.random.default_rng(5)
+    b = W.config1(seed=11, n_regions=3)
+    out = []
+    for unit in (1, 3, 8):
+        with PairHMMEngine(precision="f64", haps_per_unit=unit) as e:
+            out.append(e.compute_regions(b))
+    _check(b, out[0], oracle)
+    assert all(np.array_equal(o, out[0]) for o in out)
+
+
+def test_scalar_transitions_with_a_zero(engine, oracle):
+    """A zero insertion probability has no scaled form: the unscaled kernel takes the pair."""
+    from biovoltron_b200.pairhmm import PairHMMEngine
+    rng = np.random.default_rng(7)
+    b = W._build([_pair(rng, 120, 260), _pair(rng, 700, 900)], "scalar")
+    for trans in ((0.9998, 0.0001, 0.0001, 0.9, 0.1, 0.9, 0.1), (0.9999, 0.0, 0.0001, 0.9, 0.1, 0.9, 0.1)):
+        with PairHMMEngine(precision="f64") as e:
+            e.set_transitions(trans)
+            got = e.compute_regions(b)
+        for k in range(b.n_reads):
+            rd = b.read(k)
+            want = oracle.scalar_log10(bytes(rd[0]), bytes(rd[1]), b.hap(k), trans)
+            if np.isfinite(want):
+                assert abs(got[k] - want) <= TOL
+
+
+# strip and group edges of the long-read kernel for every block size; few pairs (blocks of 16 warps), more
+# pairs than SMs (8 and 4), unrelated pairs whose mass falls by thousands of binary orders, a read longer
+# than its haplotype, rows that cannot fold
+@pytest.mark.parametrize("copies", [1, 9, 18])
+def test_long_reads(oracle, copies):
+    from biovoltron_b200.pairhmm import PairHMMEngine
+    rng = np.random.default_rng(9)
+    regions = [_pair(rng, n, h) for n, h in ((254, 300), (255, 700), (256, 256), (383, 500), (511, 640), (512, 900),
+                                             (1023, 1100), (1024, 1300), (2047, 2100), (2048, 2300), (2049, 2200),
+                                             (4095, 4200), (4500, 5000))]
+    regions += [_pair(rng, 900, 600, related=False), _pair(rng, 1500, 1500, related=False, qlo=38, qhi=40),
+                _pair(rng, 2500, 3000, gaps=(20, 60, 10)), _pair(rng, 300, 33, related=False), _pair(rng, 400, 1),
+                _pair(rng, 600, 900, gaps=(1, 2, 10))]
+    b = W._build(regions, "long reads")
+    big = W._build(regions * copies, "long reads, several times")
+    with PairHMMEngine(precision="f64") as e:
+        got = e.compute_regions(big)
+        assert np.array_equal(got.reshape(copies, -1), np.tile(got[:b.n_pairs], (copies, 1)))
+        _check(b, got[:b.n_pairs], oracle)
+        n = e.stage(big)
+        for _ in range(2):
+            e.run()
+            assert np.array_equal(e.fetch(n), got)
+        for k in (2, 4, 8):
+            e.set_long_warps(k)
+            _check(b, e.compute_regions(b), oracle)
+    with PairHMMEngine() as e:
+        _, st = e.compute_regions(b, with_stats=True)
+        assert st["rescued"] > 0
