@@ -38,6 +38,7 @@ constexpr int kOut = 2;                // outputs: lower and upper band edge (di
 constexpr int kHistBins = 64;          // histogram window: d* - 32 .. d* + 31
 constexpr int kBandMaxSpan = 2048;     // read_len + hap_len limit of the featuriser (per-warp histogram)
 constexpr int kBandMaxHap = 1024;      // haplotype limit of the k-mer sort and the featuriser's staging
+constexpr int kLabelClasses = 8;       // launches of the label kernel (haplotype lengths up to 128, 256, .. 1024)
 constexpr int kBandWidths = 4;         // width classes of the banded kernel
 #if defined(__CUDACC__)
 __host__ __device__
@@ -85,6 +86,7 @@ struct BandCounters {
   unsigned int gap_mixed;                                 // some base's gap qualities differ from the first base's
   unsigned long long cap_count[16];                       // banded pairs rescored by the full DP, per variant
   unsigned long long cap_flagged;                         // their total
+  unsigned long long label_next[kLabelClasses];           // work-queue heads of the label kernel's launches
 };
 // work-queue slots of the rescore launches (the fallback launches use 0 .. 8, the audit 16 .. 24)
 constexpr int kCapSlot0 = 32;

@@ -101,15 +101,14 @@ bv_status Engine::compute_labels(const bv_region_batch& b, float tau, float* ms)
   int max_r = 0, max_h = 0;
   for (int64_t r = 0; r < b.num_reads; ++r) max_r = std::max<int>(max_r, (int)(b.read_offsets[r + 1] - b.read_offsets[r]));
   for (int64_t h = 0; h < b.num_haps; ++h) max_h = std::max<int>(max_h, (int)(b.hap_offsets[h + 1] - b.hap_offsets[h]));
+  const int longest = max_r;
   max_r = std::min(max_r, kBandMaxRead);
   max_h = std::min(max_h, kBandMaxHap);
-  const long long stride = (long long)(max_r + 1) * 3 * (max_h + 2);
-  const size_t per_block = (size_t)stride * sizeof(float) * label_warps_per_block();
-  const int blocks = (int)std::max<size_t>(1, std::min<size_t>((size_t)sms_ * 2, kLabelBufLimit / per_block));
+  const LabelRows rows = label_rows(max_r, longest, max_h, sms_, kLabelBufLimit);
   const int64_t n = std::max<int64_t>(n_results_, 1);
   BV_CUDA(d_lab_lo_.reserve(sizeof(int32_t) * n), "alloc labels");
   BV_CUDA(d_lab_hi_.reserve(sizeof(int32_t) * n), "alloc labels");
-  BV_CUDA(d_lab_fbuf_.reserve(per_block * blocks), "alloc label rows");
+  BV_CUDA(d_lab_fbuf_.reserve(rows.bytes), "alloc label rows");
   DeviceBatch db{};
   db.read_bases = d_read_bases_.as<uint8_t>();
   db.read_quals = d_quals4_.as<uchar4>();
@@ -118,8 +117,9 @@ bv_status Engine::compute_labels(const bv_region_batch& b, float tau, float* ms)
   db.hap_off = d_hap_off_.as<int64_t>();
   BV_CUDA(cudaEventRecord(ev_[0], stream_), "event");
   BV_CUDA(launch_posterior_spread(db, d_tables_.as<Tables>(), d_pair_read_.as<int32_t>(), d_pair_hap_.as<int32_t>(),
-                                  n_results_, tau, d_lab_fbuf_.as<float>(), stride, d_lab_lo_.as<int32_t>(),
-                                  d_lab_hi_.as<int32_t>(), blocks, stream_), "labels");
+                                  n_results_, tau, d_lab_fbuf_.as<float>(), rows, max_h,
+                                  d_bctr_.as<BandCounters>()->label_next, d_lab_lo_.as<int32_t>(),
+                                  d_lab_hi_.as<int32_t>(), stream_), "labels");
   BV_CUDA(cudaEventRecord(ev_[1], stream_), "event");
   BV_CUDA(cudaStreamSynchronize(stream_), "labels sync");
   float t = 0;

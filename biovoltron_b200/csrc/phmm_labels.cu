@@ -10,27 +10,43 @@
 //   B_X(r,c) = gp(r+1) e(r+1,c+1) B_M(r+1,c+1) + g(r+1) B_X(r+1,c) + [r==R]
 //   B_Y(r,c) = gp(r+1) e(r+1,c+1) B_M(r+1,c+1) + g(r) B_Y(r,c+1)
 //
-// One warp per pair; lane l owns columns [l*C + 1, (l+1)*C] of a row.  M and X
-// of a row depend only on the previous row (kept in shared memory); the
-// in-row Y recurrence is affine with a per-row constant (Y(c) = g Y(c-1) +
-// t(c)), solved by a warp scan over the lanes' chunks.  Every row is
-// renormalised by a power of two; the per-row normalisation of p_r makes the
-// scales cancel.  Forward rows go to a per-warp global buffer that the
-// backward reads back.
+// One warp per pair; lane l owns the C = ceil(H / 32) columns l C + 1 .. of a
+// row and keeps their states in registers (template CM >= C: one launch per
+// class of haplotype lengths; columns past the haplotype hold zeros).  M and X
+// of a row depend only on the previous row (one shuffle brings the column left
+// of the lane's first); the in-row Y recurrence is affine with a per-row
+// constant (Y(c) = g Y(c-1) + t(c)), solved by a warp scan over the lanes'
+// chunks.  Every row is renormalised by a power of two; the per-row
+// normalisation of p_r makes the scales cancel.  Forward rows go to a per-warp
+// global buffer, column-interleaved so that a warp's stores and loads are
+// whole lines, and the backward reads them once.  pstar moves with the row: a
+// lane's register for column c holds diagonal c - r, so going one row up
+// shifts it by one column, and the diagonal that leaves column 1 is final.
+//
+// Bound by latency: a row's two affine chains, its warp scan and its three
+// reductions follow one another, with 8 to 12 warps an SM to hide them (the
+// forward rows' traffic, 24 bytes a cell, is a quarter of the time).  24 k pairs
+// of 150 x 450: 10 ms.  States and pstar in shared memory (33 KB a warp, a lane
+// stride of C words and its bank conflicts) took 80; classes of 256 and 128
+// columns with a branch at every column 21; four columns a class leave the
+// branch to the last three.
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cstdint>
+#include <type_traits>
+#include <utility>
 
 #include "phmm_band.h"
 #include "phmm_common.h"
 #include "phmm_kernels.h"
+#include "phmm_mlp.h"
 
 namespace bvphmm {
 namespace {
 
 constexpr int kLabelMaxH = kBandMaxHap;   // columns per pair
 constexpr int kLabelWarps = 4;
-constexpr int kLabelCols = kLabelMaxH + 2;
 
 __device__ __forceinline__ uint32_t code_of(uint8_t b) {
   return b == 'C' ? 1u : b == 'T' ? 2u : b == 'G' ? 3u : b == 'N' ? 4u : 0u;
@@ -58,10 +74,6 @@ __device__ __forceinline__ RowC row_consts(const Tables* tb, const uchar4* quals
   return k;
 }
 
-__device__ __forceinline__ float emis(const RowC& k, uint32_t hc) {
-  return (k.rc == hc || k.rc == 4u || hc == 4u) ? k.em : k.ex;
-}
-
 // Inclusive warp scan of affine maps y -> a*y + b (lane order = left to right
 // when `forward`, right to left otherwise).  Returns the map composed over
 // the lanes before this one applied to 0, i.e. the carry-in.
@@ -85,173 +97,251 @@ __device__ __forceinline__ float warp_sum(float v) {
   return v;
 }
 
-__global__ void __launch_bounds__(kLabelWarps * 32) k_posterior_spread(DeviceBatch b, const Tables* tb,
-                                                                      const int32_t* pair_read, const int32_t* pair_hap,
-                                                                      long long n_pairs, float tau, float* fbuf,
-                                                                      long long fbuf_stride, int32_t* lo_out,
-                                                                      int32_t* hi_out) {
-  extern __shared__ __align__(16) unsigned char smem[];
+// Pairs whose C lies in (CL, CM]; `first`: this launch also marks the pairs
+// that get no label.  Warps take `grab` pairs at a time from *next.
+template <int CL, int CM>
+__global__ void __launch_bounds__(kLabelWarps * 32, CM <= 20 ? 3 : 2)
+    k_posterior_spread(DeviceBatch b, const Tables* tb, const int32_t* pair_read, const int32_t* pair_hap,
+                       long long n_pairs, float tau, float* fbuf, long long fbuf_stride, long long max_area,
+                       unsigned long long* next, int grab, bool first, int32_t* lo_out, int32_t* hi_out) {
   const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
-  float* prevM = reinterpret_cast<float*>(smem) + (size_t)wib * (6 * kLabelCols + kBandMaxSpan);
-  float* prevX = prevM + kLabelCols;
-  float* prevY = prevX + kLabelCols;
-  float* curM = prevY + kLabelCols;
-  float* curX = curM + kLabelCols;
-  float* curY = curX + kLabelCols;
-  float* pstar = curY + kLabelCols;
-  uint8_t* hcode = reinterpret_cast<uint8_t*>(reinterpret_cast<float*>(smem) + (size_t)kLabelWarps * (6 * kLabelCols + kBandMaxSpan)) +
-                   (size_t)wib * kLabelCols;
-  const long long warp = blockIdx.x * (long long)kLabelWarps + wib;
-  float* F = fbuf + warp * fbuf_stride;
-  for (long long pi = warp; pi < n_pairs; pi += (long long)gridDim.x * kLabelWarps) {
-    const int r_idx = pair_read[pi], h_idx = pair_hap[pi];
-    const int64_t ro = b.read_off[r_idx], ho = b.hap_off[h_idx];
-    const int R = (int)(b.read_off[r_idx + 1] - ro), H = (int)(b.hap_off[h_idx + 1] - ho);
-    if (R < 1 || H < 1 || H > kLabelMaxH || R + H >= kBandMaxSpan ||
-        (long long)(R + 1) * 3 * (H + 2) > fbuf_stride) {
-      if (lane == 0) { lo_out[pi] = INT32_MIN; hi_out[pi] = INT32_MIN; }
-      continue;
-    }
-    const uchar4* quals = b.read_quals + ro;
-    const uint8_t* bases = b.read_bases + ro;
-    const int C = (H + 31) / 32;
-    const int c0 = lane * C + 1, c1 = min(c0 + C - 1, H);  // this lane's columns (may be empty)
-    __syncwarp();
-    for (int c = lane; c < H; c += 32) hcode[c + 1] = (uint8_t)code_of(b.hap_bases[ho + c]);
-    for (int x = lane; x < R + H; x += 32) pstar[x] = 0.f;
-    for (int c = lane; c <= H + 1; c += 32) { prevM[c] = 0.f; prevX[c] = 0.f; prevY[c] = 1.f; curM[c] = 0.f; curX[c] = 0.f; curY[c] = 0.f; }
-    __syncwarp();
-    // ---- forward, rows 1..R; row r stored at F[r * 3 * (H+2) + {0, H+2, 2(H+2)} + c]
-    const int stride = H + 2;
-    for (int r = 1; r <= R; ++r) {
-      const RowC k = row_consts(tb, quals, bases, r);
-      // M, X from the previous row; the Y pass with its carry-in follows
-      for (int c = c0; c <= c1; ++c) {
-        const float e = emis(k, hcode[c]);
-        curM[c] = e * (k.mm * prevM[c - 1] + k.gp * (prevX[c - 1] + prevY[c - 1]));
-        curX[c] = k.mx * prevM[c] + k.g * prevX[c];
+  float* F = fbuf + (blockIdx.x * (long long)kLabelWarps + wib) * fbuf_stride + lane;
+  for (;;) {
+    long long base = 0;
+    if (lane == 0) base = (long long)atomicAdd(next, (unsigned long long)grab);
+    base = __shfl_sync(0xffffffffu, base, 0);
+    if (base >= n_pairs) break;
+    for (long long pi = base; pi < min(base + grab, n_pairs); ++pi) {
+      const int r_idx = pair_read[pi], h_idx = pair_hap[pi];
+      const int64_t ro = b.read_off[r_idx], ho = b.hap_off[h_idx];
+      const int R = (int)(b.read_off[r_idx + 1] - ro), H = (int)(b.hap_off[h_idx + 1] - ho);
+      if (R < 1 || H < 1 || H > kLabelMaxH || R + H >= kBandMaxSpan || (long long)(R + 1) * 3 * (H + 2) > max_area) {
+        if (first && lane == 0) { lo_out[pi] = INT32_MIN; hi_out[pi] = INT32_MIN; }
+        continue;
       }
-      __syncwarp();
-      // Y(c) = g Y(c-1) + my M(c-1): affine along the row
-      const float mleft = (c0 <= H && c0 > 1) ? curM[c0 - 1] : 0.f;
-      float a = 1.f, bb = 0.f;
-      {
-        float y = 0.f, m = mleft;
-        for (int c = c0; c <= c1; ++c) { y = k.g * y + k.my * m; m = curM[c]; a *= k.g; }
-        bb = y;
-      }
-      if (c0 > c1) { a = 1.f; bb = 0.f; }
-      const float carry = affine_carry(a, bb, lane, true);
-      {
-        float y = carry, m = mleft;
-        for (int c = c0; c <= c1; ++c) { y = k.g * y + k.my * m; curY[c] = y; m = curM[c]; }
-      }
-      __syncwarp();
-      float mx = 0.f;
-      for (int c = c0; c <= c1; ++c) mx = fmaxf(mx, fmaxf(curM[c], fmaxf(curX[c], curY[c])));
-      mx = warp_max(mx);
-      const float sc = mx > 0.f ? ldexpf(1.f, -ilogbf(mx)) : 1.f;
-      float* Fr = F + (size_t)r * 3 * stride;
-      for (int c = lane; c <= H; c += 32) {
-        const float m = c == 0 ? 0.f : curM[c] * sc, x = c == 0 ? 0.f : curX[c] * sc, y = c == 0 ? 0.f : curY[c] * sc;
-        prevM[c] = m; prevX[c] = x; prevY[c] = y;
-        Fr[c] = m; Fr[stride + c] = x; Fr[2 * stride + c] = y;
-      }
-      __syncwarp();
-    }
-    // ---- backward, rows R..1, B of row r+1 in prev*, posterior per row
-    for (int c = lane; c <= H + 1; c += 32) { prevM[c] = 0.f; prevX[c] = 0.f; prevY[c] = 0.f; }
-    __syncwarp();
-    RowC k1{};  // constants of row r+1
-    for (int r = R; r >= 1; --r) {
-      const RowC k0 = row_consts(tb, quals, bases, r);
-      // B_Y(c) = g(r) B_Y(c+1) + t(c), right to left, t(c) = gp(r+1) e(r+1,c+1) B_M(r+1,c+1)
-      float a = 1.f, bb = 0.f;
-      auto tval = [&](int c) -> float {
-        if (r == R || c + 1 > H) return 0.f;
-        return k1.gp * emis(k1, hcode[c + 1]) * prevM[c + 1];
+      const int C = (H + 31) / 32;
+      if (C <= CL || C > CM) continue;
+      const uchar4* quals = b.read_quals + ro;
+      const uint8_t* bases = b.read_bases + ro;
+      const int nc = max(0, min(C, H - lane * C));  // this lane's columns
+      // bit j of match[h]: column j matches read code h
+      uint32_t match[4] = {0, 0, 0, 0};
+#pragma unroll
+      for (int j = 0; j < CM; ++j)
+        if (j < nc) {
+          const uint32_t hc = code_of(b.hap_bases[ho + lane * C + j]);
+#pragma unroll
+          for (uint32_t h = 0; h < 4; ++h) match[h] |= (uint32_t)(hc == h || hc == 4u) << j;
+        }
+      auto row_match = [&](uint32_t rc) {
+        return rc == 0 ? match[0] : rc == 1 ? match[1] : rc == 2 ? match[2] : rc == 3 ? match[3] : 0xffffffffu;
       };
-      {
-        float y = 0.f;
-        for (int c = c1; c >= c0; --c) { y = k0.g * y + tval(c); a *= k0.g; }
-        bb = y;
+      float M[CM], X[CM], Y[CM];
+#pragma unroll
+      for (int j = 0; j < CM; ++j) {
+        M[j] = 0.f;
+        X[j] = 0.f;
+        Y[j] = j < nc ? 1.f : 0.f;
       }
-      if (c0 > c1) { a = 1.f; bb = 0.f; }
-      const float carry = affine_carry(a, bb, lane, false);
-      {
-        float y = carry;  // B_Y(r, c+1)
-        for (int c = c1; c >= c0; --c) {
-          const float byr = y;
-          y = k0.g * y + tval(c);
-          curY[c] = y;
-          if (r == R) {
-            curM[c] = 1.f;
-            curX[c] = 1.f;
-          } else {
-            const float nm = (c + 1 <= H) ? emis(k1, hcode[c + 1]) * prevM[c + 1] : 0.f;
-            curM[c] = k1.mm * nm + k1.mx * prevX[c] + k0.my * byr;
-            curX[c] = k1.gp * nm + k1.g * prevX[c];
+      // ---- forward, rows 1..R; row r's states at F + r * 3 * 32 C: M, X, Y, column j of all lanes together
+      const long long row_floats = 96ll * C;
+      float tM = 0.f, tX = 0.f, tY = 1.f;  // the lane's last column
+      RowC k = row_consts(tb, quals, bases, 1);
+      for (int r = 1; r <= R; ++r) {
+        const RowC kn = row_consts(tb, quals, bases, min(r + 1, R));
+        const uint32_t mm = row_match(k.rc);
+        float oM = __shfl_up_sync(0xffffffffu, tM, 1), oX = __shfl_up_sync(0xffffffffu, tX, 1);
+        float oY = __shfl_up_sync(0xffffffffu, tY, 1);
+        if (lane == 0) { oM = 0.f; oX = 0.f; oY = r == 1 ? 1.f : 0.f; }
+        float lastM = 0.f;
+#pragma unroll
+        for (int j = 0; j < CM; ++j)
+          if (j <= CL || j < C) {
+            const float e = (mm >> j & 1u) ? k.em : k.ex;
+            const float nM = e * (k.mm * oM + k.gp * (oX + oY));
+            const float nX = k.mx * M[j] + k.g * X[j];
+            oM = M[j]; oX = X[j]; oY = Y[j];
+            M[j] = j < nc ? nM : 0.f;
+            X[j] = nX;
+            lastM = M[j];
           }
+        // Y(c) = g Y(c-1) + my M(c-1): affine along the row
+        float mleft = __shfl_up_sync(0xffffffffu, lastM, 1);
+        if (lane == 0) mleft = 0.f;
+        float a = 1.f, bb = 0.f;
+        {
+          float y = 0.f, m = mleft;
+#pragma unroll
+          for (int j = 0; j < CM; ++j)
+            if (j <= CL || j < C) { y = k.g * y + k.my * m; m = M[j]; a *= k.g; }
+          bb = y;
         }
-      }
-      __syncwarp();
-      // posterior of row r
-      const float* Fr = F + (size_t)r * 3 * stride;
-      float tot = 0.f;
-      for (int c = c0; c <= c1; ++c) tot += Fr[c] * curM[c] + Fr[stride + c] * curX[c] + Fr[2 * stride + c] * curY[c];
-      tot = warp_sum(tot);
-      if (tot > 0.f) {
-        const float inv = 1.f / tot;
-        for (int c = c0; c <= c1; ++c) {
-          const float pr = (Fr[c] * curM[c] + Fr[stride + c] * curX[c] + Fr[2 * stride + c] * curY[c]) * inv;
-          const int d = c - r + (R - 1);  // index into pstar, d in [1-R, H-1]
-          pstar[d] = fmaxf(pstar[d], pr);   // each (r, c) is owned by one lane: no race within a row
+        const float carry = affine_carry(a, bb, lane, true);
+        float mx = 0.f;
+        {
+          float y = carry, m = mleft;
+#pragma unroll
+          for (int j = 0; j < CM; ++j)
+            if (j <= CL || j < C) {
+              y = k.g * y + k.my * m;
+              Y[j] = j < nc ? y : 0.f;
+              m = M[j];
+              mx = fmaxf(mx, fmaxf(M[j], fmaxf(X[j], Y[j])));
+            }
         }
+        mx = warp_max(mx);
+        const float sc = mx > 0.f ? ldexpf(1.f, -ilogbf(mx)) : 1.f;
+        float* Fr = F + r * row_floats;
+#pragma unroll
+        for (int j = 0; j < CM; ++j)
+          if (j <= CL || j < C) {
+            M[j] *= sc;
+            X[j] *= sc;
+            Y[j] *= sc;
+            Fr[j * 32] = M[j];
+            Fr[(C + j) * 32] = X[j];
+            Fr[(2 * C + j) * 32] = Y[j];
+            tM = M[j]; tX = X[j]; tY = Y[j];
+          }
+        k = kn;
       }
-      float mx = 0.f;
-      for (int c = c0; c <= c1; ++c) mx = fmaxf(mx, fmaxf(curM[c], fmaxf(curX[c], curY[c])));
-      mx = warp_max(mx);
-      const float sc = mx > 0.f ? ldexpf(1.f, -ilogbf(mx)) : 1.f;
-      __syncwarp();
-      for (int c = lane; c <= H + 1; c += 32) {
-        prevM[c] = (c >= 1 && c <= H) ? curM[c] * sc : 0.f;
-        prevX[c] = (c >= 1 && c <= H) ? curX[c] * sc : 0.f;
-        prevY[c] = (c >= 1 && c <= H) ? curY[c] * sc : 0.f;
+      // ---- backward, rows R..1: M, X hold B of row r + 1, posterior per row
+      float P[CM];  // pstar of diagonal c - r
+#pragma unroll
+      for (int j = 0; j < CM; ++j) { M[j] = 0.f; X[j] = 0.f; P[j] = 0.f; }
+      int lo = INT32_MAX, hi = INT32_MIN;
+      RowC k1{};  // constants of row r+1
+      uint32_t mm1 = 0;
+      RowC k0 = row_consts(tb, quals, bases, R);
+      for (int r = R; r >= 1; --r) {
+        const RowC kn = row_consts(tb, quals, bases, max(r - 1, 1));
+        // the column right of the lane's last: B_M of row r + 1 and whether it matches
+        float rM = __shfl_down_sync(0xffffffffu, M[0], 1);
+        const bool rbit = __shfl_down_sync(0xffffffffu, mm1, 1) & 1u;
+        if (lane == 31) rM = 0.f;
+        // B_Y(c) = g(r) B_Y(c+1) + t(c), right to left, t(c) = gp(r+1) e(r+1,c+1) B_M(r+1,c+1)
+        float a = 1.f, bb = 0.f;
+        {
+          float y = 0.f, nx = rM;
+          bool bit = rbit;
+#pragma unroll
+          for (int j = CM - 1; j >= 0; --j)
+            if (j <= CL || j < C) {
+              const float t = __fmul_rn(__fmul_rn(k1.gp, bit ? k1.em : k1.ex), nx);
+              y = __fmaf_rn(k0.g, y, t);
+              if (j < nc) a *= k0.g;
+              nx = M[j];
+              bit = mm1 >> j & 1u;
+            }
+          bb = y;
+        }
+        const float carry = affine_carry(a, bb, lane, false);
+        float mx = 0.f, tot = 0.f;
+        {
+          float y = carry, nx = rM;  // y: B_Y(r, c+1)
+          bool bit = rbit;
+#pragma unroll
+          for (int j = CM - 1; j >= 0; --j)
+            if (j <= CL || j < C) {
+              const float byr = y, e = bit ? k1.em : k1.ex, nm = e * nx;
+              const float t = __fmul_rn(__fmul_rn(k1.gp, e), nx);
+              y = __fmaf_rn(k0.g, y, t);
+              Y[j] = y;
+              nx = M[j];
+              bit = mm1 >> j & 1u;
+              const float bm = k1.mm * nm + k1.mx * X[j] + k0.my * byr;
+              const float bx = k1.gp * nm + k1.g * X[j];
+              M[j] = r == R ? (j < nc ? 1.f : 0.f) : bm;
+              X[j] = r == R ? (j < nc ? 1.f : 0.f) : bx;
+              mx = fmaxf(mx, fmaxf(M[j], fmaxf(X[j], Y[j])));
+            }
+        }
+        // posterior of row r
+        const float* Fr = F + r * row_floats;
+#pragma unroll
+        for (int j = 0; j < CM; ++j)
+          if (j <= CL || j < C) {
+            // the sum's terms, kept for the row's normalised values
+            Y[j] = Fr[j * 32] * M[j] + Fr[(C + j) * 32] * X[j] + Fr[(2 * C + j) * 32] * Y[j];
+            tot += Y[j];
+          }
+        tot = warp_sum(tot);
+        if (tot > 0.f) {
+          const float inv = 1.f / tot;
+#pragma unroll
+          for (int j = 0; j < CM; ++j)
+            if (j <= CL || j < C) P[j] = fmaxf(P[j], Y[j] * inv);
+        }
+        mx = warp_max(mx);
+        const float sc = mx > 0.f ? ldexpf(1.f, -ilogbf(mx)) : 1.f;
+#pragma unroll
+        for (int j = 0; j < CM; ++j)
+          if (j <= CL || j < C) { M[j] *= sc; X[j] *= sc; }
+        if (r > 1) {  // one row up: diagonal 1 - r leaves column 1
+          if (lane == 0 && P[0] >= tau) { lo = min(lo, 1 - r); hi = max(hi, 1 - r); }
+          float in = __shfl_down_sync(0xffffffffu, P[0], 1);
+          if (lane == 31) in = 0.f;
+#pragma unroll
+          for (int j = 0; j < CM; ++j)
+            if (j <= CL || j < C) P[j] = j + 1 < CM && (j + 1 <= CL || j + 1 < C) ? P[j + 1 < CM ? j + 1 : j] : in;
+        }
+        k1 = k0;
+        mm1 = row_match(k0.rc);
+        k0 = kn;
       }
-      k1 = k0;
-      __syncwarp();
+      // spread: lowest and highest diagonal with pstar >= tau (row 1: diagonal c - 1)
+#pragma unroll
+      for (int j = 0; j < CM; ++j)
+        if (j < nc && P[j] >= tau) { lo = min(lo, lane * C + j); hi = max(hi, lane * C + j); }
+      lo = __reduce_min_sync(0xffffffffu, lo);
+      hi = __reduce_max_sync(0xffffffffu, hi);
+      if (lane == 0) { lo_out[pi] = lo == INT32_MAX ? INT32_MIN : lo; hi_out[pi] = hi; }
     }
-    // spread: lowest and highest diagonal with pstar >= tau
-    int lo = INT32_MAX, hi = INT32_MIN;
-    for (int x = lane; x < R + H - 1; x += 32)
-      if (pstar[x] >= tau) { lo = min(lo, x - (R - 1)); hi = max(hi, x - (R - 1)); }
-    for (int o = 16; o > 0; o >>= 1) {
-      lo = min(lo, __shfl_xor_sync(0xffffffffu, lo, o));
-      hi = max(hi, __shfl_xor_sync(0xffffffffu, hi, o));
-    }
-    if (lane == 0) { lo_out[pi] = lo == INT32_MAX ? INT32_MIN : lo; hi_out[pi] = hi; }
-    __syncwarp();
   }
+}
+
+template <int CL, int CM>
+cudaError_t launch_class(const DeviceBatch& b, const Tables* tb, const int32_t* pair_read, const int32_t* pair_hap,
+                         long long n_pairs, float tau, float* fbuf, const LabelRows& f, unsigned long long* next, bool first,
+                         int32_t* lo, int32_t* hi, cudaStream_t st) {
+  const int blocks = f.blocks;
+  const int grab = (int)std::max<long long>(1, std::min<long long>(32, n_pairs / ((long long)blocks * kLabelWarps * 64)));
+  k_posterior_spread<CL, CM><<<blocks, kLabelWarps * 32, 0, st>>>(b, tb, pair_read, pair_hap, n_pairs, tau, fbuf, f.stride,
+                                                                  f.max_area, next, grab, first, lo, hi);
+  return cudaGetLastError();
 }
 
 }  // namespace
 
-int label_smem_bytes() {
-  return kLabelWarps * ((6 * kLabelCols + kBandMaxSpan) * 4 + kLabelCols);
+// Rows of the longest read and haplotype the label kernel takes; a longer
+// read may stand against a shorter haplotype as long as its rows fit that
+// area (a row holds 32 C <= H + 31 columns, 29 more than the area counts).
+LabelRows label_rows(int max_read, int longest, int max_hap, int sms, size_t max_bytes) {
+  LabelRows f{};
+  f.max_area = (long long)(max_read + 1) * 3 * (max_hap + 2);
+  f.stride = (f.max_area + 3ll * 29 * (std::min(longest, kBandMaxSpan) + 1) + 31) / 32 * 32;
+  const size_t per_block = (size_t)f.stride * sizeof(float) * kLabelWarps;
+  f.blocks = (int)std::max<size_t>(1, std::min<size_t>((size_t)sms * 3, max_bytes / per_block));
+  f.bytes = per_block * (size_t)f.blocks;
+  return f;
 }
-
-int label_warps_per_block() { return kLabelWarps; }
 
 cudaError_t launch_posterior_spread(const DeviceBatch& b, const Tables* tb, const int32_t* pair_read,
                                     const int32_t* pair_hap, long long n_pairs, float tau, float* fbuf,
-                                    long long fbuf_stride, int32_t* lo, int32_t* hi, int blocks, cudaStream_t st) {
+                                    const LabelRows& f, int max_hap, unsigned long long* next, int32_t* lo, int32_t* hi,
+                                    cudaStream_t st) {
   if (n_pairs <= 0) return cudaSuccess;
-  const int smem = label_smem_bytes();
-  cudaError_t e = raise_dynamic_smem(reinterpret_cast<const void*>(&k_posterior_spread), smem);
-  if (e != cudaSuccess) return e;
-  k_posterior_spread<<<blocks, kLabelWarps * 32, smem, st>>>(b, tb, pair_read, pair_hap, n_pairs, tau, fbuf,
-                                                             fbuf_stride, lo, hi);
-  return cudaGetLastError();
+  const int c = (std::min(max_hap, kLabelMaxH) + 31) / 32;  // classes above the longest haplotype's are empty
+  cudaError_t e = cudaSuccess;
+  auto run = [&](auto cls) {
+    constexpr int k = decltype(cls)::value;
+    if (e == cudaSuccess && (k == 0 || c > 4 * k))
+      e = launch_class<4 * k, 4 * k + 4>(b, tb, pair_read, pair_hap, n_pairs, tau, fbuf, f, next + k, k == 0, lo, hi, st);
+  };
+  [&]<int... K>(std::integer_sequence<int, K...>) {
+    (run(std::integral_constant<int, K>{}), ...);
+  }(std::make_integer_sequence<int, kLabelClasses>{});
+  return e;
 }
 
 }  // namespace bvphmm

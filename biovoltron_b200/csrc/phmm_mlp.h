@@ -38,13 +38,19 @@ cudaError_t mlp_gather(const __nv_bfloat16* feat, const float* targets, const fl
                        const MlpTrainBuffers& b, cudaStream_t st);
 cudaError_t mlp_export(const float* w, MlpParams* out, cudaStream_t st);
 
-// Label kernel (one warp per pair; each warp keeps its forward rows in
-// fbuf + warp * fbuf_stride, so fbuf holds blocks * label_warps_per_block()
-// strides of floats).
-int label_smem_bytes();
-int label_warps_per_block();
+// Label kernel (one warp per pair): the forward rows of every resident warp,
+// `stride` floats each, `bytes` in all; pairs whose (R + 1) 3 (H + 2) exceeds
+// max_area get no label.  `next`: kLabelClasses work-queue heads, zero.
+struct LabelRows {
+  long long stride, max_area;
+  size_t bytes;
+  int blocks;
+};
+// max_read, max_hap: the longest within the band's limits; longest: the batch's longest read
+LabelRows label_rows(int max_read, int longest, int max_hap, int sms, size_t max_bytes);
 cudaError_t launch_posterior_spread(const DeviceBatch& b, const Tables* tb, const int32_t* pair_read,
                                     const int32_t* pair_hap, long long n_pairs, float tau, float* fbuf,
-                                    long long fbuf_stride, int32_t* lo, int32_t* hi, int blocks, cudaStream_t st);
+                                    const LabelRows& f, int max_hap, unsigned long long* next, int32_t* lo, int32_t* hi,
+                                    cudaStream_t st);
 
 }  // namespace bvphmm
