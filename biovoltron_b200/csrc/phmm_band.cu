@@ -712,7 +712,7 @@ __global__ void __launch_bounds__(kFeatUWarps * 32, kFeatUBlocksPerSm) k_featuri
 
 // ---------------------------------------------------------------------------
 // Routing.  Pass 0 counts band items per (width class, read-length bucket)
-// and writes full-DP fallback units; pass 1 places band items at their
+// and marks the pairs left to the full DP; pass 1 places band items at their
 // bucket's offset so that each warp of the banded kernel gets reads of nearly
 // equal length.
 // ---------------------------------------------------------------------------
@@ -768,8 +768,8 @@ __global__ void __launch_bounds__(256) k_band_route(BandParams p, int pass) {
       const int H = (int)(p.batch.hap_off[h + 1] - p.batch.hap_off[h]);
       band = route_band(p, pi, R, H, cls, d_lo);
       slot = band ? cls * kRBuckets + min(R / kRBucketRows, kRBuckets - 1) : kSlotFull + full_variant(R);
-      if (pass == 0 && p.banded) p.banded[pi] = 0;  // set by band_outcome when the band's result stands
-      if (pass == 0 || band) local = atomicAdd(&cnt[slot], 1u);
+      if (pass == 0) p.state[pi] = band ? kPairPending : kPairFull;  // band_outcome says what became of it
+      if (band || pass == 0) local = atomicAdd(&cnt[slot], 1u);
     }
     __syncthreads();
     for (int x = threadIdx.x; x < kRouteSlots; x += blockDim.x) {
@@ -780,7 +780,6 @@ __global__ void __launch_bounds__(256) k_band_route(BandParams p, int pass) {
         if (pass == 0) atomicAdd(&p.bctr->band_count[cl][bucket], (unsigned long long)c);
         else base[x] = atomicAdd(&p.bctr->band_fill[cl][bucket], (unsigned long long)c);
       } else if (pass == 0) {
-        base[x] = atomicAdd(&p.bctr->full_count[x - kSlotFull], (unsigned long long)c);
         atomicAdd(&p.bctr->fallback_route, (unsigned long long)c);
       }
     }
@@ -790,16 +789,6 @@ __global__ void __launch_bounds__(256) k_band_route(BandParams p, int pass) {
         BandItem it;
         it.read = r; it.hap = h; it.out = pi; it.d_lo = d_lo; it.pad_ = 0;
         p.items[(size_t)cls * p.item_cap + base[slot] + local] = it;
-      } else if (!band && pass == 0) {
-        const int v = slot - kSlotFull;
-        const unsigned long long q = base[slot] + local;
-        if (q < (unsigned long long)p.full_cap) {
-          Unit u{};
-          u.read = r; u.hap0 = h; u.nh = 1; u.out0 = pi;
-          p.full_items[(size_t)v * p.full_cap + q] = u;
-        } else {
-          atomicOr(&p.ctr->status, 4ull);
-        }
       }
       if (band && pass == 0 && p.audit_period > 0 && pi % p.audit_period == 0) {
         const unsigned long long a = atomicAdd(&p.bctr->audit_count, 1ull);
@@ -839,22 +828,14 @@ __device__ __forceinline__ void band_outcome(const BandParams& p, int cls, const
       atomicOr(&p.ctr->status, 4ull);
     }
   } else if (fall_back) {
-    const int v = full_variant(R);
-    const unsigned long long q = atomicAdd(&p.bctr->full_count[v], 1ull);
     atomicAdd(&p.bctr->fallback_edge, 1ull);
-    if (q < (unsigned long long)p.full_cap) {
-      Unit u{};
-      u.read = it.read; u.hap0 = it.hap; u.nh = 1; u.out0 = it.out;
-      p.full_items[(size_t)v * p.full_cap + q] = u;
-    } else {
-      atomicOr(&p.ctr->status, 4ull);
-    }
+    p.state[it.out] = kPairFull;
   } else if (rescue) {
     push_rescue(p.ctr, p.rescue, p.rescue_cap, p.long_rows, R, it.read, it.hap, it.out);
     p.out[it.out] = __longlong_as_double(0x7ff8000000000000ll);
   } else {
     p.out[it.out] = (double)(log10f(tot) - p.tables->log10_init_f);
-    if (p.banded) p.banded[it.out] = 1;
+    p.state[it.out] = kPairBanded;
   }
 }
 
@@ -1258,38 +1239,66 @@ __global__ void k_gap_check(const uchar4* __restrict__ quals, long long n, BandC
   if (tid == 0) c->gap_checked = 1u;
 }
 
-// Rescore: a read's pairs are consecutive result slots.  The thread at a
-// read's first slot takes the best result over the read's pairs (NaN: an FP64
-// rescue still to come, left out) and sends every banded pair more than
-// cap_margin log10 units below it to the full DP: such a pair is a read
-// scored against a haplotype it does not come from, and a stretch of the read
-// that does not belong to the haplotype is then partly explained by paths off
-// the band (a long insertion run, or a start far off the diagonal), which the
-// ring test does not see.  The full DP's result replaces the banded one.
-__global__ void k_band_cap(BandParams p) {
+// Units for the full DP from the pairs' states: a thread per read (its pairs
+// are consecutive result slots, its haplotypes consecutive).  First round
+// (RESCORE false): the pairs the band path left to the full DP (kPairFull).
+// Second round: a banded pair more than cap_margin log10 units below its
+// read's best result (NaN: an FP64 rescue still to come, left out) is scored
+// again: such a pair is a read scored against a haplotype it does not come
+// from, and a stretch of the read that does not belong to the haplotype is
+// then partly explained by paths off the band (a long insertion run, or a start
+// far off the diagonal), which the ring test does not see.  The full DP's
+// result replaces the banded one.
+// A unit holds two of a read's pairs (as a mask of 32 haplotypes), which the
+// paired kernels score at once: the two rounds of 286 k uneven pairs (147 k of
+// them on the full DP) take 3.1 ms, against 4.2 with one pair a unit and 3.4
+// with four (longer last units); 4.3 M genome pairs (53 k) 1.18 against 1.27.
+constexpr int kFullUnit = 2;
+
+template <bool RESCORE>
+__global__ void k_full_units(BandParams p) {
+  Unit* const units = RESCORE ? p.cap_items : p.full_items;
   for (long long pi = blockIdx.x * (long long)blockDim.x + threadIdx.x; pi < p.n_pairs;
        pi += (long long)gridDim.x * blockDim.x) {
     const int r = p.pair_read[pi];
     if (pi > 0 && p.pair_read[pi - 1] == r) continue;
     long long end = pi;
     double best = -INFINITY;
+    bool any = false;
     for (; end < p.n_pairs && p.pair_read[end] == r; ++end) {
-      const double v = p.out[end];
-      if (v > best) best = v;  // NaN compares false
-    }
-    const double cut = best - (double)p.cap_margin;
-    const int R = (int)(p.batch.read_off[r + 1] - p.batch.read_off[r]);
-    const int v = full_variant(R);
-    for (long long j = pi; j < end; ++j) {
-      if (!p.banded[j] || !(p.out[j] < cut)) continue;
-      const unsigned long long q = atomicAdd(&p.bctr->cap_count[v], 1ull);
-      atomicAdd(&p.bctr->cap_flagged, 1ull);
-      if (q < (unsigned long long)p.item_cap) {
-        Unit u{};
-        u.read = r; u.hap0 = p.pair_hap[j]; u.nh = 1; u.out0 = j;
-        p.cap_items[(size_t)v * p.item_cap + q] = u;
+      if (RESCORE) {
+        const double v = p.out[end];
+        if (v > best) best = v;  // NaN compares false
+        any = true;
       } else {
-        atomicOr(&p.ctr->status, 4ull);
+        any |= p.state[end] == kPairFull;
+      }
+    }
+    if (!any) continue;
+    const double cut = best - (double)p.cap_margin;
+    const int v = full_variant((int)(p.batch.read_off[r + 1] - p.batch.read_off[r]));
+    for (long long w = pi; w < end; w += 32) {
+      uint32_t mask = 0;
+      for (int k = 0; k < 32 && w + k < end; ++k) {
+        const bool in = RESCORE ? p.state[w + k] == kPairBanded && p.out[w + k] < cut : p.state[w + k] == kPairFull;
+        mask |= (uint32_t)in << k;
+      }
+      if (mask == 0) continue;
+      const int n = __popc(mask);
+      if (RESCORE) atomicAdd(&p.bctr->cap_flagged, (unsigned long long)n);
+      const int nu = (n + kFullUnit - 1) / kFullUnit;
+      unsigned long long q = atomicAdd(RESCORE ? &p.bctr->cap_count[v] : &p.bctr->full_count[v], (unsigned long long)nu);
+      for (; mask; ++q) {
+        Unit u{};
+        u.read = r;
+        u.hap0 = p.pair_hap[w];
+        u.out0 = w;
+        for (; mask && u.nh < kFullUnit; ++u.nh) {
+          u.mask |= mask & (0u - mask);
+          mask &= mask - 1u;
+        }
+        if (q < (unsigned long long)p.full_cap) units[(size_t)v * p.full_cap + q] = u;
+        else atomicOr(&p.ctr->status, 4ull);
       }
     }
   }
@@ -1328,10 +1337,11 @@ cudaError_t launch_gap_check(const uchar4* quals, long long n_bases, BandCounter
   return cudaGetLastError();
 }
 
-cudaError_t launch_band_cap(const BandParams& p, int sms, cudaStream_t st) {
+cudaError_t launch_full_units(const BandParams& p, bool rescore, int sms, cudaStream_t st) {
   if (p.n_pairs <= 0) return cudaSuccess;
   const long long blocks = std::min<long long>((p.n_pairs + 255) / 256, (long long)sms * 8);
-  k_band_cap<<<(int)blocks, 256, 0, st>>>(p);
+  if (rescore) k_full_units<true><<<(int)blocks, 256, 0, st>>>(p);
+  else k_full_units<false><<<(int)blocks, 256, 0, st>>>(p);
   return cudaGetLastError();
 }
 

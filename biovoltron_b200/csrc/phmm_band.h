@@ -73,7 +73,7 @@ struct BandCounters {
   unsigned long long band_next[kBandWidths];              // work-queue heads of the band launches
   unsigned long long band_total[kBandWidths];             // routed items per width class
   unsigned long long promoted[kBandWidths];               // items promoted from the next narrower class
-  unsigned long long full_count[16];                      // fallback items per full-DP variant
+  unsigned long long full_count[16];                      // fallback units per full-DP variant
   unsigned long long audit_count;
   unsigned long long audit_var[16];                       // audit units per full-DP variant
   unsigned long long fallback_edge;                       // pairs sent back by the edge check
@@ -84,12 +84,16 @@ struct BandCounters {
   unsigned long long feat_slow_next;                      // its work-queue head
   unsigned int gap_checked;                               // k_gap_check ran on this batch
   unsigned int gap_mixed;                                 // some base's gap qualities differ from the first base's
-  unsigned long long cap_count[16];                       // banded pairs rescored by the full DP, per variant
-  unsigned long long cap_flagged;                         // their total
+  unsigned long long cap_count[16];                       // rescore units per full-DP variant
+  unsigned long long cap_flagged;                         // banded pairs rescored by the full DP
   unsigned long long label_next[kLabelClasses];           // work-queue heads of the label kernel's launches
 };
 // work-queue slots of the rescore launches (the fallback launches use 0 .. 8, the audit 16 .. 24)
 constexpr int kCapSlot0 = 32;
+
+// What became of a pair: still in the band path (or sent to FP64 from there), scored by the banded kernel, left
+// to the full DP.
+constexpr uint8_t kPairPending = 0, kPairBanded = 1, kPairFull = 2;
 
 struct BandParams {
   DeviceBatch batch;
@@ -115,14 +119,14 @@ struct BandParams {
   int margin;                 // diagonals added on both sides of the predicted band
   float edge_threshold;       // promotion when the ring adds more than this share of the likelihood
   float cap_margin;           // > 0: banded pairs this many log10 units below their read's best are rescored
-  uint8_t* banded;            // [n_pairs] 1 where the result came from the banded kernel
-  Unit* cap_items;            // [9][item_cap] rescore units per full-DP variant
+  uint8_t* state;             // [n_pairs] kPair...
+  Unit* cap_items;            // [9][full_cap] rescore units per full-DP variant
   int audit_period;           // every audit_period-th pair is also scored by the full DP (0: off)
   BandCounters* bctr;
   Counters* ctr;
   BandItem* items;            // [kBandWidths][capacity]
   long long item_cap;
-  Unit* full_items;           // [16][capacity] fallback units (nh = 1), per full-DP variant
+  Unit* full_items;           // [9][full_cap] fallback units per full-DP variant
   long long full_cap;
   int64_t* audit_pairs;       // [audit capacity]
   long long audit_cap;
@@ -153,9 +157,9 @@ cudaError_t launch_mlp_forward(const BandParams& p, int sms, cudaStream_t st);
 cudaError_t launch_band_route(const BandParams& p, int pass, int sms, cudaStream_t st);
 cudaError_t launch_band_scan(BandCounters* c, cudaStream_t st);
 cudaError_t launch_band_dp(const BandParams& p, int width_class, int sms, cudaStream_t st);
-// After the fallback full DP: per read, the banded pairs whose result lies more than cap_margin
-// log10 units below the read's best result go to the rescore lists (cap_items, cap_count).
-cudaError_t launch_band_cap(const BandParams& p, int sms, cudaStream_t st);
+// Units of the pairs left to the full DP (full_items, full_count) or, after those have run, of the banded pairs
+// more than cap_margin log10 units below their read's best result (cap_items, cap_count).
+cudaError_t launch_full_units(const BandParams& p, bool rescore, int sms, cudaStream_t st);
 // banded kernels: 128-thread blocks, as many as fit at once (3 per SM for W = 8, 2 for the wider classes)
 inline int band_dp_blocks(int sms, int width_class) { return sms * (width_class == 0 ? 3 : 2); }
 // warp featuriser (the slow path) grid and its per-warp scratch histograms (words)

@@ -59,12 +59,13 @@ struct Tables {
 };
 
 // One unit of full-DP work: a read scored against `nh` consecutive haplotypes
-// whose results are consecutive in the output.
+// whose results are consecutive in the output; with a mask, against haplotypes
+// hap0 + k (result out0 + k) for its nh set bits k.
 struct Unit {
   int32_t read;
   int32_t hap0;
   int32_t nh;
-  int32_t pad_;
+  uint32_t mask;
   int64_t out0;
 };
 

@@ -640,6 +640,7 @@ template <> __device__ __forceinline__ double log10_(double v) { return log10(v)
 struct Item {
   int read, hap0, nh;
   long long out0;
+  uint32_t mask = 0;  // the haplotypes' places from hap0 (0: the nh consecutive ones)
 };
 
 // Writes one pair's log10 likelihood (lane 31 holds the result).  FP32:
@@ -725,14 +726,23 @@ __device__ void process_item(const KernelParams& p, const Item& it, unsigned cha
     // single strip: rows and emission table are shared by all haplotypes
     fold = setup_rows<T, RT>(p.tables, quals, bases, R, lane * RT - pad, T(0), rw, etab, lane);
   }
-  for (int k = 0; k < it.nh; ++k) {
+  uint32_t left = it.mask;
+  auto place = [&](int n) {  // of the item's n-th haplotype
+    if (it.mask == 0) return n;
+    const int at = __ffs(left) - 1;
+    left &= left - 1u;
+    return at;
+  };
+  for (int n = 0; n < it.nh; ++n) {
+    const int k = place(n);
     const int h = it.hap0 + k;
     const int64_t ho = b.hap_off[h];
     const int H = (int)(b.hap_off[h + 1] - ho);
     if constexpr (PAIR && !MULTI && sizeof(T) == 4) {
-      if (k + 1 < it.nh && R > 0) {
-        const int64_t ho2 = b.hap_off[h + 1];
-        const int H2 = (int)(b.hap_off[h + 2] - ho2);
+      if (n + 1 < it.nh && R > 0) {
+        const int k2 = it.mask ? __ffs(left) - 1 : n + 1, h2 = it.hap0 + k2;
+        const int64_t ho2 = b.hap_off[h2];
+        const int H2 = (int)(b.hap_off[h2 + 1] - ho2);
         if (H > 0 && H2 > 0) {
           const int Hm = H > H2 ? H : H2;
           const int nsteps = (Hm + kWarp + 7) / 8 * 8;  // as the single path: H + 31 + 1 (summing row), to 8
@@ -753,9 +763,9 @@ __device__ void process_item(const KernelParams& p, const Item& it, unsigned cha
           else run_strip_pair<RT, false>(rw, y0a, y0b, el, hcp + kHapLead - lane, nsteps, lastM, lastY);
           if (lane == kWarp - 1) {
             write_result<float>(p, it.read, h, it.out0 + k, lastY.x + lastM.x, 0);
-            write_result<float>(p, it.read, h + 1, it.out0 + k + 1, lastY.y + lastM.y, 0);
+            write_result<float>(p, it.read, h2, it.out0 + k2, lastY.y + lastM.y, 0);
           }
-          ++k;
+          place(++n);  // the second haplotype is done too
           continue;
         }
       }

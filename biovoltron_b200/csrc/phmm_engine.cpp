@@ -51,9 +51,6 @@ constexpr int kMaxRowsPerLane = 8;
 constexpr int kF64Bin0 = 19;
 constexpr int kF64List = 28;
 constexpr int kMaxVariants = 28;
-// Launches in flight beside each other.  Two, four and eight lanes took 1.77, 1.74 and 1.72 ms for the
-// call on 48 uneven regions; every lane is a stream that a new context has to make (0.3 ms for four).
-constexpr int kMaxLanes = 4;
 constexpr int kRescaleTarget = 1000;  // FP64 boundary rows are scaled to ~2^1000
 
 int64_t round_up(int64_t x, int64_t m) { return (x + m - 1) / m * m; }
@@ -279,6 +276,7 @@ bv_status Engine::plan(const bv_region_batch& b) {
   const int v_multi = variant_index(false, 8, true);
   std::vector<int64_t> count(kMaxVariants, 0);
   std::vector<int> var_max_hap(kMaxVariants, 0);
+  std::fill(bin_reads_, bin_reads_ + 9, 0);
   int64_t n_long = 0, long_rows_sum = 0;  // pairs the long-read kernel may get, and their reads' bases
   // pass 1: count units per variant
   std::vector<int> region_max_hap(std::max<int64_t>(b.num_regions, 1), 0);
@@ -331,6 +329,7 @@ bv_status Engine::plan(const bv_region_batch& b) {
     const int64_t chunks = (nh + per_unit - 1) / per_unit;
     for (int64_t r = b.region_reads[g]; r < b.region_reads[g + 1]; ++r) {
       const int64_t rl = b.read_offsets[r + 1] - b.read_offsets[r];
+      ++bin_reads_[std::min<int64_t>((rows_needed((int)std::min<int64_t>(rl, 1 << 24), true, true) + kWarp - 1) / kWarp, 9) - 1];
       if (rl >= long_rows()) {
         n_long += nh;
         long_rows_sum += nh * rl;
@@ -762,11 +761,12 @@ bv_status Engine::finish(bv_phmm_stats* stats) {
     stats->fp32_skipped_cells = (int64_t)c.fp32_skipped_cells;
     stats->underflow = (int64_t)c.underflow_count;
     // band mode: k-mer tables, nibble image, read k-mers, gap check, two featurisers, MLP, route,
-    // scan, route; the banded kernels; the fallback variants; the rescore check and variants;
-    // the audit; the FP64 pass
+    // scan, route; the banded kernels; the fallback's units and bins; the rescore's;
+    // the audit's; the FP64 pass
     stats->kernel_launches = band_enabled()
-                                 ? 9 + (band_opt_.use_mlp ? 1 : 0) + kBandWidths + 9 + (band_opt_.cap_margin > 0 ? 10 : 0) +
-                                       (band_opt_.audit_period > 0 ? 11 : 0) + 1
+                                 ? 9 + (band_opt_.use_mlp ? 1 : 0) + kBandWidths + 1 + full_bins_ +
+                                       (band_opt_.cap_margin > 0 ? 1 + full_bins_ : 0) +
+                                       (band_opt_.audit_period > 0 ? 2 + full_bins_ : 0) + 1 + (long_plan_.grid > 0)
                                  : (int64_t)plans_.size() + 1 + (long_plan_.grid > 0);
     stats->ms_fp32 = ms32;
     stats->ms_fp64 = ms64;

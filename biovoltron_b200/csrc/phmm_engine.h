@@ -41,6 +41,10 @@ struct BinTune {
 };
 constexpr int kTuneBins = 8;  // rows per lane 1..8
 
+// Launches in flight beside each other.  Two, four and eight lanes took 1.77, 1.74 and 1.72 ms for the
+// call on 48 uneven regions; every lane is a stream that a new context has to make (0.3 ms for four).
+constexpr int kMaxLanes = 4;
+
 struct LaunchPlan {
   int variant = -1;
   int rows = 0;  // rows per lane of a single-strip variant (0: multi-strip)
@@ -208,6 +212,8 @@ class Engine {
   bv_status enqueue_plans(bool capturing, bool f64, KernelParams& p);
   bv_status band_prepare();
   bv_status enqueue_band(bool capturing, KernelParams& p);
+  bv_status enqueue_full(KernelParams& kp, const Unit* units, long long cap, const unsigned long long* counts, int slot0,
+                         const char* what);
   bv_status band_stats(bv_phmm_stats* stats);
   void destroy_graph();
   // Side streams: independent launches (the bins of a full-DP pass) run beside
@@ -272,10 +278,12 @@ class Engine {
   bv_band_options band_opt_{};
   bool mlp_ready_ = false;
   DevBuf d_pair_read_, d_pair_hap_, d_hap_table_, d_dstar_, d_feat_, d_mlp_out_, d_mlp_, d_bctr_;
-  DevBuf d_kmin_, d_kmax_, d_read_kmers_, d_feat_hist_, d_feat_slow_, d_hap_nib_, d_banded_, d_cap_items_;
+  DevBuf d_kmin_, d_kmax_, d_read_kmers_, d_feat_hist_, d_feat_slow_, d_hap_nib_, d_pair_state_, d_cap_items_;
   DevBuf d_band_items_, d_full_items_, d_audit_pairs_, d_audit_units_, d_audit_out_, d_audit_err_;
   long long item_cap_ = 0, full_cap_ = 0, audit_cap_ = 0;
   LaunchPlan full_plans_[9];
+  int64_t bin_reads_[9] = {};  // reads of the batch per full-DP bin (rows per lane 1 .. 8, several strips)
+  int full_bins_ = 0;          // bins that have reads
   BandParams band_params() const;
   // training
   bv_status stage_for_labels(const bv_region_batch& b);

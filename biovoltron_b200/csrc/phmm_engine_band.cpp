@@ -64,7 +64,7 @@ BandParams Engine::band_params() const {
   p.edge_threshold = (float)band_opt_.edge_threshold;
   p.audit_period = band_opt_.audit_period;
   p.cap_margin = band_opt_.cap_margin;
-  p.banded = d_banded_.as<uint8_t>();
+  p.state = d_pair_state_.as<uint8_t>();
   p.cap_items = d_cap_items_.as<Unit>();
   p.bctr = d_bctr_.as<BandCounters>();
   p.ctr = d_counters_.as<Counters>();
@@ -106,7 +106,7 @@ bv_status Engine::band_prepare() {
   audit_cap_ = band_opt_.audit_period > 0 ? n / band_opt_.audit_period + 1 : 1;
   BV_CUDA(d_band_items_.reserve(sizeof(BandItem) * kBandWidths * item_cap_), "alloc band items");
   BV_CUDA(d_full_items_.reserve(sizeof(Unit) * 9 * full_cap_), "alloc fallback units");
-  BV_CUDA(d_banded_.reserve((size_t)n), "alloc band flags");
+  BV_CUDA(d_pair_state_.reserve((size_t)n), "alloc band states");
   BV_CUDA(d_cap_items_.reserve(sizeof(Unit) * 9 * (band_opt_.cap_margin > 0 ? full_cap_ : 1)), "alloc rescore units");
   BV_CUDA(d_audit_pairs_.reserve(sizeof(int64_t) * audit_cap_), "alloc audit");
   BV_CUDA(d_audit_units_.reserve(sizeof(Unit) * 9 * audit_cap_), "alloc audit");
@@ -115,24 +115,66 @@ bv_status Engine::band_prepare() {
   // Fallback launches: one persistent launch per full-DP variant, sized for the
   // batch's longest haplotype; the unit counts are known only on the device.
   size_t need32 = d_bnd32_.capacity();
+  full_bins_ = 0;
   for (int v = 0; v < 9; ++v) {
     LaunchPlan lp;
-    lp.variant = v;
-    lp.slot = v;
     lp.multi = (v == 8);
-    lp.hap_bytes = (int)round_up((int64_t)std::max(max_hap_, 1) + (kWarp - 1) + (lp.multi ? 32 : 8) + kHapLead + 16, 16);
-    lp.warp_smem = warp_smem_bytes(v, lp.hap_bytes);
-    const int smem_block = lp.warp_smem * (kThreadsPerBlock / kWarp);
+    lp.variant = lp.multi ? v : variant_index(false, v + 1, false, true);
+    lp.slot = v;
+    lp.code_row_bytes =
+        (int)round_up((int64_t)std::max(max_hap_, 1) + (kWarp - 1) + (lp.multi ? 32 : 8) + kHapLead + 16, 16);
+    lp.hap_bytes = variant_paired(lp.variant) ? 4 * lp.code_row_bytes : lp.code_row_bytes;
+    lp.warp_smem = warp_smem_bytes(lp.variant, lp.hap_bytes);
+    int smem_block = lp.warp_smem * (kThreadsPerBlock / kWarp);
+    if (!lp.multi && smem_block > 227 * 1024) {  // haplotypes too long for a paired row: one at a time
+      lp.variant = v;
+      lp.hap_bytes = lp.code_row_bytes;
+      lp.warp_smem = warp_smem_bytes(lp.variant, lp.hap_bytes);
+      smem_block = lp.warp_smem * (kThreadsPerBlock / kWarp);
+    }
     if (smem_block > 227 * 1024) return fail(BV_ERR_INVALID_ARG, "haplotype too long for shared-memory staging");
-    BV_CUDA(prepare_variant(v, smem_block), "kernel attribute");
-    lp.grid = sms_ * std::max(1, blocks_per_sm(v, smem_block));
+    BV_CUDA(prepare_variant(lp.variant, smem_block), "kernel attribute");
+    lp.grid = sms_ * std::max(1, blocks_per_sm(lp.variant, smem_block));
     lp.bnd_cols = lp.multi ? round_up((int64_t)std::max(max_hap_, 1) + kWarp, 32) + 160 : 0;
     if (lp.multi) need32 = std::max<size_t>(need32, (size_t)lp.grid * (kThreadsPerBlock / kWarp) * lp.bnd_cols * 4 * sizeof(float));
     full_plans_[v] = lp;
+    full_bins_ += bin_reads_[v] > 0;
   }
+  if (bv_status ls = reserve_lanes(std::min(full_bins_, kMaxLanes)); ls != BV_OK) return ls;
   if (need32 > d_bnd32_.capacity()) BV_CUDA(d_bnd32_.reserve(need32), "alloc boundary buffers");
   BV_CUDA(launch_pairs_from_units(d_units_.as<Unit>(), (long long)units_.size(), d_pair_read_.as<int32_t>(),
                                   d_pair_hap_.as<int32_t>(), sms_, stream_), "pairs");
+  return BV_OK;
+}
+
+// The full DP over device-built unit lists ([9][cap] by read-length bin, the
+// counts on the device): a launch per bin that has reads in the batch, the
+// bins side by side, longest reads first.
+bv_status Engine::enqueue_full(KernelParams& kp, const Unit* units, long long cap, const unsigned long long* counts,
+                               int slot0, const char* what) {
+  const int lanes = std::min(full_bins_, kMaxLanes);
+  if (bv_status fs = fork(lanes); fs != BV_OK) return fs;
+  cudaError_t le = cudaSuccess;  // a failed launch still joins the lanes that started
+  int n = 0;
+  for (int v = 8; v >= 0 && le == cudaSuccess; --v) {
+    if (bin_reads_[v] == 0) continue;
+    const LaunchPlan& lp = full_plans_[v];
+    kp.units = units + (size_t)v * cap;
+    kp.unit_base = 0;
+    kp.n_units = 0;
+    kp.n_units_dev = counts + v;
+    kp.slot = slot0 + v;
+    kp.hap_bytes = lp.hap_bytes;
+    kp.code_row_bytes = lp.code_row_bytes;
+    kp.warp_smem_bytes = lp.warp_smem;
+    kp.bnd = lp.multi ? d_bnd32_.get() : nullptr;
+    kp.bnd_cols = lp.bnd_cols;
+    kp.rescale = 0;
+    kp.rescale_target = 0;
+    le = launch_forward(lp.variant, kp, lp.grid, lane(n++ % lanes));
+  }
+  if (bv_status js = join(lanes); js != BV_OK) return js;
+  BV_CUDA(le, what);
   return BV_OK;
 }
 
@@ -156,57 +198,23 @@ bv_status Engine::enqueue_band(bool capturing, KernelParams& kp) {
   for (int cls = 0; cls < kBandWidths; ++cls) BV_CUDA(launch_band_dp(p, cls, sms_, stream_), "band dp");
   BV_CUDA(rec(ev_[6]), "event");
   // full DP for everything the band path handed back
-  for (int v = 0; v < 9; ++v) {
-    const LaunchPlan& lp = full_plans_[v];
-    kp.units = d_full_items_.as<Unit>() + (size_t)v * full_cap_;
-    kp.unit_base = 0;
-    kp.n_units = 0;
-    kp.n_units_dev = &d_bctr_.as<BandCounters>()->full_count[v];
-    kp.slot = lp.slot;
-    kp.hap_bytes = lp.hap_bytes;
-    kp.warp_smem_bytes = lp.warp_smem;
-    kp.bnd = lp.multi ? d_bnd32_.get() : nullptr;
-    kp.bnd_cols = lp.bnd_cols;
-    kp.rescale = 0;
-    kp.rescale_target = 0;
-    BV_CUDA(launch_forward(v, kp, lp.grid, stream_), "fallback full DP");
-  }
+  BandCounters* bc = d_bctr_.as<BandCounters>();
+  BV_CUDA(launch_full_units(p, false, sms_, stream_), "full-DP units");
+  bv_status s = enqueue_full(kp, d_full_items_.as<Unit>(), full_cap_, bc->full_count, 0, "fallback full DP");
+  if (s != BV_OK) return s;
   if (band_opt_.cap_margin > 0) {
     // banded pairs far below their read's best result, scored again by the full DP
-    BV_CUDA(launch_band_cap(p, sms_, stream_), "band cap");
-    for (int v = 0; v < 9; ++v) {
-      const LaunchPlan& lp = full_plans_[v];
-      kp.units = d_cap_items_.as<Unit>() + (size_t)v * full_cap_;
-      kp.unit_base = 0;
-      kp.n_units = 0;
-      kp.n_units_dev = &d_bctr_.as<BandCounters>()->cap_count[v];
-      kp.slot = kCapSlot0 + v;
-        kp.hap_bytes = lp.hap_bytes;
-      kp.warp_smem_bytes = lp.warp_smem;
-      kp.bnd = lp.multi ? d_bnd32_.get() : nullptr;
-      kp.bnd_cols = lp.bnd_cols;
-      kp.rescale = 0;
-      kp.rescale_target = 0;
-      BV_CUDA(launch_forward(v, kp, lp.grid, stream_), "rescore full DP");
-    }
+    BV_CUDA(launch_full_units(p, true, sms_, stream_), "rescore units");
+    s = enqueue_full(kp, d_cap_items_.as<Unit>(), full_cap_, bc->cap_count, kCapSlot0, "rescore full DP");
+    if (s != BV_OK) return s;
   }
   if (band_opt_.audit_period > 0) {
     BV_CUDA(launch_audit_units(p, d_audit_units_.as<Unit>(), stream_), "audit units");
-    // the audit pairs' full DP, on the variant each read length takes
-    for (int v = 0; v < 9; ++v) {
-      KernelParams ak = kp;
-      const LaunchPlan& lp = full_plans_[v];
-      ak.units = d_audit_units_.as<Unit>() + (size_t)v * audit_cap_;
-      ak.n_units_dev = &d_bctr_.as<BandCounters>()->audit_var[v];
-      ak.slot = 16 + v;
-      ak.hap_bytes = lp.hap_bytes;
-      ak.warp_smem_bytes = lp.warp_smem;
-      ak.bnd = lp.multi ? d_bnd32_.get() : nullptr;
-      ak.bnd_cols = lp.bnd_cols;
-      ak.out = d_audit_out_.as<double>();
-      ak.rescue = nullptr;  // audit pairs that need FP64 are left out of the comparison
-      BV_CUDA(launch_forward(v, ak, lp.grid, stream_), "audit full DP");
-    }
+    KernelParams ak = kp;
+    ak.out = d_audit_out_.as<double>();
+    ak.rescue = nullptr;  // audit pairs that need FP64 are left out of the comparison
+    s = enqueue_full(ak, d_audit_units_.as<Unit>(), audit_cap_, bc->audit_var, 16, "audit full DP");
+    if (s != BV_OK) return s;
   }
   kp.n_units_dev = nullptr;
   return BV_OK;
@@ -276,7 +284,8 @@ bv_status Engine::band_routes(int64_t n, int32_t* d_lo, int32_t* width, int32_t*
     if (cnt) BV_CUDA(cudaMemcpy(u.data(), d_full_items_.as<Unit>() + (size_t)v * full_cap_, sizeof(Unit) * cnt,
                                 cudaMemcpyDeviceToHost), "fallback units");
     for (const auto& x : u)
-      if (x.out0 >= 0 && x.out0 < n && route[x.out0] == 0) route[x.out0] = 2;
+      for (int k = 0; k < 32; ++k)
+        if ((x.mask >> k & 1u) && x.out0 + k < n && route[x.out0 + k] == 0) route[x.out0 + k] = 2;
   }
   const unsigned long long nr = std::min<unsigned long long>(cc.rescue_count, (unsigned long long)std::max<int64_t>(n_results_, 1));
   std::vector<PairRef> rl(nr);
@@ -293,7 +302,8 @@ bv_status Engine::band_routes(int64_t n, int32_t* d_lo, int32_t* width, int32_t*
       if (cnt) BV_CUDA(cudaMemcpy(u.data(), d_cap_items_.as<Unit>() + (size_t)v * full_cap_, sizeof(Unit) * cnt,
                                   cudaMemcpyDeviceToHost), "rescore units");
       for (const auto& x : u)
-        if (x.out0 >= 0 && x.out0 < n && route[x.out0] == 0) route[x.out0] = 4;
+        for (int k = 0; k < 32; ++k)
+          if ((x.mask >> k & 1u) && x.out0 + k < n && route[x.out0 + k] == 0) route[x.out0 + k] = 4;
     }
   }
   for (const auto& x : rl)

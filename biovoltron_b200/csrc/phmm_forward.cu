@@ -95,7 +95,7 @@ __global__ void __launch_bounds__(kThreadsPerBlock) k_forward(KernelParams p) {
     w = __shfl_sync(0xffffffffu, w, 0);
     if (w >= n) break;
     const Unit u = p.units[p.unit_base + w];
-    process_item<T, RT, MULTI, PAIR>(p, Item{u.read, u.hap0, u.nh, u.out0}, wsm, lane, bnd);
+    process_item<T, RT, MULTI, PAIR>(p, Item{u.read, u.hap0, u.nh, u.out0, u.mask}, wsm, lane, bnd);
   }
 }
 
