@@ -31,7 +31,7 @@ size_t align256(size_t x) { return (x + 255) / 256 * 256; }
 struct TrainArena {
   size_t bytes = 0;
   MlpTrainBuffers b{};
-  void layout(char* base, int cap, int loss_slots) {
+  void layout(char* base, int cap, int loss_slots, bool eval) {
     size_t off = 0;
     auto take = [&](size_t n) {
       float* p = base ? reinterpret_cast<float*>(base + off) : nullptr;
@@ -39,23 +39,19 @@ struct TrainArena {
       return p;
     };
     b.w = take(kMlpParamCount);
-    b.wq = take(kMlpParamCount);
     b.g = take(kMlpParamCount);
     b.m = take(kMlpParamCount);
     b.v = take(kMlpParamCount);
-    b.X = take((size_t)cap * kFeat);
-    b.T = take((size_t)cap * 2);
-    b.mask = take((size_t)cap);
-    b.Z1 = take((size_t)cap * kHid);
-    b.H1 = take((size_t)cap * kHid);
-    b.Z2 = take((size_t)cap * kHid);
+    b.X = take((size_t)(eval ? cap : 0) * kFeat);
+    b.T = take((size_t)(eval ? cap : 0) * 2);
     b.H2 = take((size_t)cap * kHid);
     b.O = take((size_t)cap * kOut);
     b.dO = take((size_t)cap * kOut);
     b.dH = take((size_t)cap * kHid);
     b.dH2 = take((size_t)cap * kHid);
     b.loss = take((size_t)std::max(loss_slots, 1));
-    b.part = take((size_t)((cap + 127) / 128) * kHid * kHid);
+    b.part1 = take((size_t)((cap + 127) / 128) * kHid * kFeat);
+    b.part2 = take((size_t)((cap + 127) / 128) * kHid * kHid);
     b.tc_fail = reinterpret_cast<unsigned int*>(take(1));
     b.cap = cap;
     bytes = off;
@@ -208,12 +204,11 @@ bv_status Engine::band_mlp_eval(const float* w, const float* x, const float* t, 
   BV_CUDA(cudaSetDevice(opt_.device), "cudaSetDevice");
   if (n > (1 << 24)) return fail(BV_ERR_INVALID_ARG, "too many rows");
   TrainArena a;
-  a.layout(nullptr, (int)n, 1);
+  a.layout(nullptr, (int)n, 1, true);
   DevBuf mem;
   BV_CUDA(mem.reserve(a.bytes), "alloc eval");
-  a.layout(mem.as<char>(), (int)n, 1);
+  a.layout(mem.as<char>(), (int)n, 1, true);
   MlpTrainBuffers b = a.b;
-  b.mask = nullptr;
   BV_CUDA(cudaMemcpyAsync(b.w, w, sizeof(float) * kMlpParamCount, cudaMemcpyHostToDevice, stream_), "H2D");
   BV_CUDA(cudaMemcpyAsync(b.X, x, sizeof(float) * kFeat * n, cudaMemcpyHostToDevice, stream_), "H2D");
   BV_CUDA(cudaMemcpyAsync(b.T, t, sizeof(float) * 2 * n, cudaMemcpyHostToDevice, stream_), "H2D");
@@ -327,10 +322,10 @@ bv_status Engine::band_train(const bv_region_batch& bt, const bv_band_train_opti
   const int steps_per_epoch = (int)((nl + batch - 1) / batch);
   const int total_steps = steps_per_epoch * o.epochs;
   TrainArena a;
-  a.layout(nullptr, batch, total_steps);
+  a.layout(nullptr, batch, total_steps, false);
   DevBuf mem, d_targets, d_perm;
   BV_CUDA(mem.reserve(a.bytes), "alloc training");
-  a.layout(mem.as<char>(), batch, total_steps);
+  a.layout(mem.as<char>(), batch, total_steps, false);
   MlpTrainBuffers b = a.b;
   BV_CUDA(d_targets.reserve(targets.size() * sizeof(float)), "alloc targets");
   BV_CUDA(d_perm.reserve(sizeof(int32_t) * nl), "alloc permutation");
@@ -341,6 +336,7 @@ bv_status Engine::band_train(const bv_region_batch& bt, const bv_band_train_opti
   BV_CUDA(cudaMemsetAsync(b.v, 0, sizeof(float) * kMlpParamCount, stream_), "memset");
   BV_CUDA(cudaMemsetAsync(b.tc_fail, 0, sizeof(unsigned int), stream_), "memset");
   float* loss_hist = b.loss;
+  BV_CUDA(cudaMemsetAsync(loss_hist, 0, sizeof(float) * total_steps, stream_), "memset");
   BV_CUDA(cudaEventRecord(ev_[0], stream_), "event");
   int step = 0;
   const int warm = std::min(50, total_steps / 10 + 1);
@@ -351,13 +347,11 @@ bv_status Engine::band_train(const bv_region_batch& bt, const bv_band_train_opti
     for (int k = 0; k < steps_per_epoch; ++k, ++step) {
       const int nb = (int)std::min<int64_t>(batch, nl - (int64_t)k * batch);
       b.loss = loss_hist + step;
-      BV_CUDA(mlp_gather(d_feat_.as<__nv_bfloat16>(), d_targets.as<float>(), nullptr, d_perm.as<int32_t>() + (size_t)k * batch,
-                         nb, b, stream_), "gather");
-      BV_CUDA(mlp_forward_backward(b, nb, o.alpha, true, stream_), "forward/backward");
       const float prog = (float)step / (float)std::max(total_steps - 1, 1);
       const float lr = step < warm ? o.lr * (float)(step + 1) / (float)warm
                                    : o.lr * (0.02f + 0.98f * 0.5f * (1.f + std::cos(3.14159265f * prog)));
-      BV_CUDA(mlp_adam(b, step + 1, lr, stream_), "adam");
+      BV_CUDA(mlp_train_step(b, d_feat_.as<__nv_bfloat16>(), d_targets.as<float>(), d_perm.as<int32_t>() + (size_t)k * batch,
+                             nb, o.alpha, step + 1, lr, stream_), "train step");
     }
     BV_CUDA(cudaStreamSynchronize(stream_), "epoch sync");
   }

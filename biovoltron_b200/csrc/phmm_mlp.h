@@ -17,25 +17,28 @@ constexpr int kMlpParamCount = kHid * kFeat + kHid + kHid * kHid + kHid + kOut *
 
 struct MlpTrainBuffers {
   float* w;      // master weights
-  float* wq;     // BF16-rounded copy used by forward and backward
-  float* g;      // gradient
+  float* g;      // gradient (evaluation)
   float* m;      // Adam moments
   float* v;
-  float* X;      // [cap][kFeat] minibatch inputs
-  float* T;      // [cap][2] targets
-  float* mask;   // [cap]
-  float* Z1; float* H1; float* Z2; float* H2; float* O;
-  float* dO; float* dH; float* dH2;
+  float* X;      // [cap][kFeat] inputs and [cap][2] targets (evaluation; training gathers its rows)
+  float* T;
+  float* H2;     // [cap][kHid] second hidden layer's activations
+  float* O;      // [cap][2] outputs and their gradient
+  float* dO;
+  float* dH;     // [cap][kHid] gradients of the hidden layers' sums, second and first
+  float* dH2;
   float* loss;   // scalar
-  float* part;             // split-K partial products of the weight gradients, ceil(cap / 128) x 128 x 128
-  unsigned int* tc_fail;   // set when a tensor-core GEMM's completion wait gave up
+  float* part1;            // [ceil(cap / 128)][kHid][kFeat] partial products of W1's gradient
+  float* part2;            // [ceil(cap / 128)][kHid][kHid] and of W2's
+  unsigned int* tc_fail;   // set when a tensor-core product's completion wait gave up
   int cap;
 };
 
+// One evaluation of the objective on the n rows of X, T: outputs, loss and, with `backward`, the gradient.
 cudaError_t mlp_forward_backward(const MlpTrainBuffers& b, int n, float alpha, bool backward, cudaStream_t st);
-cudaError_t mlp_adam(const MlpTrainBuffers& b, int step, float lr, cudaStream_t st);
-cudaError_t mlp_gather(const __nv_bfloat16* feat, const float* targets, const float* mask, const int32_t* idx, int n,
-                       const MlpTrainBuffers& b, cudaStream_t st);
+// One Adam step (number `step`, from 1) on the n rows idx of feat / targets; adds the loss to *b.loss.
+cudaError_t mlp_train_step(const MlpTrainBuffers& b, const __nv_bfloat16* feat, const float* targets, const int32_t* idx,
+                           int n, float alpha, int step, float lr, cudaStream_t st);
 cudaError_t mlp_export(const float* w, MlpParams* out, cudaStream_t st);
 
 // Label kernel (one warp per pair): the forward rows of every resident warp,

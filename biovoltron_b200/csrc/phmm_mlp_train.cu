@@ -3,132 +3,425 @@
 // Master weights are FP32; every step rounds them to BF16 (the precision the
 // tensor-core inference kernel uses) and runs forward and backward in FP32 on
 // those rounded values, so the gradient is that of the deployed network
-// (straight-through rounding).  The GEMMs with 80 or 128 rows on every side
-// run on the tensor cores (tcgen05.mma kind::f16: BF16 operands, FP32
-// accumulation in tensor memory) -- the two hidden layers' forward products
-// (inputs, weights and hidden activations are BF16 values already), the
-// hidden layers' weight gradients and the back-propagated hidden gradient
-// (the FP32 gradient operands rounded to BF16, as mixed-precision training
-// does); the products with the 2-wide output layer stay FP32 SIMT.  The loss
-// is an asymmetric squared error on
+// (straight-through rounding).  The products with 80 or 128 on every side run
+// on the tensor cores (tcgen05.mma kind::f16: BF16 operands, FP32 accumulation
+// in tensor memory) -- the two hidden layers' forward products (inputs, weights
+// and hidden activations are BF16 values already), the hidden layers' weight
+// gradients and the back-propagated hidden gradient (the FP32 gradient operands
+// rounded to BF16, as mixed-precision training does); the products with the
+// 2-wide output layer stay FP32.  The loss is an asymmetric squared error on
 // the band's lower and upper edge (diagonals relative to the seed diagonal):
 //   L = mean( w_lo (o_lo - t_lo)^2 + w_hi (o_hi - t_hi)^2 ),
 //   w_lo = alpha if o_lo > t_lo (band too narrow below) else 1,
 //   w_hi = alpha if o_hi < t_hi (band too narrow above) else 1,
 // so under-covering the posterior spread costs alpha times more than
 // over-covering it.  Optimiser: Adam.
+//
+// Two launches a step.  k_mlp_rows: a block per 128 rows of the minibatch runs
+// the whole forward and backward pass of its rows with every operand in shared
+// memory, and leaves the rows' hidden gradients and its partial products of the
+// hidden weight gradients (K = its 128 rows).  k_mlp_update: sums the partial
+// products block by block and the bias and output-layer gradients row by row,
+// in a fixed order, so training is deterministic, and applies Adam.  The step
+// is a chain of five small products and a 1,024-term sum, so latency is what
+// counts: 1,024 rows take 47 us, where a launch per product, activation
+// and sum (22 of them, operands through global memory) took 273.
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 
+#include <algorithm>
+#include <cmath>
 #include <cstdint>
 
 #include "phmm_band.h"
+#include "phmm_kernels.h"
 #include "phmm_mlp.h"
 #include "phmm_tc.cuh"
 
 namespace bvphmm {
 namespace {
 
-constexpr int TS = 16;
+using namespace tc;
 
-// C[M x N] = op(A) op(B) (+ C if accumulate); A is M x K (or K x M when ta),
-// B is K x N (or N x K when tb); all row-major FP32.
-__global__ void k_gemm(const float* __restrict__ A, const float* __restrict__ B, float* __restrict__ Cm, int M, int N,
-                       int K, int ta, int tb, int accumulate) {
-  __shared__ float sa[TS][TS + 1], sb[TS][TS + 1];
-  const int row = blockIdx.y * TS + threadIdx.y, col = blockIdx.x * TS + threadIdx.x;
-  float acc = 0.f;
-  for (int k0 = 0; k0 < K; k0 += TS) {
-    const int ka = k0 + threadIdx.x, kb = k0 + threadIdx.y;
-    float va = 0.f, vb = 0.f;
-    if (row < M && ka < K) va = ta ? A[(size_t)ka * M + row] : A[(size_t)row * K + ka];
-    if (col < N && kb < K) vb = tb ? B[(size_t)col * K + kb] : B[(size_t)kb * N + col];
-    sa[threadIdx.y][threadIdx.x] = va;
-    sb[threadIdx.y][threadIdx.x] = vb;
-    __syncthreads();
+constexpr int kRows = 128;          // minibatch rows per block (the MMA's M, and K of the weight gradients)
+constexpr int kRowThreads = 256;    // warp w: rows 32 (w & 3) .., columns 64 (w >> 2) ..
+constexpr int kW1 = kHid * kFeat, kW2 = kHid * kHid;
+constexpr int kOffW1 = 0, kOffB1 = kW1, kOffW2 = kOffB1 + kHid, kOffB2 = kOffW2 + kW2, kOffW3 = kOffB2 + kHid,
+              kOffB3 = kOffW3 + kOut * kHid;
+
+struct RowsSmem {
+  __nv_bfloat16 xa[kRows * kFeat];  // inputs [row][feature]
+  __nv_bfloat16 w1[kHid * kFeat];   // W1 [out][feature]; after layer 1 the inputs transposed, [feature][row]
+  __nv_bfloat16 w2[kHid * kHid];    // W2 [out][in]
+  __nv_bfloat16 w2t[kHid * kHid];   // W2 transposed, [in][out]
+  __nv_bfloat16 ra[kRows * kHid];   // H1, later dZ2, [row][unit]
+  __nv_bfloat16 h1t[kHid * kRows];  // H1 transposed, [unit][row]
+  __nv_bfloat16 dzt[kHid * kRows];  // dZ2, later dZ1, transposed, [unit][row]
+  float b1[kHid], b2[kHid], w3[kOut][kHid], b3[kOut];
+  float err[kRows][kOut], dout[kRows][kOut];
+  uint64_t mbar;
+  uint32_t tmem_base;
+  int fail;
+};
+
+// eight consecutive values rounded to BF16 (nearest even)
+__device__ __forceinline__ uint4 pack8(const float* v) {
+  uint32_t w[4];
 #pragma unroll
-    for (int t = 0; t < TS; ++t) acc = fmaf(sa[threadIdx.y][t], sb[t][threadIdx.x], acc);
+  for (int t = 0; t < 4; ++t) {
+    const __nv_bfloat162 h = __floats2bfloat162_rn(v[2 * t], v[2 * t + 1]);
+    w[t] = *reinterpret_cast<const uint32_t*>(&h);
+  }
+  return make_uint4(w[0], w[1], w[2], w[3]);
+}
+struct Eight {
+  float v[8];
+};
+__device__ __forceinline__ Eight load8(const float* p) {  // 16-byte aligned
+  const float4 a = __ldcg(reinterpret_cast<const float4*>(p)), b = __ldcg(reinterpret_cast<const float4*>(p) + 1);
+  return Eight{{a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w}};
+}
+__device__ __forceinline__ float as_bf16(float v) { return __bfloat162float(__float2bfloat16(v)); }
+
+// D[tmem] = A . B^T over K, both operands in the canonical K-major layout.
+template <int K, int N>
+__device__ __forceinline__ void product(uint32_t d, const __nv_bfloat16* a, const __nv_bfloat16* b) {
+  const unsigned char* pa = reinterpret_cast<const unsigned char*>(a);
+  const unsigned char* pb = reinterpret_cast<const unsigned char*>(b);
+#pragma unroll
+  for (int k = 0; k < K / 16; ++k)
+    mma_f16(d, mat_desc(pa + k * 2 * kLbo, kLbo, sbo_for(K)), mat_desc(pb + k * 2 * kLbo, kLbo, sbo_for(K)),
+            instr_desc(kRows, N), k > 0);
+}
+
+__device__ __forceinline__ unsigned char* at(__nv_bfloat16* m, int row, int col, int k) {
+  return reinterpret_cast<unsigned char*>(m) + core_offset(row, col, k);
+}
+
+// Forward (and backward) pass of rows [128 blockIdx.x, ..) of the minibatch of
+// n rows.  The inputs are rows idx[r] of feat (training) or FP32 rows of X,
+// rounded here (evaluation).
+__global__ void __launch_bounds__(kRowThreads, 1)
+    k_mlp_rows(MlpTrainBuffers b, const __nv_bfloat16* __restrict__ feat, const float* __restrict__ targets,
+               const int32_t* __restrict__ idx, int n, float alpha, float inv_n, int backward) {
+  extern __shared__ __align__(1024) unsigned char smem_raw[];
+  RowsSmem& s = *reinterpret_cast<RowsSmem*>(smem_raw);
+  const int tid = threadIdx.x, warp = tid >> 5, half = warp >> 2;
+  const int row = (warp & 3) * 32 + (tid & 31);     // this thread's row (and TMEM lane)
+  const int c0 = 64 * half;                         // and columns c0 .. c0 + 63
+  const long long gr = (long long)blockIdx.x * kRows + row;
+  const bool valid = gr < n;
+  if (warp == 0) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&s.tmem_base)),
+                 "r"(256)
+                 : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+  }
+  if (tid == 0) {
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(&s.mbar)) : "memory");
+    s.fail = 0;
+  }
+  asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  // inputs: a row's ten 16-byte pieces, five a thread
+  const long long src = !valid ? 0 : idx ? idx[gr] : gr;
+#pragma unroll
+  for (int q = 0; q < kFeat / 16; ++q) {
+    const int c = 8 * (2 * q + half);
+    uint4 v = make_uint4(0, 0, 0, 0);
+    if (valid) {
+      if (feat) {
+        v = *reinterpret_cast<const uint4*>(feat + src * kFeat + c);
+      } else {
+        v = pack8(load8(b.X + src * kFeat + c).v);
+      }
+    }
+    *reinterpret_cast<uint4*>(at(s.xa, row, c, kFeat)) = v;
+  }
+  // weights, rounded: 16-byte loads, several in flight a thread
+  const float* gw1 = b.w + kOffW1;
+  const float* gw2 = b.w + kOffW2;
+#pragma unroll
+  for (int x = tid; x < kW1 / 8; x += kRowThreads) {
+    const int r = x / (kFeat / 8), c = 8 * (x % (kFeat / 8));
+    *reinterpret_cast<uint4*>(at(s.w1, r, c, kFeat)) = pack8(load8(gw1 + r * kFeat + c).v);
+  }
+#pragma unroll 4
+  for (int x = tid; x < kW2 / 8; x += kRowThreads) {
+    const int r = x / (kHid / 8), c = 8 * (x % (kHid / 8));
+    *reinterpret_cast<uint4*>(at(s.w2, r, c, kHid)) = pack8(load8(gw2 + r * kHid + c).v);
+  }
+  if (backward) {
+#pragma unroll 4
+    for (int x = tid; x < kW2 / 8; x += kRowThreads) {  // column r of W2, outputs c .. c + 7
+      const int r = x % kHid, c = 8 * (x / kHid);
+      float f[8];
+#pragma unroll
+      for (int t = 0; t < 8; ++t) f[t] = __ldcg(gw2 + (c + t) * kHid + r);
+      *reinterpret_cast<uint4*>(at(s.w2t, r, c, kHid)) = pack8(f);
+    }
+  }
+  if (tid < kHid) {
+    s.b1[tid] = b.w[kOffB1 + tid];
+    s.b2[tid] = b.w[kOffB2 + tid];
+  }
+  s.w3[half][tid & (kHid - 1)] = as_bf16(b.w[kOffW3 + tid]);
+  if (tid < kOut) s.b3[tid] = b.w[kOffB3 + tid];
+  unsigned phase = 0;
+  // every thread's shared-memory writes towards the tensor cores, then one thread issues
+  auto issue = [&](auto&& mmas) {
+    fence_async_smem();
+    fence_before_sync();
     __syncthreads();
+    fence_after_sync();
+    if (tid == 0) {
+      mmas();
+      mma_commit(&s.mbar);
+    }
+  };
+  auto wait = [&]() -> bool {
+    if (!mbar_wait_parity(&s.mbar, phase)) {
+      s.fail = 1;
+      mbar_wait_parity(&s.mbar, phase);  // again bounded: MMAs still reading shared memory
+    }
+    phase ^= 1u;
+    fence_after_sync();
+    __syncthreads();
+    return !*reinterpret_cast<volatile int*>(&s.fail);
+  };
+  issue([&] { product<kFeat, kHid>(s.tmem_base, s.xa, s.w1); });
+  const uint32_t d0 = s.tmem_base + ((uint32_t)((warp & 3) * 32) << 16), d1 = d0 + 128;
+  bool ok = wait();
+  uint32_t on1[2], on2[2];  // ReLU masks of this thread's columns
+  if (ok) {
+#pragma unroll 1
+    for (int q = 0; q < 2; ++q) {
+      float v[32];
+      tmem_ld32(d0 + (uint32_t)(c0 + 32 * q), v);
+      uint32_t m = 0;
+#pragma unroll
+      for (int j = 0; j < 32; ++j) {
+        const float z = v[j] + s.b1[c0 + 32 * q + j];
+        m |= (uint32_t)(z > 0.f) << j;
+        v[j] = fmaxf(z, 0.f);
+      }
+      on1[q] = m;
+#pragma unroll
+      for (int j = 0; j < 32; j += 8) *reinterpret_cast<uint4*>(at(s.ra, row, c0 + 32 * q + j, kHid)) = pack8(v + j);
+      if (backward) {
+#pragma unroll
+        for (int j = 0; j < 32; ++j)
+          *reinterpret_cast<__nv_bfloat16*>(at(s.h1t, c0 + 32 * q + j, row, kRows)) = __float2bfloat16(v[j]);
+      }
+    }
+    issue([&] { product<kHid, kHid>(s.tmem_base + 128, s.ra, s.w2); });
+    if (backward) {  // the inputs transposed, where W1 was
+#pragma unroll
+      for (int q = 0; q < kFeat / 16; ++q) {
+        const int c = 8 * (2 * q + half);
+        const uint4 v = *reinterpret_cast<const uint4*>(at(s.xa, row, c, kFeat));
+        const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+        for (int t = 0; t < 8; ++t)
+          *reinterpret_cast<uint16_t*>(at(s.w1, c + t, row, kRows)) = (uint16_t)(w[t >> 1] >> (16 * (t & 1)));
+      }
+    }
+    ok = wait();
   }
-  if (row < M && col < N) {
-    float* c = Cm + (size_t)row * N + col;
-    *c = accumulate ? *c + acc : acc;
+  if (ok) {
+    // output layer: this thread sums output `half` of its row, hidden units in order
+    float acc = 0.f;
+#pragma unroll 1
+    for (int q = 0; q < 4; ++q) {
+      float v[32];
+      tmem_ld32(d1 + (uint32_t)(32 * q), v);
+      uint32_t m = 0;
+#pragma unroll
+      for (int j = 0; j < 32; ++j) {
+        const float z = v[j] + s.b2[32 * q + j];
+        m |= (uint32_t)(z > 0.f) << j;
+        v[j] = as_bf16(fmaxf(z, 0.f));
+        acc = fmaf(v[j], s.w3[half][32 * q + j], acc);
+      }
+      if ((q >> 1) == half) {
+        if (q & 1) on2[1] = m;
+        else on2[0] = m;
+        if (backward && valid) {
+#pragma unroll
+          for (int j = 0; j < 32; j += 4)
+            *reinterpret_cast<float4*>(b.H2 + gr * kHid + 32 * q + j) = make_float4(v[j], v[j + 1], v[j + 2], v[j + 3]);
+        }
+      }
+    }
+    const float o = acc + s.b3[half];
+    const float t = valid ? (feat ? targets[2 * src + half] : b.T[2 * src + half]) : 0.f;
+    const float e = o - t;
+    const float w = (half == 0 ? e > 0.f : e < 0.f) ? alpha : 1.f;
+    const float d = valid ? 2.f * w * e * inv_n : 0.f;
+    s.err[row][half] = valid ? w * e * e : 0.f;
+    s.dout[row][half] = d;
+    if (valid) {
+      b.O[2 * gr + half] = o;
+      b.dO[2 * gr + half] = d;
+    }
+    __syncthreads();
+    if (half == 0) {
+      float l = s.err[row][0] + s.err[row][1];
+      for (int k = 16; k > 0; k >>= 1) l += __shfl_xor_sync(0xffffffffu, l, k);
+      if ((tid & 31) == 0) atomicAdd(b.loss, l * inv_n);
+    }
+  }
+  if (ok && backward) {
+    // dZ2 = (dO . W3) where Z2 > 0
+    const float g0 = s.dout[row][0], g1 = s.dout[row][1];
+#pragma unroll 1
+    for (int q = 0; q < 2; ++q) {
+      float v[32];
+#pragma unroll
+      for (int j = 0; j < 32; ++j) {
+        const int c = c0 + 32 * q + j;
+        const float d = fmaf(g1, s.w3[1][c], fmaf(g0, s.w3[0][c], 0.f));
+        v[j] = (on2[q] >> j & 1u) ? d : 0.f;
+        *reinterpret_cast<__nv_bfloat16*>(at(s.dzt, c, row, kRows)) = __float2bfloat16(v[j]);
+      }
+#pragma unroll
+      for (int j = 0; j < 32; j += 8) *reinterpret_cast<uint4*>(at(s.ra, row, c0 + 32 * q + j, kHid)) = pack8(v + j);
+      if (valid) {
+#pragma unroll
+        for (int j = 0; j < 32; j += 4)
+          *reinterpret_cast<float4*>(b.dH + gr * kHid + c0 + 32 * q + j) = make_float4(v[j], v[j + 1], v[j + 2], v[j + 3]);
+      }
+    }
+    issue([&] {
+      product<kHid, kHid>(s.tmem_base, s.ra, s.w2t);         // dH1 = dZ2 W2
+      product<kRows, kHid>(s.tmem_base + 128, s.dzt, s.h1t);  // this block's part of dW2 = dZ2^T H1
+    });
+    ok = wait();
+    if (ok) {
+      float* part2 = b.part2 + (size_t)blockIdx.x * kW2 + row * kHid + c0;
+#pragma unroll 1
+      for (int q = 0; q < 2; ++q) {
+        float v[32];
+        tmem_ld32(d1 + (uint32_t)(c0 + 32 * q), v);
+#pragma unroll
+        for (int j = 0; j < 32; j += 4)
+          *reinterpret_cast<float4*>(part2 + 32 * q + j) = make_float4(v[j], v[j + 1], v[j + 2], v[j + 3]);
+        tmem_ld32(d0 + (uint32_t)(c0 + 32 * q), v);
+#pragma unroll
+        for (int j = 0; j < 32; ++j) {
+          v[j] = (on1[q] >> j & 1u) ? v[j] : 0.f;  // dZ1
+          *reinterpret_cast<__nv_bfloat16*>(at(s.dzt, c0 + 32 * q + j, row, kRows)) = __float2bfloat16(v[j]);
+        }
+        if (valid) {
+#pragma unroll
+          for (int j = 0; j < 32; j += 4)
+            *reinterpret_cast<float4*>(b.dH2 + gr * kHid + c0 + 32 * q + j) =
+                make_float4(v[j], v[j + 1], v[j + 2], v[j + 3]);
+        }
+      }
+      issue([&] { product<kRows, kFeat>(s.tmem_base, s.dzt, s.w1); });  // part of dW1 = dZ1^T X
+      ok = wait();
+    }
+    if (ok) {
+      float* part1 = b.part1 + (size_t)blockIdx.x * kW1 + row * kFeat;
+#pragma unroll 1
+      for (int c = 32 * half; c < kFeat; c += 64) {  // columns 0-31 and 64-79, or 32-63
+        float v[32];
+        tmem_ld32(d0 + (uint32_t)c, v);
+#pragma unroll
+        for (int j = 0; j < 32; j += 4)
+          if (c + j < kFeat) *reinterpret_cast<float4*>(part1 + c + j) = make_float4(v[j], v[j + 1], v[j + 2], v[j + 3]);
+      }
+    }
+  }
+  if (!ok && tid == 0) atomicOr(b.tc_fail, 1u);
+  fence_before_sync();
+  __syncthreads();
+  if (warp == 0) {
+    fence_after_sync();
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(s.tmem_base), "r"(256) : "memory");
   }
 }
 
-// weight matrices to BF16, biases unchanged (the inference kernel keeps FP32 biases)
-__global__ void k_round_bf16(const float* __restrict__ w, float* __restrict__ wq, int n) {
-  const int n1 = kHid * kFeat, n2 = kHid * kHid;
-  for (int x = blockIdx.x * blockDim.x + threadIdx.x; x < n; x += gridDim.x * blockDim.x) {
-    const bool bias = (x >= n1 && x < n1 + kHid) || (x >= n1 + kHid + n2 && x < n1 + 2 * kHid + n2) ||
-                      x >= n1 + 2 * kHid + n2 + kOut * kHid;
-    wq[x] = bias ? w[x] : __bfloat162float(__float2bfloat16(w[x]));
+struct AdamArgs {
+  int on;  // 0: the gradient goes to g (evaluation)
+  float lr, b1, b2, eps, c1, c2;
+};
+
+// Gradient gg of parameter x: stored, or applied.
+__device__ __forceinline__ void apply_grad(const MlpTrainBuffers& b, int x, float gg, const AdamArgs& a) {
+  if (!a.on) {
+    b.g[x] = gg;
+    return;
   }
+  const float mm = a.b1 * b.m[x] + (1.f - a.b1) * gg;
+  const float vv = a.b2 * b.v[x] + (1.f - a.b2) * gg * gg;
+  b.m[x] = mm;
+  b.v[x] = vv;
+  b.w[x] -= a.lr * (mm * a.c1) / (sqrtf(vv * a.c2) + a.eps);
 }
 
-// Z[r][c] += bias[c]; H = relu(Z) rounded to BF16, as the inference kernel
-// stores its hidden activations (the gradient passes the rounding straight)
-__global__ void k_bias_relu(float* __restrict__ Z, const float* __restrict__ bias, float* __restrict__ Hout, int rows,
-                            int cols, int relu) {
-  for (long long x = blockIdx.x * (long long)blockDim.x + threadIdx.x; x < (long long)rows * cols;
-       x += (long long)gridDim.x * blockDim.x) {
-    const float z = Z[x] + bias[x % cols];
-    Z[x] = z;
-    if (Hout) Hout[x] = relu ? __bfloat162float(__float2bfloat16(fmaxf(z, 0.f))) : z;
+// Blocks 0 .. kUpdElem - 1: the hidden weights, a parameter a thread, the partial
+// products summed block by block.  Then a block per 32 columns of dZ1, dZ2 and
+// H2: bias gradients (column sums) and the output layer's (sums of dO times H2),
+// row by row: the rows are brought to shared memory kSumRows at a time, then
+// one thread a sum adds them in order.
+constexpr int kUpdThreads = 256;
+constexpr int kUpdElem = (kW1 + kW2) / kUpdThreads;
+constexpr int kSumRows = 1024;
+constexpr int kSumCols = 32;
+constexpr int kUpdSmem = kSumRows * (kSumCols + kOut) * (int)sizeof(float);
+static_assert(kOffW2 % 4 == 0, "16-byte loads of W2");
+static_assert((kW1 + kW2) % kUpdThreads == 0, "whole blocks of hidden weights");
+
+__global__ void __launch_bounds__(kUpdThreads) k_mlp_update(MlpTrainBuffers b, int n, AdamArgs a) {
+  extern __shared__ __align__(16) float tile[];
+  const int tid = threadIdx.x;
+  if (blockIdx.x < kUpdElem) {
+    const int x = blockIdx.x * kUpdThreads + tid;
+    const bool second = x >= kW1;
+    const int e = second ? x - kW1 : x, size = second ? kW2 : kW1;
+    const float* part = (second ? b.part2 : b.part1) + e;
+    const int parts = (n + kRows - 1) / kRows;
+    float acc = 0.f;
+#pragma unroll 8
+    for (int k = 0; k < parts; ++k) acc += part[(size_t)k * size];
+    apply_grad(b, (second ? kOffW2 : kOffW1) + e, acc, a);
+    return;
   }
-}
-
-__global__ void k_relu_bwd(float* __restrict__ dH, const float* __restrict__ Z, long long n) {
-  for (long long x = blockIdx.x * (long long)blockDim.x + threadIdx.x; x < n; x += (long long)gridDim.x * blockDim.x)
-    if (!(Z[x] > 0.f)) dH[x] = 0.f;
-}
-
-// db[c] = sum_r dZ[r][c]
-__global__ void k_colsum(const float* __restrict__ dZ, float* __restrict__ db, int rows, int cols) {
-  const int c = blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= cols) return;
-  float s = 0.f;
-  for (int r = 0; r < rows; ++r) s += dZ[(size_t)r * cols + c];
-  db[c] = s;
-}
-
-__global__ void k_loss(const float* __restrict__ O, const float* __restrict__ T, const float* __restrict__ mask,
-                       float* __restrict__ dO, float* __restrict__ loss, int rows, float alpha, float inv_n) {
-  float l = 0.f;
-  for (int r = blockIdx.x * blockDim.x + threadIdx.x; r < rows; r += gridDim.x * blockDim.x) {
-    const float m = mask ? mask[r] : 1.f;
-    const float e0 = O[2 * r] - T[2 * r], e1 = O[2 * r + 1] - T[2 * r + 1];
-    const float w0 = e0 > 0.f ? alpha : 1.f, w1 = e1 < 0.f ? alpha : 1.f;
-    dO[2 * r] = m * 2.f * w0 * e0 * inv_n;
-    dO[2 * r + 1] = m * 2.f * w1 * e1 * inv_n;
-    l += m * (w0 * e0 * e0 + w1 * e1 * e1);
+  const int q = blockIdx.x - kUpdElem, what = q / (kHid / kSumCols), col = kSumCols * (q % (kHid / kSumCols));
+  const float* rows = (what == 0 ? b.dH2 : what == 1 ? b.dH : b.H2) + col;
+  float* dout = tile + kSumRows * kSumCols;
+  // what 0, 1: thread c < 32 sums column c; 2: thread 32 o + c sums dO[o] H2[c], threads 64 + o sum dO[o]
+  const int c = tid & 31, o = tid >> 5;
+  const bool sums = what < 2 ? tid < 32 : tid < 64, sums_o = what == 2 && col == 0 && tid >= 64 && tid < 64 + kOut;
+  float acc = 0.f;
+  for (int r0 = 0; r0 < n; r0 += kSumRows) {
+    const int nr = min(kSumRows, n - r0);
+    __syncthreads();
+#pragma unroll 16
+    for (int x = tid; x < nr * (kSumCols / 4); x += kUpdThreads) {
+      const int r = x / (kSumCols / 4), k = 4 * (x % (kSumCols / 4));
+      *reinterpret_cast<float4*>(tile + r * kSumCols + k) =
+          __ldcg(reinterpret_cast<const float4*>(rows + (size_t)(r0 + r) * kHid + k));
+    }
+    if (what == 2)
+      for (int x = tid; x < nr * kOut; x += kUpdThreads) dout[x] = __ldcg(b.dO + (size_t)r0 * kOut + x);
+    __syncthreads();
+    if (sums) {
+      if (what < 2) {
+#pragma unroll 16
+        for (int r = 0; r < nr; ++r) acc += tile[r * kSumCols + c];
+      } else {
+#pragma unroll 16
+        for (int r = 0; r < nr; ++r) acc = fmaf(dout[r * kOut + o], tile[r * kSumCols + c], acc);
+      }
+    } else if (sums_o) {
+#pragma unroll 16
+      for (int r = 0; r < nr; ++r) acc += dout[r * kOut + tid - 64];
+    }
   }
-  for (int o = 16; o > 0; o >>= 1) l += __shfl_xor_sync(0xffffffffu, l, o);
-  if ((threadIdx.x & 31) == 0) atomicAdd(loss, l * inv_n);
-}
-
-__global__ void k_adam(float* __restrict__ w, const float* __restrict__ g, float* __restrict__ m, float* __restrict__ v,
-                       int n, float lr, float b1, float b2, float eps, float c1, float c2) {
-  for (int x = blockIdx.x * blockDim.x + threadIdx.x; x < n; x += gridDim.x * blockDim.x) {
-    const float gg = g[x];
-    const float mm = b1 * m[x] + (1.f - b1) * gg;
-    const float vv = b2 * v[x] + (1.f - b2) * gg * gg;
-    m[x] = mm;
-    v[x] = vv;
-    w[x] -= lr * (mm * c1) / (sqrtf(vv * c2) + eps);
-  }
-}
-
-__global__ void k_gather_rows(const __nv_bfloat16* __restrict__ feat, const float* __restrict__ targets,
-                              const float* __restrict__ mask, const int32_t* __restrict__ idx, int n, float* __restrict__ X,
-                              float* __restrict__ T, float* __restrict__ Mk) {
-  for (int x = blockIdx.x * blockDim.x + threadIdx.x; x < n * kFeat; x += gridDim.x * blockDim.x) {
-    const int r = x / kFeat, c = x % kFeat;
-    const long long src = idx ? idx[r] : r;
-    X[x] = __bfloat162float(feat[src * kFeat + c]);
-    if (c < 2) T[2 * r + c] = targets[2 * src + c];
-    if (c == 0) Mk[r] = mask ? mask[src] : 1.f;
-  }
+  if (sums) apply_grad(b, what == 0 ? kOffB1 + col + c : what == 1 ? kOffB2 + col + c : kOffW3 + o * kHid + col + c, acc, a);
+  if (sums_o) apply_grad(b, kOffB3 + tid - 64, acc, a);
 }
 
 __global__ void k_export_params(const float* __restrict__ w, MlpParams* __restrict__ out) {
@@ -144,215 +437,37 @@ __global__ void k_export_params(const float* __restrict__ w, MlpParams* __restri
   }
 }
 
-inline dim3 grid2(int M, int N) { return dim3((N + TS - 1) / TS, (M + TS - 1) / TS); }
 
-// ---- tensor-core GEMM ---------------------------------------------------------
-// C = A . B^T over K with FP32 operands read through strides and rounded to
-// BF16 while they are staged: A(r, k) = A[r sar + k sak] for r < m_valid and
-// k < k_valid (else 0), B(n, k) = B[n sbn + k sbk] for k < k_valid; C FP32
-// row-major (ldc = N), rows past m_valid not written.  N a multiple of 16, at
-// most 128.  Block (x, y) takes rows 128 x .. 128 x + 127 and the K range
-// y kspan .. (y + 1) kspan (kspan a multiple of 16) and writes its product to
-// C + y c_split (split K: the partial products are summed in a fixed order by
-// k_sum_splits).  Four warps: K in chunks of up to 64 staged into shared
-// memory in the canonical K-major layout without swizzling, one thread issues
-// the chunk's MMAs (K = 16 each) into the FP32 accumulator in tensor memory
-// and commits them to an mbarrier, every thread waits (bounded: a wait that
-// gives up sets *fail and the block skips its epilogue), and the warps drain
-// the accumulator with tcgen05.ld (warp w: rows 32 w .. 32 w + 31).
-constexpr int kTcKc = 64;
-struct GemmTcSmem {
-  __nv_bfloat16 a[128 * kTcKc];
-  __nv_bfloat16 b[128 * kTcKc];
-  uint64_t mbar;
-  uint32_t tmem_base;
-  int fail;
-};
-struct GemmTcArgs {
-  const float* A;
-  long long sar, sak;
-  const float* B;
-  long long sbn, sbk;
-  float* C;
-  long long c_split;
-  int m_valid, N, k_valid, kspan;
-};
-
-// eight consecutive k of one row, rounded to BF16 (nearest even), zero where invalid
-__device__ __forceinline__ uint4 stage8(const float* base, long long sk, bool row_ok, int k, int k_valid) {
-  uint32_t w[4];
-#pragma unroll
-  for (int t = 0; t < 4; ++t) {
-    const int k0 = k + 2 * t, k1 = k0 + 1;
-    const float v0 = row_ok && k0 < k_valid ? base[(long long)k0 * sk] : 0.f;
-    const float v1 = row_ok && k1 < k_valid ? base[(long long)k1 * sk] : 0.f;
-    const __nv_bfloat162 h = __floats2bfloat162_rn(v0, v1);
-    w[t] = *reinterpret_cast<const uint32_t*>(&h);
-  }
-  return make_uint4(w[0], w[1], w[2], w[3]);
+cudaError_t launch_rows(const MlpTrainBuffers& b, const __nv_bfloat16* feat, const float* targets, const int32_t* idx, int n,
+                        float alpha, bool backward, cudaStream_t st) {
+  const cudaError_t e = raise_dynamic_smem(reinterpret_cast<const void*>(&k_mlp_rows), (int)sizeof(RowsSmem));
+  if (e != cudaSuccess) return e;
+  k_mlp_rows<<<(n + kRows - 1) / kRows, kRowThreads, sizeof(RowsSmem), st>>>(b, feat, targets, idx, n, alpha, 1.f / (float)n,
+                                                                           backward);
+  return cudaGetLastError();
 }
-
-__global__ void __launch_bounds__(128, 1) k_gemm_tc(GemmTcArgs g, unsigned int* fail) {
-  using namespace tc;
-  __shared__ __align__(1024) GemmTcSmem s;
-  const int tid = threadIdx.x, warp = tid >> 5;
-  const int row0 = blockIdx.x * 128;
-  const int kb = blockIdx.y * g.kspan, ke = min(kb + g.kspan, g.k_valid);
-  if (warp == 0) {
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&s.tmem_base)),
-                 "r"(128)
-                 : "memory");
-    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
-  }
-  if (tid == 0) {
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(&s.mbar)) : "memory");
-    s.fail = 0;
-  }
-  asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-  fence_before_sync();
-  __syncthreads();
-  fence_after_sync();
-  const uint32_t tmem = s.tmem_base;
-  const uint32_t idesc = instr_desc(128, g.N);
-  unsigned char* sa = reinterpret_cast<unsigned char*>(s.a);
-  unsigned char* sb = reinterpret_cast<unsigned char*>(s.b);
-  unsigned phase = 0;
-  bool any = false;  // the accumulator holds a product
-  for (int k0 = kb; k0 < kb + g.kspan; k0 += kTcKc) {
-    const int kc = min(kTcKc, kb + g.kspan - k0);  // a multiple of 16
-    const int pieces = kc / 8;                     // 16-byte row pieces per row
-    for (int x = tid; x < 128 * pieces; x += 128) {
-      const int r = x / pieces, c = 8 * (x % pieces);
-      const int gr = row0 + r;
-      *reinterpret_cast<uint4*>(sa + core_offset(r, c, kc)) =
-          stage8(g.A + (long long)gr * g.sar, g.sak, gr < g.m_valid, k0 + c, ke);
-    }
-    for (int x = tid; x < g.N * pieces; x += 128) {
-      const int r = x / pieces, c = 8 * (x % pieces);
-      *reinterpret_cast<uint4*>(sb + core_offset(r, c, kc)) = stage8(g.B + (long long)r * g.sbn, g.sbk, true, k0 + c, ke);
-    }
-    fence_async_smem();
-    fence_before_sync();
-    __syncthreads();
-    if (tid == 0) {
-      fence_after_sync();
-      const uint32_t sbo = sbo_for(kc);
-      for (int k = 0; k < kc / 16; ++k)
-        mma_f16(tmem, mat_desc(sa + k * 2 * kLbo, kLbo, sbo), mat_desc(sb + k * 2 * kLbo, kLbo, sbo), idesc,
-                any || k > 0);
-      mma_commit(&s.mbar);
-    }
-    any = true;
-    if (!mbar_wait_parity(&s.mbar, phase)) {
-      s.fail = 1;
-      mbar_wait_parity(&s.mbar, phase);  // again bounded: the MMAs still reading this chunk
-    }
-    phase ^= 1u;
-    fence_after_sync();
-    __syncthreads();  // the chunk's shared memory is free for the next one
-    if (*reinterpret_cast<volatile int*>(&s.fail)) break;
-  }
-  if (!*reinterpret_cast<volatile int*>(&s.fail)) {
-    const int r = row0 + tid;
-    float* C = g.C + blockIdx.y * g.c_split;
-    const uint32_t trow = tmem + ((uint32_t)(warp * 32) << 16);
-    for (int c0 = 0; c0 < g.N; c0 += 32) {
-      float v[32];
-      if (any) {
-        tmem_ld32(trow + (uint32_t)c0, v);
-      } else {
-#pragma unroll
-        for (int j = 0; j < 32; ++j) v[j] = 0.f;
-      }
-      if (r < g.m_valid) {
-#pragma unroll
-        for (int j = 0; j < 32; ++j)
-          if (c0 + j < g.N) C[(size_t)r * g.N + c0 + j] = v[j];
-      }
-    }
-  } else if (tid == 0) {
-    atomicOr(fail, 1u);
-  }
-  fence_before_sync();
-  __syncthreads();
-  if (warp == 0) {
-    fence_after_sync();
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(s.tmem_base), "r"(128) : "memory");
-  }
-}
-
-// out[x] = sum over s of part[s * n + x], s = 0, 1, .. in order
-__global__ void k_sum_splits(const float* __restrict__ part, int splits, int n, float* __restrict__ out) {
-  for (int x = blockIdx.x * blockDim.x + threadIdx.x; x < n; x += gridDim.x * blockDim.x) {
-    float acc = 0.f;
-    for (int sp = 0; sp < splits; ++sp) acc += part[(size_t)sp * n + x];
-    out[x] = acc;
-  }
-}
-
-// C[m x N] = A . B^T on the tensor cores (one K range)
-inline void gemm_tc(GemmTcArgs g, unsigned int* fail, cudaStream_t st) {
-  if (g.m_valid <= 0 || g.k_valid <= 0) return;
-  g.c_split = 0;
-  g.kspan = (g.k_valid + 15) / 16 * 16;
-  k_gemm_tc<<<dim3((g.m_valid + 127) / 128, 1), 128, 0, st>>>(g, fail);
-}
-// C[128 x N] = A . B^T with K = the batch split into ranges of 128 (partials in `part`, summed in order)
-inline void gemm_tc_splitk(GemmTcArgs g, float* part, unsigned int* fail, cudaStream_t st) {
-  if (g.m_valid <= 0 || g.k_valid <= 0) return;
-  float* C = g.C;
-  const int splits = (g.k_valid + 127) / 128;
-  g.C = part;
-  g.c_split = (long long)g.m_valid * g.N;
-  g.kspan = 128;
-  k_gemm_tc<<<dim3((g.m_valid + 127) / 128, splits), 128, 0, st>>>(g, fail);
-  k_sum_splits<<<64, 256, 0, st>>>(part, splits, g.m_valid * g.N, C);
+cudaError_t launch_update(const MlpTrainBuffers& b, int n, const AdamArgs& a, cudaStream_t st) {
+  const cudaError_t e = raise_dynamic_smem(reinterpret_cast<const void*>(&k_mlp_update), kUpdSmem);
+  if (e != cudaSuccess) return e;
+  k_mlp_update<<<kUpdElem + 3 * (kHid / kSumCols), kUpdThreads, kUpdSmem, st>>>(b, n, a);
+  return cudaGetLastError();
 }
 
 }  // namespace
 
 cudaError_t mlp_forward_backward(const MlpTrainBuffers& b, int n, float alpha, bool backward, cudaStream_t st) {
-  const dim3 blk(TS, TS);
-  const int o1 = 0, ob1 = kHid * kFeat, o2 = ob1 + kHid, ob2 = o2 + kHid * kHid, o3 = ob2 + kHid, ob3 = o3 + kOut * kHid;
-  k_round_bf16<<<64, 256, 0, st>>>(b.w, b.wq, kMlpParamCount);
-  // forward: the hidden layers on the tensor cores (X and the rounded weights are BF16 values)
-  gemm_tc({b.X, kFeat, 1, b.wq + o1, kFeat, 1, b.Z1, 0, n, kHid, kFeat, 0}, b.tc_fail, st);
-  k_bias_relu<<<256, 256, 0, st>>>(b.Z1, b.wq + ob1, b.H1, n, kHid, 1);
-  gemm_tc({b.H1, kHid, 1, b.wq + o2, kHid, 1, b.Z2, 0, n, kHid, kHid, 0}, b.tc_fail, st);
-  k_bias_relu<<<256, 256, 0, st>>>(b.Z2, b.wq + ob2, b.H2, n, kHid, 1);
-  k_gemm<<<grid2(n, kOut), blk, 0, st>>>(b.H2, b.wq + o3, b.O, n, kOut, kHid, 0, 1, 0);
-  k_bias_relu<<<256, 256, 0, st>>>(b.O, b.wq + ob3, nullptr, n, kOut, 0);
-  cudaMemsetAsync(b.loss, 0, sizeof(float), st);
-  k_loss<<<64, 256, 0, st>>>(b.O, b.T, b.mask, b.dO, b.loss, n, alpha, 1.f / (float)n);
-  if (!backward) return cudaGetLastError();
-  // backward: dW = dZ^T H, db = colsum(dZ), dH_prev = dZ W
-  k_gemm<<<grid2(kOut, kHid), blk, 0, st>>>(b.dO, b.H2, b.g + o3, kOut, kHid, n, 1, 0, 0);
-  k_colsum<<<1, 32, 0, st>>>(b.dO, b.g + ob3, n, kOut);
-  k_gemm<<<grid2(n, kHid), blk, 0, st>>>(b.dO, b.wq + o3, b.dH, n, kHid, kOut, 0, 0, 0);
-  k_relu_bwd<<<256, 256, 0, st>>>(b.dH, b.Z2, (long long)n * kHid);
-  // dW2 = dZ2^T H1 (K = the batch, split in ranges of 128)
-  gemm_tc_splitk({b.dH, 1, kHid, b.H1, 1, kHid, b.g + o2, 0, kHid, kHid, n, 0}, b.part, b.tc_fail, st);
-  k_colsum<<<(kHid + 127) / 128, 128, 0, st>>>(b.dH, b.g + ob2, n, kHid);
-  // dH1 = dZ2 W2 (B(i, o) = W2[o][i])
-  gemm_tc({b.dH, kHid, 1, b.wq + o2, 1, kHid, b.dH2, 0, n, kHid, kHid, 0}, b.tc_fail, st);
-  k_relu_bwd<<<256, 256, 0, st>>>(b.dH2, b.Z1, (long long)n * kHid);
-  // dW1 = dZ1^T X
-  gemm_tc_splitk({b.dH2, 1, kHid, b.X, 1, kFeat, b.g + o1, 0, kHid, kFeat, n, 0}, b.part, b.tc_fail, st);
-  k_colsum<<<(kHid + 127) / 128, 128, 0, st>>>(b.dH2, b.g + ob1, n, kHid);
-  return cudaGetLastError();
+  cudaError_t e = cudaMemsetAsync(b.loss, 0, sizeof(float), st);
+  if (e == cudaSuccess) e = launch_rows(b, nullptr, nullptr, nullptr, n, alpha, backward, st);
+  if (e == cudaSuccess && backward) e = launch_update(b, n, AdamArgs{}, st);
+  return e;
 }
 
-cudaError_t mlp_adam(const MlpTrainBuffers& b, int step, float lr, cudaStream_t st) {
+cudaError_t mlp_train_step(const MlpTrainBuffers& b, const __nv_bfloat16* feat, const float* targets, const int32_t* idx,
+                           int n, float alpha, int step, float lr, cudaStream_t st) {
   const float b1 = 0.9f, b2 = 0.999f;
-  const float c1 = 1.f / (1.f - powf(b1, (float)step)), c2 = 1.f / (1.f - powf(b2, (float)step));
-  k_adam<<<64, 256, 0, st>>>(b.w, b.g, b.m, b.v, kMlpParamCount, lr, b1, b2, 1e-8f, c1, c2);
-  return cudaGetLastError();
-}
-
-cudaError_t mlp_gather(const __nv_bfloat16* feat, const float* targets, const float* mask, const int32_t* idx, int n,
-                       const MlpTrainBuffers& b, cudaStream_t st) {
-  k_gather_rows<<<256, 256, 0, st>>>(feat, targets, mask, idx, n, b.X, b.T, b.mask);
-  return cudaGetLastError();
+  const AdamArgs a{1, lr, b1, b2, 1e-8f, 1.f / (1.f - powf(b1, (float)step)), 1.f / (1.f - powf(b2, (float)step))};
+  const cudaError_t e = launch_rows(b, feat, targets, idx, n, alpha, true, st);
+  return e == cudaSuccess ? launch_update(b, n, a, st) : e;
 }
 
 cudaError_t mlp_export(const float* w, MlpParams* out, cudaStream_t st) {
