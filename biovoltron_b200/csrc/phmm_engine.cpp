@@ -16,6 +16,8 @@
 
 #include "phmm_rows.h"
 
+#include <emmintrin.h>
+
 #include <algorithm>
 #include <chrono>
 #include <memory>
@@ -25,22 +27,26 @@
 namespace bvphmm {
 
 cudaError_t DevBuf::reserve(size_t bytes) {
-  if (bytes <= cap_ && p_) return cudaSuccess;
+  if (bytes <= cap_ && own_) {
+    p_ = own_;
+    return cudaSuccess;
+  }
   release();
   size_t want = std::max<size_t>(bytes, 256);
-  cudaError_t e = cudaMalloc(&p_, want);
+  cudaError_t e = cudaMalloc(&own_, want);
   if (e != cudaSuccess) {
-    p_ = nullptr;
-    cap_ = 0;
+    own_ = nullptr;
     return e;
   }
+  p_ = own_;
   cap_ = want;
   return cudaSuccess;
 }
 
 void DevBuf::release() {
-  if (p_) cudaFree(p_);
+  if (own_) cudaFree(own_);
   p_ = nullptr;
+  own_ = nullptr;
   cap_ = 0;
 }
 
@@ -52,6 +58,17 @@ constexpr int kF64Bin0 = 19;
 constexpr int kF64List = 28;
 constexpr int kMaxVariants = 28;
 constexpr int kRescaleTarget = 1000;  // FP64 boundary rows are scaled to ~2^1000
+
+// Small batches.  Eight copies from pageable memory, a packing kernel and two
+// copies back cost more host time than the kernels of one window take; a batch
+// whose inputs fit kStageBytes is laid out in page-locked memory instead
+// (qualities packed there) and sent as one copy, and results that fit
+// kSmallOutBytes come back with the counters in one.  Beyond that size the
+// packing loop is slower than the copies it saves.
+constexpr size_t kStageBytes = 512 << 10;
+constexpr size_t kSmallOutBytes = 256 << 10;
+constexpr size_t kCountersBytes = 512;
+static_assert(sizeof(Counters) <= kCountersBytes, "results lie behind the counters");
 
 int64_t round_up(int64_t x, int64_t m) { return (x + m - 1) / m * m; }
 
@@ -163,7 +180,7 @@ bv_status Engine::init() {
   BV_CUDA(d_tables_.reserve(sizeof(Tables)), "tables alloc");
   BV_CUDA(cudaMemcpyAsync(d_tables_.get(), h_tables_.get(), sizeof(Tables), cudaMemcpyHostToDevice, stream_),
           "tables copy");
-  BV_CUDA(d_counters_.reserve(sizeof(Counters)), "counters alloc");
+  BV_CUDA(d_counters_.reserve(kCountersBytes + kSmallOutBytes), "counters alloc");
   BV_CUDA(cudaStreamSynchronize(stream_), "init sync");
   return BV_OK;
 }
@@ -471,6 +488,61 @@ bv_status Engine::plan(const bv_region_batch& b) {
   return BV_OK;
 }
 
+bv_status Engine::reserve_host() {
+  if (h_counters_) return BV_OK;
+  unsigned char* p = nullptr;
+  BV_CUDA(cudaMallocHost(reinterpret_cast<void**>(&p), kCountersBytes + kSmallOutBytes + kStageBytes), "pinned buffers");
+  h_counters_ = reinterpret_cast<Counters*>(p);
+  h_stage_ = p + kCountersBytes + kSmallOutBytes;
+  return BV_OK;
+}
+
+// The next piece of the staged image: its host place, `dev` viewing its place
+// on the device; nullptr when the image is full.
+void* Engine::stage_piece(size_t bytes, DevBuf& dev) {
+  const size_t at = stage_used_;
+  const size_t end = (at + bytes + 255) / 256 * 256;
+  if (end > kStageBytes) return nullptr;
+  stage_used_ = end;
+  dev.view(d_stage_.as<unsigned char>() + at);
+  return h_stage_ + at;
+}
+
+// A small batch's inputs into the image (upload_plan sends it).
+bv_status Engine::stage_inputs(const bv_region_batch& b) {
+  if (bv_status s = reserve_host(); s != BV_OK) return s;
+  BV_CUDA(d_stage_.reserve(kStageBytes), "alloc inputs");
+  stage_used_ = 0;
+  const size_t rb = (size_t)n_read_bytes_, hb = (size_t)n_hap_bytes_;
+  auto put = [&](DevBuf& dev, const void* src, size_t bytes, size_t room) {
+    void* p = stage_piece(room, dev);
+    if (bytes) std::memcpy(p, src, bytes);
+  };
+  put(d_read_off_, b.read_offsets, n_reads_ > 0 ? sizeof(int64_t) * (n_reads_ + 1) : 0, sizeof(int64_t) * (n_reads_ + 1));
+  put(d_hap_off_, b.hap_offsets, n_haps_ > 0 ? sizeof(int64_t) * (n_haps_ + 1) : 0, sizeof(int64_t) * (n_haps_ + 1));
+  put(d_read_bases_, b.read_bases, rb, rb + 16);  // tail padding for the k-mer kernel's word loads
+  put(d_hap_bases_, b.hap_bases, hb, hb + 16);
+  uchar4* q = static_cast<uchar4*>(stage_piece(4 * rb + 16, d_quals4_));
+  size_t x = 0;
+  const __m128i gi = _mm_set1_epi8((char)gap_ins_), gd = _mm_set1_epi8((char)gap_del_), gc = _mm_set1_epi8((char)gap_gcp_);
+  auto load = [&](const uint8_t* p) { return _mm_loadu_si128(reinterpret_cast<const __m128i*>(p + x)); };
+  for (; x + 16 <= rb; x += 16) {  // 16 bases' four qualities interleaved
+    const __m128i vq = load(b.read_q), vi = uniform_gaps_ ? gi : load(b.read_i);
+    const __m128i vd = uniform_gaps_ ? gd : load(b.read_d), vc = uniform_gaps_ ? gc : load(b.read_c);
+    const __m128i qi0 = _mm_unpacklo_epi8(vq, vi), qi1 = _mm_unpackhi_epi8(vq, vi);
+    const __m128i dc0 = _mm_unpacklo_epi8(vd, vc), dc1 = _mm_unpackhi_epi8(vd, vc);
+    __m128i* o = reinterpret_cast<__m128i*>(q + x);
+    _mm_store_si128(o, _mm_unpacklo_epi16(qi0, dc0));
+    _mm_store_si128(o + 1, _mm_unpackhi_epi16(qi0, dc0));
+    _mm_store_si128(o + 2, _mm_unpacklo_epi16(qi1, dc1));
+    _mm_store_si128(o + 3, _mm_unpackhi_epi16(qi1, dc1));
+  }
+  for (; x < rb; ++x)
+    q[x] = uniform_gaps_ ? uchar4{b.read_q[x], gap_ins_, gap_del_, gap_gcp_}
+                         : uchar4{b.read_q[x], b.read_i[x], b.read_d[x], b.read_c[x]};
+  return BV_OK;
+}
+
 // Inputs: the byte arrays and offsets go to the device as soon as the batch
 // is validated, so the copies run while the host plans the launches.
 bv_status Engine::upload_inputs(const bv_region_batch& b) {
@@ -479,22 +551,35 @@ bv_status Engine::upload_inputs(const bv_region_batch& b) {
   n_read_bytes_ = b.num_reads > 0 ? b.read_offsets[b.num_reads] : 0;
   n_hap_bytes_ = b.num_haps > 0 ? b.hap_offsets[b.num_haps] : 0;
   const size_t rb = (size_t)std::max<int64_t>(n_read_bytes_, 1);
-  BV_CUDA(d_read_bases_.reserve(rb + 16), "alloc reads");  // tail padding for the k-mer kernel's word loads
   // uniform gap penalties: no per-base i, d, c arrays to copy (see bv_region_batch)
   uniform_gaps_ = !b.read_i && !b.read_d && !b.read_c;
   gap_ins_ = b.gap_ins;
   gap_del_ = b.gap_del;
   gap_gcp_ = b.gap_gcp;
-  BV_CUDA(d_q_.reserve(rb), "alloc q");
-  if (!uniform_gaps_) {
-    BV_CUDA(d_i_.reserve(rb), "alloc i");
-    BV_CUDA(d_d_.reserve(rb), "alloc d");
-    BV_CUDA(d_c_.reserve(rb), "alloc c");
+  small_in_ = 5 * rb + (size_t)n_hap_bytes_ + sizeof(int64_t) * (size_t)(n_reads_ + n_haps_ + 2) + 2048 <= kStageBytes;
+  if (small_in_) return stage_inputs(b);
+  // one allocation for all of them: a new context's first call, and one that grows its buffers, pays for
+  // one instead of nine
+  size_t total = 0;
+  for (int pass = 0; pass < 2; ++pass) {
+    if (pass == 1) BV_CUDA(d_inputs_.reserve(total), "alloc inputs");
+    total = 0;
+    auto piece = [&](DevBuf& dev, size_t bytes) {
+      if (pass == 1) dev.view(d_inputs_.as<unsigned char>() + total);
+      total += (bytes + 255) / 256 * 256;
+    };
+    piece(d_read_bases_, rb + 16);  // tail padding for the k-mer kernel's word loads
+    piece(d_q_, rb);
+    if (!uniform_gaps_) {
+      piece(d_i_, rb);
+      piece(d_d_, rb);
+      piece(d_c_, rb);
+    }
+    piece(d_quals4_, rb * 4);
+    piece(d_read_off_, sizeof(int64_t) * (n_reads_ + 1));
+    piece(d_hap_bases_, (size_t)std::max<int64_t>(n_hap_bytes_, 1));
+    piece(d_hap_off_, sizeof(int64_t) * (n_haps_ + 1));
   }
-  BV_CUDA(d_quals4_.reserve(rb * 4), "alloc quals");
-  BV_CUDA(d_read_off_.reserve(sizeof(int64_t) * (n_reads_ + 1)), "alloc read offsets");
-  BV_CUDA(d_hap_bases_.reserve((size_t)std::max<int64_t>(n_hap_bytes_, 1)), "alloc haps");
-  BV_CUDA(d_hap_off_.reserve(sizeof(int64_t) * (n_haps_ + 1)), "alloc hap offsets");
   BV_CUDA(cudaEventRecord(ev_[0], stream_), "event");
   // Offsets are copied verbatim; the byte arrays are copied from index 0 so
   // offsets index them directly.
@@ -522,8 +607,20 @@ bv_status Engine::upload_inputs(const bv_region_batch& b) {
 // qualities.  Nothing here waits for the copies; run() reads the copy time
 // once its own synchronisation has passed.
 bv_status Engine::upload_plan() {
-  BV_CUDA(d_units_.reserve(sizeof(Unit) * std::max<size_t>(units_.size(), 1)), "alloc units");
-  BV_CUDA(d_out_.reserve(sizeof(double) * (size_t)std::max<int64_t>(n_results_, 1)), "alloc results");
+  bool units_staged = false;
+  if (small_in_) {
+    const size_t bytes = sizeof(Unit) * units_.size();
+    if (void* p = stage_piece(std::max<size_t>(bytes, 1), d_units_)) {
+      if (bytes) std::memcpy(p, units_.data(), bytes);
+      units_staged = true;
+    }
+    BV_CUDA(cudaEventRecord(ev_[0], stream_), "event");
+    BV_CUDA(cudaMemcpyAsync(d_stage_.get(), h_stage_, stage_used_, cudaMemcpyHostToDevice, stream_), "H2D");
+  }
+  if (!units_staged) BV_CUDA(d_units_.reserve(sizeof(Unit) * std::max<size_t>(units_.size(), 1)), "alloc units");
+  small_out_ = sizeof(double) * (size_t)n_results_ <= kSmallOutBytes;
+  if (small_out_) d_out_.view(d_counters_.as<unsigned char>() + kCountersBytes);
+  else BV_CUDA(d_out_.reserve(sizeof(double) * (size_t)std::max<int64_t>(n_results_, 1)), "alloc results");
   BV_CUDA(d_rescue_.reserve(sizeof(PairRef) * (size_t)std::max<int64_t>(n_results_, 1)), "alloc rescue list");
   // strip-boundary buffers for the multi-strip launches
   size_t need32 = 0;
@@ -533,7 +630,7 @@ bv_status Engine::upload_plan() {
   const size_t need64 = std::max((size_t)rescue_plan_.grid * (kThreadsPerBlock / kWarp) * (size_t)rescue_plan_.bnd_cols,
                                  (size_t)long_plan_.grid * (size_t)long_plan_.bnd_cols) * 4 * sizeof(double);
   BV_CUDA(d_bnd64_.reserve(need64), "alloc FP64 boundary buffers");
-  if (!units_.empty())
+  if (!units_.empty() && !units_staged)
     BV_CUDA(cudaMemcpyAsync(d_units_.get(), units_.data(), sizeof(Unit) * units_.size(), cudaMemcpyHostToDevice,
                             stream_), "H2D");
   if (!f64_items_.empty())
@@ -543,7 +640,8 @@ bv_status Engine::upload_plan() {
     BV_CUDA(cudaMemcpyAsync(d_rescue_.as<PairRef>() + (std::max<int64_t>(n_results_, 1) - (int64_t)f64_long_items_.size()),
                             f64_long_items_.data(), sizeof(PairRef) * f64_long_items_.size(), cudaMemcpyHostToDevice,
                             stream_), "H2D");
-  if (uniform_gaps_)
+  if (small_in_) {  // packed in the image
+  } else if (uniform_gaps_)
     BV_CUDA(launch_pack_quals_uniform(d_q_.as<uint8_t>(), gap_ins_, gap_del_, gap_gcp_, d_quals4_.as<uchar4>(),
                                       n_read_bytes_, sms_, stream_), "pack quals");
   else
@@ -698,11 +796,11 @@ bv_status Engine::run(bv_phmm_stats* stats) {
   return finish(stats);
 }
 
-bv_status Engine::launch() {
+bv_status Engine::launch(int64_t n_out) {
   if (!staged_) return fail(BV_ERR_INVALID_ARG, "no staged batch");
   BV_CUDA(cudaSetDevice(opt_.device), "cudaSetDevice");
   run_t0_ = std::chrono::steady_clock::now();
-  if (!h_counters_) BV_CUDA(cudaMallocHost(reinterpret_cast<void**>(&h_counters_), sizeof(Counters)), "pinned counters");
+  if (bv_status hs = reserve_host(); hs != BV_OK) return hs;
   // The first run of a staged batch launches directly; later runs replay a
   // captured graph of the same launch sequence.
   if (runs_since_stage_ == 0 || !graph_exec_) {
@@ -728,8 +826,9 @@ bv_status Engine::launch() {
   }
   ++runs_since_stage_;
   // page-locked destination: the copy is queued, the host goes on
-  BV_CUDA(cudaMemcpyAsync(h_counters_, d_counters_.get(), sizeof(Counters), cudaMemcpyDeviceToHost, stream_),
-          "counters D2H");
+  BV_CUDA(cudaMemcpyAsync(h_counters_, d_counters_.get(),
+                          n_out > 0 ? kCountersBytes + sizeof(double) * (size_t)n_out : sizeof(Counters),
+                          cudaMemcpyDeviceToHost, stream_), "counters D2H");
   return BV_OK;
 }
 
@@ -820,14 +919,20 @@ bv_status Engine::compute(const bv_region_batch& b, double* out, bv_phmm_stats* 
   }
   bv_status s = stage(b, false);  // run() synchronises before this call returns
   if (s != BV_OK) return s;
-  s = run(stats);
+  s = launch(small_out_ ? n_results_ : 0);
+  if (s == BV_OK) s = finish(stats);
   if (s != BV_OK) {
     cudaStreamSynchronize(stream_);  // no copy from the caller's arrays outlives the call
     return s;
   }
   const auto t1 = std::chrono::steady_clock::now();
-  s = fetch(out, n_results_);
-  if (s != BV_OK) return s;
+  if (small_out_) {
+    if (n_results_ > 0)
+      std::memcpy(out, reinterpret_cast<unsigned char*>(h_counters_) + kCountersBytes, sizeof(double) * (size_t)n_results_);
+  } else {
+    s = fetch(out, n_results_);
+    if (s != BV_OK) return s;
+  }
   if (stats) {
     const auto t2 = std::chrono::steady_clock::now();
     stats->ms_d2h = std::chrono::duration<double, std::milli>(t2 - t1).count();

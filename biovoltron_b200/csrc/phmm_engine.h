@@ -15,7 +15,8 @@
 
 namespace bvphmm {
 
-// Grow-only device allocation.
+// Grow-only device allocation, or (view) a place in another buffer until the
+// next reserve().
 class DevBuf {
  public:
   DevBuf() = default;
@@ -24,13 +25,15 @@ class DevBuf {
   ~DevBuf() { release(); }
   cudaError_t reserve(size_t bytes);
   void release();
+  void view(void* p) { p_ = p; }
   void* get() const { return p_; }
   template <typename T> T* as() const { return static_cast<T*>(p_); }
   size_t capacity() const { return cap_; }
 
  private:
-  void* p_ = nullptr;
-  size_t cap_ = 0;
+  void* p_ = nullptr;    // own_, or the place viewed
+  void* own_ = nullptr;
+  size_t cap_ = 0;       // of own_
 };
 
 // Launch parameters of one rows-per-lane bin (single-strip FP32 full DP),
@@ -139,7 +142,9 @@ class Engine {
 
   bv_status stage(const bv_region_batch& b, bool wait = true);
   bv_status run(bv_phmm_stats* stats);  // launch + finish
-  bv_status launch();                    // queue one run of the staged batch; does not wait
+  // queue one run of the staged batch and the copy of its counters (and, for results that lie behind
+  // them, of the first n_out results) to page-locked memory; does not wait
+  bv_status launch(int64_t n_out = 0);
   bv_status finish(bv_phmm_stats* stats);  // wait for the queued run, check it, fill stats
   bv_status fetch(double* out, int64_t n);
   bv_status fetch_async(double* out, int64_t n);  // queued behind the run; finish() or a sync waits for it
@@ -207,6 +212,7 @@ class Engine {
   int64_t* chunk_offsets() const { return h_chunk_off_; }
   bv_status plan(const bv_region_batch& b);
   bv_status upload_inputs(const bv_region_batch& b);
+  bv_status stage_inputs(const bv_region_batch& b);
   bv_status upload_plan();
   bv_status enqueue_kernels(bool capturing);
   bv_status enqueue_plans(bool capturing, bool f64, KernelParams& p);
@@ -267,7 +273,15 @@ class Engine {
   bool staged_ = false;
   float ms_h2d_ = 0;
   bool h2d_time_pending_ = false;  // ms_h2d_ is read after the next synchronisation
-  Counters* h_counters_ = nullptr;  // page-locked copy of the device counters
+  // Page-locked: the device counters' copy, small results behind it (kCountersBytes on), and the image of a
+  // small batch's inputs (h_stage_), which goes to the device (d_stage_) as one copy.
+  Counters* h_counters_ = nullptr;
+  unsigned char* h_stage_ = nullptr;
+  DevBuf d_stage_, d_inputs_;  // the inputs' places on the device: of a small batch, of a larger one
+  size_t stage_used_ = 0;
+  bool small_in_ = false, small_out_ = false;
+  bv_status reserve_host();
+  void* stage_piece(size_t bytes, DevBuf& dev);
   int64_t* h_chunk_off_ = nullptr;  // page-locked rebased offsets of the chunk this context stages
   int64_t chunk_off_cap_ = 0;
   std::chrono::steady_clock::time_point run_t0_{};
