@@ -468,8 +468,23 @@ bv_status Engine::plan(const bv_region_batch& b) {
       long_block_ *= 2;
     long_smem_ = long_smem_bytes(rp.hap_bytes, long_block_);
     if (long_smem_ <= 227 * 1024) {
-      BV_CUDA(prepare_long(long_smem_, long_block_), "kernel attribute");
-      long_plan_.grid = (int)std::min<int64_t>(n_long, (int64_t)sms_ * std::max(1, long_blocks_per_sm(long_smem_, long_block_)));
+      // A cluster of blocks a pair: the largest that leaves every pair a cluster of its own (a second round
+      // of clusters costs more than their width saves) and every block strips.  FP64 pass of reads of up to
+      // 10 kb with 1 / 2 / 4 / 8 blocks a pair, ms: 8 pairs 8.4 / - / - / 2.8, 20 pairs 9.5 / 5.5 / 3.4 / 5.6, 40
+      // pairs 11.1 / 6.8 / 8.4 / 7.6 (74, 33 and 15 clusters of 2, 4 and 8 run at once), 148 pairs 11.8 / 11.5
+      // / 15.4 / 25.0.
+      long_cluster_ = 1;
+      int64_t teams = (int64_t)sms_ * std::max(1, long_blocks_per_sm(long_smem_, long_block_));
+      for (int c = kLongMaxBlocks; c > 1 && long_block_ == 16 && !long_set_; c /= 2) {
+        if (8 * c >= strips) continue;
+        const int active = long_clusters(long_smem_, long_block_, c);
+        if (n_long > active) continue;
+        long_cluster_ = c;
+        teams = active;
+        break;
+      }
+      BV_CUDA(prepare_long(long_smem_, long_block_, long_cluster_), "kernel attribute");
+      long_plan_.grid = (int)std::min<int64_t>(n_long, teams) * long_cluster_;
       long_plan_.hap_bytes = rp.hap_bytes;
       long_plan_.bnd_cols = rp.bnd_cols;
       long_plan_.f64 = true;
@@ -771,7 +786,7 @@ bv_status Engine::enqueue_kernels(bool capturing) {
       KernelParams q = p;
       q.hap_bytes = long_plan_.hap_bytes;
       q.bnd_cols = long_plan_.bnd_cols;
-      BV_CUDA(launch_forward_long(q, long_plan_.grid, long_smem_, long_block_, stream_), "FP64 long-read launch");
+      BV_CUDA(launch_forward_long(q, long_plan_.grid, long_smem_, long_block_, long_cluster_, stream_), "FP64 long-read launch");
     }
     BV_CUDA(launch_f64(0, p, lp.grid, stream_), "FP64 forward launch");
     p.cells_ctr = nullptr;

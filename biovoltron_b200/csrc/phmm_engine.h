@@ -259,6 +259,7 @@ class Engine {
   int long_warps_ = kLongWarps;
   bool long_set_ = false;
   int long_block_ = kLongWarps;
+  int long_cluster_ = 1;  // blocks per pair
   int long_rows() const { return long_set_ ? long_warps_ * 128 : kF64ShortMax + 1; }
   int long_smem_ = 0;
   int64_t n_results_ = 0;

@@ -49,9 +49,12 @@ cudaError_t launch_f64(int rt, const KernelParams& p, int grid, cudaStream_t st)
 constexpr int kLongWarps = 4;
 bool long_warps_valid(int warps);
 int long_smem_bytes(int hap_bytes, int warps);
-cudaError_t prepare_long(int smem, int warps);
+// `blocks` > 1 (16 warps each): clusters of that many blocks per pair, grid a multiple of it.
+constexpr int kLongMaxBlocks = 8;
+cudaError_t prepare_long(int smem, int warps, int blocks);
 int long_blocks_per_sm(int smem, int warps);
-cudaError_t launch_forward_long(const KernelParams& p, int grid, int smem, int warps, cudaStream_t st);
+int long_clusters(int smem, int warps, int blocks);  // clusters that run at once
+cudaError_t launch_forward_long(const KernelParams& p, int grid, int smem, int warps, int blocks, cudaStream_t st);
 
 // Variant table: (precision, rows per lane, multi-strip, two haplotypes per
 // warp).  Paired variants exist for FP32 single strip only.

@@ -29,13 +29,20 @@
 // column) and falls by at most 2^-500, so nothing that matters leaves the
 // range whatever the length of the read.
 //
+// Few pairs: a cluster of up to eight blocks takes a pair, its warps numbered
+// through, so that 16 x blocks strips run at once; the boundary rows between
+// two blocks go through the producer's global buffer like a group's last row,
+// with the chunk counter in global memory (release / acquire).  The cluster
+// guarantees that its blocks run at the same time; pairs are dealt to clusters
+// in snake order, longest first, and the blocks meet at the end of each.
+//
 // A pair with a row that cannot be folded, or whose result is not a positive
 // finite number, is handed back to k_f64_list (its list entry marked), which
 // runs after this kernel.
 //
 // Bound by the issue slots of the FP64 instructions (two each): 40 reads of up to
-// 10 kb take 12.0 ms with 16 warps a pair (28 with 4), 2,000 of them 77 ms, where
-// the unscaled form with four warps, emissions in shared memory and one scale
+// 10 kb take 6.8 ms with two blocks of 16 warps a pair (11 with one, 28 with four
+// warps), 8 of them 2.8 ms with eight blocks, 2,000 of them 77 ms, where the unscaled form with four warps, emissions in shared memory and one scale
 // a group of strips took 58 and 169.
 //
 // The haplotype codes are staged once per pair for all warps.  Every wait is
@@ -78,9 +85,8 @@ struct LongLayout {
 
 struct LongShared {  // at LongLayout::kScalars
   long long item;
-  int done;  // chunks the group-ending strips have written to the boundary buffer
+  int done;  // chunks the block's last warp has written to the boundary buffer
   int fail;
-  int redo;  // the pair goes back to k_f64_list
 };
 
 struct LongIO {
@@ -92,8 +98,12 @@ struct LongIO {
   int* chout_e;
   uint64_t* out_full;
   uint64_t* out_empty;
-  double2* bnd;         // the block's boundary buffer and its chunks' exponents
+  double2* bnd;         // the block's boundary buffer, its chunks' exponents and (clusters) how many are written
   int* bnd_e;
+  int* bnd_done;
+  const double2* src;   // the buffer warp 0 reads: the block's own, or the block's before it in the cluster
+  const int* src_e;
+  const int* src_done;
   double2* stage;       // the warp's staged chunk
 };
 enum LongMode { kZero = 0, kChan = 1, kGlobal = 2 };  // where a strip's input comes from (kZero: none), its output goes
@@ -107,16 +117,33 @@ __device__ __forceinline__ void wait_flip(uint64_t* mb, unsigned& bits, int i, v
   if (!*fail && !mbar_wait(mb, (bits >> i) & 1u)) *fail = 1;
   bits ^= 1u << i;
 }
-// Waits until the group-ending strips have written `need` chunks.
-__device__ __forceinline__ void wait_done(volatile int* done, int need, volatile int* fail) {
+// Waits until `need` chunks of a boundary buffer have been written (CL: by a
+// block of the cluster, the count in global memory).
+template <bool CL>
+__device__ __forceinline__ void wait_done(const int* done, int need, volatile int* fail) {
   for (unsigned it = 0; it < kBulkWaitLimit && !*fail; ++it) {
-    if (*done >= need) {
-      __threadfence_block();
+    int n;
+    if (CL) asm volatile("ld.acquire.gpu.global.s32 %0, [%1];" : "=r"(n) : "l"(done) : "memory");
+    else n = *(const volatile int*)done;
+    if (n >= need) {
+      if (!CL) __threadfence_block();
       return;
     }
     __nanosleep(100);
   }
   *fail = 1;
+}
+template <bool CL>
+__device__ __forceinline__ void post_done(int* done, int n) {
+  if (CL) {
+    asm volatile("st.release.gpu.global.s32 [%0], %1;" ::"l"(done), "r"(n) : "memory");
+  } else {
+    __threadfence_block();
+    *(volatile int*)done = n;
+  }
+}
+__device__ __forceinline__ void cluster_sync() {
+  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 
 // Exponent of a non-negative value (kNoExp for zero and below 2^-1022).
@@ -177,6 +204,7 @@ __device__ __forceinline__ void run_chunk(const F64Rows<kLongRT>& w, F64State<kL
 // 31) are the parities of the channel barriers' next phases.  Returns the
 // strip's exponent; sumM, sumX: lane 31's last row summed over the haplotype's
 // columns (last strip only).
+template <bool CL>
 __device__ __forceinline__ int run_strip_long(const F64Rows<kLongRT>& w, const unsigned char* __restrict__ hc_lane, int H,
                                               int nch, int lane, LongMode in, LongMode out, bool last, int in_done,
                                               int out_done, int l0, int j0, double y0, int y0_exp, const LongIO& io,
@@ -206,13 +234,13 @@ __device__ __forceinline__ int run_strip_long(const F64Rows<kLongRT>& w, const u
     __syncwarp();
     if (lane == 0) mbar_arrive(io.in_empty);
   } else if (in == kGlobal) {
-    if (lane == 0) wait_done(&sh.done, in_done + min(2, nch), fail);
+    if (lane == 0) wait_done<CL>(io.src_done, in_done + min(2, nch), fail);
     __syncwarp();
-    carry = __ldcg(io.bnd + lane);
-    carry_e = __ldcg(io.bnd_e);
+    carry = __ldcg(io.src + lane);
+    carry_e = __ldcg(io.src_e);
     if (nch > 1) {
-      ahead = __ldcg(io.bnd + 32 + lane);
-      ahead_e = __ldcg(io.bnd_e + 1);
+      ahead = __ldcg(io.src + 32 + lane);
+      ahead_e = __ldcg(io.src_e + 1);
     }
   }
   if (!first) E = carry_e;
@@ -236,10 +264,10 @@ __device__ __forceinline__ int run_strip_long(const F64Rows<kLongRT>& w, const u
         nx_e = ahead_e;
       }
       if (k + 2 < nch) {
-        if (lane == 0) wait_done(&sh.done, in_done + k + 3, fail);
+        if (lane == 0) wait_done<CL>(io.src_done, in_done + k + 3, fail);
         __syncwarp();
-        ahead = __ldcg(io.bnd + 32 * (k + 2) + lane);
-        ahead_e = __ldcg(io.bnd_e + k + 2);
+        ahead = __ldcg(io.src + 32 * (k + 2) + lane);
+        ahead_e = __ldcg(io.src_e + k + 2);
       }
     }
     {
@@ -306,8 +334,7 @@ __device__ __forceinline__ int run_strip_long(const F64Rows<kLongRT>& w, const u
         mbar_arrive(io.out_full + slot);
       } else if (out == kGlobal) {
         io.bnd_e[k] = E;
-        __threadfence_block();
-        *(volatile int*)&sh.done = out_done + k + 1;
+        post_done<CL>(io.bnd_done, out_done + k + 1);
       }
     }
     __syncwarp();  // lane 0 has read the staged entries
@@ -315,9 +342,9 @@ __device__ __forceinline__ int run_strip_long(const F64Rows<kLongRT>& w, const u
   return E;
 }
 
-// One block of K warps per long pair (the FP64 list's long part, read from
-// the list's far end).
-template <int K>
+// A block of K warps (CL: a cluster of such blocks) per long pair: the FP64
+// list's long part, read from the list's far end.
+template <int K, bool CL>
 __global__ void __launch_bounds__(K * kWarp, 16 / K) k_forward_long(KernelParams p) {
   using L = LongLayout<K>;
   extern __shared__ __align__(16) unsigned char smem[];
@@ -346,28 +373,57 @@ __global__ void __launch_bounds__(K * kWarp, 16 / K) k_forward_long(KernelParams
     io.out_full = full + w * kLongSlots;
     io.out_empty = empty + w * kLongSlots;
   }
-  // bnd_cols rows of 32 bytes: 16 bytes an entry, the exponents behind them
-  io.bnd = reinterpret_cast<double2*>(p.bnd) + (size_t)blockIdx.x * p.bnd_cols * 2;
+  // the blocks of a pair: rank in the cluster, their number, the cluster's and the clusters' number
+  int rank = 0, blocks = 1;
+  if (CL) {
+    asm("mov.u32 %0, %%cluster_ctarank;" : "=r"(rank));
+    asm("mov.u32 %0, %%cluster_nctarank;" : "=r"(blocks));
+  }
+  const int team = blockIdx.x / blocks, teams = gridDim.x / blocks;
+  const int W = K * blocks, gw = rank * K + w;  // warps per pair, this warp's number
+  // a buffer: bnd_cols rows of 32 bytes: 16 bytes an entry, the exponents behind them, the count at the end
+  auto buffer = [&](int block) { return reinterpret_cast<double2*>(p.bnd) + (size_t)block * p.bnd_cols * 2; };
+  auto count_of = [&](double2* buf) { return reinterpret_cast<int*>(buf + 2 * p.bnd_cols) - 4; };
+  io.bnd = buffer(blockIdx.x);
   io.bnd_e = reinterpret_cast<int*>(io.bnd + p.bnd_cols);
+  io.bnd_done = CL ? count_of(io.bnd) : &sh.done;
+  const int before = (rank + blocks - 1) % blocks;  // whose last warp feeds this block's first
+  double2* const src = buffer(team * blocks + before);
+  io.src = src;
+  io.src_e = reinterpret_cast<const int*>(src + p.bnd_cols);
+  io.src_done = CL ? count_of(src) : &sh.done;
+  if (threadIdx.x == 0) *io.bnd_done = 0;
+  int in_base = 0, out_base = 0;  // chunks of earlier pairs (the counts run on over the pairs)
   io.stage = reinterpret_cast<double2*>(base) + w * 32;
   unsigned fph = 0;                        // lane 0: input channel slots' next full phases
   unsigned eph = (1u << kLongSlots) - 1u;  // lane 31: output slots; their first wait passes at once
   volatile int* fail = &sh.fail;
   const DeviceBatch& b = p.batch;
   const unsigned long long n_long = min(p.ctr->rescue_long_count, (unsigned long long)p.rescue_cap);
-  for (;;) {
-    if (threadIdx.x == 0) sh.item = (long long)atomicAdd(&p.ctr->rescue_long_next, 1ull);
-    __syncthreads();
-    const long long wi = sh.item;
-    if (wi >= (long long)n_long || *fail) break;
-    const PairRef pr = p.rescue[p.rescue_cap - 1 - wi];
+  __syncwarp();
+  if (CL) cluster_sync();  // every count is zero
+  for (long long round = 0;; ++round) {
+    long long wi;
+    if (CL) {
+      // dealt in snake order; every block of a cluster takes the same pairs, and leaves after the same one
+      wi = round * teams + (round & 1 ? teams - 1 - team : team);
+      if (round * teams >= (long long)n_long) break;
+      if (wi >= (long long)n_long) continue;
+    } else {
+      if (threadIdx.x == 0) sh.item = (long long)atomicAdd(&p.ctr->rescue_long_next, 1ull);
+      __syncthreads();
+      wi = sh.item;
+      if (wi >= (long long)n_long || *fail) break;
+    }
+    PairRef pr = p.rescue[p.rescue_cap - 1 - wi];
+    if (CL && pr.read < 0) pr.read = ~pr.read;  // another block of the cluster is through and has handed it back
     const int64_t ro = b.read_off[pr.read], ho = b.hap_off[pr.hap];
     const int R = (int)(b.read_off[pr.read + 1] - ro), H = (int)(b.hap_off[pr.hap + 1] - ho);
     const uchar4* quals = b.read_quals + ro;
     const uint8_t* bases = b.read_bases + ro;
     if (H == 0 || R == 0) {
       if (threadIdx.x == 0) p.out[pr.out] = -INFINITY;
-      __syncthreads();
+      if (!CL) __syncthreads();
       continue;
     }
     const int nch = (H + kWarp - 1 + 31) / 32;
@@ -377,46 +433,63 @@ __global__ void __launch_bounds__(K * kWarp, 16 / K) k_forward_long(KernelParams
     const int y0_exp = kF64InitExp - kTop;
     const double y0 = ldexp(p.tables->init_d, -y0_exp) / (double)H;
     stage_hap_block(b.hap_bases + ho, H, hc, 32 * nch + kHapLead);
-    if (threadIdx.x == 0) {
-      sh.done = 0;
-      sh.redo = 0;
-    }
     __syncthreads();
-    for (int s = w; s < nstrips; s += K) {
+    for (int s = gw; s < nstrips; s += W) {
       F64Rows<kLongRT> rw;
-      const bool fold =
-          f64_setup<kLongRT, false>(p.tables, quals, bases, R, s * kStrip + lane * kLongRT - pad, rw);
-      if (!fold) sh.redo = 1;
+      // a row that cannot be folded makes the result NaN
+      if (!f64_setup<kLongRT, false>(p.tables, quals, bases, R, s * kStrip + lane * kLongRT - pad, rw))
+        rw.em[0] = rw.ex[0] = __longlong_as_double(0x7ff8000000000000ll);
       const LongMode in = s == 0 ? kZero : (w == 0 ? kGlobal : kChan);
       const bool last = s == nstrips - 1;
       const LongMode out = last ? kZero : (w == K - 1 ? kGlobal : kChan);
       double sumM, sumX;
-      const int E = run_strip_long(rw, hc + kHapLead - lane, H, nch, lane, in, out, last, (s / K - 1) * nch,
-                                   (s / K) * nch, pad / kLongRT, pad % kLongRT, y0, y0_exp, io, sh, fph, eph, sumM, sumX);
+      const int E = run_strip_long<CL>(rw, hc + kHapLead - lane, H, nch, lane, in, out, last,
+                                       in_base + (s > 0 ? (s - 1) / W * nch : 0), out_base + s / W * nch,
+                                       pad / kLongRT, pad % kLongRT, y0, y0_exp, io, sh, fph, eph, sumM, sumX);
       if (last && lane == kWarp - 1) {
         const double pmx = p.tables->const_mode ? p.tables->cd[1] : p.tables->ph2pr_d[quals[R - 1].y & kQualMask];
         const double res = sumM + pmx * sumX;
-        if (!(res > 0.0 && isfinite(res))) {
-          sh.redo = 1;
-        } else if (!*(volatile int*)&sh.redo) {
+        if (res > 0.0 && isfinite(res)) {
           write_result<double>(p, pr.read, pr.hap, pr.out, res, E);
           if (p.cells_ctr) atomicAdd(p.cells_ctr, (unsigned long long)R * (unsigned long long)H);
+        } else {
+          // handed back: the entry is marked (read index complemented) for k_f64_list
+          p.rescue[p.rescue_cap - 1 - wi].read = ~pr.read;
         }
       }
     }
-    __syncthreads();
-    // handed back: the entry is marked (read index complemented) for k_f64_list
-    if (threadIdx.x == 0 && sh.redo) p.rescue[p.rescue_cap - 1 - wi].read = ~pr.read;
+    // strips but the last that end in a block's last warp: those numbers W i + (rank + 1) K - 1 < nstrips - 1
+    auto ended = [&](int r) { return (max(0, nstrips - 1 - ((r + 1) * K - 1)) + W - 1) / W * nch; };
+    in_base += ended(before);
+    out_base += ended(rank);
+    __syncwarp();
+    if (CL) cluster_sync();  // the buffers are read
+    else __syncthreads();
   }
   if (threadIdx.x == 0 && *fail) atomicOr(&p.ctr->status, 8ull);
 }
 
-template <int K>
-int blocks_for(int smem) {
-  int nb = 0;
-  if (raise_dynamic_smem(reinterpret_cast<const void*>(&k_forward_long<K>), smem) != cudaSuccess) return 0;
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_forward_long<K>, K * kWarp, smem) != cudaSuccess) return 0;
-  return nb;
+template <int K, bool CL>
+const void* kernel() { return reinterpret_cast<const void*>(&k_forward_long<K, CL>); }
+const void* kernel_of(int warps, int blocks) {
+  if (blocks > 1) return warps == 16 ? kernel<16, true>() : nullptr;
+  return warps == 2 ? kernel<2, false>() : warps == 4 ? kernel<4, false>() : warps == 8 ? kernel<8, false>() : kernel<16, false>();
+}
+cudaLaunchConfig_t config_of(int grid, int smem, int warps, int blocks, cudaStream_t st, cudaLaunchAttribute* attr) {
+  cudaLaunchConfig_t c{};
+  c.gridDim = dim3(grid);
+  c.blockDim = dim3(warps * kWarp);
+  c.dynamicSmemBytes = (size_t)smem;
+  c.stream = st;
+  if (blocks > 1) {
+    attr->id = cudaLaunchAttributeClusterDimension;
+    attr->val.clusterDim.x = (unsigned)blocks;
+    attr->val.clusterDim.y = 1;
+    attr->val.clusterDim.z = 1;
+    c.attrs = attr;
+    c.numAttrs = 1;
+  }
+  return c;
 }
 }  // namespace
 
@@ -429,24 +502,30 @@ int long_smem_bytes(int hap_bytes, int warps) {
                                     : LongLayout<16>::kBytes);
 }
 
-cudaError_t prepare_long(int smem, int warps) {
-  const void* f = warps == 2   ? reinterpret_cast<const void*>(&k_forward_long<2>)
-                  : warps == 4 ? reinterpret_cast<const void*>(&k_forward_long<4>)
-                  : warps == 8 ? reinterpret_cast<const void*>(&k_forward_long<8>)
-                               : reinterpret_cast<const void*>(&k_forward_long<16>);
-  return raise_dynamic_smem(f, smem);
-}
+cudaError_t prepare_long(int smem, int warps, int blocks) { return raise_dynamic_smem(kernel_of(warps, blocks), smem); }
 
 int long_blocks_per_sm(int smem, int warps) {
-  return warps == 2 ? blocks_for<2>(smem) : warps == 4 ? blocks_for<4>(smem) : warps == 8 ? blocks_for<8>(smem) : blocks_for<16>(smem);
+  int nb = 0;
+  if (prepare_long(smem, warps, 1) != cudaSuccess) return 0;
+  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, kernel_of(warps, 1), warps * kWarp, smem) != cudaSuccess) return 0;
+  return nb;
 }
 
-cudaError_t launch_forward_long(const KernelParams& p, int grid, int smem, int warps, cudaStream_t st) {
-  if (warps == 2) k_forward_long<2><<<grid, 2 * kWarp, smem, st>>>(p);
-  else if (warps == 4) k_forward_long<4><<<grid, 4 * kWarp, smem, st>>>(p);
-  else if (warps == 8) k_forward_long<8><<<grid, 8 * kWarp, smem, st>>>(p);
-  else k_forward_long<16><<<grid, 16 * kWarp, smem, st>>>(p);
-  return cudaGetLastError();
+int long_clusters(int smem, int warps, int blocks) {
+  int n = 0;
+  cudaLaunchAttribute attr{};
+  if (prepare_long(smem, warps, blocks) != cudaSuccess) return 0;
+  const cudaLaunchConfig_t c = config_of(blocks, smem, warps, blocks, nullptr, &attr);
+  if (cudaOccupancyMaxActiveClusters(&n, kernel_of(warps, blocks), &c) != cudaSuccess) return 0;
+  return n;
+}
+
+cudaError_t launch_forward_long(const KernelParams& p, int grid, int smem, int warps, int blocks, cudaStream_t st) {
+  cudaLaunchAttribute attr{};
+  const cudaLaunchConfig_t c = config_of(grid, smem, warps, blocks, st, &attr);
+  KernelParams q = p;
+  void* args[] = {&q};
+  return cudaLaunchKernelExC(&c, kernel_of(warps, blocks), args);
 }
 
 }  // namespace bvphmm

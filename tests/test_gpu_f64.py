@@ -92,10 +92,10 @@ def test_scalar_transitions_with_a_zero(engine, oracle):
                 assert abs(got[k] - want) <= TOL
 
 
-# strip and group edges of the long-read kernel for every block size; few pairs (blocks of 16 warps), more
-# pairs than SMs (8 and 4), unrelated pairs whose mass falls by thousands of binary orders, a read longer
+# strip and group edges of the long-read kernel; few pairs (clusters of four and two blocks of 16 warps, one
+# round of them and two), more pairs (one block a pair), unrelated pairs whose mass falls by thousands of binary orders, a read longer
 # than its haplotype, rows that cannot fold
-@pytest.mark.parametrize("copies", [1, 9, 18])
+@pytest.mark.parametrize("copies", [1, 3, 5, 9, 18])
 def test_long_reads(oracle, copies):
     from biovoltron_b200.pairhmm import PairHMMEngine
     rng = np.random.default_rng(9)
@@ -121,3 +121,15 @@ def test_long_reads(oracle, copies):
     with PairHMMEngine() as e:
         _, st = e.compute_regions(b, with_stats=True)
         assert st["rescued"] > 0
+
+
+def test_long_read_on_eight_blocks(oracle):
+    """Reads of more strips than four blocks have warps, and the strip counts around eight blocks' 128."""
+    from biovoltron_b200.pairhmm import PairHMMEngine
+    rng = np.random.default_rng(10)
+    b = W._build([_pair(rng, n, h) for n, h in ((16383, 1200), (16384, 900), (16500, 700), (8300, 8400), (254, 300))],
+                 "very long reads")
+    with PairHMMEngine(precision="f64") as e:
+        got = e.compute_regions(b)
+        _check(b, got, oracle)
+        assert np.array_equal(e.compute_regions(b), got)
