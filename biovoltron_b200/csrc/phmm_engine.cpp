@@ -51,7 +51,6 @@ void DevBuf::release() {
 }
 
 namespace {
-constexpr int kMaxRowsPerLane = 8;
 // Launch bins: the FP32 variants (variant_index), then FP64 mode's bins of 1 .. 8 rows a lane; reads of
 // several strips go to the FP64 list.
 constexpr int kF64Bin0 = 19;
@@ -331,65 +330,85 @@ bv_status Engine::plan(const bv_region_batch& b) {
     if (opt_.haps_per_warp == 1 || per_unit < 2 || rt < 1 || rt > kTuneBins) return false;
     return opt_.haps_per_warp == 2 || tune_[rt].haps_per_warp == 2;
   };
-  auto variant_of = [&](int64_t rlen) {
-    if (f64_units) return rlen <= kF64ShortMax ? kF64Bin0 + (int)((rlen + 3 + kWarp - 1) / kWarp) : kF64List;
-    // rows of the single-strip FP32 kernel: row 0, the read, the summing row
-    // and one padding row on top (phmm_device.cuh, rows_needed)
-    const int64_t rows = rows_needed((int)std::min<int64_t>(rlen, 1 << 24), true, true);
-    const int64_t rt = (rows + kWarp - 1) / kWarp;
-    return rt <= kMaxRowsPerLane ? variant_index(false, (int)rt, false, pair_rows(rt)) : v_multi;
-  };
+  // A read's bin: rows per lane of the single-strip kernels (row 0, the read, the summing row and one padding
+  // row on top: phmm_device.cuh, rows_needed), kBins for reads of several strips; and the launch it takes.
+  auto bin_of = [](int64_t rlen) { return (int)std::min<int64_t>((rlen + 3 + kWarp - 1) / kWarp, kBins); };
+  int bin_variant[kBins + 1] = {};
+  for (int rt = 1; rt <= kBins; ++rt)
+    bin_variant[rt] = f64_units      ? (rt < kBins ? kF64Bin0 + rt : kF64List)
+                      : rt == kBins ? v_multi
+                                    : variant_index(false, rt, false, pair_rows(rt));
+  // pass over the reads: units per bin and, per region, where its units of each bin start
+  std::vector<uint32_t>* const base = region_base_;
+  for (int rt = 1; rt <= kBins; ++rt) base[rt].clear();
+  int64_t res = 0, bin_units[kBins + 1] = {};
+  std::vector<int64_t>& res_off = region_res_;
+  res_off.assign((size_t)std::max<int64_t>(b.num_regions, 1), 0);
   for (int64_t g = 0; g < b.num_regions; ++g) {
-    const int64_t nh = b.region_haps[g + 1] - b.region_haps[g];
-    const int64_t nr = b.region_reads[g + 1] - b.region_reads[g];
+    const int64_t h0 = b.region_haps[g], nh = b.region_haps[g + 1] - h0;
+    const int64_t r0 = b.region_reads[g], nr = b.region_reads[g + 1] - r0;
+    res_off[g] = res;
+    res += nr * nh;
     if (nh == 0 || nr == 0) continue;
+    // reads and haplotypes are contiguous
+    n_cells_ += (b.read_offsets[r0 + nr] - b.read_offsets[r0]) * (b.hap_offsets[h0 + nh] - b.hap_offsets[h0]);
     const int64_t chunks = (nh + per_unit - 1) / per_unit;
-    for (int64_t r = b.region_reads[g]; r < b.region_reads[g + 1]; ++r) {
+    int64_t cnt[kBins + 1] = {};
+    for (int64_t r = r0; r < r0 + nr; ++r) {
       const int64_t rl = b.read_offsets[r + 1] - b.read_offsets[r];
-      ++bin_reads_[std::min<int64_t>((rows_needed((int)std::min<int64_t>(rl, 1 << 24), true, true) + kWarp - 1) / kWarp, 9) - 1];
+      ++cnt[bin_of(rl)];
+      max_read = std::max(max_read, rl);
       if (rl >= long_rows()) {
         n_long += nh;
         long_rows_sum += nh * rl;
       }
-      const int v = variant_of(rl);
+    }
+    for (int rt = 1; rt <= kBins; ++rt) {
+      if (cnt[rt] == 0) continue;
+      bin_reads_[rt - 1] += cnt[rt];
+      const int v = bin_variant[rt];
       if (v == kF64List) continue;
-      count[v] += chunks;
+      if (base[rt].empty()) base[rt].assign((size_t)b.num_regions, 0);
+      base[rt][g] = (uint32_t)bin_units[rt];
+      bin_units[rt] += cnt[rt] * chunks;
+      count[v] += cnt[rt] * chunks;
       var_max_hap[v] = std::max(var_max_hap[v], region_max_hap[g]);
     }
   }
+  n_results_ = res;
+  for (int rt = 1; rt <= kBins; ++rt)
+    if (bin_units[rt] > UINT32_MAX) return fail(BV_ERR_INVALID_ARG, "too many pairs");
   std::vector<int64_t> start(kMaxVariants + 1, 0);
   for (int v = 0; v < kMaxVariants; ++v) start[v + 1] = start[v] + count[v];
-  if (!all_f64 || f64_units) units_.resize(start[kMaxVariants]);
-  std::vector<int64_t> fill(start.begin(), start.end() - 1);
-  // pass 2: fill units (or FP64 items) in result order within each bucket
-  int64_t res = 0;
-  for (int64_t g = 0; g < b.num_regions; ++g) {
+  // the units, in result order within each bin: on the device (k_make_units, from the region arrays) or, for a
+  // small batch, here; the FP64 list's pairs here
+  n_units_ = !all_f64 || f64_units ? start[kMaxVariants] : 0;
+  unit_haps_ = per_unit;
+  for (int rt = 1; rt <= kBins; ++rt) bin_start_[rt] = base[rt].empty() || n_units_ == 0 ? -1 : start[bin_variant[rt]];
+  const bool lists = all_f64 && (!f64_units || bin_reads_[kBins - 1] > 0);
+  if (small_in_) units_.resize((size_t)n_units_);
+  for (int64_t g = 0; (small_in_ || lists) && g < b.num_regions; ++g) {
     const int64_t h0 = b.region_haps[g], nh = b.region_haps[g + 1] - h0;
-    const int64_t r0 = b.region_reads[g], nr = b.region_reads[g + 1] - r0;
-    const int64_t hap_bases = nh > 0 ? b.hap_offsets[h0 + nh] - b.hap_offsets[h0] : 0;  // haplotypes are contiguous
-    for (int64_t r = r0; r < r0 + nr; ++r) {
+    int64_t out = res_off[g], fill[kBins + 1];
+    for (int rt = 1; rt <= kBins; ++rt) fill[rt] = bin_start_[rt] < 0 ? 0 : bin_start_[rt] + base[rt][g];
+    for (int64_t r = b.region_reads[g]; r < b.region_reads[g + 1]; ++r, out += nh) {
       const int64_t rl = b.read_offsets[r + 1] - b.read_offsets[r];
-      n_cells_ += rl * hap_bases;
-      max_read = std::max(max_read, rl);
-      const int v = variant_of(rl);
-      if (all_f64 && (!f64_units || v == kF64List)) {
+      const int rt = bin_of(rl);
+      if (lists && (!f64_units || rt == kBins)) {
         auto& list = rl >= long_rows() ? f64_long_items_ : f64_items_;
-        for (int64_t k = 0; k < nh; ++k)
-          list.push_back(PairRef{(int32_t)r, (int32_t)(h0 + k), res + (r - r0) * nh + k});
+        for (int64_t k = 0; k < nh; ++k) list.push_back(PairRef{(int32_t)r, (int32_t)(h0 + k), out + k});
         continue;
       }
-      for (int64_t k = 0; k < nh; k += per_unit) {
+      for (int64_t k = 0; small_in_ && k < nh; k += per_unit) {
         Unit u{};
         u.read = (int32_t)r;
         u.hap0 = (int32_t)(h0 + k);
         u.nh = (int32_t)std::min<int64_t>(per_unit, nh - k);
-        u.out0 = res + (r - r0) * nh + k;
-        units_[fill[v]++] = u;
+        u.out0 = out + k;
+        units_[(size_t)fill[rt]++] = u;
       }
     }
-    res += nr * nh;
   }
-  n_results_ = res;
   // launch plans
   int slot = 0;
   for (int v = 0; v < kMaxVariants && (!all_f64 || f64_units); ++v) {
@@ -621,7 +640,7 @@ bv_status Engine::upload_inputs(const bv_region_batch& b) {
 // The plan's device side: work units, result and list buffers, and the packed
 // qualities.  Nothing here waits for the copies; run() reads the copy time
 // once its own synchronisation has passed.
-bv_status Engine::upload_plan() {
+bv_status Engine::upload_plan(const bv_region_batch& b) {
   bool units_staged = false;
   if (small_in_) {
     const size_t bytes = sizeof(Unit) * units_.size();
@@ -632,7 +651,7 @@ bv_status Engine::upload_plan() {
     BV_CUDA(cudaEventRecord(ev_[0], stream_), "event");
     BV_CUDA(cudaMemcpyAsync(d_stage_.get(), h_stage_, stage_used_, cudaMemcpyHostToDevice, stream_), "H2D");
   }
-  if (!units_staged) BV_CUDA(d_units_.reserve(sizeof(Unit) * std::max<size_t>(units_.size(), 1)), "alloc units");
+  if (!units_staged) BV_CUDA(d_units_.reserve(sizeof(Unit) * (size_t)std::max<int64_t>(n_units_, 1)), "alloc units");
   small_out_ = sizeof(double) * (size_t)n_results_ <= kSmallOutBytes;
   if (small_out_) d_out_.view(d_counters_.as<unsigned char>() + kCountersBytes);
   else BV_CUDA(d_out_.reserve(sizeof(double) * (size_t)std::max<int64_t>(n_results_, 1)), "alloc results");
@@ -645,9 +664,42 @@ bv_status Engine::upload_plan() {
   const size_t need64 = std::max((size_t)rescue_plan_.grid * (kThreadsPerBlock / kWarp) * (size_t)rescue_plan_.bnd_cols,
                                  (size_t)long_plan_.grid * (size_t)long_plan_.bnd_cols) * 4 * sizeof(double);
   BV_CUDA(d_bnd64_.reserve(need64), "alloc FP64 boundary buffers");
-  if (!units_.empty() && !units_staged)
+  if (small_in_ && !units_staged && n_units_ > 0)
     BV_CUDA(cudaMemcpyAsync(d_units_.get(), units_.data(), sizeof(Unit) * units_.size(), cudaMemcpyHostToDevice,
                             stream_), "H2D");
+  if (!small_in_ && n_units_ > 0) {
+    // the region arrays in one copy: reads, haplotypes and results before each region, unit bases per bin
+    const size_t ng = (size_t)b.num_regions;
+    MakeUnits m{};
+    m.n_regions = b.num_regions;
+    m.per_unit = unit_haps_;
+    int bins = 0;
+    for (int rt = 1; rt <= kBins; ++rt) {
+      m.column[rt] = bin_start_[rt] < 0 ? -1 : bins;
+      if (bin_start_[rt] >= 0) m.start[bins++] = bin_start_[rt];
+    }
+    const size_t bytes = sizeof(int64_t) * (3 * ng + 2) + sizeof(uint32_t) * ng * (size_t)bins;
+    region_img_.resize(bytes);
+    unsigned char* p = region_img_.data();
+    auto put = [&](const void* src, size_t n) {
+      std::memcpy(p, src, n);
+      p += n;
+    };
+    put(b.region_reads, sizeof(int64_t) * (ng + 1));
+    put(b.region_haps, sizeof(int64_t) * (ng + 1));
+    put(region_res_.data(), sizeof(int64_t) * ng);
+    for (int rt = 1; rt <= kBins; ++rt)
+      if (bin_start_[rt] >= 0) put(region_base_[rt].data(), sizeof(uint32_t) * ng);
+    BV_CUDA(d_regions_.reserve(bytes), "alloc regions");
+    BV_CUDA(cudaMemcpyAsync(d_regions_.get(), region_img_.data(), bytes, cudaMemcpyHostToDevice, stream_), "H2D");
+    m.region_reads = d_regions_.as<int64_t>();
+    m.region_haps = m.region_reads + ng + 1;
+    m.region_res = m.region_haps + ng + 1;
+    m.base = reinterpret_cast<const uint32_t*>(m.region_res + ng);
+    m.read_off = d_read_off_.as<int64_t>();
+    m.units = d_units_.as<Unit>();
+    BV_CUDA(launch_make_units(m, sms_, stream_), "units");
+  }
   if (!f64_items_.empty())
     BV_CUDA(cudaMemcpyAsync(d_rescue_.get(), f64_items_.data(), sizeof(PairRef) * f64_items_.size(),
                             cudaMemcpyHostToDevice, stream_), "H2D");
@@ -678,7 +730,7 @@ bv_status Engine::stage(const bv_region_batch& b, bool wait) {
   if (s != BV_OK) return s;
   s = upload_inputs(b);
   if (s == BV_OK) s = plan(b);
-  if (s == BV_OK) s = upload_plan();
+  if (s == BV_OK) s = upload_plan(b);
   if (s == BV_OK && band_enabled()) s = band_prepare();
   if (s != BV_OK) {
     cudaStreamSynchronize(stream_);

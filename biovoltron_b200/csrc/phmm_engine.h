@@ -213,7 +213,7 @@ class Engine {
   bv_status plan(const bv_region_batch& b);
   bv_status upload_inputs(const bv_region_batch& b);
   bv_status stage_inputs(const bv_region_batch& b);
-  bv_status upload_plan();
+  bv_status upload_plan(const bv_region_batch& b);
   bv_status enqueue_kernels(bool capturing);
   bv_status enqueue_plans(bool capturing, bool f64, KernelParams& p);
   bv_status band_prepare();
@@ -248,7 +248,14 @@ class Engine {
   DevBuf d_units_, d_out_, d_rescue_, d_counters_, d_bnd32_, d_bnd64_, d_f64_items_;
 
   // staged batch
-  std::vector<Unit> units_;
+  std::vector<Unit> units_;  // of a small batch; larger ones' are made on the device
+  int64_t n_units_ = 0;
+  int unit_haps_ = 1;                          // haplotypes per unit
+  int64_t bin_start_[kBins + 1] = {};          // first unit of a bin (-1: the bin has none)
+  std::vector<uint32_t> region_base_[kBins + 1];  // per region, its first unit within the bin (used bins only)
+  std::vector<int64_t> region_res_;            // per region, its first result
+  std::vector<unsigned char> region_img_;
+  DevBuf d_regions_;
   std::vector<PairRef> f64_items_;  // pairs sent straight to FP64 (precision F64)
   std::vector<PairRef> f64_long_items_;  // the long reads among them, ascending cells (the list's far end first)
   std::vector<LaunchPlan> plans_;

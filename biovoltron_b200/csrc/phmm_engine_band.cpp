@@ -48,7 +48,7 @@ BandParams Engine::band_params() const {
   p.hap_table = d_hap_table_.as<uint32_t>();
   p.hap_nib = d_hap_nib_.as<uint32_t>();
   p.units = d_units_.as<Unit>();
-  p.n_units = (long long)units_.size();
+  p.n_units = n_units_;
   p.read_kmers = d_read_kmers_.as<uint32_t>();
   p.feat_hist = d_feat_hist_.as<uint32_t>();
   p.feat_slow = d_feat_slow_.as<int64_t>();
@@ -142,7 +142,7 @@ bv_status Engine::band_prepare() {
   }
   if (bv_status ls = reserve_lanes(std::min(full_bins_, kMaxLanes)); ls != BV_OK) return ls;
   if (need32 > d_bnd32_.capacity()) BV_CUDA(d_bnd32_.reserve(need32), "alloc boundary buffers");
-  BV_CUDA(launch_pairs_from_units(d_units_.as<Unit>(), (long long)units_.size(), d_pair_read_.as<int32_t>(),
+  BV_CUDA(launch_pairs_from_units(d_units_.as<Unit>(), n_units_, d_pair_read_.as<int32_t>(),
                                   d_pair_hap_.as<int32_t>(), sms_, stream_), "pairs");
   return BV_OK;
 }

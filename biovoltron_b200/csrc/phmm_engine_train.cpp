@@ -79,7 +79,7 @@ bv_status Engine::stage_for_labels(const bv_region_batch& b) {
   if (s != BV_OK) return s;
   s = plan(b);
   if (s != BV_OK) return s;
-  s = upload_plan();
+  s = upload_plan(b);
   if (s != BV_OK) return s;
   s = band_prepare();
   if (s != BV_OK) return s;

@@ -9,6 +9,26 @@ namespace bvphmm {
 
 constexpr int kThreadsPerBlock = 128;
 
+// Read-length bins of the full DP: 1 .. 8 rows a lane in one strip, then reads of several strips.
+constexpr int kBins = 9;
+
+// Makes a batch's units from its region arrays: bin rt's units start at
+// start[column[rt]] (column -1: no units), region g's at base[column * n_regions
+// + g] within them, read by read, per_unit haplotypes each.
+struct MakeUnits {
+  const int64_t* region_reads;  // [n_regions + 1]
+  const int64_t* region_haps;   // [n_regions + 1]
+  const int64_t* region_res;    // [n_regions] first result
+  const uint32_t* base;         // [columns][n_regions]
+  const int64_t* read_off;
+  Unit* units;
+  long long n_regions;
+  long long start[kBins];
+  int column[kBins + 1];
+  int per_unit;
+};
+cudaError_t launch_make_units(const MakeUnits& m, int sms, cudaStream_t st);
+
 struct KernelParams {
   DeviceBatch batch;
   const Tables* tables;

@@ -42,3 +42,30 @@ def test_unit_sizes_and_lanes(engine, oracle, n_reads, n_haps, lens):
             for _ in range(3):  # direct launches, then the captured graph with its parallel branches
                 e.run()
                 assert np.array_equal(e.fetch(n), got)
+
+
+# units made on the device (batches over 512 KB of inputs) against those the host fills (small ones): regions
+# without reads or haplotypes, read counts around a warp, haplotype counts around a unit, every bin
+@pytest.mark.parametrize("precision,band", [("auto", False), ("f64", False), ("auto", True)])
+def test_units_made_on_the_device(precision, band):
+    from biovoltron_b200.pairhmm import PairHMMEngine
+    rng = np.random.default_rng(12)
+    lens = [1, 29, 30, 61, 62, 94, 125, 126, 157, 158, 190, 222, 252, 253, 254, 300]
+    regions = []
+    for k in range(160):
+        nr, nh = (0, 1, 31, 32, 33, 70)[k % 6], (0, 1, 2, 7, 8, 9, 17)[k % 7]
+        reads, haps = _region(rng, nr, max(nh, 1), np.roll(lens, k), 330)
+        regions.append((reads, haps[:nh]))
+    b = W._build(regions, "units")
+    assert b.nbytes() > 1 << 20
+    with PairHMMEngine(precision=precision) as e:
+        if band:
+            e.set_band_options(enabled=True, cap_margin=0)
+        got = e.compute_regions(b)
+        parts = [W.subsample_regions(b, range(g, g + 8)) for g in range(0, 160, 8)]
+        assert all(5 * p.read_bases.size + p.hap_bases.size < 400_000 for p in parts)
+        assert np.array_equal(got, np.concatenate([e.compute_regions(p) for p in parts]))
+        n = e.stage(b)
+        for _ in range(2):
+            e.run()
+            assert np.array_equal(e.fetch(n), got)
