@@ -11,12 +11,15 @@
 // renormalised between strips (process_item<double, 4, multi-strip>).
 //
 // Bound by issue: an FP64 instruction takes two slots, and a step of five rows a
-// lane has 28 of them beside 31 others (the emission selects, shuffles, the
-// code's load); the FP64 pipe is 50 % busy.  75 k pairs of 50-250 bases take
-// 3.4 ms, where the unscaled two-strip kernel took 11.0; the rescue of 84
-// pairs of 46 k takes 0.1 instead of 0.28 ms.
+// lane has 28 of them.  The emissions come from a table in shared memory, a
+// load for two rows, where a select in registers costs two instructions a row
+// (31 others a step); a column outside the haplotype then has emission zero,
+// so nothing has to be injected on the way in.  75 k pairs of 50-250 bases
+// take 3.05 ms (selects: 3.4; the unscaled two-strip kernel: 11.0); the rescue
+// of 84 pairs of 46 k takes 0.1 instead of 0.28 ms.
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cstdint>
 
 #include "phmm_f64.cuh"
@@ -25,39 +28,35 @@
 namespace bvphmm {
 namespace {
 
-// The pair (rows set up in w) over its H columns.  Lane 31 returns the
-// summing row's total.
+// The pair (rows set up in w, emissions in el's table) over its H columns.
+// Lane 31 returns the summing row's total.
 template <int RT>
-__device__ __forceinline__ double f64_sweep(const F64Rows<RT>& w, const unsigned char* hc_lane, int H, int l0, int j0,
-                                            double y0, int lane) {
+__device__ __forceinline__ double f64_sweep(const F64Rows<RT>& w, const ELane el, const unsigned char* hc_lane, int H,
+                                            int r0j, double y0) {
   F64State<RT> st;
 #pragma unroll
   for (int j = 0; j < RT; ++j) {
     st.M[j] = 0.0;
     st.X[j] = 0.0;
-    st.Y[j] = (l0 == 0 && lane == 0 && j == j0) ? y0 : 0.0;
+    st.Y[j] = j == r0j ? y0 : 0.0;
   }
-  st.zx = 0.0;  // nothing lies above column 0
-  st.zm = 0.0;
-  auto step = [&](int s, bool ramp) {
-    double dm, dx, dy;
-    f64_cells(w, st, hc_lane[s], dm, dx, dy);
-    if (ramp && lane == l0 && s == l0 - 1) {  // row 0 reaches column 0
-#pragma unroll
-      for (int j = 0; j < RT; ++j)
-        if (j == j0) st.Y[j] = y0;
-    }
-    const double2 z = shfl_up_d2(f64_sums(w, st, dm, dx, dy));
-    st.zx = z.x;
-    st.zm = z.y;
-  };
+  double2 z = shfl_up_d2(f64_sums(w, st, 0.0, 0.0, st.Y[RT - 1]));
+  st.zx = z.x;
+  st.zm = z.y;
   // lane 31's last row (the summing row) takes column H + 1 at step H + 31
-  const int nsteps = H + kWarp;
-  int s = 0;
-#pragma unroll 2
-  for (; s < kWarp; ++s) step(s, true);
-#pragma unroll 4
-  for (; s < nsteps; ++s) step(s, false);
+  const int nsteps = (H + kWarp + 3) / 4 * 4;
+#pragma unroll 1
+  for (int s = 0; s < nsteps; s += 4) {
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      double e[RT], dm, dx, dy;
+      load_emissions<double, RT>(el, (unsigned)hc_lane[s + u] * ETab<double, RT>::kCodeStride, e);
+      f64_column(w, st, [&](int j) { return e[j]; }, dm, dx, dy);
+      z = shfl_up_d2(f64_sums(w, st, dm, dx, dy));
+      st.zx = z.x;
+      st.zm = z.y;
+    }
+  }
   return st.Y[RT - 1] + st.M[RT - 1];
 }
 
@@ -65,7 +64,7 @@ __device__ __forceinline__ double f64_sweep(const F64Rows<RT>& w, const unsigned
 // has to go to the unscaled kernel.
 template <int RT>
 __device__ __forceinline__ bool f64_pair(const KernelParams& p, const F64Rows<RT>& w, bool fold, int read, int R, int hap,
-                                         long long out, unsigned char* hc, int lane) {
+                                         long long out, unsigned char* hc, const ELane el, int lane) {
   const int64_t ho = p.batch.hap_off[hap];
   const int H = (int)(p.batch.hap_off[hap + 1] - ho);
   if (H == 0 || R == 0) {
@@ -74,11 +73,11 @@ __device__ __forceinline__ bool f64_pair(const KernelParams& p, const F64Rows<RT
   }
   if (!fold) return false;
   __syncwarp();
-  stage_hap(p.batch.hap_bases + ho, H, hc, H + kWarp + kHapLead, lane);
+  stage_hap(p.batch.hap_bases + ho, H, hc, H + kWarp + 4 + kHapLead, lane);
   __syncwarp();
   const int pad = kWarp * RT - (R + 2);  // rows on top of row 0: >= 1 (the read fits RT rows a lane)
   const double y0 = ldexp(p.tables->init_d, kF64Start - kF64InitExp) / (double)H;
-  const double res = f64_sweep<RT>(w, hc + kHapLead - lane, H, pad / RT, pad % RT, y0, lane);
+  const double res = f64_sweep<RT>(w, el, hc + kHapLead - lane, H, pad - lane * RT, y0);
   const bool ok = __shfl_sync(0xffffffffu, res >= kF64MinResult && isfinite(res), kWarp - 1);
   if (ok && lane == kWarp - 1) {
     write_result<double>(p, read, hap, out, res, kF64InitExp - kF64Start);
@@ -87,10 +86,23 @@ __device__ __forceinline__ bool f64_pair(const KernelParams& p, const F64Rows<RT
   return ok;
 }
 
+// Sets up a read's rows and their emission table (behind the haplotype codes).
 template <int RT>
-__device__ __forceinline__ bool f64_read(const KernelParams& p, int64_t ro, int R, int lane, F64Rows<RT>& w) {
-  return __all_sync(0xffffffffu, f64_setup<RT, true>(p.tables, p.batch.read_quals + ro, p.batch.read_bases + ro, R,
-                                                     lane * RT - (kWarp * RT - (R + 2)), w));
+__device__ __forceinline__ bool f64_read(const KernelParams& p, int64_t ro, int R, int lane, unsigned char* etab,
+                                         F64Rows<RT>& w) {
+  __syncwarp();
+  const bool fold = __all_sync(0xffffffffu, f64_setup<RT, true>(p.tables, p.batch.read_quals + ro,
+                                                                p.batch.read_bases + ro, R,
+                                                                lane * RT - (kWarp * RT - (R + 2)), w));
+#pragma unroll
+  for (int h = 0; h < kCodes; ++h) {
+    const uint32_t hit = __byte_perm(w.ma, w.mb, h);
+    double v[RT];
+#pragma unroll
+    for (int j = 0; j < RT; ++j) v[j] = h == kPadCode && !w.sums[j] ? 0.0 : (hit & (1u << j)) ? w.em[j] : w.ex[j];
+    store_emissions<double, RT>(etab, lane, h, v);
+  }
+  return fold;
 }
 
 // Units of one bin (reads of the same rows per lane).
@@ -108,9 +120,11 @@ __global__ void __launch_bounds__(kThreadsPerBlock, RT <= 5 ? 4 : 3) k_f64_units
     const int64_t ro = p.batch.read_off[u.read];
     const int R = (int)(p.batch.read_off[u.read + 1] - ro);
     F64Rows<RT> w;
-    const bool fold = f64_read<RT>(p, ro, R, lane, w);
+    unsigned char* etab = hc + p.hap_bytes;
+    const bool fold = f64_read<RT>(p, ro, R, lane, etab, w);
+    const ELane el = elane<double, RT>(etab, lane);
     for (int k = 0; k < u.nh; ++k) {
-      if (f64_pair<RT>(p, w, fold, u.read, R, u.hap0 + k, u.out0 + k, hc, lane) || lane != 0) continue;
+      if (f64_pair<RT>(p, w, fold, u.read, R, u.hap0 + k, u.out0 + k, hc, el, lane) || lane != 0) continue;
       // to the FP64 list, marked as seen (the read index complemented)
       const unsigned long long at = atomicAdd(&p.ctr->rescue_count, 1ull);
       if (at < (unsigned long long)p.rescue_cap) {
@@ -155,12 +169,12 @@ __global__ void __launch_bounds__(kThreadsPerBlock, 3) k_f64_list(KernelParams p
     if (!seen && R <= kF64ShortMax) {
       if (R + 3 <= 5 * kWarp) {
         F64Rows<5> w;
-        const bool fold = f64_read<5>(p, ro, R, lane, w);
-        done = f64_pair<5>(p, w, fold, pr.read, R, pr.hap, pr.out, wsm, lane);
+        const bool fold = f64_read<5>(p, ro, R, lane, wsm + p.hap_bytes, w);
+        done = f64_pair<5>(p, w, fold, pr.read, R, pr.hap, pr.out, wsm, elane<double, 5>(wsm + p.hap_bytes, lane), lane);
       } else {
         F64Rows<8> w;
-        const bool fold = f64_read<8>(p, ro, R, lane, w);
-        done = f64_pair<8>(p, w, fold, pr.read, R, pr.hap, pr.out, wsm, lane);
+        const bool fold = f64_read<8>(p, ro, R, lane, wsm + p.hap_bytes, w);
+        done = f64_pair<8>(p, w, fold, pr.read, R, pr.hap, pr.out, wsm, elane<double, 8>(wsm + p.hap_bytes, lane), lane);
       }
     }
     if (!done) process_item<double, 4, true>(p, Item{pr.read, pr.hap, 1, pr.out}, wsm, lane, bnd);
@@ -186,9 +200,12 @@ const void* kernel_of(int rt) { return rt == 0 ? reinterpret_cast<const void*>(&
 
 }  // namespace
 
+// Four warps fit a block for every haplotype length that is accepted (BV_PHMM_MAX_HAP_LEN: 172 KB).
 int f64_warp_smem(int rt, int hap_bytes) {
   using S = WarpSmem<double, 4>;
-  return rt == 0 ? hap_bytes + S::kEtabBytes + S::kRingBytes : hap_bytes;
+  // the list's short reads need the table of eight rows a lane, its long ones that of four and the rings
+  const int list = std::max(ETab<double, 8>::kBytes, S::kEtabBytes + S::kRingBytes);
+  return hap_bytes + (rt == 0 ? list : kCodes * kWarp * rt * (int)sizeof(double));  // ETab<double, rt>::kBytes
 }
 
 int f64_blocks_per_sm(int rt, int smem_per_block) {

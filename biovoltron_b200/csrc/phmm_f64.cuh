@@ -14,15 +14,14 @@
 //   zm = M(r-1,c-1) + cx'(r) Xh(r-1,c-1) + cy'(r) Yh(r-1,c-1),
 // so four shuffles a step.
 //
-// Emissions are chosen in registers: a byte per haplotype code holds the
-// lane's match bits, one byte permute picks it, and every row selects between
-// its two values.  (From a table in shared memory, as the FP32 kernels have
-// them, an FP64 lookup moves 256 bytes a row and warp: two wavefronts against
-// the ten FP64-pipe cycles of the row on each of the four schedulers, so the
-// load pipe would be the limit.)  A column outside the haplotype therefore
-// has no zero emission; instead row 0's Y stays zero up to column -1 (the
-// caller injects it, `inject`), which keeps every cell of a column <= 0 zero,
-// and nothing is summed past the last column.
+// The single-strip kernels read the emissions from a table in shared memory
+// (ETab, zero outside the haplotype except in the summing row).  The long-read
+// kernel, 16 warps on an SM's shared memory, chooses them in registers: a byte
+// per haplotype code holds the lane's match bits, one byte permute picks it,
+// and every row selects between its two values.  A column outside the
+// haplotype then has no zero emission; its cells stay zero because nothing
+// above or left of column 1 is non-zero, and nothing is summed past the last
+// column.
 //
 // The folded form needs pMM >= kFoldMin in every row and the scaled states
 // need head-room, so callers start from 2^kF64Start / H (not 2^1020 / H) and
@@ -45,6 +44,7 @@ struct F64Rows {
   double cx[RT], cy[RT], kap[RT], g[RT], em[RT], ex[RT];
   double cxN, cyN, kapN;  // the row below the lane's last
   uint32_t ma, mb;        // match bits (bit j: row j) per haplotype code: bytes A C T G, N pad
+  bool sums[RT];          // the summing row
 };
 
 struct F64Row {
@@ -114,6 +114,7 @@ __device__ __forceinline__ bool f64_setup(const Tables* __restrict__ tb, const u
     w.cx[j] = o.cx; w.cy[j] = o.cy; w.kap[j] = o.kap; w.g[j] = o.g; w.em[j] = o.em; w.ex[j] = o.ex;
     const uint32_t hit = o.code < 4 ? 1u << (8 * o.code) : o.code == 4 ? 0x01010101u : 0u;
     w.ma |= hit << j;
+    w.sums[j] = SUM && rbase + j == R + 1;
     ok &= o.ok;
   }
   const F64Row n = f64_row<SUM>(tb, quals, bases, R, rbase + RT);
@@ -135,16 +136,14 @@ __device__ __forceinline__ double2 f64_sums(const F64Rows<RT>& w, const F64State
   return make_double2(fma_(w.kapN, st.X[RT - 1], st.M[RT - 1]), fma_(w.cyN, dy, fma_(w.cxN, dx, dm)));
 }
 
-// One column: the RT cells below the sums (st.zx, st.zm).  Returns the last
-// row's previous column in dm, dx, dy.
-template <int RT>
-__device__ __forceinline__ void f64_cells(const F64Rows<RT>& w, F64State<RT>& st, uint32_t code, double& dm, double& dx,
-                                          double& dy) {
-  const uint32_t hit = __byte_perm(w.ma, w.mb, code);
+// One column: the RT cells below the sums (st.zx, st.zm), e(j) the emission of
+// the lane's row j.  Returns the last row's previous column in dm, dx, dy.
+template <int RT, typename Emission>
+__device__ __forceinline__ void f64_column(const F64Rows<RT>& w, F64State<RT>& st, Emission&& e, double& dm, double& dx,
+                                           double& dy) {
   double um, ux;
   {
-    const double e = (hit & 1u) ? w.em[0] : w.ex[0];
-    const double mn = e * st.zm;
+    const double mn = e(0) * st.zm;
     const double yn = fma_(w.g[0], st.Y[0], st.M[0]);
     dm = st.M[0]; dx = st.X[0]; dy = st.Y[0];
     um = mn; ux = st.zx;
@@ -152,14 +151,21 @@ __device__ __forceinline__ void f64_cells(const F64Rows<RT>& w, F64State<RT>& st
   }
 #pragma unroll
   for (int j = 1; j < RT; ++j) {
-    const double e = (hit & (1u << j)) ? w.em[j] : w.ex[j];
-    const double mn = e * fma_(w.cy[j], dy, fma_(w.cx[j], dx, dm));
+    const double mn = e(j) * fma_(w.cy[j], dy, fma_(w.cx[j], dx, dm));
     const double xn = fma_(w.kap[j], ux, um);
     const double yn = fma_(w.g[j], st.Y[j], st.M[j]);
     dm = st.M[j]; dx = st.X[j]; dy = st.Y[j];
     um = mn; ux = xn;
     st.M[j] = mn; st.X[j] = xn; st.Y[j] = yn;
   }
+}
+
+// Emissions selected in registers by the code's match bits.
+template <int RT>
+__device__ __forceinline__ void f64_cells(const F64Rows<RT>& w, F64State<RT>& st, uint32_t code, double& dm, double& dx,
+                                          double& dy) {
+  const uint32_t hit = __byte_perm(w.ma, w.mb, code);
+  f64_column(w, st, [&](int j) { return (hit & (1u << j)) ? w.em[j] : w.ex[j]; }, dm, dx, dy);
 }
 
 __device__ __forceinline__ double2 shfl_up_d2(double2 v) {

@@ -133,3 +133,12 @@ def test_long_read_on_eight_blocks(oracle):
         got = e.compute_regions(b)
         _check(b, got, oracle)
         assert np.array_equal(e.compute_regions(b), got)
+
+
+def test_longest_haplotypes(oracle):
+    """The longest haplotypes that are accepted: a block's four of them and the emission tables of seven and eight rows a lane."""
+    from biovoltron_b200.pairhmm import PairHMMEngine
+    rng = np.random.default_rng(12)
+    b = W._build([_pair(rng, n, 32768) for n in (100, 157, 190, 253)], "long haplotypes")
+    with PairHMMEngine(precision="f64") as e:
+        _check(b, e.compute_regions(b), oracle)
