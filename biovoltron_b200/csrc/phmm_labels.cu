@@ -16,20 +16,25 @@
 // of a row depend only on the previous row (one shuffle brings the column left
 // of the lane's first); the in-row Y recurrence is affine with a per-row
 // constant (Y(c) = g Y(c-1) + t(c)), solved by a warp scan over the lanes'
-// chunks.  Every row is renormalised by a power of two; the per-row
-// normalisation of p_r makes the scales cancel.  Forward rows go to a per-warp
-// global buffer, column-interleaved so that a warp's stores and loads are
-// whole lines, and the backward reads them once.  pstar moves with the row: a
-// lane's register for column c holds diagonal c - r, so going one row up
-// shifts it by one column, and the diagonal that leaves column 1 is final.
+// chunks.  Every row is renormalised by a power of two, folded into the next
+// row's constants; the per-row normalisation of p_r makes the scales cancel.
+// Forward rows go to a per-warp global buffer, M and X column-interleaved so
+// that a warp's stores are whole lines, and of Y only what enters each lane's
+// first column: the backward pass, which reads a row once, runs Y's chain again.
+// It reads from two row buffers in shared memory, filled with cp.async two rows
+// ahead.  pstar moves with the row: a lane's register for column c holds
+// diagonal c - r, so going one row up shifts it by one column, and the diagonal
+// that leaves column 1 is final.
 //
-// Bound by latency: a row's two affine chains, its warp scan and its three
-// reductions follow one another, with 8 to 12 warps an SM to hide them (the
-// forward rows' traffic, 24 bytes a cell, is a quarter of the time).  24 k pairs
-// of 150 x 450: 10 ms.  States and pstar in shared memory (33 KB a warp, a lane
-// stride of C words and its bank conflicts) took 80; classes of 256 and 128
-// columns with a branch at every column 21; four columns a class leave the
-// branch to the last three.
+// Bound by issue (70 %, 12 warps an SM at 168 registers; 16 warps at 128 give 1 %,
+// classes of 20 columns lose by spilling) and by the forward rows' traffic, 16
+// bytes a cell: 26 GB of 24 k uneven pairs (1.6 G cells), 3.9 of 6.5 ms.  Reading the
+// rows where they are used took 9.5 ms (half the stalls waited for them), with
+// the row buffers and one-instruction maxima 7.9, without Y's rows 6.9.
+// Earlier forms: states and pstar in shared memory (33 KB a warp, a lane stride of
+// C words and its bank conflicts) 80 ms; classes of 256 and 128 columns with a
+// branch at every column 21; four columns a class leave the branch to the last
+// three.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -53,7 +58,7 @@ __device__ __forceinline__ uint32_t code_of(uint8_t b) {
 }
 
 struct RowC {
-  float mm, gp, mx, my, g, em, ex;
+  float mm, gp, mx, my, g, gx, em, ex;
   uint32_t rc;
 };
 
@@ -64,6 +69,7 @@ __device__ __forceinline__ RowC row_consts(const Tables* tb, const uchar4* quals
   const int mx = max(qi, qd), mn = min(qi, qd);
   k.mm = tb->mm_f[((mx * (mx + 1)) >> 1) + mn];
   k.g = tb->ph2pr_f[q.w & kQualMask];
+  k.gx = k.g;
   k.gp = 1.f - k.g;
   k.mx = tb->ph2pr_f[qi];
   k.my = tb->ph2pr_f[qd];
@@ -74,28 +80,62 @@ __device__ __forceinline__ RowC row_consts(const Tables* tb, const uchar4* quals
   return k;
 }
 
-// Inclusive warp scan of affine maps y -> a*y + b (lane order = left to right
-// when `forward`, right to left otherwise).  Returns the map composed over
-// the lanes before this one applied to 0, i.e. the carry-in.
-__device__ __forceinline__ float affine_carry(float a, float b, int lane, bool forward) {
+// Inclusive warp scans of affine maps y -> a*y + b, `a` the same in every lane
+// (a lane that takes a step has a full window of maps beside it: its factor is
+// a power that all lanes know).  They return the map composed over the lanes
+// before this one applied to 0, i.e. the carry-in.
+__device__ __forceinline__ float carry_from_left(float a, float b, int lane) {
   for (int o = 1; o < 32; o <<= 1) {
-    const float ao = forward ? __shfl_up_sync(0xffffffffu, a, o) : __shfl_down_sync(0xffffffffu, a, o);
-    const float bo = forward ? __shfl_up_sync(0xffffffffu, b, o) : __shfl_down_sync(0xffffffffu, b, o);
-    const bool has = forward ? lane >= o : lane + o < 32;
-    if (has) { b = a * bo + b; a = a * ao; }
+    const float bo = __shfl_up_sync(0xffffffffu, b, o);
+    if (lane >= o) b = a * bo + b;
+    a = a * a;
   }
-  const float prev = forward ? __shfl_up_sync(0xffffffffu, b, 1) : __shfl_down_sync(0xffffffffu, b, 1);
-  return (forward ? lane == 0 : lane == 31) ? 0.f : prev;
+  const float prev = __shfl_up_sync(0xffffffffu, b, 1);
+  return lane == 0 ? 0.f : prev;
+}
+// Right to left.  Lanes past the haplotype's end have b = 0, so that the one
+// lane with fewer columns, and with it a smaller power, needs none of its own.
+__device__ __forceinline__ float carry_from_right(float a, float b, int lane) {
+  for (int o = 1; o < 32; o <<= 1) {
+    const float bo = __shfl_down_sync(0xffffffffu, b, o);
+    if (lane + o < 32) b = a * bo + b;
+    a = a * a;
+  }
+  const float prev = __shfl_down_sync(0xffffffffu, b, 1);
+  return lane == 31 ? 0.f : prev;
+}
+// The constants of a row that reads the states of a neighbouring row, those
+// states to be multiplied by the power of two sc: exact, and cheaper than a
+// product for every state.  (g also leads Y along its own row, which has no
+// factor: gx is X's.)
+__device__ __forceinline__ RowC scaled(RowC k, float sc) {
+  k.mm *= sc;
+  k.gp *= sc;
+  k.mx *= sc;
+  k.gx *= sc;
+  return k;
 }
 
+// Of values >= 0: their bits are in the same order.
 __device__ __forceinline__ float warp_max(float v) {
-  for (int o = 16; o > 0; o >>= 1) v = fmaxf(v, __shfl_xor_sync(0xffffffffu, v, o));
-  return v;
+  return __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(v)));
 }
 __device__ __forceinline__ float warp_sum(float v) {
   for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
   return v;
 }
+
+__device__ __forceinline__ void cp_async16(float* dst, const float* src) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src)
+               : "memory");
+}
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+// Until at most one group is in flight.
+__device__ __forceinline__ void cp_async_wait1() { asm volatile("cp.async.wait_group 1;" ::: "memory"); }
+
+// A warp's two row buffers of the backward pass, floats.
+template <int CM>
+constexpr int kRowBufFloats = 2 * (64 * CM + 32);
 
 // Pairs whose C lies in (CL, CM]; `first`: this launch also marks the pairs
 // that get no label.  Warps take `grab` pairs at a time from *next.
@@ -106,6 +146,8 @@ __global__ void __launch_bounds__(kLabelWarps * 32, CM <= 20 ? 3 : 2)
                        unsigned long long* next, int grab, bool first, int32_t* lo_out, int32_t* hi_out) {
   const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
   float* F = fbuf + (blockIdx.x * (long long)kLabelWarps + wib) * fbuf_stride + lane;
+  extern __shared__ __align__(16) float row_bufs[];
+  float* S = row_bufs + wib * kRowBufFloats<CM>;
   for (;;) {
     long long base = 0;
     if (lane == 0) base = (long long)atomicAdd(next, (unsigned long long)grab);
@@ -143,8 +185,8 @@ __global__ void __launch_bounds__(kLabelWarps * 32, CM <= 20 ? 3 : 2)
         X[j] = 0.f;
         Y[j] = j < nc ? 1.f : 0.f;
       }
-      // ---- forward, rows 1..R; row r's states at F + r * 3 * 32 C: M, X, Y, column j of all lanes together
-      const long long row_floats = 96ll * C;
+      // ---- forward, rows 1..R; row r at F + r * row_floats: M, X (column j of all lanes together), Y's carries
+      const long long row_floats = 64ll * C + 32;
       float tM = 0.f, tX = 0.f, tY = 1.f;  // the lane's last column
       RowC k = row_consts(tb, quals, bases, 1);
       for (int r = 1; r <= R; ++r) {
@@ -159,7 +201,7 @@ __global__ void __launch_bounds__(kLabelWarps * 32, CM <= 20 ? 3 : 2)
           if (j <= CL || j < C) {
             const float e = (mm >> j & 1u) ? k.em : k.ex;
             const float nM = e * (k.mm * oM + k.gp * (oX + oY));
-            const float nX = k.mx * M[j] + k.g * X[j];
+            const float nX = k.mx * M[j] + k.gx * X[j];
             oM = M[j]; oX = X[j]; oY = Y[j];
             M[j] = j < nc ? nM : 0.f;
             X[j] = nX;
@@ -170,21 +212,20 @@ __global__ void __launch_bounds__(kLabelWarps * 32, CM <= 20 ? 3 : 2)
         if (lane == 0) mleft = 0.f;
         float a = 1.f, bb = 0.f;
         {
-          float y = 0.f, m = mleft;
+          float m = mleft;
 #pragma unroll
           for (int j = 0; j < CM; ++j)
-            if (j <= CL || j < C) { y = k.g * y + k.my * m; m = M[j]; a *= k.g; }
-          bb = y;
+            if (j <= CL || j < C) { bb = __fmaf_rn(k.g, bb, __fmul_rn(k.my, m)); m = M[j]; a *= k.g; }
         }
-        const float carry = affine_carry(a, bb, lane, true);
+        const float carry = carry_from_left(a, bb, lane);
         float mx = 0.f;
         {
           float y = carry, m = mleft;
 #pragma unroll
           for (int j = 0; j < CM; ++j)
             if (j <= CL || j < C) {
-              y = k.g * y + k.my * m;
-              Y[j] = j < nc ? y : 0.f;
+              y = __fmaf_rn(k.g, y, __fmul_rn(k.my, m));
+              Y[j] = y;
               m = M[j];
               mx = fmaxf(mx, fmaxf(M[j], fmaxf(X[j], Y[j])));
             }
@@ -192,25 +233,40 @@ __global__ void __launch_bounds__(kLabelWarps * 32, CM <= 20 ? 3 : 2)
         mx = warp_max(mx);
         const float sc = mx > 0.f ? ldexpf(1.f, -ilogbf(mx)) : 1.f;
         float* Fr = F + r * row_floats;
+        Fr[64 * C] = carry;
 #pragma unroll
         for (int j = 0; j < CM; ++j)
           if (j <= CL || j < C) {
-            M[j] *= sc;
-            X[j] *= sc;
-            Y[j] *= sc;
             Fr[j * 32] = M[j];
             Fr[(C + j) * 32] = X[j];
-            Fr[(2 * C + j) * 32] = Y[j];
             tM = M[j]; tX = X[j]; tY = Y[j];
           }
-        k = kn;
+        k = scaled(kn, sc);
       }
       // ---- backward, rows R..1: M, X hold B of row r + 1, posterior per row
+      // forward row r is copied to buffer r & 1 while row r + 2 and r + 1 are computed
+      auto fetch = [&](int r) {
+        if (r >= 1) {
+          const float* src = F - lane + r * row_floats;
+          float* dst = S + (r & 1) * (64 * CM + 32);
+#pragma unroll
+          for (int i = 0; i < (16 * CM + 8 + 31) / 32; ++i) {
+            const int at = i * 32 + lane;
+            if (at < 16 * C + 8) cp_async16(dst + 4 * at, src + 4 * at);
+          }
+        }
+        cp_async_commit();  // a group a row, empty past the first
+      };
+      __syncwarp();
+      fetch(R);
+      fetch(R - 1);
       float P[CM];  // pstar of diagonal c - r
 #pragma unroll
-      for (int j = 0; j < CM; ++j) { M[j] = 0.f; X[j] = 0.f; P[j] = 0.f; }
+      for (int j = 0; j < CM; ++j) { M[j] = 0.f; X[j] = j < nc ? 1.f : 0.f; P[j] = 0.f; }
       int lo = INT32_MAX, hi = INT32_MIN;
-      RowC k1{};  // constants of row r+1
+      RowC k1{};  // constants of row r+1; above row R a row whose B_X = 1 gives B_M = B_X = 1 there
+      k1.mx = 1.f;
+      k1.gx = 1.f;
       uint32_t mm1 = 0;
       RowC k0 = row_consts(tb, quals, bases, R);
       for (int r = R; r >= 1; --r) {
@@ -222,20 +278,19 @@ __global__ void __launch_bounds__(kLabelWarps * 32, CM <= 20 ? 3 : 2)
         // B_Y(c) = g(r) B_Y(c+1) + t(c), right to left, t(c) = gp(r+1) e(r+1,c+1) B_M(r+1,c+1)
         float a = 1.f, bb = 0.f;
         {
-          float y = 0.f, nx = rM;
+          float nx = rM;
           bool bit = rbit;
 #pragma unroll
           for (int j = CM - 1; j >= 0; --j)
             if (j <= CL || j < C) {
               const float t = __fmul_rn(__fmul_rn(k1.gp, bit ? k1.em : k1.ex), nx);
-              y = __fmaf_rn(k0.g, y, t);
-              if (j < nc) a *= k0.g;
+              bb = __fmaf_rn(k0.g, bb, t);
+              a *= k0.g;
               nx = M[j];
               bit = mm1 >> j & 1u;
             }
-          bb = y;
         }
-        const float carry = affine_carry(a, bb, lane, false);
+        const float carry = carry_from_right(a, bb, lane);
         float mx = 0.f, tot = 0.f;
         {
           float y = carry, nx = rM;  // y: B_Y(r, c+1)
@@ -249,43 +304,44 @@ __global__ void __launch_bounds__(kLabelWarps * 32, CM <= 20 ? 3 : 2)
               Y[j] = y;
               nx = M[j];
               bit = mm1 >> j & 1u;
-              const float bm = k1.mm * nm + k1.mx * X[j] + k0.my * byr;
-              const float bx = k1.gp * nm + k1.g * X[j];
-              M[j] = r == R ? (j < nc ? 1.f : 0.f) : bm;
-              X[j] = r == R ? (j < nc ? 1.f : 0.f) : bx;
+              M[j] = k1.mm * nm + k1.mx * X[j] + k0.my * byr;
+              X[j] = k1.gp * nm + k1.gx * X[j];
               mx = fmaxf(mx, fmaxf(M[j], fmaxf(X[j], Y[j])));
             }
         }
         // posterior of row r
-        const float* Fr = F + r * row_floats;
-#pragma unroll
-        for (int j = 0; j < CM; ++j)
-          if (j <= CL || j < C) {
-            // the sum's terms, kept for the row's normalised values
-            Y[j] = Fr[j * 32] * M[j] + Fr[(C + j) * 32] * X[j] + Fr[(2 * C + j) * 32] * Y[j];
-            tot += Y[j];
-          }
-        tot = warp_sum(tot);
-        if (tot > 0.f) {
-          const float inv = 1.f / tot;
+        cp_async_wait1();
+        __syncwarp();
+        const float* Fr = S + (r & 1) * (64 * CM + 32) + lane;
+        {
+          float y = Fr[64 * C], m = lane == 0 ? 0.f : Fr[(C - 1) * 32 - 1];
 #pragma unroll
           for (int j = 0; j < CM; ++j)
-            if (j <= CL || j < C) P[j] = fmaxf(P[j], Y[j] * inv);
+            if (j <= CL || j < C) {
+              y = __fmaf_rn(k0.g, y, __fmul_rn(k0.my, m));
+              m = Fr[j * 32];
+              // the sum's terms, kept for the row's normalised values
+              Y[j] = m * M[j] + Fr[(C + j) * 32] * X[j] + y * Y[j];
+              tot += Y[j];
+            }
         }
-        mx = warp_max(mx);
-        const float sc = mx > 0.f ? ldexpf(1.f, -ilogbf(mx)) : 1.f;
-#pragma unroll
-        for (int j = 0; j < CM; ++j)
-          if (j <= CL || j < C) { M[j] *= sc; X[j] *= sc; }
-        if (r > 1) {  // one row up: diagonal 1 - r leaves column 1
-          if (lane == 0 && P[0] >= tau) { lo = min(lo, 1 - r); hi = max(hi, 1 - r); }
+        __syncwarp();
+        fetch(r - 2);
+        tot = warp_sum(tot);
+        // one row up: the diagonals move by one column (P: row r + 1's)
+        {
           float in = __shfl_down_sync(0xffffffffu, P[0], 1);
           if (lane == 31) in = 0.f;
+          const float inv = tot > 0.f ? 1.f / tot : 0.f;
 #pragma unroll
           for (int j = 0; j < CM; ++j)
-            if (j <= CL || j < C) P[j] = j + 1 < CM && (j + 1 <= CL || j + 1 < C) ? P[j + 1 < CM ? j + 1 : j] : in;
+            if (j <= CL || j < C)
+              P[j] = fmaxf(j + 1 < CM && (j + 1 <= CL || j + 1 < C) ? P[j + 1 < CM ? j + 1 : j] : in, Y[j] * inv);
         }
-        k1 = k0;
+        if (r > 1 && lane == 0 && P[0] >= tau) { lo = min(lo, 1 - r); hi = max(hi, 1 - r); }  // leaves column 1
+        mx = warp_max(mx);
+        const float sc = mx > 0.f ? ldexpf(1.f, -ilogbf(mx)) : 1.f;
+        k1 = scaled(k0, sc);
         mm1 = row_match(k0.rc);
         k0 = kn;
       }
@@ -306,7 +362,10 @@ cudaError_t launch_class(const DeviceBatch& b, const Tables* tb, const int32_t* 
                          int32_t* lo, int32_t* hi, cudaStream_t st) {
   const int blocks = f.blocks;
   const int grab = (int)std::max<long long>(1, std::min<long long>(32, n_pairs / ((long long)blocks * kLabelWarps * 64)));
-  k_posterior_spread<CL, CM><<<blocks, kLabelWarps * 32, 0, st>>>(b, tb, pair_read, pair_hap, n_pairs, tau, fbuf, f.stride,
+  const int smem = kLabelWarps * kRowBufFloats<CM> * (int)sizeof(float);
+  if (cudaError_t e = raise_dynamic_smem(reinterpret_cast<const void*>(&k_posterior_spread<CL, CM>), smem); e != cudaSuccess)
+    return e;
+  k_posterior_spread<CL, CM><<<blocks, kLabelWarps * 32, smem, st>>>(b, tb, pair_read, pair_hap, n_pairs, tau, fbuf, f.stride,
                                                                   f.max_area, next, grab, first, lo, hi);
   return cudaGetLastError();
 }
@@ -315,11 +374,12 @@ cudaError_t launch_class(const DeviceBatch& b, const Tables* tb, const int32_t* 
 
 // Rows of the longest read and haplotype the label kernel takes; a longer
 // read may stand against a shorter haplotype as long as its rows fit that
-// area (a row holds 32 C <= H + 31 columns, 29 more than the area counts).
+// area.  (The buffer's rows hold M and X of 32 C <= H + 31 columns and 32
+// carries: 2 (H + 2) + 90 floats at most, where the area counts 3 (H + 2).)
 LabelRows label_rows(int max_read, int longest, int max_hap, int sms, size_t max_bytes) {
   LabelRows f{};
   f.max_area = (long long)(max_read + 1) * 3 * (max_hap + 2);
-  f.stride = (f.max_area + 3ll * 29 * (std::min(longest, kBandMaxSpan) + 1) + 31) / 32 * 32;
+  f.stride = (f.max_area / 3 * 2 + 90ll * (std::min(longest, kBandMaxSpan) + 1) + 31) / 32 * 32;
   const size_t per_block = (size_t)f.stride * sizeof(float) * kLabelWarps;
   f.blocks = (int)std::max<size_t>(1, std::min<size_t>((size_t)sms * 3, max_bytes / per_block));
   f.bytes = per_block * (size_t)f.blocks;

@@ -41,3 +41,21 @@ def test_label_classes(oracle, hap_len):
         d = np.arange(len(pstar)) + dmin
         strict, loose = d[pstar >= tau * 1.05], d[pstar >= tau * 0.95]
         assert loose.min() <= lo[k] <= strict.min() and strict.max() <= hi[k] <= loose.max(), k
+
+
+def test_reads_of_a_few_rows(oracle):
+    """One to four rows (the backward pass copies rows two ahead), against the oracle's posterior."""
+    from biovoltron_b200.pairhmm import PairHMMEngine
+    rng = np.random.default_rng(2)
+    hap = W._random_seq(rng, 70)
+    reads = [(hap[20:20 + n].copy(), *W._quals(rng, n, 20, 40)) for n in (1, 2, 3, 4)]
+    b = W._build([(reads, [hap, hap[:40].copy()])], "short reads")
+    tau = 1e-3
+    with PairHMMEngine() as e:
+        _, lo, hi = e.band_labels(b, tau=tau)
+    tcs = TestcaseArray(b, *b.pair_index())
+    for k in range(b.n_pairs):
+        dmin, pstar = oracle.posterior_diag(tcs, k)
+        d = np.arange(len(pstar)) + dmin
+        strict, loose = d[pstar >= tau * 1.05], d[pstar >= tau * 0.95]
+        assert loose.min() <= lo[k] <= strict.min() and strict.max() <= hi[k] <= loose.max(), k
