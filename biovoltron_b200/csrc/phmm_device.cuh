@@ -631,6 +631,64 @@ __device__ __forceinline__ void run_strip_pair(const Rows<float, RT>& rw, const 
   lastY = Y[RT - 1];
 }
 
+// One haplotype of a read (FP32 single strip), for launches with too few pairs
+// to fill the device: bound by a step's latency (the shuffle, then the X chain
+// down the lane's rows), not by issue.  The lane above sends the top row's two
+// sums as in run_strip_pair (two shuffles instead of run_strip's three), and the
+// emissions of step s + 1 and the code of step s + 2 are loaded before step s is
+// computed.  Five rows a lane, 512 pairs: 44.6 ns a step where run_strip takes
+// 48.8; kept out of the paired kernels, whose registers it would raise (96 to 105
+// there: 4 % of a large batch).  The codes are read two columns past the last step's.
+template <int RT, bool FOLD>
+__device__ __forceinline__ void run_strip_one(const Rows<float, RT>& rw, const ELane el,
+                                              const unsigned char* __restrict__ hc_lane, int nsteps, float& lastM,
+                                              float& lastY) {
+  constexpr unsigned kStride = WarpSmem<float, RT>::kCodeStride;
+  constexpr int CH = 8;
+  float M[RT], X[RT], Y[RT];
+#pragma unroll
+  for (int j = 0; j < RT; ++j) { M[j] = 0.f; X[j] = 0.f; Y[j] = rw.y0[j]; }
+  const float mmN = __shfl_down_sync(0xffffffffu, rw.mm[0], 1), cxN = __shfl_down_sync(0xffffffffu, rw.cx[0], 1);
+  const float cyN = __shfl_down_sync(0xffffffffu, rw.cy[0], 1), kapN = __shfl_down_sync(0xffffffffu, rw.kap[0], 1);
+  auto msum = [&](float mm, float cx, float cy, float m, float x, float y) {
+    if constexpr (FOLD) return fma_(cy, y, fma_(cx, x, m));
+    else return fma_(mm, m, fma_(cx, x, cy * y));
+  };
+  float zx = __shfl_up_sync(0xffffffffu, fma_(kapN, X[RT - 1], M[RT - 1]), 1);
+  float zm = __shfl_up_sync(0xffffffffu, msum(mmN, cxN, cyN, M[RT - 1], X[RT - 1], Y[RT - 1]), 1);
+  float en[RT];  // the next step's emissions
+  load_emissions<float, RT>(el, (unsigned)hc_lane[0] * kStride, en);
+  unsigned code = hc_lane[1];
+  for (int s0 = 0; s0 < nsteps; s0 += CH) {
+#pragma unroll
+    for (int u = 0; u < CH; ++u) {
+      float e[RT];
+#pragma unroll
+      for (int j = 0; j < RT; ++j) e[j] = en[j];
+      load_emissions<float, RT>(el, code * kStride, en);
+      code = hc_lane[s0 + u + 2];
+      float dm = M[0], dx = X[0], dy = Y[0];
+      float um = e[0] * zm, ux = zx;
+      Y[0] = fma_(rw.g[0], Y[0], M[0]);
+      M[0] = um;
+      X[0] = ux;
+#pragma unroll
+      for (int j = 1; j < RT; ++j) {
+        const float mn = e[j] * msum(rw.mm[j], rw.cx[j], rw.cy[j], dm, dx, dy);
+        const float xn = fma_(rw.kap[j], ux, um);
+        const float yn = fma_(rw.g[j], Y[j], M[j]);
+        dm = M[j]; dx = X[j]; dy = Y[j];
+        um = mn; ux = xn;
+        M[j] = mn; X[j] = xn; Y[j] = yn;
+      }
+      zx = __shfl_up_sync(0xffffffffu, fma_(kapN, X[RT - 1], M[RT - 1]), 1);
+      zm = __shfl_up_sync(0xffffffffu, msum(mmN, cxN, cyN, dm, dx, dy), 1);
+    }
+  }
+  lastM = M[RT - 1];
+  lastY = Y[RT - 1];
+}
+
 template <typename T> __device__ __forceinline__ T log10_(T v);
 template <> __device__ __forceinline__ float log10_(float v) { return log10f(v); }
 template <> __device__ __forceinline__ double log10_(double v) { return log10(v); }
@@ -782,7 +840,7 @@ __device__ void process_item(const KernelParams& p, const Item& it, unsigned cha
     // last read row by one column, so FP32 runs one step more.
     const int nsteps = (H + kWarp - 1 + (SumRow<T>::value ? 1 : 0) + CHK - 1) / CHK * CHK;
     __syncwarp();
-    stage_hap(b.hap_bases + ho, H, hc, nsteps + kHapLead, lane);
+    stage_hap(b.hap_bases + ho, H, hc, nsteps + 2 + kHapLead, lane);  // run_strip_one reads two columns ahead
     if (!MULTI) {
       // the initial row's Y depends on the haplotype length
       const int r0j = pad - lane * RT;  // j of row 0 within this lane, if here
@@ -838,6 +896,9 @@ __device__ void process_item(const KernelParams& p, const Item& it, unsigned cha
           }
         }
       }
+    } else if constexpr (sizeof(T) == 4 && !PAIR) {
+      if (fold) run_strip_one<RT, true>(rw, el, hc + kHapLead - lane, nsteps, lastM, lastY);
+      else run_strip_one<RT, false>(rw, el, hc + kHapLead - lane, nsteps, lastM, lastY);
     } else {
       if (fold)
         run_strip<T, RT, false, 8, true>(rw, el, hc + kHapLead - lane, nsteps, lane, nullptr, nullptr, T(1), lastM,

@@ -467,7 +467,9 @@ bv_status Engine::plan(const bv_region_batch& b) {
   rp.warp_smem = f64_warp_smem(0, rp.hap_bytes);
   const int smem_block = rp.warp_smem * (kThreadsPerBlock / kWarp);
   if (smem_block > 227 * 1024) return fail(BV_ERR_INVALID_ARG, "haplotype too long for shared-memory staging");
-  rp.grid = sms_ * std::max(1, f64_blocks_per_sm(0, smem_block));
+  // (no more warps than pairs: an empty list after 60 pairs takes 4 instead of 8 us)
+  rp.grid = (int)std::min<int64_t>((int64_t)sms_ * std::max(1, f64_blocks_per_sm(0, smem_block)),
+                                   std::max<int64_t>(1, (n_results_ + kThreadsPerBlock / kWarp - 1) / (kThreadsPerBlock / kWarp)));
   rp.bnd_cols = bnd_cols_for(std::max(max_hap_, 1));
   rescue_plan_ = rp;
   // FP64 long reads: one block per pair, longest pairs first (the long list is
@@ -893,9 +895,11 @@ bv_status Engine::launch(int64_t n_out) {
   }
   ++runs_since_stage_;
   // page-locked destination: the copy is queued, the host goes on
-  BV_CUDA(cudaMemcpyAsync(h_counters_, d_counters_.get(),
-                          n_out > 0 ? kCountersBytes + sizeof(double) * (size_t)n_out : sizeof(Counters),
-                          cudaMemcpyDeviceToHost, stream_), "counters D2H");
+  const size_t back = n_out > 0 ? kCountersBytes + sizeof(double) * (size_t)n_out : sizeof(Counters);
+  // A small batch's come back by a kernel: a copy engine's start and end cost 8 us more.  Not beside large
+  // batches, whose persistent blocks it would queue behind.
+  if (small_in_) BV_CUDA(launch_copy_small(d_counters_.get(), h_counters_, back, stream_), "counters D2H");
+  else BV_CUDA(cudaMemcpyAsync(h_counters_, d_counters_.get(), back, cudaMemcpyDeviceToHost, stream_), "counters D2H");
   return BV_OK;
 }
 

@@ -163,6 +163,19 @@ __global__ void k_pack_quals_uniform(const uint8_t* __restrict__ q, uint8_t gi, 
     out[x] = make_uchar4(q[x], gi, gd, gc);
 }
 
+// Small copies to and from page-locked memory (16-byte units).
+__global__ void k_copy_small(const uint4* __restrict__ src, uint4* __restrict__ dst, int n) {
+  const int x = blockIdx.x * blockDim.x + threadIdx.x;
+  if (x < n) dst[x] = src[x];
+}
+
+cudaError_t launch_copy_small(const void* src, void* dst, size_t bytes, cudaStream_t st) {
+  const int n = (int)((bytes + 15) / 16);
+  if (n <= 0) return cudaSuccess;
+  k_copy_small<<<(n + 127) / 128, 128, 0, st>>>(static_cast<const uint4*>(src), static_cast<uint4*>(dst), n);
+  return cudaGetLastError();
+}
+
 __global__ void k_set_u64(unsigned long long* dst, unsigned long long v) { *dst = v; }
 
 cudaError_t launch_set_u64(unsigned long long* dst, unsigned long long v, cudaStream_t st) {

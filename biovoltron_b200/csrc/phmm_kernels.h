@@ -88,6 +88,8 @@ cudaError_t raise_dynamic_smem(const void* func, int bytes);
 // Sets the variant's dynamic shared-memory limit; call before launching or capturing it.
 cudaError_t prepare_variant(int variant, int smem_per_block);
 cudaError_t launch_forward(int variant, const KernelParams& p, int grid, cudaStream_t st);
+// Copies `bytes` (rounded up to 16; both sides 16-byte aligned) by a kernel.
+cudaError_t launch_copy_small(const void* src, void* dst, size_t bytes, cudaStream_t st);
 cudaError_t launch_pack_quals(const uint8_t* q, const uint8_t* i, const uint8_t* d, const uint8_t* c, uchar4* out,
                               long long n, int sms, cudaStream_t st);
 // The same with the insertion, deletion and continuation qualities constant.

@@ -69,3 +69,28 @@ def test_units_made_on_the_device(precision, band):
         for _ in range(2):
             e.run()
             assert np.array_equal(e.fetch(n), got)
+
+
+# one haplotype a warp (few pairs) against two, bit for bit: rows that cannot be folded (indel qualities of 0-3),
+# N in reads and haplotypes, haplotypes of one base and shorter than the read, every bin's longest read
+@pytest.mark.parametrize("gap", [45, 2, 0])
+def test_one_haplotype_a_warp(oracle, gap):
+    from biovoltron_b200.pairhmm import PairHMMEngine
+    rng = np.random.default_rng(40 + gap)
+    regions = []
+    for n in (1, 29, 61, 93, 125, 157, 189, 221, 253):
+        reads, haps = _region(rng, 2, 3, [n], n + 40)
+        reads = [(r, q, np.full(len(r), gap, np.uint8), np.full(len(r), gap, np.uint8), c) for r, q, _, _, c in reads]
+        reads[0][0][len(reads[0][0]) // 2] = ord("N")
+        haps[1][5:7] = ord("N")
+        regions.append((reads, haps + [haps[0][:1].copy(), haps[0][:n // 2 + 1].copy()]))
+    b = W._build(regions, "one haplotype a warp")
+    out = []
+    for warp in (1, 2):
+        with PairHMMEngine(haps_per_unit=4, haps_per_warp=warp) as e:
+            out.append(e.compute_regions(b))
+    assert np.array_equal(out[0], out[1])
+    truth = oracle.log10_rescaled(TestcaseArray.for_batch(b))
+    fin = np.isfinite(truth)
+    assert np.array_equal(np.isfinite(out[0]), fin)
+    assert np.max(np.abs(out[0][fin] - truth[fin])) <= TOL_FP32
