@@ -22,6 +22,7 @@
 #include <chrono>
 #include <memory>
 #include <cstring>
+#include <numeric>
 #include <string>
 
 namespace bvphmm {
@@ -489,23 +490,48 @@ bv_status Engine::plan(const bv_region_batch& b) {
       long_block_ *= 2;
     long_smem_ = long_smem_bytes(rp.hap_bytes, long_block_);
     if (long_smem_ <= 227 * 1024) {
-      // A cluster of blocks a pair: the largest that leaves every pair a cluster of its own (a second round
-      // of clusters costs more than their width saves) and every block strips.  FP64 pass of reads of up to
-      // 10 kb with 1 / 2 / 4 / 8 blocks a pair, ms: 8 pairs 8.4 / - / - / 2.8, 20 pairs 9.5 / 5.5 / 3.4 / 5.6, 40
-      // pairs 11.1 / 6.8 / 8.4 / 7.6 (74, 33 and 15 clusters of 2, 4 and 8 run at once), 148 pairs 11.8 / 11.5
-      // / 15.4 / 25.0.
-      long_cluster_ = 1;
-      int64_t teams = (int64_t)sms_ * std::max(1, long_blocks_per_sm(long_smem_, long_block_));
-      for (int c = kLongMaxBlocks; c > 1 && long_block_ == 16 && !long_set_; c /= 2) {
-        if (8 * c >= strips) continue;
-        const int active = long_clusters(long_smem_, long_block_, c);
-        if (n_long > active) continue;
-        long_cluster_ = c;
-        teams = active;
-        break;
+      // Up to a few hundred pairs: a cluster of blocks for each, the blocks dealt by the pairs' costs (long_cost):
+      // the lowest limit for which all pairs' blocks together are at most the SMs, or 2/5 of them more than there
+      // are pairs.  FP64 pass of reads of up to 10 kb, one block a pair -> this, ms: 40 pairs 11.1 -> 3.5, 90 12.2 ->
+      // 6.0, 148 11.9 -> 9.6, 256 15.9 -> 11.5, 512 25.7 -> 20.1 (one cluster size for all pairs: 40 pairs 6.8, 90
+      // 12.2; totals of 112 to 400 blocks tried at 40 to 256 pairs).  Pairs of one length get a block each: then,
+      // and beyond, the blocks take the next pair from the list.
+      std::fill(long_grid_, long_grid_ + 4, 0);
+      int64_t budget = 0;
+      if (long_block_ == 16 && !long_set_ && n_long <= kLongMembers)
+        budget = std::max<int64_t>(sms_, n_long + sms_ * 2 / 5);
+      if (n_long <= budget) {
+        std::vector<std::pair<int64_t, int64_t>> pairs;  // read and haplotype lengths
+        std::vector<long long> limits;
+        for (int64_t g = 0; g < b.num_regions; ++g)
+          for (int64_t r = b.region_reads[g]; r < b.region_reads[g + 1]; ++r) {
+            const int64_t rl = b.read_offsets[r + 1] - b.read_offsets[r];
+            for (int64_t h = b.region_haps[g]; rl >= long_rows() && h < b.region_haps[g + 1]; ++h) {
+              pairs.emplace_back(rl, b.hap_offsets[h + 1] - b.hap_offsets[h]);
+              for (int c = 1; c <= kLongMaxBlocks; c *= 2) limits.push_back(long_cost(rl, pairs.back().second, c));
+            }
+          }
+        std::sort(limits.begin(), limits.end());
+        auto blocks = [&](long long limit) {
+          int64_t n = 0;
+          for (const auto& [rl, hl] : pairs) n += long_blocks(rl, hl, limit);
+          return n;
+        };
+        long_limit_ = *std::partition_point(limits.begin(), limits.end() - 1, [&](long long t) { return blocks(t) > budget; });
+        for (const auto& [rl, hl] : pairs) {
+          const int c = long_blocks(rl, hl, long_limit_);
+          long_grid_[c == 8 ? 0 : c == 4 ? 1 : c == 2 ? 2 : 3] += c;
+        }
+        if (long_grid_[3] == n_long) long_grid_[3] = 0;
       }
-      BV_CUDA(prepare_long(long_smem_, long_block_, long_cluster_), "kernel attribute");
-      long_plan_.grid = (int)std::min<int64_t>(n_long, teams) * long_cluster_;
+      long_plan_.grid = std::accumulate(long_grid_, long_grid_ + 4, 0);
+      if (long_plan_.grid > 0) {
+        BV_CUDA(prepare_long(long_smem_, long_block_, 1), "kernel attribute");
+        if (bv_status ls = reserve_lanes(4); ls != BV_OK) return ls;
+      } else {
+        BV_CUDA(prepare_long(long_smem_, long_block_, 0), "kernel attribute");
+        long_plan_.grid = (int)std::min<int64_t>(n_long, (int64_t)sms_ * std::max(1, long_blocks_per_sm(long_smem_, long_block_)));
+      }
       long_plan_.hap_bytes = rp.hap_bytes;
       long_plan_.bnd_cols = rp.bnd_cols;
       long_plan_.f64 = true;
@@ -840,7 +866,20 @@ bv_status Engine::enqueue_kernels(bool capturing) {
       KernelParams q = p;
       q.hap_bytes = long_plan_.hap_bytes;
       q.bnd_cols = long_plan_.bnd_cols;
-      BV_CUDA(launch_forward_long(q, long_plan_.grid, long_smem_, long_block_, long_cluster_, stream_), "FP64 long-read launch");
+      if (long_grid_[0] + long_grid_[1] + long_grid_[2] + long_grid_[3] == 0) {
+        BV_CUDA(launch_forward_long(q, long_plan_.grid, long_smem_, long_block_, 0, stream_), "FP64 long-read launch");
+      } else {  // the largest clusters first, the smaller ones beside them
+        q.long_cost = long_limit_;
+        if (bv_status fs = fork(4); fs != BV_OK) return fs;
+        cudaError_t le = cudaSuccess;  // a failed launch still joins the lanes that started
+        for (int k = 0; k < 4 && le == cudaSuccess; ++k) {
+          if (long_grid_[k] == 0) continue;
+          le = launch_forward_long(q, long_grid_[k], long_smem_, long_block_, 8 >> k, lane(k));
+          q.bnd = static_cast<unsigned char*>(q.bnd) + (size_t)long_grid_[k] * (size_t)q.bnd_cols * 4 * sizeof(double);
+        }
+        if (bv_status js = join(4); js != BV_OK) return js;
+        BV_CUDA(le, "FP64 long-read launch");
+      }
     }
     BV_CUDA(launch_f64(0, p, lp.grid, stream_), "FP64 forward launch");
     p.cells_ctr = nullptr;
@@ -930,14 +969,16 @@ bv_status Engine::finish(bv_phmm_stats* stats) {
     }
     stats->fp32_skipped_cells = (int64_t)c.fp32_skipped_cells;
     stats->underflow = (int64_t)c.underflow_count;
+    const int clusters = (int)(4 - std::count(long_grid_, long_grid_ + 4, 0));
+    const int long_launches = long_plan_.grid == 0 ? 0 : clusters > 0 ? clusters : 1;
     // band mode: k-mer tables, nibble image, read k-mers, gap check, two featurisers, MLP, route,
     // scan, route; the banded kernels; the fallback's units and bins; the rescore's;
     // the audit's; the FP64 pass
     stats->kernel_launches = band_enabled()
                                  ? 9 + (band_opt_.use_mlp ? 1 : 0) + kBandWidths + 1 + full_bins_ +
                                        (band_opt_.cap_margin > 0 ? 1 + full_bins_ : 0) +
-                                       (band_opt_.audit_period > 0 ? 2 + full_bins_ : 0) + 1 + (long_plan_.grid > 0)
-                                 : (int64_t)plans_.size() + 1 + (long_plan_.grid > 0);
+                                       (band_opt_.audit_period > 0 ? 2 + full_bins_ : 0) + 1 + long_launches
+                                 : (int64_t)plans_.size() + 1 + long_launches;
     stats->ms_fp32 = ms32;
     stats->ms_fp64 = ms64;
     if (band_enabled()) {

@@ -266,7 +266,9 @@ class Engine {
   int long_warps_ = kLongWarps;
   bool long_set_ = false;
   int long_block_ = kLongWarps;
-  int long_cluster_ = 1;  // blocks per pair
+  // clusters of 8, 4, 2 and 1 blocks a pair: each launch's grid (all 0: a block a pair), and the cost limit
+  int long_grid_[4] = {};
+  long long long_limit_ = 0;
   int long_rows() const { return long_set_ ? long_warps_ * 128 : kF64ShortMax + 1; }
   int long_smem_ = 0;
   int64_t n_results_ = 0;

@@ -50,6 +50,7 @@ struct KernelParams {
   int rescale;            // renormalise between strips (FP64, multi-strip)
   int rescale_target;     // binary exponent the boundary maximum is scaled to
   unsigned long long* cells_ctr;  // if set, FP64 launches add read x haplotype length per pair here
+  long long long_cost;    // long-read kernel on clusters: the cost limit that gives each pair its blocks
   int long_rows;          // > 0: FP32 results of reads this long or longer go to the FP64 list's long part
 };
 
@@ -69,8 +70,23 @@ cudaError_t launch_f64(int rt, const KernelParams& p, int grid, cudaStream_t st)
 constexpr int kLongWarps = 4;
 bool long_warps_valid(int warps);
 int long_smem_bytes(int hap_bytes, int warps);
-// `blocks` > 1 (16 warps each): clusters of that many blocks per pair, grid a multiple of it.
+// `blocks` > 0 (16 warps each): clusters of that many blocks per pair, grid a multiple of it; the launch takes
+// the listed pairs (kLongMembers at most) whose long_blocks is `blocks`.  0: a block per pair, all pairs.
 constexpr int kLongMaxBlocks = 8;
+constexpr int kLongMembers = 512;
+// Wavefront steps of a pair on `blocks` blocks: strips of 128 rows on 16 x blocks
+// warps, each strip some 96 columns behind the one above it.
+__host__ __device__ inline long long long_cost(long long R, long long H, int blocks) {
+  const long long strips = (R + 128) / 128, W = 16 * blocks, full = (strips - 1) / W;
+  return full * (H > 96 * W ? H : 96 * W) + H + 96 * (strips - full * W);
+}
+// The fewest blocks (1, 2, 4, 8) that keep a pair's cost within the limit, or make it as small as it gets.
+__host__ __device__ inline int long_blocks(long long R, long long H, long long limit) {
+  int best = 1;
+  for (int c = 2; c <= kLongMaxBlocks && long_cost(R, H, best) > limit; c *= 2)
+    if (long_cost(R, H, c) < long_cost(R, H, best)) best = c;
+  return best;
+}
 cudaError_t prepare_long(int smem, int warps, int blocks);
 int long_blocks_per_sm(int smem, int warps);
 int long_clusters(int smem, int warps, int blocks);  // clusters that run at once

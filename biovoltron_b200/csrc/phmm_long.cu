@@ -29,20 +29,23 @@
 // column) and falls by at most 2^-500, so nothing that matters leaves the
 // range whatever the length of the read.
 //
-// Few pairs: a cluster of up to eight blocks takes a pair, its warps numbered
-// through, so that 16 x blocks strips run at once; the boundary rows between
+// Up to a few hundred pairs: a cluster of up to eight blocks takes a pair, its warps numbered
+// through, so that 16 x blocks strips run at once (long reads get more blocks
+// than short ones: a launch for each cluster size, side by side, each picking
+// its pairs from the list); the boundary rows between
 // two blocks go through the producer's global buffer like a group's last row,
 // with the chunk counter in global memory (release / acquire).  The cluster
-// guarantees that its blocks run at the same time; pairs are dealt to clusters
-// in snake order, longest first, and the blocks meet at the end of each.
+// guarantees that its blocks run at the same time; a launch's pairs are dealt
+// to its clusters in snake order, costliest first, and the blocks meet at the
+// end of each.
 //
 // A pair with a row that cannot be folded, or whose result is not a positive
 // finite number, is handed back to k_f64_list (its list entry marked), which
 // runs after this kernel.
 //
 // Bound by the issue slots of the FP64 instructions (two each): 40 reads of up to
-// 10 kb take 6.8 ms with two blocks of 16 warps a pair (11 with one, 28 with four
-// warps), 8 of them 2.8 ms with eight blocks, 2,000 of them 77 ms, where the unscaled form with four warps, emissions in shared memory and one scale
+// 10 kb take 3.5 ms with one to eight blocks of 16 warps a pair (6.8 with two
+// each, 11 with one, 28 with four warps), 8 of them 2.8 ms with eight blocks, 2,000 of them 77 ms, where the unscaled form with four warps, emissions in shared memory and one scale
 // a group of strips took 58 and 169.
 //
 // The haplotype codes are staged once per pair for all warps.  Every wait is
@@ -401,14 +404,38 @@ __global__ void __launch_bounds__(K * kWarp, 16 / K) k_forward_long(KernelParams
   const DeviceBatch& b = p.batch;
   const unsigned long long n_long = min(p.ctr->rescue_long_count, (unsigned long long)p.rescue_cap);
   __syncwarp();
-  if (CL) cluster_sync();  // every count is zero
+  __shared__ long long member_cost[CL ? kLongMembers : 1];  // the listed pairs' costs, -1: other launches'
+  __shared__ int members[CL ? kLongMembers : 1], n_members;
+  if (CL) {
+    // this launch's pairs, the costliest first (every block of every cluster finds the same order)
+    const int n = (int)min(n_long, (unsigned long long)kLongMembers);
+    long long cost = -1;
+    if (threadIdx.x == 0) n_members = 0;
+    if (threadIdx.x < n) {
+      const PairRef pr = p.rescue[p.rescue_cap - 1 - threadIdx.x];
+      const int read = pr.read < 0 ? ~pr.read : pr.read;  // handed back by another cluster already
+      const long long R = b.read_off[read + 1] - b.read_off[read], H = b.hap_off[pr.hap + 1] - b.hap_off[pr.hap];
+      if (long_blocks(R, H, p.long_cost) == blocks) cost = long_cost(R, H, blocks);
+      member_cost[threadIdx.x] = cost;
+    }
+    __syncthreads();
+    if (cost >= 0) {
+      int at = 0;
+      for (int t = 0; t < n; ++t) at += member_cost[t] > cost || (member_cost[t] == cost && t < threadIdx.x);
+      members[at] = threadIdx.x;
+      atomicAdd(&n_members, 1);
+    }
+    __syncthreads();
+    cluster_sync();  // every count is zero
+  }
   for (long long round = 0;; ++round) {
     long long wi;
     if (CL) {
       // dealt in snake order; every block of a cluster takes the same pairs, and leaves after the same one
-      wi = round * teams + (round & 1 ? teams - 1 - team : team);
-      if (round * teams >= (long long)n_long) break;
-      if (wi >= (long long)n_long) continue;
+      const long long m = round * teams + (round & 1 ? teams - 1 - team : team);
+      if (round * teams >= n_members) break;
+      if (m >= n_members) continue;
+      wi = members[m];
     } else {
       if (threadIdx.x == 0) sh.item = (long long)atomicAdd(&p.ctr->rescue_long_next, 1ull);
       __syncthreads();
@@ -472,7 +499,7 @@ __global__ void __launch_bounds__(K * kWarp, 16 / K) k_forward_long(KernelParams
 template <int K, bool CL>
 const void* kernel() { return reinterpret_cast<const void*>(&k_forward_long<K, CL>); }
 const void* kernel_of(int warps, int blocks) {
-  if (blocks > 1) return warps == 16 ? kernel<16, true>() : nullptr;
+  if (blocks > 0) return warps == 16 ? kernel<16, true>() : nullptr;
   return warps == 2 ? kernel<2, false>() : warps == 4 ? kernel<4, false>() : warps == 8 ? kernel<8, false>() : kernel<16, false>();
 }
 cudaLaunchConfig_t config_of(int grid, int smem, int warps, int blocks, cudaStream_t st, cudaLaunchAttribute* attr) {
@@ -481,7 +508,7 @@ cudaLaunchConfig_t config_of(int grid, int smem, int warps, int blocks, cudaStre
   c.blockDim = dim3(warps * kWarp);
   c.dynamicSmemBytes = (size_t)smem;
   c.stream = st;
-  if (blocks > 1) {
+  if (blocks > 0) {
     attr->id = cudaLaunchAttributeClusterDimension;
     attr->val.clusterDim.x = (unsigned)blocks;
     attr->val.clusterDim.y = 1;
@@ -506,8 +533,8 @@ cudaError_t prepare_long(int smem, int warps, int blocks) { return raise_dynamic
 
 int long_blocks_per_sm(int smem, int warps) {
   int nb = 0;
-  if (prepare_long(smem, warps, 1) != cudaSuccess) return 0;
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, kernel_of(warps, 1), warps * kWarp, smem) != cudaSuccess) return 0;
+  if (prepare_long(smem, warps, 0) != cudaSuccess) return 0;
+  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, kernel_of(warps, 0), warps * kWarp, smem) != cudaSuccess) return 0;
   return nb;
 }
 

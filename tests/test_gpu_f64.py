@@ -142,3 +142,24 @@ def test_longest_haplotypes(oracle):
     b = W._build([_pair(rng, n, 32768) for n in (100, 157, 190, 253)], "long haplotypes")
     with PairHMMEngine(precision="f64") as e:
         _check(b, e.compute_regions(b), oracle)
+
+
+@pytest.mark.parametrize("pairs", [100, 512, 513])
+def test_long_reads_of_very_different_lengths(oracle, pairs):
+    """Cluster launches of every size side by side (a few long reads among many short ones), up to the most pairs
+    they take and one more."""
+    from biovoltron_b200.pairhmm import PairHMMEngine
+    rng = np.random.default_rng(13)
+    some = [_pair(rng, n, n + 100) for n in (6000, 4100, 2300, 1000, 520, 254, 300)]
+    some.append(_pair(rng, 3000, 900, related=False))
+    regions = some + [some[4 + k % 3] for k in range(pairs - len(some))]
+    b = W._build(regions, "very different lengths")
+    with PairHMMEngine(precision="f64") as e:
+        got = e.compute_regions(b)
+        first = W._build(some, "one of each")
+        _check(first, got[:len(some)], oracle)
+        assert np.array_equal(got[len(some):], np.array([got[4 + k % 3] for k in range(pairs - len(some))]))
+        n = e.stage(b)
+        for _ in range(3):
+            e.run()
+            assert np.array_equal(e.fetch(n), got)
