@@ -94,3 +94,25 @@ def test_one_haplotype_a_warp(oracle, gap):
     fin = np.isfinite(truth)
     assert np.array_equal(np.isfinite(out[0]), fin)
     assert np.max(np.abs(out[0][fin] - truth[fin])) <= TOL_FP32
+
+
+# reads of several strips that stay in FP32, at the strips' edges (256 rows, the initial and the summing row among
+# them), haplotypes shorter than a 32-column chunk and around its multiples, rows that cannot be folded
+@pytest.mark.parametrize("gap", [45, 2])
+@pytest.mark.parametrize("read_len", [254, 255, 256, 510, 511, 512, 766, 767])
+def test_strips(oracle, read_len, gap):
+    from biovoltron_b200.pairhmm import PairHMMEngine
+    rng = np.random.default_rng(read_len + gap)
+    regions = []
+    for hap_len in (read_len, read_len + 1, read_len + 31, read_len + 32, read_len + 33, read_len + 200):
+        hap = W._random_seq(rng, hap_len)
+        q, i, d, c = W._quals(rng, read_len, 40, 45)
+        i, d = np.full(read_len, gap, np.uint8), np.full(read_len, gap, np.uint8)
+        regions.append(([(hap[:read_len].copy(), q, i, d, c)], [hap, hap[:read_len].copy(), hap[:20].copy()]))
+    b = W._build(regions, "strips")
+    truth = oracle.log10_rescaled(TestcaseArray.for_batch(b))
+    with PairHMMEngine() as e:
+        got, st = e.compute_regions(b, with_stats=True)
+        assert np.max(np.abs(got - truth)) <= TOL_FP32
+        if gap == 45:  # the reads match: only the haplotypes of 20 bases need FP64
+            assert st["rescued"] <= len(regions)
