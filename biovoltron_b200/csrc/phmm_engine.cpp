@@ -491,15 +491,16 @@ bv_status Engine::plan(const bv_region_batch& b) {
     long_smem_ = long_smem_bytes(rp.hap_bytes, long_block_);
     if (long_smem_ <= 227 * 1024) {
       // Up to a few hundred pairs: a cluster of blocks for each, the blocks dealt by the pairs' costs (long_cost):
-      // the lowest limit for which all pairs' blocks together are at most the SMs, or 2/5 of them more than there
-      // are pairs.  FP64 pass of reads of up to 10 kb, one block a pair -> this, ms: 40 pairs 11.1 -> 3.5, 90 12.2 ->
+      // the lowest limit for which all pairs' blocks together are at most the SMs (but eight: a cluster's have to be
+      // neighbours, and one that finds no place waits for the others: 40 pairs 4.4-4.8 instead of 3.5-3.7 ms), or
+      // 2/5 of them more than there are pairs.  FP64 pass of reads of up to 10 kb, one block a pair -> this, ms: 40 pairs 11.1 -> 3.7, 90 12.2 ->
       // 6.0, 148 11.9 -> 9.6, 256 15.9 -> 11.5, 512 25.7 -> 20.1 (one cluster size for all pairs: 40 pairs 6.8, 90
       // 12.2; totals of 112 to 400 blocks tried at 40 to 256 pairs).  Pairs of one length get a block each: then,
       // and beyond, the blocks take the next pair from the list.
       std::fill(long_grid_, long_grid_ + 4, 0);
       int64_t budget = 0;
       if (long_block_ == 16 && !long_set_ && n_long <= kLongMembers)
-        budget = std::max<int64_t>(sms_, n_long + sms_ * 2 / 5);
+        budget = std::max<int64_t>(sms_ - 8, n_long + sms_ * 2 / 5);
       if (n_long <= budget) {
         std::vector<std::pair<int64_t, int64_t>> pairs;  // read and haplotype lengths
         std::vector<long long> limits;

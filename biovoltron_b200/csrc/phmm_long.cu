@@ -44,7 +44,7 @@
 // runs after this kernel.
 //
 // Bound by the issue slots of the FP64 instructions (two each): 40 reads of up to
-// 10 kb take 3.5 ms with one to eight blocks of 16 warps a pair (6.8 with two
+// 10 kb take 3.7 ms with one to eight blocks of 16 warps a pair (6.8 with two
 // each, 11 with one, 28 with four warps), 8 of them 2.8 ms with eight blocks, 2,000 of them 77 ms, where the unscaled form with four warps, emissions in shared memory and one scale
 // a group of strips took 58 and 169.
 //
