@@ -521,7 +521,7 @@ def main():
                        "parallelism": f"dp{world} (independent regions, one replica per GPU)",
                        "generate_s": round(t_gen, 1),
                        "launch_shapes": tuning or "engine defaults (2 haplotypes per warp, 4 warps per block)",
-                       "long_read_kernel": long_tuning or "engine default (4 warps per pair, reads of 512 bases on)"},
+                       "long_read_kernel": long_tuning or "engine default (2 to 16 warps per pair or a cluster, reads of 254 bases on)"},
         }
         if plain is not None:
             pl = plain["steps"][-1]
@@ -583,8 +583,8 @@ def main():
         if fp64_cells > 0 and fp64_ms > 0:
             a64 = FLOPS_PER_CELL * fp64_cells / (fp64_ms / 1e3) / 1e12
             line["roofline_fp64"] = {"bound": "fp64",
-                                     "kernel": "k_forward_long<4> (reads >= 512 bases, a block of four warps per "
-                                               "pair) and k_forward<double, 4, multi-strip> (FP64 pass)",
+                                     "kernel": "k_forward_long (reads of several strips, several warps per pair), "
+                                               "k_f64_units and k_f64_list (FP64 pass)",
                                      "achieved": a64, "peak": fp64_peak, "unit": "TFLOP/s",
                                      "frac": (a64 / fp64_peak) if fp64_peak else None,
                                      "cells": fp64_cells, "ms": fp64_ms, "flops_per_cell": FLOPS_PER_CELL}

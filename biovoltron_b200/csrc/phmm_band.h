@@ -4,12 +4,12 @@
 //   k_pairs_from_units  expand work units into one (read, hap) per result slot
 //   k_hap_table         per haplotype: 11-mer hash table (code -> positions)
 //   k_read_kmers        per read position: 11-mer code
-//   k_featurize_t       one thread per pair: shared 11-mer diagonal votes ->
+//   k_featurize_u       a warp per work unit: shared 11-mer diagonal votes ->
 //                       features, seed diagonal d* (the votes' mode), band
 //                       extent (voted diagonals and read-end triangles); a
-//                       pair voting for more diagonals than a thread keeps
-//                       goes to k_featurize_slow (one warp per pair, a
-//                       histogram in global scratch), with the same results
+//                       pair with a repeated 11-mer goes to k_featurize_slow
+//                       (one warp per pair, a histogram in global scratch),
+//                       with the same results
 //   k_mlp_forward       per pair: BF16 MLP 80-128-128-2 (FP32 accumulation) ->
 //                       lower and upper band edge relative to d*
 //   k_band_route        band (by width class and read-length bucket) or full DP
