@@ -130,6 +130,12 @@ bv_status Engine::compute_chunked(Engine& other, const bv_region_batch& b, doubl
     // last user of this context's offset buffer, has been drained
     ck[k].build(b, e.chunk_offsets());
     s = e.stage(ck[k].view, false);
+    // Chunk k - 1's kernels first: side by side both chunks end late, and the device then waits for the host,
+    // which stages chunk k + 1 once k - 1 has ended (60,000 regions of a 30x genome, 9 chunks: 110 -> 101 ms).
+    // The last chunk may run beside the one before (8,000 regions, 2 chunks: 14.8 ms, in order 15.7).
+    if (s == BV_OK && k >= 1 && k + 1 < ck.size() &&
+        cudaStreamWaitEvent(e.stream_, eng[(k - 1) % 2]->ev_[4], 0) != cudaSuccess)
+      s = e.fail(BV_ERR_CUDA, "chunk order");
     if (s == BV_OK) s = e.launch();
     if (s != BV_OK) return abort(fail(s, e.last_error()));
     if (k >= 1) {
