@@ -23,11 +23,20 @@
 // Scale.  Every strip keeps its own power of two E (true values are stored
 // values * 2^E) and a chunk carries the E it was written with.  Before a
 // chunk the warp looks at the largest exponent among its states and the
-// incoming sums and, when that has left [2^-100, 2^400], moves it to 2^200: all
-// states are multiplied by one exact power of two.  Inside a chunk (32
-// columns) a state grows by at most ~2^350 (a gap's continuation undone once a
-// column) and falls by at most 2^-500, so nothing that matters leaves the
-// range whatever the length of the read.
+// incoming sums and, when that has left [2^600, 2^1010], moves it to 2^1000: all
+// states are multiplied by exact powers of two.  E holds for all 128 rows of
+// the strip, and the top rows are the largest: a path that loses a whole strip
+// (a stretch of the read that does not align, insertion runs too dear to bridge
+// it: 11 to 15 binary orders a row at base qualities 25 to 40) has to fit below
+// them, and may still be the one that counts in the end.  So the largest state
+// stands at the top of the range: 2,000 binary orders a strip are kept, as by
+// the unscaled form, whose strips start at 2^1000 too (from 2^200, an exponent
+// that leaves room for growth, 922 to 1,422 are, and a read of 300 bases whose
+// bases 45-172 do not align scored 10^-436 instead of 10^-384).  What lies
+// further below is lost there as here.  Inside a chunk (32 columns) states grow
+// by little: all of a row's mass comes from the row above it, and X / pMX by
+// what the insertion quality jumps from one row to the next; beyond 2^13 they
+// overflow and the pair is handed back.
 //
 // Up to a few hundred pairs: a cluster of up to eight blocks takes a pair, its warps numbered
 // through, so that 16 x blocks strips run at once (long reads get more blocks
@@ -39,9 +48,11 @@
 // to its clusters in snake order, costliest first, and the blocks meet at the
 // end of each.
 //
-// A pair with a row that cannot be folded, or whose result is not a positive
-// finite number, is handed back to k_f64_list (its list entry marked), which
-// runs after this kernel.
+// A pair with a row that cannot be folded, with a row between two strips whose
+// largest sum lies below 2^-960 in the largest scale of the strip that wrote it
+// (so that what that strip lost may count), or whose result lies below 2^-960 in
+// the last strip's scale or is not finite, is handed back to k_f64_list (its
+// list entry marked), which runs after this kernel.
 //
 // Bound by the issue slots of the FP64 instructions (two each): 40 reads of up to
 // 10 kb take 3.7 ms with one to eight blocks of 16 warps a pair (6.8 with two
@@ -67,8 +78,9 @@ constexpr int kLongRT = 4;                // rows per lane
 constexpr int kStrip = kWarp * kLongRT;   // rows per strip
 constexpr int kLongSlots = 4;             // chunk slots per channel
 constexpr int kChunkB = 32 * 16;          // one 32-column chunk of (zx, zm)
-constexpr int kTop = 200;                 // exponent the largest state is moved to
-constexpr int kTopMax = 400, kTopMin = -100;
+constexpr int kTop = 1000;                // exponent the largest state is moved to
+constexpr int kTopMax = 1010, kTopMin = 600;
+constexpr int kMinExp = -960;             // of a row's largest sum, and of the result
 constexpr int kNoExp = -(1 << 24);        // "no value": below every exponent
 
 // Dynamic shared memory of a block of K warps, after the staged haplotype
@@ -154,10 +166,18 @@ __device__ __forceinline__ int exp_of(double v) {
   const int e = (__double2hiint(v) >> 20) & 0x7ff;
   return e == 0 ? kNoExp : e - 1023;
 }
-// 2^d, exact; zero below 2^-1000 (a value that far below the others does not count).
-__device__ __forceinline__ double pow2(int d) {
-  return d < -1000 ? 0.0 : __hiloint2double((min(d, 1000) + 1023) << 20, 0);
-}
+// 2^d, exact; zero below 2^-1022.  d <= 1000.
+__device__ __forceinline__ double pow2(int d) { return d < -1022 ? 0.0 : __hiloint2double((d + 1023) << 20, 0); }
+// v 2^d: a strip's scale may move by more than one power of two holds.
+struct Pow2 {
+  double a, b;
+  __device__ __forceinline__ explicit Pow2(int d) {
+    d = max(-2100, min(d, 2000));  // below: zero, as it should be; above: no value that is kept needs more
+    a = pow2(d / 2);
+    b = pow2(d - d / 2);
+  }
+  __device__ __forceinline__ double operator()(double v) const { return v * a * b; }
+};
 
 // The 32 steps of a chunk.  hc: the lane's first column code; stage: what lane
 // 0 consumes; o: where lane 31's last row goes (kChan: shared, kGlobal: global
@@ -246,6 +266,8 @@ __device__ __forceinline__ int run_strip_long(const F64Rows<kLongRT>& w, const u
       ahead_e = __ldcg(io.src_e + 1);
     }
   }
+  // the largest sum of the row above (this lane's share), the largest scale it came in
+  int row_top = max(exp_of(carry.x), exp_of(carry.y)) + carry_e, row_e = carry_e;
   if (!first) E = carry_e;
   else io.stage[lane] = make_double2(0.0, 0.0);
   double2 z = make_double2(0.0, 0.0);  // nothing lies above column 0
@@ -281,36 +303,39 @@ __device__ __forceinline__ int run_strip_long(const F64Rows<kLongRT>& w, const u
       top += E;
       top = max(top, max(exp_of(nx.x), exp_of(nx.y)) + nx_e);
       if (lane == kWarp - 1) top = max(top, max(exp_of(carry.x), exp_of(carry.y)) + carry_e);
-      top = __reduce_max_sync(0xffffffffu, top);
+      // (The broadcast says that the value is the warp's.  Without it the warp runs a strip's later chunks in parts:
+      // the 40 pairs 8.4 instead of 3.7 ms.)
+      top = __shfl_sync(0xffffffffu, __reduce_max_sync(0xffffffffu, top), 0);
       if (top > kNoExp / 2 && (top - E > kTopMax || top - E < kTopMin)) {
-        const int d = min(E - (top - kTop), 1000);  // stored values times 2^d
-        const double f = pow2(d);
+        const int d = min(E - (top - kTop), 2000);  // stored values times 2^d
+        const Pow2 f(d);
 #pragma unroll
         for (int j = 0; j < kLongRT; ++j) {
-          st.M[j] *= f;
-          st.X[j] *= f;
-          st.Y[j] *= f;
+          st.M[j] = f(st.M[j]);
+          st.X[j] = f(st.X[j]);
+          st.Y[j] = f(st.Y[j]);
         }
-        z.x *= f;
-        z.y *= f;
-        sumM *= f;
-        sumX *= f;
-        y0 *= f;
+        z.x = f(z.x);
+        z.y = f(z.y);
+        sumM = f(sumM);
+        sumX = f(sumX);
+        y0 = f(y0);
         E -= d;
       }
     }
     if (!first) {
       // lane 0's inputs of this chunk: the carried entry, then the next chunk's first 31
-      const double f = pow2(nx_e - E);
-      const double2 v = make_double2(nx.x * f, nx.y * f);
-      if (lane < kWarp - 1) {
-        io.stage[lane + 1] = v;
-      } else {
-        const double fc = pow2(carry_e - E);
-        io.stage[0] = make_double2(carry.x * fc, carry.y * fc);
-      }
+      const bool edge = lane == kWarp - 1;
+      const Pow2 f((edge ? carry_e : nx_e) - E);
+      io.stage[edge ? 0 : lane + 1] = make_double2(f(edge ? carry.x : nx.x), f(edge ? carry.y : nx.y));
       carry = nx;
       carry_e = nx_e;
+      row_top = max(row_top, max(exp_of(nx.x), exp_of(nx.y)) + nx_e);
+      row_e = max(row_e, nx_e);
+      if (k + 1 == nch && __reduce_max_sync(0xffffffffu, row_top) < row_e + kMinExp) {
+        sumM = __longlong_as_double(0x7ff8000000000000ll);  // a NaN in the chunk's first column, or in the result
+        st.M[kLongRT - 1] = sumM;
+      }
     }
     const int slot = k % kLongSlots;
     if (lane == kWarp - 1 && out == kChan) {
@@ -351,7 +376,7 @@ template <int K, bool CL>
 __global__ void __launch_bounds__(K * kWarp, 16 / K) k_forward_long(KernelParams p) {
   using L = LongLayout<K>;
   extern __shared__ __align__(16) unsigned char smem[];
-  const int lane = threadIdx.x & (kWarp - 1), w = threadIdx.x >> 5;
+  const int lane = threadIdx.x & (kWarp - 1), w = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0);
   unsigned char* hc = smem;
   unsigned char* base = smem + p.hap_bytes;
   uint64_t* bars = reinterpret_cast<uint64_t*>(base + L::kBars);
@@ -445,7 +470,8 @@ __global__ void __launch_bounds__(K * kWarp, 16 / K) k_forward_long(KernelParams
     PairRef pr = p.rescue[p.rescue_cap - 1 - wi];
     if (CL && pr.read < 0) pr.read = ~pr.read;  // another block of the cluster is through and has handed it back
     const int64_t ro = b.read_off[pr.read], ho = b.hap_off[pr.hap];
-    const int R = (int)(b.read_off[pr.read + 1] - ro), H = (int)(b.hap_off[pr.hap + 1] - ho);
+    const int R = __shfl_sync(0xffffffffu, (int)(b.read_off[pr.read + 1] - ro), 0);
+    const int H = __shfl_sync(0xffffffffu, (int)(b.hap_off[pr.hap + 1] - ho), 0);
     const uchar4* quals = b.read_quals + ro;
     const uint8_t* bases = b.read_bases + ro;
     if (H == 0 || R == 0) {
@@ -456,8 +482,8 @@ __global__ void __launch_bounds__(K * kWarp, 16 / K) k_forward_long(KernelParams
     const int nch = (H + kWarp - 1 + 31) / 32;
     const int nstrips = (R + 1 + kStrip - 1) / kStrip;
     const int pad = nstrips * kStrip - (R + 1);  // padding rows on top of row 0
-    // initial row: init / H, stored with exponent y0_exp
-    const int y0_exp = kF64InitExp - kTop;
+    // initial row: init / H, stored with exponent y0_exp, just below 2^1009
+    const int y0_exp = kF64InitExp - kTop - 8 - (31 - __clz(H));
     const double y0 = ldexp(p.tables->init_d, -y0_exp) / (double)H;
     stage_hap_block(b.hap_bases + ho, H, hc, 32 * nch + kHapLead);
     __syncthreads();
@@ -476,7 +502,7 @@ __global__ void __launch_bounds__(K * kWarp, 16 / K) k_forward_long(KernelParams
       if (last && lane == kWarp - 1) {
         const double pmx = p.tables->const_mode ? p.tables->cd[1] : p.tables->ph2pr_d[quals[R - 1].y & kQualMask];
         const double res = sumM + pmx * sumX;
-        if (res > 0.0 && isfinite(res)) {
+        if (res >= pow2(kMinExp) && isfinite(res)) {
           write_result<double>(p, pr.read, pr.hap, pr.out, res, E);
           if (p.cells_ctr) atomicAdd(p.cells_ctr, (unsigned long long)R * (unsigned long long)H);
         } else {

@@ -163,3 +163,69 @@ def test_long_reads_of_very_different_lengths(oracle, pairs):
         for _ in range(3):
             e.run()
             assert np.array_equal(e.fetch(n), got)
+
+
+def _strip_bases(n, strip):
+    """The read bases [a, b) whose rows the long-read kernel's strip holds (128 rows, row 0 and the padding on top)."""
+    pad = -(n + 1) % 128
+    return max(0, 128 * strip - pad - 1), 128 * (strip + 1) - pad - 1
+
+
+def _blocked(rng, n, q, gcp, strips, rival):
+    """A read of A and C; a haplotype that is the read but for whole strips of other bases, so that a path along it
+    loses 1,000 to 1,600 binary orders within a strip; with `rival` a second copy behind it that loses 600 to 800 in
+    each of two strips, so that the lower of two paths after one strip is the better one after both."""
+    read = rng.choice(np.frombuffer(b"AC", np.uint8), n)
+    first = read.copy()
+    for s in strips:
+        a, b = _strip_bases(n, s)
+        first[a:b] = rng.choice(np.frombuffer(b"GT", np.uint8), b - a)
+    hap = [W._random_seq(rng, 40), first, W._random_seq(rng, 40)]
+    if rival:
+        second = read.copy()
+        for s in (strips[0], strips[0] + 1):
+            a, b = _strip_bases(n, s)
+            at = a + rng.choice(b - a, 70, replace=False)
+            second[at] = rng.choice(np.frombuffer(b"GT", np.uint8), 70)
+        hap.append(second)
+    q, i, d, c = W._quals(rng, n, q, q, gcp=gcp)
+    return [(read, q, i, d, c)], [np.concatenate(hap)]
+
+
+# strips whose rows cost more than half of FP64's exponent range (a stretch of the read that does not align and
+# insertion runs too dear to bridge it), read lengths of three, five and twenty strips, the second and the last but one
+# of them, or two at once; one path, or two of which the one that is lower after the strip wins in the end
+@pytest.mark.parametrize("rival", [False, True])
+@pytest.mark.parametrize("n", [300, 600, 2500])
+def test_long_reads_that_lose_most_of_the_range_in_a_strip(oracle, n, rival):
+    from biovoltron_b200.pairhmm import PairHMMEngine
+    rng = np.random.default_rng(n)
+    last = (n + 1 + 127) // 128 - 1
+    regions = [_blocked(rng, n, q, gcp, strips, rival)
+               for q, gcp in ((25, 40), (26, 30), (28, 45), (30, 40), (30, 60))
+               for strips in ([1], [last - 1], [last - 1] if rival else [1, last])]
+    if n <= 600:  # a read that belongs to nothing in a short haplotype
+        regions.append(_pair(rng, n, 180, related=False, gaps=(45, 45, 30), qlo=30, qhi=34))
+    b = W._build(regions, "range within a strip")
+    for precision in ("f64", "auto"):  # every pair in FP64, and the rescue
+        with PairHMMEngine(precision=precision) as e:
+            got, st = e.compute_regions(b, with_stats=True)
+            assert st["rescued"] == b.n_pairs
+            _check(b, got, oracle)
+            for k in (2, 4, 8):
+                if n >= 128 * k:  # the long-read kernel's edge
+                    e.set_long_warps(k)
+                    _check(b, e.compute_regions(b), oracle)
+
+
+def test_constant_transitions_that_lose_most_of_the_range_in_a_strip(oracle):
+    """Insertion runs that are dear by a small insertion-to-insertion probability."""
+    from biovoltron_b200.pairhmm import PairHMMEngine
+    rng = np.random.default_rng(17)
+    b = W._build([_blocked(rng, 300, q, 10, [1], False) for q in (25, 28, 30)], "scalar, range within a strip")
+    trans = (0.9998, 0.0001, 0.0001, 0.999999, 0.000001, 0.9, 0.1)
+    with PairHMMEngine(precision="f64") as e:
+        e.set_transitions(trans)
+        got = e.compute_regions(b)
+    want = [oracle.scalar_log10(bytes(b.read(k)[0]), bytes(b.read(k)[1]), b.hap(k), trans) for k in range(b.n_reads)]
+    assert np.max(np.abs(got - want)) <= TOL
