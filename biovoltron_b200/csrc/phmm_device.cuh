@@ -992,14 +992,22 @@ __device__ void process_item(const KernelParams& p, const Item& it, unsigned cha
           }
         }
         in_scale = T(1);
-        if (p.rescale && st + 1 < nstrips) {
+        if (sizeof(T) == 8 && p.rescale && st + 1 < nstrips) {
           const T m = __shfl_sync(0xffffffffu, bmax, kWarp - 1);
           if (m > T(0)) {
             int e2;
             frexp((double)m, &e2);
             // keep the row maximum near 2^(target) so the next strip has headroom
-            const int shift = e2 - p.rescale_target;
+            int shift = e2 - p.rescale_target;
             kexp += shift;
+            // a row that a strip has left below 2^-23 or so needs more than one factor: raised where it lies
+            for (; shift < -1000; shift += 1000) {
+              for (int x = lane; x < nsteps + 96; x += kWarp) {
+                bnd[(size_t)x * 4 + 0] *= (T)0x1p1000;
+                bnd[(size_t)x * 4 + 1] *= (T)0x1p1000;
+                bnd[(size_t)x * 4 + 2] *= (T)0x1p1000;
+              }
+            }
             in_scale = (T)ldexp(1.0, -shift);
           }
         }

@@ -229,3 +229,18 @@ def test_constant_transitions_that_lose_most_of_the_range_in_a_strip(oracle):
         got = e.compute_regions(b)
     want = [oracle.scalar_log10(bytes(b.read(k)[0]), bytes(b.read(k)[1]), b.hap(k), trans) for k in range(b.n_reads)]
     assert np.max(np.abs(got - want)) <= TOL
+
+
+# the unscaled strips, which reads below the long-read kernel's edge take (512 bases with 4 warps, 1,024 with 8) and
+# pairs that other kernels hand back: a row between two strips below 2^-24 needs a factor of more than 2^1023
+@pytest.mark.parametrize("n", [300, 600])
+def test_unscaled_strips_that_lose_most_of_the_range(oracle, n):
+    from biovoltron_b200.pairhmm import PairHMMEngine
+    rng = np.random.default_rng(n)
+    regions = [_blocked(rng, n, q, gcp, strips, False) for q, gcp in ((15, 30), (20, 30), (25, 40), (28, 45), (30, 60))
+               for strips in ([1], [1, (n + 128) // 128 - 1])]
+    regions += [_pair(rng, n, 180, related=False, gaps=(45, 45, gcp), qlo=30, qhi=34) for gcp in (20, 25, 30)]
+    b = W._build(regions, "unscaled strips")
+    with PairHMMEngine(precision="f64") as e:
+        e.set_long_warps(8)
+        _check(b, e.compute_regions(b), oracle)
