@@ -863,8 +863,15 @@ static __device__ __noinline__ bool fp32_result_below_threshold(const Tables* tb
   return growth < 100.f && 2.f * mass * exp2f(growth) < (float)kMinAccepted;
 }
 
+// FP64 strips: a row between two strips, or a result, below kF64MinRow in its
+// strip's scale (whose rows start at 2^rescale_target) has lost its precision,
+// or all of it, to the end of the range.  With RT > 1 nothing is written then
+// and the return value is false: process_item_f64 runs the item again in strips
+// of 32 rows, which lose a quarter as much.
+constexpr double kF64MinRow = 0x1p-960;
+
 template <typename T, int RT, bool MULTI, bool PAIR = false>
-__device__ void process_item(const KernelParams& p, const Item& it, unsigned char* wsm, int lane, T* bnd) {
+__device__ bool process_item(const KernelParams& p, const Item& it, unsigned char* wsm, int lane, T* bnd) {
   using S = WarpSmem<T, RT>;
   const DeviceBatch& b = p.batch;
   const int64_t ro = b.read_off[it.read];
@@ -956,6 +963,7 @@ __device__ void process_item(const KernelParams& p, const Item& it, unsigned cha
     T lastM, lastY, sumM, sumX, bmax;
     long long kexp = 0;  // stored values are true values * 2^-kexp
     bool handed_over = false;  // FP32: the pair went to the FP64 list before its last strip
+    [[maybe_unused]] bool lost = false;  // FP64
     if constexpr (MULTI) {
       // boundary row of "strip -1": all zero
       for (int x = lane; x < nsteps + 96; x += kWarp) {
@@ -994,6 +1002,8 @@ __device__ void process_item(const KernelParams& p, const Item& it, unsigned cha
         in_scale = T(1);
         if (sizeof(T) == 8 && p.rescale && st + 1 < nstrips) {
           const T m = __shfl_sync(0xffffffffu, bmax, kWarp - 1);
+          lost |= m < (T)kF64MinRow;
+          if (RT > 1 && lost) break;
           if (m > T(0)) {
             int e2;
             frexp((double)m, &e2);
@@ -1023,6 +1033,10 @@ __device__ void process_item(const KernelParams& p, const Item& it, unsigned cha
         run_strip<T, RT, false, 8>(rw, el, hc + kHapLead - lane, nsteps, lane, nullptr, nullptr, T(1), lastM,
                                    lastY, sumM, sumX, bmax);
     }
+    if constexpr (sizeof(T) == 8 && MULTI && RT > 1) {
+      lost |= __shfl_sync(0xffffffffu, sumM + sumX, kWarp - 1) < (T)kF64MinRow;
+      if (lost && p.rescale) return false;
+    }
     if (lane == kWarp - 1) {
       // FP32: the summing row's Y + M; FP64: the accumulated last-row sums;
       // a pair handed over early counts as below the rescue threshold.
@@ -1031,6 +1045,19 @@ __device__ void process_item(const KernelParams& p, const Item& it, unsigned cha
       if (is_f64 && p.cells_ctr) atomicAdd(p.cells_ctr, (unsigned long long)R * (unsigned long long)H);
     }
   }
+  return true;
+}
+
+// A pair in FP64, unscaled, in strips of 128 rows or, where those lose more than
+// the range holds, of 32.  (Out of line: hardly any pair needs it.)
+static __device__ __noinline__ void process_item_short_strips(const KernelParams& p, const Item& it, unsigned char* wsm,
+                                                              int lane, double* bnd) {
+  __syncwarp();
+  process_item<double, 1, true>(p, it, wsm, lane, bnd);
+}
+__device__ __forceinline__ void process_item_f64(const KernelParams& p, const Item& it, unsigned char* wsm, int lane,
+                                                 double* bnd) {
+  if (!process_item<double, 4, true>(p, it, wsm, lane, bnd)) process_item_short_strips(p, it, wsm, lane, bnd);
 }
 
 }  // namespace bvphmm

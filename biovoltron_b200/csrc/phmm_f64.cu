@@ -143,7 +143,7 @@ __global__ void __launch_bounds__(kThreadsPerBlock, RT <= 5 ? 4 : 3) k_f64_units
 // long-read kernel, which runs before, handed back.  A warp per pair: five
 // rows a lane for the reads that fit them, eight for the other short ones,
 // the unscaled strips for the rest.
-__global__ void __launch_bounds__(kThreadsPerBlock, 3) k_f64_list(KernelParams p) {
+__global__ void __launch_bounds__(kThreadsPerBlock, 3) k_f64_list(const __grid_constant__ KernelParams p) {
   extern __shared__ __align__(16) unsigned char smem[];
   const int lane = threadIdx.x & (kWarp - 1), wib = threadIdx.x >> 5;
   unsigned char* wsm = smem + (size_t)wib * p.warp_smem_bytes;
@@ -177,7 +177,7 @@ __global__ void __launch_bounds__(kThreadsPerBlock, 3) k_f64_list(KernelParams p
         done = f64_pair<8>(p, w, fold, pr.read, R, pr.hap, pr.out, wsm, elane<double, 8>(wsm + p.hap_bytes, lane), lane);
       }
     }
-    if (!done) process_item<double, 4, true>(p, Item{pr.read, pr.hap, 1, pr.out}, wsm, lane, bnd);
+    if (!done) process_item_f64(p, Item{pr.read, pr.hap, 1, pr.out}, wsm, lane, bnd);
     // the long part's mark is cleared: a replayed batch finds the list as it was staged
     if (!front && lane == 0) p.rescue[at].read = pr.read;
   }

@@ -95,7 +95,7 @@ __global__ void k_noalloc_reset(Counters* c) {
 // Each warp takes pairs from the list; a pair whose indices or haplotype
 // length fall outside the bounds the scratch was sized for is skipped, its
 // output (when addressable) set to NaN and the status flagged.
-__global__ void __launch_bounds__(kThreadsPerBlock) k_forward_f64_noalloc(KernelParams p, long long n_pairs,
+__global__ void __launch_bounds__(kThreadsPerBlock) k_forward_f64_noalloc(const __grid_constant__ KernelParams p, long long n_pairs,
                                                                           long long n_reads, long long n_haps,
                                                                           long long n_out) {
   extern __shared__ __align__(16) unsigned char smem[];
@@ -128,7 +128,7 @@ __global__ void __launch_bounds__(kThreadsPerBlock) k_forward_f64_noalloc(Kernel
     it.hap0 = pr.hap;
     it.nh = 1;
     it.out0 = pr.out;
-    process_item<double, kRT, true>(p, it, wsm, lane, bnd);
+    process_item_f64(p, it, wsm, lane, bnd);
   }
 }
 

@@ -244,3 +244,35 @@ def test_unscaled_strips_that_lose_most_of_the_range(oracle, n):
     with PairHMMEngine(precision="f64") as e:
         e.set_long_warps(8)
         _check(b, e.compute_regions(b), oracle)
+
+
+def _hopeless(rng):
+    """Reads that lose more than 2,000 binary orders in 128 rows: bases of one kind against haplotypes of another, with
+    insertion runs as dear as mismatches."""
+    regions = []
+    for n, q, gcp in ((200, 55, 70), (254, 50, 60), (300, 48, 60), (600, 50, 50), (900, 60, 70)):
+        read = rng.choice(np.frombuffer(b"AC", np.uint8), n)
+        qs, i, d, c = W._quals(rng, n, q, q, gcp=gcp)
+        regions.append(([(read, qs, i, d, c)], [rng.choice(np.frombuffer(b"GT", np.uint8), h) for h in (n // 3, n + 70)]))
+    return W._build(regions, "hopeless reads")
+
+
+def test_strips_that_lose_more_than_the_range(oracle):
+    """What no strip of 128 rows holds is scored in strips of 32."""
+    from biovoltron_b200.pairhmm import PairHMMEngine
+    b = _hopeless(np.random.default_rng(19))
+    for precision in ("f64", "auto"):
+        with PairHMMEngine(precision=precision) as e:
+            got, st = e.compute_regions(b, with_stats=True)
+            _check(b, got, oracle)
+            assert st["underflow"] == 0 and st["rescued_cells"] == b.n_cells()
+            n = e.stage(b)
+            for _ in range(2):
+                e.run()
+                assert np.array_equal(e.fetch(n), got)
+
+
+def test_no_allocation_entry_point_on_hopeless_reads(monkeypatch):
+    import test_zz_no_alloc as no_alloc
+    monkeypatch.setattr(no_alloc, "_batch", lambda: _hopeless(np.random.default_rng(19)))
+    no_alloc.test_noalloc_matches_allocating_entry_point()
