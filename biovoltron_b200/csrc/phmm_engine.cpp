@@ -319,13 +319,12 @@ bv_status Engine::plan(const bv_region_batch& b) {
   for (int64_t g = 0; g < b.num_regions; ++g)
     n_pairs += (b.region_reads[g + 1] - b.region_reads[g]) * (b.region_haps[g + 1] - b.region_haps[g]);
   const int64_t warps = (int64_t)sms_ * 16;
-  // FP64 mode: reads that fit a strip run in units too, one haplotype at a time
-  const bool f64_units = all_f64 && !band_enabled();
-  const bool few = n_pairs * 2 <= warps && opt_.haps_per_warp != 2 && !band_enabled() && !tuning_;
-  const int per_unit = band_enabled() ? max_unit
-                       : f64_units    ? (int)std::min<int64_t>(max_unit, std::max<int64_t>(1, n_pairs / (warps * 8)))
-                       : few          ? 1
-                                      : (int)std::min<int64_t>(max_unit, std::max<int64_t>(2, n_pairs / (warps * 8) / 2 * 2));
+  // (FP64 mode: reads that fit a strip run in units too, one haplotype at a time)
+  const bool few = n_pairs * 2 <= warps && opt_.haps_per_warp != 2 && !band_runs() && !tuning_;
+  const int per_unit = band_runs() ? max_unit
+                       : all_f64   ? (int)std::min<int64_t>(max_unit, std::max<int64_t>(1, n_pairs / (warps * 8)))
+                       : few       ? 1
+                                   : (int)std::min<int64_t>(max_unit, std::max<int64_t>(2, n_pairs / (warps * 8) / 2 * 2));
   // two haplotypes per warp (paired variants) unless the options or the bin's tuning ask for one
   auto pair_rows = [&](int64_t rt) {
     if (opt_.haps_per_warp == 1 || per_unit < 2 || rt < 1 || rt > kTuneBins) return false;
@@ -336,7 +335,7 @@ bv_status Engine::plan(const bv_region_batch& b) {
   auto bin_of = [](int64_t rlen) { return (int)std::min<int64_t>((rlen + 3 + kWarp - 1) / kWarp, kBins); };
   int bin_variant[kBins + 1] = {};
   for (int rt = 1; rt <= kBins; ++rt)
-    bin_variant[rt] = f64_units      ? (rt < kBins ? kF64Bin0 + rt : kF64List)
+    bin_variant[rt] = all_f64       ? (rt < kBins ? kF64Bin0 + rt : kF64List)
                       : rt == kBins ? v_multi
                                     : variant_index(false, rt, false, pair_rows(rt));
   // pass over the reads: units per bin and, per region, where its units of each bin start
@@ -383,10 +382,10 @@ bv_status Engine::plan(const bv_region_batch& b) {
   for (int v = 0; v < kMaxVariants; ++v) start[v + 1] = start[v] + count[v];
   // the units, in result order within each bin: on the device (k_make_units, from the region arrays) or, for a
   // small batch, here; the FP64 list's pairs here
-  n_units_ = !all_f64 || f64_units ? start[kMaxVariants] : 0;
+  n_units_ = start[kMaxVariants];
   unit_haps_ = per_unit;
   for (int rt = 1; rt <= kBins; ++rt) bin_start_[rt] = base[rt].empty() || n_units_ == 0 ? -1 : start[bin_variant[rt]];
-  const bool lists = all_f64 && (!f64_units || bin_reads_[kBins - 1] > 0);
+  const bool lists = all_f64 && bin_reads_[kBins - 1] > 0;
   if (small_in_) units_.resize((size_t)n_units_);
   for (int64_t g = 0; (small_in_ || lists) && g < b.num_regions; ++g) {
     const int64_t h0 = b.region_haps[g], nh = b.region_haps[g + 1] - h0;
@@ -395,7 +394,7 @@ bv_status Engine::plan(const bv_region_batch& b) {
     for (int64_t r = b.region_reads[g]; r < b.region_reads[g + 1]; ++r, out += nh) {
       const int64_t rl = b.read_offsets[r + 1] - b.read_offsets[r];
       const int rt = bin_of(rl);
-      if (lists && (!f64_units || rt == kBins)) {
+      if (lists && rt == kBins) {
         auto& list = rl >= long_rows() ? f64_long_items_ : f64_items_;
         for (int64_t k = 0; k < nh; ++k) list.push_back(PairRef{(int32_t)r, (int32_t)(h0 + k), out + k});
         continue;
@@ -410,9 +409,10 @@ bv_status Engine::plan(const bv_region_batch& b) {
       }
     }
   }
+  unit_pairs_ = res - (int64_t)(f64_items_.size() + f64_long_items_.size());
   // launch plans
   int slot = 0;
-  for (int v = 0; v < kMaxVariants && (!all_f64 || f64_units); ++v) {
+  for (int v = 0; v < kMaxVariants; ++v) {
     if (count[v] == 0) continue;
     LaunchPlan lp;
     lp.variant = v;
@@ -760,7 +760,7 @@ bv_status Engine::stage(const bv_region_batch& b, bool wait) {
   s = upload_inputs(b);
   if (s == BV_OK) s = plan(b);
   if (s == BV_OK) s = upload_plan(b);
-  if (s == BV_OK && band_enabled()) s = band_prepare();
+  if (s == BV_OK && band_runs()) s = band_prepare();
   if (s != BV_OK) {
     cudaStreamSynchronize(stream_);
     return s;
@@ -773,7 +773,7 @@ bv_status Engine::stage(const bv_region_batch& b, bool wait) {
 
 // The staged bins' launches (of FP32 units, or of FP64 mode's).
 bv_status Engine::enqueue_plans(bool capturing, bool f64, KernelParams& p) {
-  if (band_enabled() || plans_.empty() || plans_[0].f64 != f64) return BV_OK;
+  if (band_runs() || plans_.empty() || plans_[0].f64 != f64) return BV_OK;
   if (tune_timing_ && !capturing) {
     while (tune_ev_.size() < 2 * plans_.size()) {
       cudaEvent_t e;
@@ -843,7 +843,7 @@ bv_status Engine::enqueue_kernels(bool capturing) {
   p.long_rows = long_plan_.grid > 0 ? long_rows() : 0;
   p.warps_per_block = kThreadsPerBlock / kWarp;  // band-path fallback and audit launches
   BV_CUDA(rec(ev_[2]), "event");
-  if (band_enabled()) {
+  if (band_runs()) {
     bv_status bs = enqueue_band(capturing, p);
     if (bs != BV_OK) return bs;
   }
@@ -886,7 +886,7 @@ bv_status Engine::enqueue_kernels(bool capturing) {
     p.cells_ctr = nullptr;
   }
   BV_CUDA(rec(ev_[4]), "event");
-  if (band_enabled() && band_opt_.audit_period > 0) {
+  if (band_runs() && band_opt_.audit_period > 0) {
     BV_CUDA(launch_audit_compare(band_params(), d_audit_err_.as<double>(), stream_), "audit compare");
   }
   return BV_OK;
@@ -952,7 +952,7 @@ bv_status Engine::finish(bv_phmm_stats* stats) {
   const Counters c = *h_counters_;
   if (c.status != 0) return status_fail(c.status);
   if (stats) *stats = bv_phmm_stats{};
-  if (stats && band_enabled()) {
+  if (stats && band_runs()) {
     bv_status bs = band_stats(stats);
     if (bs != BV_OK) return bs;
   }
@@ -964,7 +964,7 @@ bv_status Engine::finish(bv_phmm_stats* stats) {
     stats->cells = n_cells_;
     stats->rescued = (int64_t)(c.rescue_count + c.rescue_long_count);
     stats->rescued_cells = (int64_t)c.rescued_cells;
-    if (opt_.precision == BV_PRECISION_F64 && !band_enabled()) {  // every pair, on the list or in units
+    if (opt_.precision == BV_PRECISION_F64) {  // every pair, on the list or in units
       stats->rescued = n_results_;
       stats->rescued_cells = n_cells_;
     }
@@ -975,14 +975,14 @@ bv_status Engine::finish(bv_phmm_stats* stats) {
     // band mode: k-mer tables, nibble image, read k-mers, gap check, two featurisers, MLP, route,
     // scan, route; the banded kernels; the fallback's units and bins; the rescore's;
     // the audit's; the FP64 pass
-    stats->kernel_launches = band_enabled()
+    stats->kernel_launches = band_runs()
                                  ? 9 + (band_opt_.use_mlp ? 1 : 0) + kBandWidths + 1 + full_bins_ +
                                        (band_opt_.cap_margin > 0 ? 1 + full_bins_ : 0) +
                                        (band_opt_.audit_period > 0 ? 2 + full_bins_ : 0) + 1 + long_launches
                                  : (int64_t)plans_.size() + 1 + long_launches;
     stats->ms_fp32 = ms32;
     stats->ms_fp64 = ms64;
-    if (band_enabled()) {
+    if (band_runs()) {
       float seed = 0, band = 0, full = 0;
       cudaEventElapsedTime(&seed, ev_[2], ev_[5]);
       cudaEventElapsedTime(&band, ev_[5], ev_[6]);

@@ -178,6 +178,8 @@ class Engine {
   int device() const { return opt_.device; }
   bv_status set_band_options(const bv_band_options& o);
   bool band_enabled() const { return band_opt_.enabled != 0; }
+  // FP64 precision scores every pair in FP64: an enabled band waits for a context of the default precision.
+  bool band_runs() const { return band_enabled() && opt_.precision != BV_PRECISION_F64; }
   bv_status band_train(const bv_region_batch& b, const bv_band_train_options& o, bv_band_train_report* rep);
   bv_status band_labels(const bv_region_batch& b, float tau, int32_t* dstar, int32_t* lo, int32_t* hi, float* feat,
                         int32_t* kmin, int32_t* kmax);
@@ -250,6 +252,7 @@ class Engine {
   // staged batch
   std::vector<Unit> units_;  // of a small batch; larger ones' are made on the device
   int64_t n_units_ = 0;
+  int64_t unit_pairs_ = 0;                     // results the units cover (FP64 precision: not those on the lists)
   int unit_haps_ = 1;                          // haplotypes per unit
   int64_t bin_start_[kBins + 1] = {};          // first unit of a bin (-1: the bin has none)
   std::vector<uint32_t> region_base_[kBins + 1];  // per region, its first unit within the bin (used bins only)

@@ -84,6 +84,8 @@ BandParams Engine::band_params() const {
 
 bv_status Engine::band_prepare() {
   const int64_t n = std::max<int64_t>(n_results_, 1);
+  // every slot's read and haplotype come from the units (launch_pairs_from_units)
+  if (unit_pairs_ != n_results_) return fail(BV_ERR_INTERNAL, "work units do not cover the batch");
   BV_CUDA(prepare_band_kernels(), "band kernel attributes");
   BV_CUDA(d_pair_read_.reserve(sizeof(int32_t) * n), "alloc pairs");
   BV_CUDA(d_pair_hap_.reserve(sizeof(int32_t) * n), "alloc pairs");
@@ -258,6 +260,12 @@ bv_status Engine::band_stats(bv_phmm_stats* st) {
 bv_status Engine::band_routes(int64_t n, int32_t* d_lo, int32_t* width, int32_t* route) {
   if (!band_enabled() || !staged_) return fail(BV_ERR_INVALID_ARG, "no band-mode batch has run");
   if (n != n_results_) return fail(BV_ERR_INVALID_ARG, "result count");
+  if (!band_runs()) {  // FP64 precision: every pair in FP64
+    std::fill(d_lo, d_lo + n, 0);
+    std::fill(width, width + n, 0);
+    std::fill(route, route + n, 3);
+    return BV_OK;
+  }
   BandCounters bc{};
   Counters cc{};
   BV_CUDA(cudaMemcpy(&bc, d_bctr_.get(), sizeof(bc), cudaMemcpyDeviceToHost), "band counters");

@@ -77,7 +77,11 @@ bv_status Engine::stage_for_labels(const bv_region_batch& b) {
   if (s != BV_OK) return s;
   s = upload_inputs(b);
   if (s != BV_OK) return s;
+  // planned in the default precision whatever the context's: every pair has to have a unit
+  const int32_t precision = opt_.precision;
+  opt_.precision = BV_PRECISION_AUTO;
   s = plan(b);
+  opt_.precision = precision;
   if (s != BV_OK) return s;
   s = upload_plan(b);
   if (s != BV_OK) return s;

@@ -53,7 +53,8 @@ typedef enum bv_status {
 
 enum bv_phmm_precision {
   BV_PRECISION_AUTO = 0, /* FP32, FP64 for pairs below the rescue threshold (AvxPairHMM default) */
-  BV_PRECISION_F64 = 1   /* FP64 for every pair (AvxPairHMM::initNative(use_double = true)) */
+  BV_PRECISION_F64 = 1   /* FP64 for every pair (AvxPairHMM::initNative(use_double = true)); the band, if it is
+                            enabled, is not used (band labels and training do not depend on the precision) */
 };
 
 enum bv_phmm_mode {

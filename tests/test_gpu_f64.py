@@ -276,3 +276,55 @@ def test_no_allocation_entry_point_on_hopeless_reads(monkeypatch):
     import test_zz_no_alloc as no_alloc
     monkeypatch.setattr(no_alloc, "_batch", lambda: _hopeless(np.random.default_rng(19)))
     no_alloc.test_noalloc_matches_allocating_entry_point()
+
+
+# reads at the edge of a single strip (253 bases: a unit in FP64 mode; 254: the FP64 list), with some the band takes
+def _band_batch():
+    rng = np.random.default_rng(23)
+    regions = []
+    for n in (100, 253, 254, 150, 300):
+        hap = W._random_seq(rng, 400)
+        reads = [(W._mutate_read(rng, hap, 40, n, 0.01, 0.0, 1, 1), ) for _ in range(3)]
+        regions.append(([(r[0], *W._quals(rng, len(r[0]), 10, 40)) for r in reads],
+                        [hap, W._substitute(rng, hap, 0.01)]))
+    return W._build(regions, "single-strip edge")
+
+
+@pytest.mark.parametrize("chunks", [0, 2])
+def test_fp64_precision_with_the_band_enabled(chunks):
+    """Every pair in FP64, whatever the band's options: the values of a context without the band."""
+    from biovoltron_b200.pairhmm import PairHMMEngine
+    b = _band_batch()
+    with PairHMMEngine(precision="f64") as e:
+        want = e.compute_regions(b)
+    for mode in ("band", "full"):
+        with PairHMMEngine(precision="f64", mode=mode, pipeline_chunks=chunks, pipeline_min_pairs=1) as e:
+            if mode == "full":
+                e.set_band_options(fixed_half=8, margin=2, audit_period=2)
+            got, st = e.compute_regions(b, with_stats=True)
+            assert np.array_equal(got, want)
+            assert st["rescued"] == st["pairs"] == b.n_pairs and st["band_pairs"] == st["band_fallback"] == 0
+            n = e.stage(b)
+            for _ in range(3):
+                e.run()
+                assert np.array_equal(e.fetch(n), want)
+            d_lo, width, route = e.band_routes()
+            assert np.all(route == 3) and not d_lo.any() and not width.any()
+
+
+def test_labels_and_training_in_an_fp64_context():
+    """Band labels and weights do not depend on the context's precision."""
+    from biovoltron_b200.pairhmm import PairHMMEngine
+    b = _band_batch()
+    out = []
+    for precision in ("auto", "f64"):
+        with PairHMMEngine(precision=precision) as e:
+            labels = e.band_labels(b, features=True, extent=True)
+            e.band_train(b, epochs=2, batch_size=16)
+            out.append([*labels, e.band_weights()])
+            scored = e.compute_regions(b)  # the context's precision again
+    for x, y in zip(*out):
+        assert np.array_equal(x, y)
+    assert np.all(out[0][1] > np.iinfo(np.int32).min)
+    with PairHMMEngine(precision="f64") as e:
+        assert np.array_equal(e.compute_regions(b), scored)
