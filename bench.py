@@ -413,7 +413,7 @@ def main():
     def configure(e):
         if tuning:
             e.set_tuning(tuning)
-        if long_tuning:
+        if long_tuning and long_tuning["fixed"]:
             e.set_long_warps(long_tuning["warps_per_pair"])
 
     h2d_link = pinned_h2d_gbps(local)

@@ -403,6 +403,8 @@ bv_status bv_phmm_set_long_warps(bv_phmm_ctx* ctx, int32_t warps) {
 
 int32_t bv_phmm_get_long_warps(const bv_phmm_ctx* ctx) { return ctx ? ctx->engine.long_warps() : 0; }
 
+int32_t bv_phmm_long_warps_fixed(const bv_phmm_ctx* ctx) { return ctx && ctx->engine.long_warps_fixed() ? 1 : 0; }
+
 bv_status bv_phmm_autotune_long(bv_phmm_ctx* ctx, const bv_region_batch* sample, int32_t repeats, int32_t* warps_out,
                                 double* ms_out) {
   if (!ctx || !sample || !warps_out || !ms_out) return BV_ERR_INVALID_ARG;

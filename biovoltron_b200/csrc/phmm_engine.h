@@ -196,11 +196,14 @@ class Engine {
   bv_status autotune(const bv_region_batch& sample, int repeats, bv_phmm_tune_entry* out, int32_t* n_out);
   bv_status set_tuning(const bv_phmm_tune_entry* entries, int32_t n);
   bv_status get_tuning(bv_phmm_tune_entry* out, int32_t* n_out);
-  // Warps per pair of the FP64 long-read kernel (2, 4 or 8; reads of at least
-  // 128 x warps bases take it), set directly or chosen by timing the FP64 pass
-  // of a sample for each (ms[0..2]: 2, 4, 8 warps; 0 where not timed).
+  // Warps per pair of the FP64 long-read kernel: fixed (2, 4 or 8; reads of at
+  // least 128 x warps bases take it), or chosen by plan() for each batch (0, the
+  // default).  autotune_long times the FP64 pass of a sample for plan()'s choice
+  // and each fixed number (ms[0..2]: 2, 4, 8 warps; 0 where not timed) and
+  // installs the fastest.  long_warps(): the fixed number, or the last one.
   bv_status set_long_warps(int warps);
   int long_warps() const { return long_warps_; }
+  bool long_warps_fixed() const { return long_set_; }
   bv_status autotune_long(const bv_region_batch& sample, int repeats, int32_t* warps_out, double* ms_out);
 
  private:
@@ -218,6 +221,7 @@ class Engine {
   bv_status upload_plan(const bv_region_batch& b);
   bv_status enqueue_kernels(bool capturing);
   bv_status enqueue_plans(bool capturing, bool f64, KernelParams& p);
+  void install_long_warps(int warps, bool fixed);
   bv_status band_prepare();
   bv_status enqueue_band(bool capturing, KernelParams& p);
   bv_status enqueue_full(KernelParams& kp, const Unit* units, long long cap, const unsigned long long* counts, int slot0,

@@ -148,38 +148,43 @@ bv_status Engine::autotune(const bv_region_batch& sample, int repeats, bv_phmm_t
 }
 
 bv_status Engine::set_long_warps(int warps) {
-  if (warps != 2 && warps != 4 && warps != 8) return fail(BV_ERR_INVALID_ARG, "long-read warps per pair must be 2, 4 or 8");
-  if (warps != long_warps_ || !long_set_) {
-    long_warps_ = warps;
-    long_set_ = true;
-    ++config_version_;
-    staged_ = false;  // the FP64 lists and launch plan depend on it: stage again
-    destroy_graph();
-  }
+  if (warps != 0 && warps != 2 && warps != 4 && warps != 8)
+    return fail(BV_ERR_INVALID_ARG, "long-read warps per pair must be 0 (chosen per batch), 2, 4 or 8");
+  install_long_warps(warps > 0 ? warps : kLongWarps, warps > 0);
   return BV_OK;
 }
 
-// The long-read kernel's shape: for each candidate warps per pair (and with
-// it the long-read edge, 128 x warps bases) the sample is staged in FP64 mode
-// -- every pair on the FP64 kernels, long reads on the long-read kernel, the
-// rest on the short reads' kernels -- and its FP64 pass timed (repeats runs after
-// a warm-up, median); the fastest is installed.
+void Engine::install_long_warps(int warps, bool fixed) {
+  if (warps == long_warps_ && fixed == long_set_) return;
+  long_warps_ = warps;
+  long_set_ = fixed;
+  ++config_version_;
+  staged_ = false;  // the FP64 lists and launch plan depend on it: stage again
+  destroy_graph();
+}
+
+// The long-read kernel's shape.  The sample is staged in FP64 mode -- every
+// pair on the FP64 kernels, long reads on the long-read kernel, the rest on the
+// short reads' kernels -- for plan()'s own choice and for each fixed number of
+// warps per pair (and with it the long-read edge, 128 x warps bases), and its
+// FP64 pass timed (`repeats` runs after a warm-up, median).  The fastest fixed
+// number is installed if it beats plan()'s choice, which is in force otherwise;
+// a sample that no fixed number has a read for changes nothing.
 bv_status Engine::autotune_long(const bv_region_batch& sample, int repeats, int32_t* warps_out, double* ms_out) {
   if (!warps_out || !ms_out) return fail(BV_ERR_INVALID_ARG, "null output");
   if (repeats < 1 || repeats > 64) return fail(BV_ERR_INVALID_ARG, "repeats out of range");
   if (band_enabled()) return fail(BV_ERR_INVALID_ARG, "autotune runs the full-DP path: disable the band first");
-  const int cands[3] = {2, 4, 8};
-  for (int c = 0; c < 3; ++c) ms_out[c] = 0.0;
+  const int cands[4] = {0, 2, 4, 8};  // 0: plan()'s choice
+  double ms[4] = {0.0, 0.0, 0.0, 0.0};
   const int saved_warps = long_warps_;
   const bool saved_set = long_set_;
-  long_set_ = true;
   const int32_t saved_precision = opt_.precision;
   opt_.precision = BV_PRECISION_F64;
-  int best = saved_warps;
-  double best_ms = 1e300;
+  int best = 0;  // index of the fastest fixed number (0: none timed)
   bv_status s = BV_OK;
-  for (int c = 0; c < 3 && s == BV_OK; ++c) {
-    long_warps_ = cands[c];
+  for (int c = 0; c < 4 && s == BV_OK; ++c) {
+    long_set_ = cands[c] > 0;
+    if (long_set_) long_warps_ = cands[c];
     s = stage(sample);
     if (s != BV_OK) break;
     if (long_plan_.grid == 0) continue;  // no read this long, or its haplotypes too long for the kernel
@@ -202,25 +207,24 @@ bv_status Engine::autotune_long(const bv_region_batch& sample, int repeats, int3
         s = status_fail(cc.status);
         break;
       }
-      float ms = 0;
-      cudaEventElapsedTime(&ms, ev_[3], ev_[4]);
-      if (k > 0) t.push_back(ms);
+      float one = 0;
+      cudaEventElapsedTime(&one, ev_[3], ev_[4]);
+      if (k > 0) t.push_back(one);
     }
     if (s != BV_OK || t.empty()) break;
     std::nth_element(t.begin(), t.begin() + t.size() / 2, t.end());
-    ms_out[c] = t[t.size() / 2];
-    if (ms_out[c] < best_ms) {
-      best_ms = ms_out[c];
-      best = cands[c];
-    }
+    ms[c] = t[t.size() / 2];
+    if (c > 0 && (best == 0 || ms[c] < ms[best])) best = c;
   }
   opt_.precision = saved_precision;
-  long_warps_ = s == BV_OK ? best : saved_warps;
-  if (s != BV_OK) long_set_ = saved_set;
+  const bool tuned = s == BV_OK && best > 0;
+  long_warps_ = tuned ? cands[best] : saved_warps;
+  long_set_ = tuned ? !(ms[0] > 0.0 && ms[0] <= ms[best]) : saved_set;
   staged_ = false;  // the sample was staged in FP64 mode
   destroy_graph();
   ++config_version_;
   *warps_out = long_warps_;
+  for (int c = 0; c < 3; ++c) ms_out[c] = s == BV_OK ? ms[c + 1] : 0.0;
   return s;
 }
 

@@ -438,17 +438,22 @@ bv_status bv_phmm_autotune(bv_phmm_ctx* ctx, const bv_region_batch* sample, int3
  * not listed keep their values (defaults: two haplotypes per warp, 4 warps). */
 bv_status bv_phmm_set_tuning(bv_phmm_ctx* ctx, const bv_phmm_tune_entry* entries, int32_t num);
 bv_status bv_phmm_get_tuning(bv_phmm_ctx* ctx, bv_phmm_tune_entry* out, int32_t* num_out);
-/* The FP64 long-read kernel: a block of `warps` warps per pair (2, 4 or 8)
- * runs reads of at least 128 x warps bases, strip w of every group of `warps`
- * strips on warp w.  Until it is set or tuned (get then says 4) every read of
- * more than 253 bases takes the kernel, with 2 to 16 warps chosen from the
- * batch.  bv_phmm_autotune_long stages `sample`
- * in FP64 mode for each choice (the long-read edge moves with it), times the
- * FP64 pass (`repeats` runs, median), installs the fastest and writes it to
- * *warps_out and the times to ms_out[0..2] (2, 4, 8 warps; 0 where the
- * sample has no read that long).  No counterpart in the reference. */
+/* The FP64 long-read kernel.  By default every read of more than 253 bases
+ * takes it, with 2 to 16 warps per pair or a cluster of blocks, chosen from the
+ * batch.  A fixed number of `warps` (2, 4 or 8) is a block of that many warps
+ * per pair, for reads of at least 128 x warps bases; 0 goes back to the choice
+ * per batch.  get returns the fixed number (4 until one was set or tuned), and
+ * bv_phmm_long_warps_fixed whether it is in force (1) or the choice per batch (0).
+ * bv_phmm_autotune_long stages `sample` in FP64 mode for the choice per batch
+ * and for each fixed number (the long-read edge moves with it) and times the
+ * FP64 pass (`repeats` runs, median).  It writes the fastest fixed number to
+ * *warps_out and the times to ms_out[0..2] (2, 4, 8 warps; 0 where the sample
+ * has no read that long), and puts the faster of that number and the choice per
+ * batch in force.  A sample without a read long enough for any fixed number
+ * leaves everything as it was.  No counterpart in the reference. */
 bv_status bv_phmm_set_long_warps(bv_phmm_ctx* ctx, int32_t warps);
 int32_t bv_phmm_get_long_warps(const bv_phmm_ctx* ctx);
+int32_t bv_phmm_long_warps_fixed(const bv_phmm_ctx* ctx);
 bv_status bv_phmm_autotune_long(bv_phmm_ctx* ctx, const bv_region_batch* sample, int32_t repeats, int32_t* warps_out,
                                 double* ms_out);
 

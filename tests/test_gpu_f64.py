@@ -328,3 +328,31 @@ def test_labels_and_training_in_an_fp64_context():
     assert np.all(out[0][1] > np.iinfo(np.int32).min)
     with PairHMMEngine(precision="f64") as e:
         assert np.array_equal(e.compute_regions(b), scored)
+
+
+def test_long_read_tuner_keeps_the_choice_per_batch():
+    """A sample without long reads changes nothing; a fixed number of warps is in force only if it was the faster; 0
+    goes back to the choice per batch.  (The launches of a batch tell the choices apart: clusters of several sizes.)"""
+    from biovoltron_b200.pairhmm import PairHMMEngine
+    rng = np.random.default_rng(29)
+    short = W._build([_pair(rng, 150, 300) for _ in range(4)], "short")
+    b = W._build([_pair(rng, n, n + 200) for n in (6000, 3000, 1500, 700, 300) for _ in range(4)], "long")
+    with PairHMMEngine(precision="f64") as e:
+        want, st = e.compute_regions(b, with_stats=True)
+        launches = st["kernel_launches"]
+        assert e.long_warps() == 4 and not e.long_warps_fixed()
+        rep = e.autotune_long(short, repeats=1)
+        assert not rep["fixed"] and rep["warps_per_pair"] == e.long_warps() == 4 and not any(rep["fp64_ms"].values())
+        got, st = e.compute_regions(b, with_stats=True)
+        assert np.array_equal(got, want) and st["kernel_launches"] == launches
+        e.set_long_warps(8)
+        assert e.long_warps_fixed() and e.compute_regions(b, with_stats=True)[1]["kernel_launches"] != launches
+        assert e.autotune_long(short, repeats=1)["fixed"] and e.long_warps() == 8
+        rep = e.autotune_long(b, repeats=3)  # clusters are several times faster than any block here
+        assert not rep["fixed"] and rep["warps_per_pair"] in (2, 4, 8) and all(rep["fp64_ms"].values())
+        assert e.compute_regions(b, with_stats=True)[1]["kernel_launches"] == launches
+        e.set_long_warps(2)
+        assert e.long_warps_fixed()
+        e.set_long_warps(0)
+        assert not e.long_warps_fixed() and e.long_warps() == 4
+        assert np.array_equal(e.compute_regions(b), want)
