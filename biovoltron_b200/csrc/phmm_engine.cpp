@@ -304,6 +304,9 @@ bv_status Engine::plan(const bv_region_batch& b) {
     region_max_hap[g] = mh;
     max_hap_ = std::max(max_hap_, mh);
   }
+  // A read's bin: rows per lane of the single-strip kernels (row 0, the read, the summing row and one padding
+  // row on top: phmm_device.cuh, rows_needed), kBins for reads of several strips.
+  auto bin_of = [](int64_t rlen) { return (int)std::min<int64_t>((rlen + 3 + kWarp - 1) / kWarp, kBins); };
   // Haplotypes per unit: as many as the options allow when the batch still
   // gives every resident warp (about 16 an SM) eight units, so that the last
   // units of a launch do not leave the chip idle; fewer for smaller batches
@@ -320,7 +323,14 @@ bv_status Engine::plan(const bv_region_batch& b) {
     n_pairs += (b.region_reads[g + 1] - b.region_reads[g]) * (b.region_haps[g + 1] - b.region_haps[g]);
   const int64_t warps = (int64_t)sms_ * 16;
   // (FP64 mode: reads that fit a strip run in units too, one haplotype at a time)
-  const bool few = n_pairs * 2 <= warps && opt_.haps_per_warp != 2 && !band_runs() && !tuning_;
+  bool few = n_pairs * 2 <= warps && opt_.haps_per_warp != 2 && !band_runs() && !tuning_;
+  // ... unless a read's bin was set or tuned to two haplotypes a warp, and they fit
+  const bool two_fit = 4 * (4 * hap_bytes_for(max_hap_, 8) + warp_smem_bytes(variant_index(false, kTuneBins, false, true), 0)) <= 227 * 1024;
+  for (int64_t g = 0; few && two_fit && g < b.num_regions; ++g)
+    for (int64_t r = b.region_reads[g]; few && r < b.region_reads[g + 1]; ++r) {
+      const int rt = bin_of(b.read_offsets[r + 1] - b.read_offsets[r]);
+      few = !(rt <= kTuneBins && tune_[rt].set && tune_[rt].haps_per_warp == 2);
+    }
   const int per_unit = band_runs() ? max_unit
                        : all_f64   ? (int)std::min<int64_t>(max_unit, std::max<int64_t>(1, n_pairs / (warps * 8)))
                        : few       ? 1
@@ -330,10 +340,7 @@ bv_status Engine::plan(const bv_region_batch& b) {
     if (opt_.haps_per_warp == 1 || per_unit < 2 || rt < 1 || rt > kTuneBins) return false;
     return opt_.haps_per_warp == 2 || tune_[rt].haps_per_warp == 2;
   };
-  // A read's bin: rows per lane of the single-strip kernels (row 0, the read, the summing row and one padding
-  // row on top: phmm_device.cuh, rows_needed), kBins for reads of several strips; and the launch it takes.
-  auto bin_of = [](int64_t rlen) { return (int)std::min<int64_t>((rlen + 3 + kWarp - 1) / kWarp, kBins); };
-  int bin_variant[kBins + 1] = {};
+  int bin_variant[kBins + 1] = {};  // the launch a bin takes
   for (int rt = 1; rt <= kBins; ++rt)
     bin_variant[rt] = all_f64       ? (rt < kBins ? kF64Bin0 + rt : kF64List)
                       : rt == kBins ? v_multi

@@ -41,6 +41,7 @@ class DevBuf {
 struct BinTune {
   int haps_per_warp = 2;    // 1: one haplotype per warp; 2: two (packed FP32x2)
   int warps_per_block = 4;  // 1..4
+  bool set = false;         // by the caller or the autotuner
 };
 constexpr int kTuneBins = 8;  // rows per lane 1..8
 

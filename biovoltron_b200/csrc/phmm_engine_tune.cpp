@@ -29,6 +29,7 @@ bv_status Engine::set_tuning(const bv_phmm_tune_entry* e, int32_t n) {
   for (int32_t i = 0; i < n; ++i) {
     tune_[e[i].rows_per_lane].haps_per_warp = e[i].haps_per_warp;
     tune_[e[i].rows_per_lane].warps_per_block = e[i].warps_per_block;
+    tune_[e[i].rows_per_lane].set = true;
   }
   ++config_version_;
   staged_ = false;  // the launch plan depends on it: stage again
@@ -135,6 +136,7 @@ bv_status Engine::autotune(const bv_region_batch& sample, int repeats, bv_phmm_t
     if (best_c[rt] < 0) continue;
     tune_[rt].haps_per_warp = cands[best_c[rt]].hpw;
     tune_[rt].warps_per_block = cands[best_c[rt]].wpb;
+    tune_[rt].set = true;
     bv_phmm_tune_entry t{};
     t.rows_per_lane = rt;
     t.haps_per_warp = tune_[rt].haps_per_warp;

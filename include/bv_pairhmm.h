@@ -435,7 +435,11 @@ typedef struct bv_phmm_tune_entry {
 bv_status bv_phmm_autotune(bv_phmm_ctx* ctx, const bv_region_batch* sample, int32_t repeats, bv_phmm_tune_entry* out,
                            int32_t* num_out);
 /* Installs (set) or reads (get) per-bin launch parameters; entries for bins
- * not listed keep their values (defaults: two haplotypes per warp, 4 warps). */
+ * not listed keep their values (defaults: two haplotypes per warp, 4 warps).
+ * A batch with fewer pairs than half the warps the device holds (1,184) runs one
+ * haplotype per warp while the bins of its reads have the default; an entry
+ * that was set or tuned is taken as it is, and bv_phmm_options.haps_per_warp
+ * goes before both. */
 bv_status bv_phmm_set_tuning(bv_phmm_ctx* ctx, const bv_phmm_tune_entry* entries, int32_t num);
 bv_status bv_phmm_get_tuning(bv_phmm_ctx* ctx, bv_phmm_tune_entry* out, int32_t* num_out);
 /* The FP64 long-read kernel.  By default every read of more than 253 bases

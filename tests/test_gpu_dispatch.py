@@ -116,3 +116,18 @@ def test_strips(oracle, read_len, gap):
         assert np.max(np.abs(got - truth)) <= TOL_FP32
         if gap == 45:  # the reads match: only the haplotypes of 20 bases need FP64
             assert st["rescued"] <= len(regions)
+
+
+def test_set_shapes_in_a_small_batch():
+    """A small batch with shapes set for its bin, for another bin, for all of them, one or two haplotypes a warp: the
+    same values; haplotypes too long for two a warp are accepted either way."""
+    from biovoltron_b200.pairhmm import PairHMMEngine
+    rng = np.random.default_rng(50)
+    batches = [W._build([_region(rng, 64, 8, [150], 300)], "window"), W._build([_region(rng, 2, 3, [150], 20000)], "long")]
+    out = []
+    for bins, haps in (((), 2), ((3,), 2), ((5,), 2), (range(1, 9), 2), (range(1, 9), 1)):
+        with PairHMMEngine() as e:
+            e.set_tuning([{"rows_per_lane": rt, "haps_per_warp": haps, "warps_per_block": 2} for rt in bins])
+            out.append([e.compute_regions(b) for b in batches])
+    for o in out[1:]:
+        assert all(np.array_equal(x, y) for x, y in zip(o, out[0]))
