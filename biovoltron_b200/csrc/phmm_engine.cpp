@@ -678,6 +678,7 @@ bv_status Engine::upload_inputs(const bv_region_batch& b) {
 // once its own synchronisation has passed.
 bv_status Engine::upload_plan(const bv_region_batch& b) {
   bool units_staged = false;
+  stage_launches_ = small_in_ ? 0 : (n_units_ > 0) + (n_read_bytes_ > 0);  // units, packed qualities
   if (small_in_) {
     const size_t bytes = sizeof(Unit) * units_.size();
     if (void* p = stage_piece(std::max<size_t>(bytes, 1), d_units_)) {
@@ -982,11 +983,13 @@ bv_status Engine::finish(bv_phmm_stats* stats) {
     // band mode: k-mer tables, nibble image, read k-mers, gap check, two featurisers, MLP, route,
     // scan, route; the banded kernels; the fallback's units and bins; the rescore's;
     // the audit's; the FP64 pass
+    // (in both modes: the FP64 lists' counts, and a small batch's way back)
+    const int small_launches = !f64_items_.empty() + !f64_long_items_.empty() + small_in_;
     stats->kernel_launches = band_runs()
                                  ? 9 + (band_opt_.use_mlp ? 1 : 0) + kBandWidths + 1 + full_bins_ +
                                        (band_opt_.cap_margin > 0 ? 1 + full_bins_ : 0) +
-                                       (band_opt_.audit_period > 0 ? 2 + full_bins_ : 0) + 1 + long_launches
-                                 : (int64_t)plans_.size() + 1 + long_launches;
+                                       (band_opt_.audit_period > 0 ? 2 + full_bins_ : 0) + 1 + long_launches + small_launches
+                                 : (int64_t)plans_.size() + 1 + long_launches + small_launches;
     stats->ms_fp32 = ms32;
     stats->ms_fp64 = ms64;
     if (band_runs()) {
@@ -1054,6 +1057,7 @@ bv_status Engine::compute(const bv_region_batch& b, double* out, bv_phmm_stats* 
     if (s != BV_OK) return s;
   }
   if (stats) {
+    stats->kernel_launches += stage_launches_;
     const auto t2 = std::chrono::steady_clock::now();
     stats->ms_d2h = std::chrono::duration<double, std::milli>(t2 - t1).count();
     stats->ms_total = std::chrono::duration<double, std::milli>(t2 - t0).count();

@@ -298,6 +298,7 @@ class Engine {
   DevBuf d_stage_, d_inputs_;  // the inputs' places on the device: of a small batch, of a larger one
   size_t stage_used_ = 0;
   bool small_in_ = false, small_out_ = false;
+  int stage_launches_ = 0;  // kernels that staging the batch launched
   bv_status reserve_host();
   void* stage_piece(size_t bytes, DevBuf& dev);
   int64_t* h_chunk_off_ = nullptr;  // page-locked rebased offsets of the chunk this context stages

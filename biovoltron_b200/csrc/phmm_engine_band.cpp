@@ -146,6 +146,7 @@ bv_status Engine::band_prepare() {
   if (need32 > d_bnd32_.capacity()) BV_CUDA(d_bnd32_.reserve(need32), "alloc boundary buffers");
   BV_CUDA(launch_pairs_from_units(d_units_.as<Unit>(), n_units_, d_pair_read_.as<int32_t>(),
                                   d_pair_hap_.as<int32_t>(), sms_, stream_), "pairs");
+  ++stage_launches_;
   return BV_OK;
 }
 

@@ -116,6 +116,7 @@ bv_status Engine::compute_chunked(Engine& other, const bv_region_batch& b, doubl
     bv_status r = e.fetch(out + ck[k].out0, ck[k].n_out);
     if (r != BV_OK) return fail(r, e.last_error());
     r = e.finish(&cs[k]);
+    cs[k].kernel_launches += e.stage_launches_;
     return r == BV_OK ? r : fail(r, e.last_error());
   };
   auto abort = [&](bv_status r) {

@@ -88,7 +88,7 @@ typedef struct bv_phmm_stats {
   int64_t band_pairs;     /* pairs scored by the banded kernel */
   int64_t band_fallback;  /* banded pairs sent back to the full DP */
   int64_t band_cells;     /* cells the banded kernel computed */
-  int64_t kernel_launches;
+  int64_t kernel_launches; /* kernels the run launched; a call that stages its batch too counts those of the staging */
   double ms_h2d;          /* host->device copies (events on the context stream) */
   double ms_fp32;         /* all FP32 kernels (band mode: seeding, banded DP and fallback full DP) */
   double ms_fp64;         /* FP64 rescue kernel */

@@ -61,3 +61,15 @@ def test_small_and_large_in_turn(engine):
     finally:
         engine.set_band_options(enabled=False)
     assert np.array_equal(engine.compute_regions(small), a)
+
+
+def test_launches_are_counted(engine):
+    """One bin: its kernel, the FP64 list's, and a small batch's copy back; a larger batch's staging makes the units and
+    packs the qualities."""
+    for n_reads, staging in ((20, 0), (1200, 2)):
+        b = _batch(n_reads, 8, 150, 300, 5, False)
+        _, st = engine.compute_regions(b, with_stats=True)
+        run = 2 + (staging == 0)
+        assert st["kernel_launches"] == run + staging
+        engine.stage(b)
+        assert engine.run()["kernel_launches"] == run
