@@ -381,9 +381,10 @@ __device__ __forceinline__ void stage_hap_pair(const uint8_t* __restrict__ ha, i
   }
 }
 
-// One strip of the wavefront.  MULTI: lane 0 reads the row above the strip
-// from `bnd` (the previous strip's bottom row, or zeros for the first strip)
-// and lane 31 writes this strip's bottom row back to `bnd`, both through
+// One strip of the wavefront: a whole read in FP32, or a strip of several in
+// FP64 (MULTI; FP32's are run_strip_below's).  MULTI: lane 0 reads the row above
+// the strip from `bnd` (the previous strip's bottom row, or zeros for the first
+// strip) and lane 31 writes this strip's bottom row back to `bnd`, both through
 // shared-memory rings.  Column c of the boundary row is buffer row c + 31.
 // On return, lane 31 holds its bottom row's final M and Y (the summing row's
 // result for FP32), the per-step sums of M and X over the bottom row (FP64,
@@ -396,8 +397,7 @@ __device__ __forceinline__ void run_strip(const Rows<T, RT>& rw, const ELane el,
                                           T& lastY, T& sumM, T& sumX, T& bmax,
                                           unsigned long long* status = nullptr) {
   using S = WarpSmem<T, RT>;
-  constexpr bool kScale = sizeof(T) == 8;  // only the FP64 path renormalises
-  constexpr bool kSums = !SumRow<T>::value;
+  static_assert(MULTI == (sizeof(T) == 8) && !(MULTI && FOLD), "FP32 whole reads, FP64 strips");
   T M[RT], X[RT], Y[RT];
 #pragma unroll
   for (int j = 0; j < RT; ++j) { M[j] = T(0); X[j] = T(0); Y[j] = rw.y0[j]; }
@@ -429,14 +429,11 @@ __device__ __forceinline__ void run_strip(const Rows<T, RT>& rw, const ELane el,
       mbar_init(mb + 1, 1);
       fence_for_bulk();
       bulk_g2s(ring_in, bnd + (size_t)32 * 4, kChunkBytes, mb);
-      dM = bnd[31 * 4 + 0]; dX = bnd[31 * 4 + 1]; dY = bnd[31 * 4 + 2];
-      if constexpr (kScale) { dM *= in_scale; dX *= in_scale; dY *= in_scale; }
+      dM = bnd[31 * 4 + 0] * in_scale; dX = bnd[31 * 4 + 1] * in_scale; dY = bnd[31 * 4 + 2] * in_scale;
       bulk_ok &= mbar_wait(mb, 0);
       phase ^= 1u;
     }
     __syncwarp();
-  } else if constexpr (!SumRow<T>::value) {
-    if (lane == 0) { upM = T(0); dM = T(0); }
   }
 
   for (int s0 = 0; s0 < nsteps; s0 += CH) {
@@ -450,8 +447,7 @@ __device__ __forceinline__ void run_strip(const Rows<T, RT>& rw, const ELane el,
       if constexpr (MULTI) {
         if (lane == 0) {
           const T* rin = ring_in + ((((s0 >> 5) & 1) * 32) + u) * 4;
-          upM = rin[0]; upX = rin[1]; upY = rin[2];
-          if constexpr (kScale) { upM *= in_scale; upX *= in_scale; upY *= in_scale; }
+          upM = rin[0] * in_scale; upX = rin[1] * in_scale; upY = rin[2] * in_scale;
         }
       }
       T e[RT];
@@ -478,7 +474,7 @@ __device__ __forceinline__ void run_strip(const Rows<T, RT>& rw, const ELane el,
         um = mn; ux = xn;
         M[j] = mn; X[j] = xn; Y[j] = yn;
       }
-      if constexpr (kSums) {
+      if constexpr (MULTI) {
         sumM += M[RT - 1];
         sumX += X[RT - 1];
       }
@@ -489,14 +485,11 @@ __device__ __forceinline__ void run_strip(const Rows<T, RT>& rw, const ELane el,
         if (lane == kWarp - 1) {
           T* ro = ring_out + u * 4;
           ro[0] = M[RT - 1]; ro[1] = X[RT - 1]; ro[2] = Y[RT - 1];
-          if constexpr (kScale) bmax = fmax(bmax, fmax(M[RT - 1], fmax(X[RT - 1], Y[RT - 1])));
+          bmax = fmax(bmax, fmax(M[RT - 1], fmax(X[RT - 1], Y[RT - 1])));
         }
       }
       dM = upM; dX = upX; dY = upY;
       upM = nM; upX = nX; upY = nY;
-      if constexpr (!MULTI && !SumRow<T>::value) {
-        if (lane == 0) upM = T(0);
-      }
     }
     if constexpr (MULTI) {
       // End of a 32-step chunk: flush its bottom row (buffer rows s0+1 ..
@@ -505,12 +498,8 @@ __device__ __forceinline__ void run_strip(const Rows<T, RT>& rw, const ELane el,
       __syncwarp();
       T* dstb = bnd + (size_t)(s0 + 1 + lane) * 4;
       const T* srco = ring_out + lane * 4;
-      if constexpr (sizeof(T) == 4) {
-        *reinterpret_cast<float4*>(dstb) = *reinterpret_cast<const float4*>(srco);
-      } else {
-        reinterpret_cast<double2*>(dstb)[0] = reinterpret_cast<const double2*>(srco)[0];
-        reinterpret_cast<double2*>(dstb)[1] = reinterpret_cast<const double2*>(srco)[1];
-      }
+      reinterpret_cast<double2*>(dstb)[0] = reinterpret_cast<const double2*>(srco)[0];
+      reinterpret_cast<double2*>(dstb)[1] = reinterpret_cast<const double2*>(srco)[1];
       __threadfence_block();
       if (lane == 0) {
         const int h = (s0 / 32 + 1) & 1;  // the prefetched half
@@ -689,7 +678,7 @@ __device__ __forceinline__ void run_strip_one(const Rows<float, RT>& rw, const E
   lastY = Y[RT - 1];
 }
 
-// One strip of a read of several (FP32), as run_strip's multi-strip form: the
+// One strip of a read of several (FP32), as run_strip's FP64 form: the
 // row above from `bnd` through the ring, the bottom row back to it.  Few long
 // reads leave a warp alone on its scheduler, so a step's latency is what counts:
 // sums instead of states from the lane above, emissions, codes and the row above
@@ -981,10 +970,7 @@ __device__ bool process_item(const KernelParams& p, const Item& it, unsigned cha
         if constexpr (sizeof(T) == 4) {
           if (fold) run_strip_below<RT, true>(rw, el, hc + kHapLead - lane, nsteps, lane, bnd, ring, lastM, lastY, &p.ctr->status);
           else run_strip_below<RT, false>(rw, el, hc + kHapLead - lane, nsteps, lane, bnd, ring, lastM, lastY, &p.ctr->status);
-        } else if (fold)
-          run_strip<T, RT, true, 32, true>(rw, el, hc + kHapLead - lane, nsteps, lane, bnd, ring, in_scale, lastM,
-                                           lastY, sumM, sumX, bmax, &p.ctr->status);
-        else
+        } else
           run_strip<T, RT, true, 32>(rw, el, hc + kHapLead - lane, nsteps, lane, bnd, ring, in_scale, lastM,
                                      lastY, sumM, sumX, bmax, &p.ctr->status);
         __syncwarp();

@@ -252,7 +252,7 @@ class Engine {
   DevBuf d_gt_kept_count_, d_gt_kept_reads_, d_gt_allele_lik_, d_gt_geno_lik_;
   bool jacobian_ready_ = false;
   DevBuf d_tables_, d_read_bases_, d_q_, d_i_, d_d_, d_c_, d_quals4_, d_read_off_, d_hap_bases_, d_hap_off_;
-  DevBuf d_units_, d_out_, d_rescue_, d_counters_, d_bnd32_, d_bnd64_, d_f64_items_;
+  DevBuf d_units_, d_out_, d_rescue_, d_counters_, d_bnd32_, d_bnd64_;
 
   // staged batch
   std::vector<Unit> units_;  // of a small batch; larger ones' are made on the device
@@ -268,7 +268,7 @@ class Engine {
   std::vector<PairRef> f64_long_items_;  // the long reads among them, ascending cells (the list's far end first)
   std::vector<LaunchPlan> plans_;
   LaunchPlan rescue_plan_;
-  LaunchPlan long_plan_;  // FP64 long reads, a block of long_warps_ warps per pair (grid 0: none)
+  LaunchPlan long_plan_;  // FP64 long reads: blocks of long_block_ warps or clusters (long_grid_); grid 0: none
   // Warps per pair of the long-read kernel as set or tuned (2, 4 or 8), and whether they were: until
   // then plan() picks the block (long_block_) and every read longer than a strip takes the kernel.
   int long_warps_ = kLongWarps;

@@ -68,7 +68,6 @@ cudaError_t launch_f64(int rt, const KernelParams& p, int grid, cudaStream_t st)
 // pair are set or tuned uses that many, for reads of at least 128 x warps
 // bases.
 constexpr int kLongWarps = 4;
-bool long_warps_valid(int warps);
 int long_smem_bytes(int hap_bytes, int warps);
 // `blocks` > 0 (16 warps each): clusters of that many blocks per pair, grid a multiple of it; the launch takes
 // the listed pairs (kLongMembers at most) whose long_blocks is `blocks`.  0: a block per pair, all pairs.
@@ -89,7 +88,6 @@ __host__ __device__ inline int long_blocks(long long R, long long H, long long l
 }
 cudaError_t prepare_long(int smem, int warps, int blocks);
 int long_blocks_per_sm(int smem, int warps);
-int long_clusters(int smem, int warps, int blocks);  // clusters that run at once
 cudaError_t launch_forward_long(const KernelParams& p, int grid, int smem, int warps, int blocks, cudaStream_t st);
 
 // Variant table: (precision, rows per lane, multi-strip, two haplotypes per

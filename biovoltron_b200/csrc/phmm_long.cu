@@ -546,8 +546,6 @@ cudaLaunchConfig_t config_of(int grid, int smem, int warps, int blocks, cudaStre
 }
 }  // namespace
 
-bool long_warps_valid(int warps) { return warps == 2 || warps == 4 || warps == 8 || warps == 16; }
-
 int long_smem_bytes(int hap_bytes, int warps) {
   return hap_bytes + (warps == 2    ? LongLayout<2>::kBytes
                       : warps == 4  ? LongLayout<4>::kBytes
@@ -562,15 +560,6 @@ int long_blocks_per_sm(int smem, int warps) {
   if (prepare_long(smem, warps, 0) != cudaSuccess) return 0;
   if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, kernel_of(warps, 0), warps * kWarp, smem) != cudaSuccess) return 0;
   return nb;
-}
-
-int long_clusters(int smem, int warps, int blocks) {
-  int n = 0;
-  cudaLaunchAttribute attr{};
-  if (prepare_long(smem, warps, blocks) != cudaSuccess) return 0;
-  const cudaLaunchConfig_t c = config_of(blocks, smem, warps, blocks, nullptr, &attr);
-  if (cudaOccupancyMaxActiveClusters(&n, kernel_of(warps, blocks), &c) != cudaSuccess) return 0;
-  return n;
 }
 
 cudaError_t launch_forward_long(const KernelParams& p, int grid, int smem, int warps, int blocks, cudaStream_t st) {
