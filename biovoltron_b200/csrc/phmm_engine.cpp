@@ -614,7 +614,9 @@ bv_status Engine::stage_inputs(const bv_region_batch& b) {
 }
 
 // Inputs: the byte arrays and offsets go to the device as soon as the batch
-// is validated, so the copies run while the host plans the launches.
+// is validated.  From page-locked arrays the copies run while the host plans the
+// launches; from pageable ones a copy holds the host until it is staged (0.2 ms
+// for 48 uneven regions, 1.1 for 256).
 bv_status Engine::upload_inputs(const bv_region_batch& b) {
   n_reads_ = b.num_reads;
   n_haps_ = b.num_haps;

@@ -8,7 +8,8 @@
 // A pair that cannot take the folded form (a row with pMM < kFoldMin), whose
 // result lies below 2^-600 (from a start of 2^900) or is not finite, and a
 // read of several strips runs the unscaled recurrence strip after strip,
-// renormalised between strips (process_item<double, 4, multi-strip>).
+// renormalised between strips (process_item_f64: 128 rows a strip, 32 where those
+// lose more than the range holds).
 //
 // Bound by issue: an FP64 instruction takes two slots, and a step of five rows a
 // lane has 28 of them.  The emissions come from a table in shared memory, a

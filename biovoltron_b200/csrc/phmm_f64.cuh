@@ -26,7 +26,7 @@
 // The folded form needs pMM >= kFoldMin in every row and the scaled states
 // need head-room, so callers start from 2^kF64Start / H (not 2^1020 / H) and
 // hand a pair whose result is not safely inside the range to the unscaled,
-// per-strip renormalised form (process_item<double, 4, multi-strip>).
+// per-strip renormalised form (process_item_f64).
 #pragma once
 #include "phmm_device.cuh"
 

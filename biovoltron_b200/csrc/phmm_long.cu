@@ -184,9 +184,8 @@ struct Pow2 {
 // memory).  RAMP: row 0 (lane l0, register j0) reaches column 0 at step l0 - 1.
 // LAST: the last row is summed over the columns up to H (lane 31 is at column
 // u + c31).  Specialised so that a step issues nothing but its cells, four
-// shuffles, one load and one store: with these choices made inside the loop a
-// step took 86 instructions, 23 of them FP64, instead of 60, and the 40 pairs
-// below 15.7 ms instead of 12.0.
+// shuffles, one load and one store: with these choices made inside the loop 40
+// reads of up to 10 kb on a block of 16 warps each took 15.7 ms instead of 12.0.
 template <LongMode OUT, bool RAMP, bool LAST>
 __device__ __forceinline__ void run_chunk(const F64Rows<kLongRT>& w, F64State<kLongRT>& st, double2& z,
                                           const unsigned char* __restrict__ hc, const double2* __restrict__ stage,

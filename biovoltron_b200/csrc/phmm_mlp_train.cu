@@ -22,7 +22,8 @@
 // memory, and leaves the rows' hidden gradients and its partial products of the
 // hidden weight gradients (K = its 128 rows).  k_mlp_update: sums the partial
 // products block by block and the bias and output-layer gradients row by row,
-// in a fixed order, so training is deterministic, and applies Adam.  The step
+// in a fixed order, so the weights are the same in every run, and applies Adam.
+// (The reported loss is summed with atomics: its last bits may differ.)  The step
 // is a chain of five small products and a 1,024-term sum, so latency is what
 // counts: 1,024 rows take 47 us, where a launch per product, activation
 // and sum (22 of them, operands through global memory) took 273.

@@ -10,7 +10,7 @@
 // into that memory without the library reserving anything.
 //
 // How.  bv_phmm_forward_f64_noalloc runs a variant of the FP64 multi-strip
-// forward pass (process_item<double, 4, multi-strip>, phmm_device.cuh): the
+// forward pass (process_item_f64, phmm_device.cuh): the
 // scratch that kernel normally takes from context-owned allocations -- the
 // work-queue counters, the probability tables and one strip-boundary buffer
 // per resident warp -- lives here in one file-scope __device__ array of fixed
