@@ -23,20 +23,22 @@
 // Scale.  Every strip keeps its own power of two E (true values are stored
 // values * 2^E) and a chunk carries the E it was written with.  Before a
 // chunk the warp looks at the largest exponent among its states and the
-// incoming sums and, when that has left [2^600, 2^1010], moves it to 2^1000: all
+// incoming sums and, when that has left [2^560, 2^975], moves it to 2^965: all
 // states are multiplied by exact powers of two.  E holds for all 128 rows of
 // the strip, and the top rows are the largest: a path that loses a whole strip
 // (a stretch of the read that does not align, insertion runs too dear to bridge
 // it: 11 to 15 binary orders a row at base qualities 25 to 40) has to fit below
 // them, and may still be the one that counts in the end.  So the largest state
-// stands at the top of the range: 2,000 binary orders a strip are kept, as by
-// the unscaled form, whose strips start at 2^1000 too (from 2^200, an exponent
-// that leaves room for growth, 922 to 1,422 are, and a read of 300 bases whose
-// bases 45-172 do not align scored 10^-436 instead of 10^-384).  What lies
-// further below is lost there as here.  Inside a chunk (32 columns) states grow
-// by little: all of a row's mass comes from the row above it, and X / pMX by
-// what the insertion quality jumps from one row to the next; beyond 2^13 they
-// overflow and the pair is handed back.
+// stands near the top of the range: some 1,980 binary orders a strip are kept,
+// about as many as by the unscaled form (from 2^200, an exponent that leaves
+// room for any growth, 922 to 1,422 are: a read of 300 bases whose bases 45-172
+// do not align scored 10^-436 instead of 10^-384).  What lies further below is
+// lost there as here.  Inside a chunk (32 columns) states grow by little: all of
+// a row's mass comes from the row above it, and X / pMX by what the insertion
+// quality falls from one row to the next, 2^43 at most.  A strip follows E
+// wherever the incoming row leads: far from the alignment, where nothing is left
+// in range, a chunk keeps the E of before, and the alignment may come back in a
+// scale thousands of binary orders away.
 //
 // Up to a few hundred pairs: a cluster of up to eight blocks takes a pair, its warps numbered
 // through, so that 16 x blocks strips run at once (long reads get more blocks
@@ -49,8 +51,8 @@
 // end of each.
 //
 // A pair with a row that cannot be folded, with a row between two strips whose
-// largest sum lies below 2^-960 in the largest scale of the strip that wrote it
-// (so that what that strip lost may count), or whose result lies below 2^-960 in
+// largest sum lies below 2^-960 in the largest scale that the strip above wrote
+// sums in (so that what it lost may count), or whose result lies below 2^-960 in
 // the last strip's scale or is not finite, is handed back to k_f64_list (its
 // list entry marked), which runs after this kernel.
 //
@@ -78,8 +80,8 @@ constexpr int kLongRT = 4;                // rows per lane
 constexpr int kStrip = kWarp * kLongRT;   // rows per strip
 constexpr int kLongSlots = 4;             // chunk slots per channel
 constexpr int kChunkB = 32 * 16;          // one 32-column chunk of (zx, zm)
-constexpr int kTop = 1000;                // exponent the largest state is moved to
-constexpr int kTopMax = 1010, kTopMin = 600;
+constexpr int kTop = 965;                 // exponent the largest state is moved to
+constexpr int kTopMax = 975, kTopMin = 560;
 constexpr int kMinExp = -960;             // of a row's largest sum, and of the result
 constexpr int kNoExp = -(1 << 24);        // "no value": below every exponent
 
@@ -172,7 +174,7 @@ __device__ __forceinline__ double pow2(int d) { return d < -1022 ? 0.0 : __hiloi
 struct Pow2 {
   double a, b;
   __device__ __forceinline__ explicit Pow2(int d) {
-    d = max(-2100, min(d, 2000));  // below: zero, as it should be; above: no value that is kept needs more
+    d = max(-2100, min(d, 2000));  // below: zero, as it should be; above: only zeros come
     a = pow2(d / 2);
     b = pow2(d - d / 2);
   }
@@ -265,8 +267,8 @@ __device__ __forceinline__ int run_strip_long(const F64Rows<kLongRT>& w, const u
       ahead_e = __ldcg(io.src_e + 1);
     }
   }
-  // the largest sum of the row above (this lane's share), the largest scale it came in
-  int row_top = max(exp_of(carry.x), exp_of(carry.y)) + carry_e, row_e = carry_e;
+  // the row above from column 2 on: its largest sum (this lane's share), the largest scale that sums came in
+  int row_top = 2 * kNoExp, row_e = 2 * kNoExp;
   if (!first) E = carry_e;
   else io.stage[lane] = make_double2(0.0, 0.0);
   double2 z = make_double2(0.0, 0.0);  // nothing lies above column 0
@@ -306,7 +308,7 @@ __device__ __forceinline__ int run_strip_long(const F64Rows<kLongRT>& w, const u
       // the 40 pairs 8.4 instead of 3.7 ms.)
       top = __shfl_sync(0xffffffffu, __reduce_max_sync(0xffffffffu, top), 0);
       if (top > kNoExp / 2 && (top - E > kTopMax || top - E < kTopMin)) {
-        const int d = min(E - (top - kTop), 2000);  // stored values times 2^d
+        const int d = E - (top - kTop);  // stored values times 2^d (beyond 2^2000 only when they are all zero)
         const Pow2 f(d);
 #pragma unroll
         for (int j = 0; j < kLongRT; ++j) {
@@ -329,8 +331,9 @@ __device__ __forceinline__ int run_strip_long(const F64Rows<kLongRT>& w, const u
       io.stage[edge ? 0 : lane + 1] = make_double2(f(edge ? carry.x : nx.x), f(edge ? carry.y : nx.y));
       carry = nx;
       carry_e = nx_e;
-      row_top = max(row_top, max(exp_of(nx.x), exp_of(nx.y)) + nx_e);
-      row_e = max(row_e, nx_e);
+      const int at = max(exp_of(nx.x), exp_of(nx.y)) + nx_e;
+      row_top = max(row_top, at);
+      row_e = max(row_e, __any_sync(0xffffffffu, at > kNoExp / 2) ? nx_e : 2 * kNoExp);  // (a branch here costs 2 %)
       if (k + 1 == nch && __reduce_max_sync(0xffffffffu, row_top) < row_e + kMinExp) {
         sumM = __longlong_as_double(0x7ff8000000000000ll);  // a NaN in the chunk's first column, or in the result
         st.M[kLongRT - 1] = sumM;
@@ -481,7 +484,7 @@ __global__ void __launch_bounds__(K * kWarp, 16 / K) k_forward_long(KernelParams
     const int nch = (H + kWarp - 1 + 31) / 32;
     const int nstrips = (R + 1 + kStrip - 1) / kStrip;
     const int pad = nstrips * kStrip - (R + 1);  // padding rows on top of row 0
-    // initial row: init / H, stored with exponent y0_exp, just below 2^1009
+    // initial row: init / H, stored with exponent y0_exp, just below 2^(kTop + 9)
     const int y0_exp = kF64InitExp - kTop - 8 - (31 - __clz(H));
     const double y0 = ldexp(p.tables->init_d, -y0_exp) / (double)H;
     stage_hap_block(b.hap_bases + ho, H, hc, 32 * nch + kHapLead);

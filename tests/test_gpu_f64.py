@@ -218,6 +218,24 @@ def test_long_reads_that_lose_most_of_the_range_in_a_strip(oracle, n, rival):
                     _check(b, e.compute_regions(b), oracle)
 
 
+@pytest.mark.parametrize("gcp", [30, 40, 60])
+def test_long_reads_with_dear_gaps(oracle, gcp):
+    """Reads of up to 10 kb whose insertion runs cost 10 to 20 binary orders a base: far from the alignment nothing stays
+    in range, and a strip's scale has to follow the row above when the alignment comes back, thousands of binary orders
+    away.  Insertion qualities of one value, and jumping between rows."""
+    from dataclasses import replace
+    from biovoltron_b200.pairhmm import PairHMMEngine
+    b = W.config2(seed=40, n_pairs=12)
+    rng = np.random.default_rng(gcp)
+    b = replace(b, read_c=np.full_like(b.read_c, gcp))
+    for b in (b, replace(b, read_i=rng.integers(8, 46, b.read_i.size).astype(np.uint8))):
+        with PairHMMEngine(precision="f64") as e:
+            _check(b, e.compute_regions(b), oracle)
+            for k in (2, 8):
+                e.set_long_warps(k)
+                _check(b, e.compute_regions(b), oracle)
+
+
 def test_constant_transitions_that_lose_most_of_the_range_in_a_strip(oracle):
     """Insertion runs that are dear by a small insertion-to-insertion probability."""
     from biovoltron_b200.pairhmm import PairHMMEngine
