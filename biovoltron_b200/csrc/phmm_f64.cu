@@ -5,7 +5,7 @@
 // k_f64_units runs FP64 mode's work units, a bin of rows per lane at a time;
 // k_f64_list drains the list of pairs the other kernels send to FP64 (the
 // FP32 kernels' rescues, the pairs the unit and long-read kernels hand back).
-// A pair that cannot take the folded form (a row with pMM < kFoldMin), whose
+// A pair that cannot take the folded form (a row with pMM < kF64FoldMin), whose
 // result lies below 2^-600 (from a start of 2^900) or is not finite, and a
 // read of several strips runs the unscaled recurrence strip after strip,
 // renormalised between strips (process_item_f64: 128 rows a strip, 32 where those

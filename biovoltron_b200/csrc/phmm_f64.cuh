@@ -23,7 +23,7 @@
 // above or left of column 1 is non-zero, and nothing is summed past the last
 // column.
 //
-// The folded form needs pMM >= kFoldMin in every row and the scaled states
+// The folded form needs pMM >= kF64FoldMin in every row and the scaled states
 // need head-room, so callers start from 2^kF64Start / H (not 2^1020 / H) and
 // hand a pair whose result is not safely inside the range to the unscaled,
 // per-strip renormalised form (process_item_f64).
@@ -38,6 +38,11 @@ namespace bvphmm {
 constexpr int kF64Start = 900;
 constexpr int kF64InitExp = 1020;  // log2 of Tables::init_d
 constexpr double kF64MinResult = 2.409919865102884e-181;  // 2^-600
+// Rows whose pMM is smaller (indel qualities of 3 and less: pMM is zero, or 0.0061
+// at least) do not fold.  FP64 holds coefficients of 1 / pMM, 2^8 at most, without
+// loss; at FP32's limit of 0.5, 40 reads of up to 10 kb with some indel qualities
+// of 5 and 6 were handed to the unscaled form and took 129 instead of 3.8 ms.
+constexpr double kF64FoldMin = 0x1p-8;
 
 template <int RT>
 struct F64Rows {
@@ -95,7 +100,7 @@ __device__ __forceinline__ F64Row f64_row(const Tables* __restrict__ tb, const u
     o.em = (1.0 - eps) * mm;
     o.ex = eps / 3.0 * mm;
     o.code = base_code(bases[r - 1]);
-    o.ok = mm >= (double)kFoldMin;
+    o.ok = mm >= kF64FoldMin;
   }
   return o;
 }

@@ -236,6 +236,25 @@ def test_long_reads_with_dear_gaps(oracle, gcp):
                 _check(b, e.compute_regions(b), oracle)
 
 
+# indel qualities whose pMM is small: the smallest that is positive (1 and 7: 0.006), zero (not folded), and both among
+# others; single strips, the list, long reads
+@pytest.mark.parametrize("gaps", [(1, 7, 10), (5, 2, 20), (4, 4, 10), (1, 6, 10), (0, 127, 30)])
+def test_rows_with_a_small_match_probability(oracle, gaps):
+    from biovoltron_b200.pairhmm import PairHMMEngine
+    rng = np.random.default_rng(sum(gaps))
+    regions = []
+    for n in (60, 150, 253, 254, 700, 1500):
+        for related in (True, False):
+            reads, haps = _pair(rng, n, n + 150, related=related, gaps=gaps)
+            r, q, i, d, c = reads[0]
+            some = rng.random(len(r)) < 0.3
+            regions.append((reads + [(r, q, np.where(some, i, 40).astype(np.uint8), np.where(some, d, 45).astype(np.uint8), c)],
+                            haps))
+    b = W._build(regions, "small pMM")
+    with PairHMMEngine(precision="f64") as e:
+        _check(b, e.compute_regions(b), oracle)
+
+
 def test_constant_transitions_that_lose_most_of_the_range_in_a_strip(oracle):
     """Insertion runs that are dear by a small insertion-to-insertion probability."""
     from biovoltron_b200.pairhmm import PairHMMEngine
